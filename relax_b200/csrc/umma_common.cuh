@@ -19,6 +19,13 @@ enum ScaleSrc : int { kSrcGlobal = 0, kSrcSmemNK = 1, kSrcSmemKN = 2 };
 
 #ifdef __CUDACC__
 // ---------------------------------------------------------------- PTX wrappers
+// one lane of a converged warp, in the form from which the compiler knows that a single thread runs
+// the branch (tcgen05 operands then stay in uniform registers)
+__device__ __forceinline__ bool elect_one() {
+  uint32_t p;
+  asm volatile("{\n\t.reg .pred p;\n\telect.sync _|p, 0xffffffff;\n\tselp.u32 %0, 1, 0, p;\n\t}" : "=r"(p));
+  return p != 0;
+}
 // 16-byte asynchronous copy global -> shared; bytes beyond src_bytes are written as zero
 __device__ __forceinline__ void cp_async16(void* smem_dst, const void* gsrc, uint32_t src_bytes) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_u32(smem_dst)), "l"(gsrc), "r"(src_bytes)

@@ -3,9 +3,9 @@
 //   out^T tile [128 weight rows x up to 256 batch rows] = W_tile [128 x K] * x_tile^T [K x 256]
 //
 // Measured on B200: one tcgen05.mma (kind::f16, M = 128, K = 16, A from tensor memory) occupies
-// the tensor pipe for 108 clocks for any N up to 192 and for 136 clocks at N = 256, so the batch
-// is the instruction's N and is made as wide as it goes (256): one instruction then does
-// 128 x 256 x 16 MACs.  The dequantised weights are the A operand and never touch shared memory:
+// the tensor pipe for N / 2 clocks (N = 16: 9, 32: 16, 64: 32, 128: 64, 256: 128).  The batch is the
+// instruction's N and is made as wide as it goes (256), because every weight element is decoded
+// once per batch tile.  The dequantised weights are the A operand and never touch shared memory:
 // decode warps write them straight into tensor memory (tcgen05.st), the MMA reads A from TMEM and
 // B (= x) from a 128B-swizzled K-major tile in shared memory, the fp32 accumulator sits in 256
 // TMEM columns.
@@ -117,6 +117,7 @@ using ug::tc_ld16;
 using ug::tc_mma_ts;
 using ug::tc_st32;
 using ug::tc_wait_st;
+using ug::elect_one;
 using ug::tmem_alloc;
 using ug::tmem_dealloc;
 using ug::tmem_relinquish;
@@ -348,67 +349,85 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else if (warp == 1) {
-    // ============================================================ MMA issuer (one thread)
-    if (lane == 0) {
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(nb >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
-      int xs = 0;
-      uint32_t xph = 0;
-      uint32_t q = 0;       // running 64-k block counter (selects the A buffer)
-      uint32_t tile_i = 0;  // tiles done by this CTA
-      int ws = 0;
-      uint32_t wph = 0;
-      (void)ws;
-      (void)wph;
-      for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x, ++tile_i) {
-        if (!mbar_wait_parked(d_empty, (tile_i & 1u) ^ 1u, p.status)) {
+    // ============================================================ MMA issuer (one elected thread)
+    // The whole warp runs the loop and waits; elect.sync picks the issuing thread.  Written as
+    // `if (lane == 0)` with descriptors rebuilt per instruction, the issue loop itself took 108
+    // clocks per MMA and hid that an MMA of width N occupies the pipe for N / 2 clocks only
+    // (measured: 16 at N = 32, 64 at 128, 128 at 256).
+    const uint32_t idesc = (1u << 4) | ((uint32_t)(nb >> 3) << 17) | ((uint32_t)(128 >> 4) << 24);
+    const bool leader = elect_one();
+    const uint64_t x_desc0 = make_b_desc(smem_u32(x_ring));
+    const uint64_t w_desc0 = make_b_desc(smem_u32(w_ring));
+    uint64_t x_desc = x_desc0;
+    int xs = 0;
+    uint32_t xph = 0;
+    uint32_t ab = 0, aph = 0;  // A buffer and its phase
+    uint32_t dph = 1;          // accumulator hand-back phase
+    int ws = 0;
+    uint32_t wph = 0;
+    (void)ws;
+    (void)wph;
+    (void)w_desc0;
+    for (int t = blockIdx.x; ok && t < total_tiles; t += gridDim.x, dph ^= 1u) {
+      if (!mbar_wait_parked(d_empty, dph, p.status)) {
+        ok = false;
+        break;
+      }
+      tc_fence_after();
+      const int kb_first = kb_lo(t % S), kb_end = kb_lo(t % S + 1);
+      uint32_t acc_on = 0u;
+      for (int kb = kb_first; kb < kb_end; ++kb) {
+        if (!um_wait(&x_full[xs], xph, p.status)) {
+          ok = false;
+          break;
+        }
+        if (kDense) {
+          if (!um_wait(&w_full[ws], wph, p.status)) {
+            ok = false;
+            break;
+          }
+        } else if (!um_wait(&a_full[ab], aph, p.status)) {
           ok = false;
           break;
         }
         tc_fence_after();
-        const int kb_first = kb_lo(t % S), kb_end = kb_lo(t % S + 1);
-        for (int kb = kb_first; kb < kb_end; ++kb, ++q) {
-          if (!um_wait(&x_full[xs], xph, p.status)) {
-            ok = false;
-            break;
-          }
-          const uint32_t ab = q % kNumA;
-          if (kDense) {
-            if (!um_wait(&w_full[ws], wph, p.status)) {
-              ok = false;
-              break;
-            }
-          } else if (!um_wait(&a_full[ab], (q / kNumA) & 1u, p.status)) {
-            ok = false;
-            break;
-          }
-          tc_fence_after();
-          const uint32_t xbase = smem_u32(x_ring + (size_t)xs * x_stage_bytes);
-          if (kDense) {
-            const uint32_t wbase = smem_u32(w_ring + (size_t)ws * kWStageBytes);
+        if (kDense) {
+          const uint64_t w_desc = w_desc0 + (uint64_t)(ws * (kWStageBytes >> 4));
+          if (leader) {
+            tc_mma_ss(d_col0, w_desc, x_desc, idesc, acc_on);
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              tc_mma_ss(d_col0, make_b_desc(wbase + j * 32), make_b_desc(xbase + j * 32), idesc,
-                        (kb == kb_first && j == 0) ? 0u : 1u);
+            for (int j = 1; j < 4; ++j) tc_mma_ss(d_col0, w_desc + j * 2, x_desc + j * 2, idesc, 1u);
             tc_commit(&w_empty[ws]);
-            if (++ws == kWStages) {
-              ws = 0;
-              wph ^= 1u;
-            }
-          } else {
-            const uint32_t a_tmem = a_col0 + ab * 32;
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              tc_mma_ts(d_col0, a_tmem + j * 8, make_b_desc(xbase + j * 32), idesc, (kb == kb_first && j == 0) ? 0u : 1u);
-            tc_commit(&a_empty[ab]);
+            tc_commit(&x_empty[xs]);
           }
-          tc_commit(&x_empty[xs]);
-          if (++xs == x_stages) {
-            xs = 0;
-            xph ^= 1u;
+          if (++ws == kWStages) {
+            ws = 0;
+            wph ^= 1u;
+          }
+        } else {
+          const uint32_t a_tmem = a_col0 + ab * 32;
+          if (leader) {
+            tc_mma_ts(d_col0, a_tmem, x_desc, idesc, acc_on);
+#pragma unroll
+            for (int j = 1; j < 4; ++j) tc_mma_ts(d_col0, a_tmem + j * 8, x_desc + j * 2, idesc, 1u);
+            tc_commit(&a_empty[ab]);
+            tc_commit(&x_empty[xs]);
+          }
+          if (++ab == kNumA) {
+            ab = 0;
+            aph ^= 1u;
           }
         }
-        if (ok) tc_commit(d_full);
+        acc_on = 1u;
+        x_desc += (uint64_t)(x_stage_bytes >> 4);
+        if (++xs == x_stages) {
+          xs = 0;
+          xph ^= 1u;
+          x_desc = x_desc0;
+        }
       }
+      if (ok && leader) tc_commit(d_full);
+      __syncwarp();
     }
   } else if (warp == 2) {
     // ============================================================ scale / zero tiles of each chunk
