@@ -10,6 +10,7 @@
 #include "gemv.h"
 #include "gemv_cluster.cuh"
 #include "umma_gemm.cuh"
+#include "gemv_rk.cuh"
 #include "gemv_sk.cuh"
 #include "gemm_tc.h"
 #include "preprocess.h"
@@ -419,14 +420,17 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
     p.k = (int)d->k;
     p.group = group;
     p.zero_const = d->zero_const;
-    // Which decode kernel: the stream-k kernel whenever x can be fetched as TMA tiles of whole
-    // 64-k blocks (always for int4); the cluster kernel - split-k partials meeting in distributed
-    // shared memory - for the remaining int8 shapes (k a multiple of 32 only).  Measured on B200
-    // with launch overlap: stream-k is ahead at every size, 8.3 against 9.3 us at k = n = 4096.
+    // Which decode kernel: up to eight rows (one MMA wide) the small-batch kernel; above that the
+    // stream-k kernel whenever x can be fetched as TMA tiles of whole 64-k blocks (always for int4), and
+    // the cluster kernel - split-k partials meeting in distributed shared memory - for the remaining
+    // int8 shapes (k a multiple of 32 only).  Measured with launch overlap at one row, small-batch
+    // against stream-k: k = n = 4096 3.9 / 8.1 us, n 22016 13.9 / 19.1, k 11008 x n 4096 8.0 / 13.4.
+    if (p.m <= rk::kMaxBatch && !ar)
+      return gemv_rk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
     if (p.k % 64 == 0) {
       unsigned* flags = reinterpret_cast<unsigned*>(sc->counters) + kSkFlagOffset;
       return gemv_sk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, sc->partials, sc->partial_bytes, flags,
-                         kSkFlagCount, ar, nullptr, stream);
+                         kSkFlagCount, ar, stream);
     }
     return gemv_cluster_run(p, d->weight_bits, zero_mode(d), sc->sm_count, stream);
   }
@@ -613,24 +617,10 @@ int rb200_group_gemm(const rb200_group_gemm_desc* d, void* stream_v) {
   const int zmode = (packed && (d->zeros || !int_zero)) ? kZeroGeneral : kZeroConstInt;
   const int64_t w_expert_bytes = d->n * d->k * d->weight_bits / 8;
   if (packed && d->total_rows <= 32 && d->k % 64 == 0 && d->n % 16 == 0 && aligned16(d->x) && aligned16(d->out)) {
-    // Decode-size batch: the weights of an expert with rows are streamed once by the decode
-    // kernel (one launch per expert; a launch whose expert has no rows returns at once), instead
-    // of padding a handful of rows to a tensor-core tile of 192.
-    unsigned* flags = reinterpret_cast<unsigned*>(sc->counters) + kSkFlagOffset;
-    for (int e = 0; e < (int)d->num_experts; ++e) {
-      GemvParams pe = p;
-      pe.w = p.w + (int64_t)e * w_expert_bytes;
-      pe.s = p.s + (int64_t)e * d->scale_stride_e;
-      if (p.z) pe.z = p.z + (int64_t)e * d->scale_stride_e;
-      sk::GroupCtx g;
-      g.indptr = d->indptr;
-      g.expert = e;
-      g.has_prev = d->indptr_has_prev ? 1 : 0;
-      if (gemv_sk_run(pe, d->weight_bits, zmode, sc->sm_count, sc->partials, sc->partial_bytes, flags, kSkFlagCount,
-                      nullptr, &g, static_cast<cudaStream_t>(stream_v)) != 0)
-        return -1;
-    }
-    return 0;
+    // Decode-size batch: one launch of the small-batch kernel streams the weights of every expert
+    // that has rows (eight experts of k 4096 x n 14336, 16 rows: 75 us; one launch per expert 150 us).
+    return gemv_rk_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0, (int)d->num_experts,
+                       w_expert_bytes, d->scale_stride_e, static_cast<cudaStream_t>(stream_v));
   }
   return umma_group_gemm_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0,
                              (int)d->num_experts, w_expert_bytes,

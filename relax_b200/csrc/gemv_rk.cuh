@@ -1,0 +1,516 @@
+// Decode-path kernel for at most eight batch rows: row blocks per CTA, k split over its warps.
+//
+//   out[m, n] = epilogue(sum_k x[m, k] * wq[n, k]),  m <= 8 (the n of one m16n8k16 MMA)
+//
+// Bound: HBM (the packed weight once) and, close behind, instruction issue: the exact two-rounding
+// decode is 52 of the 61 instructions a 512-byte tile needs (4 MMAs, 3 loads, 2 scale selects).
+// So nothing else is in the loop: no shared memory, no barriers, no copies through the async
+// engine.  A warp reads fragment tiles with 128-bit loads that are whole 512-byte lines in the
+// fragment layout, straight into the registers the MMA takes them from, one chunk (four tiles)
+// ahead of the arithmetic; activations come from L1 / L2 once per chunk and serve all row blocks
+// of the pass.  The first chunks are prefetched into L2 before the wait on the previous kernel: a
+// prefetch returns no data to this kernel, so it is safe whatever that kernel still writes.
+//
+// Measured (graph of launches over 400 MB of weights, launch overlap on, one row): int4 group 32
+// k 4096 x n 4096 3.9 us (8.1 in the stream-k kernel), x 12288 9.0 (13.6), x 22016 13.9 (19.1),
+// k 11008 x n 4096 8.0 (13.4); int8 k 8192 x n 28672, eight rows, 37.7 us = 6.2 TB/s (48.6).
+// What bounds int4: about 155 clocks per tile and SM sub-partition, of which the 32 fp16 and 35
+// integer instructions take two each and overlap only in part (a loop of alternating lop3 and
+// mul.f16x2 issues one per 1.7 clocks where either alone takes 2.0).
+//
+// Work split: a row block (16 output rows) belongs to one CTA, its k range to the CTA's eight warps,
+// whose partial sums meet in shared memory in warp order: no partial ever leaves the SM, there is
+// no flag, fence or second pass, and the result does not depend on the grid.
+//
+// Grouped (expert) form: the row blocks of all experts that have rows form one list, read from
+// indptr on the device, so that a whole expert layer is one launch.
+#pragma once
+
+#include <type_traits>
+
+#include "dequant.cuh"
+#include "gemv.h"
+
+namespace rb200 {
+namespace rk {
+
+constexpr int kRows = 2;         // row blocks of one pass: activations fetched once serve both
+constexpr int kMaxBatch = 8;
+constexpr int kLeadChunks = 2;   // chunks between an L2 prefetch and the load
+constexpr int kMaxEntries = 96;  // grouped form: (expert, eight batch rows) pairs; 64 experts, 32 rows in all
+
+// where a lane gets its scales / zero points from
+enum ScaleSrc : int {
+  kChannel = 0,  // one per output row
+  kRow32 = 1,    // int4, group 32, [N, K/32]: the eight groups of a chunk are one 16-byte load
+  kHalf = 2,     // groups of whole chunk halves (two tiles), any strides: one 16-bit load per row and half
+  kGeneral = 3,  // any strides and group size: one 16-bit load per row and tile
+};
+
+struct Params {
+  GemvParams g;
+  int group_shift;         // log2 of the group size, or -1
+  unsigned per_cta, extra; // ungrouped: row blocks per CTA, and how many CTAs take one more
+  int s_n, s_g;            // scale strides in elements
+  int early;               // the host promises that weights were not written by the previous kernel
+  const int64_t* indptr;   // grouped form: end rows per expert (device), else nullptr
+  int has_prev, num_experts;
+  int64_t w_expert_bytes, s_expert_stride;
+};
+
+int launch_i4(const Params& pp, int zmode, int src, int warps, int grid, cudaStream_t stream);
+int launch_i8(const Params& pp, int zmode, int src, int warps, int grid, cudaStream_t stream);
+
+#ifdef __CUDACC__
+
+__device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];"
+               : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w)
+               : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ uint2 ld_nc_v2(const void* p) {
+  uint2 v;
+  asm volatile("ld.global.nc.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(p));
+  return v;
+}
+__device__ __forceinline__ void prefetch_l2(const void* p) {
+  asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
+}
+
+template <int kXV>
+struct XHalf {
+  uint4 v[2][kXV];
+};
+
+// kWarps: warps per CTA = k slices of a row block (16 warps per SM either way)
+template <int BITS, int ZMODE, int SRC, bool GROUPED, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const Params pp) {
+  constexpr int kFrag = BITS == 4 ? 64 : 32;
+  constexpr int kLaneK = kFrag / 4;
+  constexpr int kXV = BITS == 4 ? 2 : 1;  // 16-byte pieces of x per lane and tile
+  constexpr bool kZ = ZMODE == kZeroGeneral;
+  __shared__ __align__(16) float4 red[2][kWarps][kRows][32];
+  __shared__ int s_entries, s_m_lo[kMaxEntries], s_m_n[kMaxEntries], s_expert[kMaxEntries];
+  const GemvParams& p = pp.g;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int NB = p.n / 16, KB = p.k / kFrag;
+  constexpr bool grouped = GROUPED;
+
+  griddep_launch_dependents();
+  int entries = 1;
+  if (grouped) {
+    griddep_wait();  // the row table is the routing kernel's output
+    if (warp == 0) {
+      int n_e = 0;
+      for (int e0 = 0; e0 < pp.num_experts; e0 += 32) {
+        const int e = e0 + lane;
+        int r0 = 0, r1 = 0;
+        if (e < pp.num_experts) {
+          r0 = (e || pp.has_prev) ? (int)pp.indptr[e - 1] : 0;
+          r1 = min((int)pp.indptr[e], p.m);  // never past the rows x / out hold
+        }
+        const int mine = r1 > r0 ? (r1 - r0 + kMaxBatch - 1) / kMaxBatch : 0;
+        int incl = mine;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, incl, o);
+          if (lane >= o) incl += v;
+        }
+        for (int i = 0; i < mine; ++i) {
+          const int slot = n_e + incl - mine + i;
+          if (slot < kMaxEntries) {
+            s_m_lo[slot] = r0 + i * kMaxBatch;
+            s_m_n[slot] = min(kMaxBatch, r1 - r0 - i * kMaxBatch);
+            s_expert[slot] = e;
+          }
+        }
+        n_e += __shfl_sync(0xffffffffu, incl, 31);
+      }
+      if (lane == 0) s_entries = min(n_e, kMaxEntries);
+    }
+    __syncthreads();
+    entries = s_entries;
+  }
+  // this CTA's row blocks, numbered entry by entry
+  unsigned pos, pos_end;
+  if (grouped) {
+    const unsigned total = (unsigned)entries * (unsigned)NB;  // total * grid fits 32 bits (checked by the host)
+    pos = blockIdx.x * total / gridDim.x;
+    pos_end = (blockIdx.x + 1) * total / gridDim.x;
+  } else {
+    pos = blockIdx.x * pp.per_cta + min(blockIdx.x, pp.extra);
+    pos_end = pos + pp.per_cta + (blockIdx.x < pp.extra ? 1u : 0u);
+  }
+  if (pos >= pos_end) return;
+
+  const ZeroConsts zc = make_zero_consts(ZMODE, p.zero_const);
+  const uint32_t zconst_h2 = h2_bcast(__float2half_rn(p.zero_const));
+  const uint32_t half_sel = (t >> 1) ? 0x3232u : 0x1010u;
+  const int unit16 = frag_unit_pos(lane) * 16;
+  const bool has_zeros = kZ && p.z != nullptr;
+
+  // this warp's whole chunks (four fragment tiles); the tiles of a short last chunk go to the last warp
+  const int full_chunks = KB / 4;
+  const int c0 = warp * full_chunks / kWarps, c1 = (warp + 1) * full_chunks / kWarps;
+
+  // What a pass works on: up to two row blocks of one entry.
+  struct Pass {
+    int nb0, rn, m_lo, m_n, e;
+  };
+  auto get_pass = [&](unsigned at) {
+    Pass q;
+    const int entry = grouped ? (int)(at / (unsigned)NB) : 0;
+    q.nb0 = (int)(at - (unsigned)entry * (unsigned)NB);
+    // a short last row tile has another chunk stride: a pass stays on one side of it
+    const int to_tile_end = 8 - (q.nb0 & 7);
+    q.rn = min(min(kRows, (int)(pos_end - at)), min(NB - q.nb0, to_tile_end));
+    q.e = grouped ? s_expert[entry] : 0;
+    q.m_lo = grouped ? s_m_lo[entry] : 0;
+    q.m_n = grouped ? s_m_n[entry] : p.m;
+    return q;
+  };
+  const int row8 = pp.s_n * 8;  // elements from row g's scale to row g + 8's
+
+  // Two register sets, one per half of a chunk (two tiles of each row block); a set is loaded for the
+  // next chunk as soon as it has been decoded, so a chunk per row block is always on its way.  The
+  // row blocks of a pass lie in one 128-row tile, so one pointer and immediate offsets reach all of
+  // a chunk's tiles.
+  uint4 w[2][kRows][2];
+  uint2 sv[2][kRows][2], zv[2][kRows][2];      // kRow32: rows g, g + 8: the half's four groups
+  uint32_t sg[2][kRows][2], zg[2][kRows][2];   // kGeneral: per tile, row g low, row g + 8 high
+  uint32_t ch_s[kRows], ch_z[kRows];           // kChannel
+  const uint8_t* wp = nullptr;                 // next chunk to load
+  const __half *sp[kRows][2], *zp[kRows][2];   // scales of rows g, g + 8 (kRow32: of the next chunk)
+  int stride = 0;                              // bytes from a chunk to the next
+
+  auto load_set = [&](auto set_tag, auto rn_tag, int c) {
+    constexpr int S = decltype(set_tag)::value, RN = decltype(rn_tag)::value;
+#pragma unroll
+    for (int r = 0; r < RN; ++r) {
+      w[S][r][0] = ld_stream_v4(wp + r * 2048 + S * 1024);
+      w[S][r][1] = ld_stream_v4(wp + r * 2048 + S * 1024 + 512);
+      if (SRC == kRow32) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          sv[S][r][i] = ld_nc_v2(sp[r][i] + S * 4);
+          if (has_zeros) zv[S][r][i] = ld_nc_v2(zp[r][i] + S * 4);
+        }
+      } else if (SRC == kHalf || SRC == kGeneral) {
+#pragma unroll
+        for (int j = 0; j < (SRC == kHalf ? 1 : 2); ++j) {
+          const unsigned k = (unsigned)((c * 4 + S * 2 + j) * kFrag + t * kLaneK);
+          const unsigned grp = pp.group_shift >= 0 ? k >> pp.group_shift : k / (unsigned)p.group;
+          const unsigned o = grp * (unsigned)pp.s_g;
+          sg[S][r][j] = ld_nc_u16(sp[r][0] + o) | (ld_nc_u16(sp[r][1] + o) << 16);
+          if (has_zeros) zg[S][r][j] = ld_nc_u16(zp[r][0] + o) | (ld_nc_u16(zp[r][1] + o) << 16);
+        }
+      }
+    }
+    if (S == 1) {
+      wp += stride;
+      if (SRC == kRow32) {
+#pragma unroll
+        for (int r = 0; r < RN; ++r)
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            sp[r][i] += 8;
+            if (has_zeros) zp[r][i] += 8;
+          }
+      }
+    }
+  };
+  using I0 = std::integral_constant<int, 0>;
+  using I1 = std::integral_constant<int, 1>;
+  using I2 = std::integral_constant<int, 2>;
+  auto start_pass = [&](const Pass& q) {
+    stride = min(8, NB - (q.nb0 & ~7)) * 2048;
+    wp = p.w + (grouped ? q.e * pp.w_expert_bytes : 0) + 
+         (int64_t)((q.nb0 & ~7) * KB + c0 * (stride >> 9) + (q.nb0 & 7) * 4) * 512 + unit16;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      const int nb = q.nb0 + min(r, q.rn - 1);
+      const int64_t o = (grouped ? q.e * pp.s_expert_stride : 0) + (nb * 16 + g) * pp.s_n + (SRC == kRow32 ? c0 * 8 : 0);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        sp[r][i] = p.s + o + i * row8;
+        zp[r][i] = p.z + o + i * row8;
+      }
+      if (SRC == kChannel) {
+        ch_s[r] = ld_nc_u16(sp[r][0]) | (ld_nc_u16(sp[r][1]) << 16);
+        if (has_zeros) ch_z[r] = ld_nc_u16(zp[r][0]) | (ld_nc_u16(zp[r][1]) << 16);
+      }
+    }
+    if (c0 < c1) {
+      if (q.rn == 2) {
+        load_set(I0{}, I2{}, c0);
+        load_set(I1{}, I2{}, c0);
+      } else {
+        load_set(I0{}, I1{}, c0);
+        load_set(I1{}, I1{}, c0);
+      }
+    }
+  };
+
+  // L2 prefetch: a lane asks for one of the 16 lines of either row block's chunk.  int8 tiles take a
+  // third of the arithmetic of int4 tiles per byte, so there the loads need this lead to keep HBM
+  // busy (k 8192 x n 28672: 54 -> 38 us); for int4 it only cost instructions (14.8 against 13.7 us at
+  // k 4096 x n 22016).
+  constexpr bool kLead = BITS == 8;
+  const int ahead = min(kLeadChunks, c1 - c0);
+  auto line_of = [&](const Pass& q, int c) -> const uint8_t* {
+    const int st = min(8, NB - (q.nb0 & ~7)) * 4;
+    return p.w + (grouped ? q.e * pp.w_expert_bytes : 0) +
+           (int64_t)((q.nb0 & ~7) * KB + c * st + (q.nb0 & 7) * 4) * 512 + lane * 128;
+  };
+  Pass q = get_pass(pos);
+  if (!grouped && pp.early) start_pass(q);
+  if (kLead || !pp.early) {
+    // before the wait: a prefetch returns nothing to this kernel, so it is safe whatever the previous
+    // kernel still writes
+    const uint8_t* line = line_of(q, c0);
+    for (int c = 0; c < ahead; ++c, line += min(8, NB - (q.nb0 & ~7)) * 2048)
+      if (lane < 16 * q.rn) prefetch_l2(line);
+  }
+  if (!grouped) griddep_wait();
+  if (grouped || !pp.early) start_pass(q);
+
+  int buf = 0;
+  for (;;) {
+    float acc[kRows][2][4];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) acc[r][0][c] = acc[r][1][c] = 0.0f;
+    // lanes of absent batch rows fetch row 0: their columns of the result are never stored
+    const __half* x0 = p.x + (q.m_lo + (g < q.m_n ? g : 0)) * (unsigned)p.ldx + t * kLaneK;
+
+    auto mma_tile = [&](int r, const uint4& wv, uint32_t s_g, uint32_t s_g8, uint32_t z_g, uint32_t z_g8,
+                        const uint4 (&xv)[kXV]) {
+      uint32_t a[4];
+      if (BITS == 4) {
+        decode_int4_word<ZMODE>(wv.x, zc, s_g, s_g8, z_g, z_g8, a);
+        mma_16816(acc[r][0], a, xv[0].x, xv[0].y);
+        decode_int4_word<ZMODE>(wv.y, zc, s_g, s_g8, z_g, z_g8, a);
+        mma_16816(acc[r][1], a, xv[0].z, xv[0].w);
+        decode_int4_word<ZMODE>(wv.z, zc, s_g, s_g8, z_g, z_g8, a);
+        mma_16816(acc[r][0], a, xv[kXV - 1].x, xv[kXV - 1].y);
+        decode_int4_word<ZMODE>(wv.w, zc, s_g, s_g8, z_g, z_g8, a);
+        mma_16816(acc[r][1], a, xv[kXV - 1].z, xv[kXV - 1].w);
+      } else {
+        decode_int8_pair<ZMODE>(wv.x, wv.y, zc, s_g, s_g8, z_g, z_g8, a);
+        mma_16816(acc[r][0], a, xv[0].x, xv[0].y);
+        decode_int8_pair<ZMODE>(wv.z, wv.w, zc, s_g, s_g8, z_g, z_g8, a);
+        mma_16816(acc[r][1], a, xv[0].z, xv[0].w);
+      }
+    };
+    const __half* xp = x0 + c0 * (kFrag * 4);
+    // activations of either half: int8 fetches them half a chunk ahead, int4 has no registers to spare
+    // for that and fetches them where they are used
+    constexpr bool kXAhead = BITS == 8;
+    XHalf<kXV> xa, xb;
+    auto load_x = [&](XHalf<kXV>& xv, int half) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int i = 0; i < kXV; ++i) xv.v[j][i] = ld_nc_v4(xp + (half * 2 + j) * kFrag + i * 8);
+    };
+    auto half_step = [&](auto set_tag, auto rn_tag, const XHalf<kXV>& xv) {
+      constexpr int S = decltype(set_tag)::value, RN = decltype(rn_tag)::value;
+#pragma unroll
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int r = 0; r < RN; ++r) {
+          uint32_t s_g, s_g8, z_g = zconst_h2, z_g8 = zconst_h2;
+          if (SRC == kRow32) {
+            const uint32_t a = j == 0 ? sv[S][r][0].x : sv[S][r][0].y, b = j == 0 ? sv[S][r][1].x : sv[S][r][1].y;
+            s_g = prmt(a, a, half_sel);
+            s_g8 = prmt(b, b, half_sel);
+            if (has_zeros) {
+              const uint32_t za = j == 0 ? zv[S][r][0].x : zv[S][r][0].y, zb = j == 0 ? zv[S][r][1].x : zv[S][r][1].y;
+              z_g = prmt(za, za, half_sel);
+              z_g8 = prmt(zb, zb, half_sel);
+            }
+          } else {
+            const uint32_t a = SRC == kChannel ? ch_s[r] : sg[S][r][SRC == kHalf ? 0 : j];
+            s_g = prmt(a, a, 0x1010u);
+            s_g8 = prmt(a, a, 0x3232u);
+            if (has_zeros) {
+              const uint32_t b = SRC == kChannel ? ch_z[r] : zg[S][r][SRC == kHalf ? 0 : j];
+              z_g = prmt(b, b, 0x1010u);
+              z_g8 = prmt(b, b, 0x3232u);
+            }
+          }
+          mma_tile(r, w[S][r][j], s_g, s_g8, z_g, z_g8, xv.v[j]);
+        }
+    };
+    Pass q_next;
+    const bool more = pos + (unsigned)q.rn < pos_end;
+    const uint8_t* line = nullptr;
+    int line_step = stride;
+    bool line_on = lane < 16 * q.rn;
+    if constexpr (kLead) {
+      q_next = get_pass(min(pos + (unsigned)q.rn, pos_end - 1));
+      line = line_of(q, c0 + ahead);
+    }
+    auto all_chunks = [&](auto rn_tag) {
+#pragma unroll 1
+      for (int c = c0; c < c1; ++c) {
+        const bool again = c + 1 < c1;
+        if constexpr (kLead) {
+          if (c + ahead == c1) {  // on into the next pass
+            line = line_of(q_next, c0);
+            line_step = min(8, NB - (q_next.nb0 & ~7)) * 2048;
+            line_on = more && lane < 16 * q_next.rn;
+          }
+          if (line_on) prefetch_l2(line);
+          line += line_step;
+        }
+        load_x(kXAhead ? xb : xa, kXAhead ? 1 : 0);
+        half_step(I0{}, rn_tag, xa);
+        if (again) load_set(I0{}, rn_tag, c + 1);
+        if (kXAhead) {
+          if (again) xp += kFrag * 4;
+          load_x(xa, 0);
+        } else {
+          load_x(xb, 1);
+          xp += kFrag * 4;
+        }
+        half_step(I1{}, rn_tag, xb);
+        if (again) load_set(I1{}, rn_tag, c + 1);
+      }
+    };
+    if (c0 < c1) {
+      if (kXAhead) load_x(xa, 0);
+      if (q.rn == 2) all_chunks(I2{});
+      else all_chunks(I1{});
+    }
+
+    if (warp == kWarps - 1) {  // tiles of a short last chunk
+      for (int kb = full_chunks * 4; kb < KB; ++kb) {
+        uint4 xt[kXV];
+#pragma unroll
+        for (int i = 0; i < kXV; ++i) xt[i] = ld_nc_v4(x0 + kb * kFrag + i * 8);
+        const unsigned k = (unsigned)(kb * kFrag + t * kLaneK);
+        const unsigned grp = SRC == kChannel ? 0u : (pp.group_shift >= 0 ? k >> pp.group_shift : k / (unsigned)p.group);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+          if (r >= q.rn) break;
+          const uint4 wt = ld_stream_v4(p.w + (grouped ? q.e * pp.w_expert_bytes : 0) +
+                                        frag_tile_offset(q.nb0 + r, kb, NB, KB) + unit16);
+          const int64_t o = (grouped ? q.e * pp.s_expert_stride : 0) + ((q.nb0 + r) * 16 + g) * pp.s_n +
+                            grp * (unsigned)pp.s_g;
+          const uint32_t a = ld_nc_u16(p.s + o), b = ld_nc_u16(p.s + o + row8);
+          const uint32_t za = has_zeros ? ld_nc_u16(p.z + o) * 0x10001u : zconst_h2;
+          const uint32_t zb = has_zeros ? ld_nc_u16(p.z + o + row8) * 0x10001u : zconst_h2;
+          mma_tile(r, wt, a * 0x10001u, b * 0x10001u, za, zb, xt);
+        }
+      }
+    }
+
+    // the next pass's first loads leave before this one's sums are put together
+    const Pass done = q;
+    pos += (unsigned)q.rn;
+    if (more) {
+      if constexpr (kLead) q = q_next;
+      else q = get_pass(pos);
+      start_pass(q);
+    }
+
+    // the eight k slices meet in warp order
+#pragma unroll
+    for (int r = 0; r < kRows; ++r)
+      red[buf][warp][r][lane] = make_float4(acc[r][0][0] + acc[r][1][0], acc[r][0][1] + acc[r][1][1],
+                                            acc[r][0][2] + acc[r][1][2], acc[r][0][3] + acc[r][1][3]);
+    __syncthreads();
+    if (warp < done.rn) {
+      float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int i = 0; i < kWarps; ++i) {
+        const float4 f = red[buf][i][warp][lane];
+        v[0] += f.x;
+        v[1] += f.y;
+        v[2] += f.z;
+        v[3] += f.w;
+      }
+      const int nb = done.nb0 + warp;
+      if (p.epi.act == kActSwiglu) {
+        // rows g / g + 8 of the block are gate_f / up_f of f = 8 nb + g (interleaved repack)
+#pragma unroll
+        for (int cc = 0; cc < 2; ++cc) {
+          const int m = t * 2 + cc;
+          if (m < done.m_n)
+            p.out[(int64_t)(done.m_lo + m) * p.ldo + nb * 8 + g] = __float2half_rn(silu_mul(v[cc], v[cc + 2]));
+        }
+      } else {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int m = t * 2 + (i & 1);
+          const int64_t n = (int64_t)nb * 16 + g + (i >> 1) * 8;
+          if (m < done.m_n)
+            p.out[(int64_t)(done.m_lo + m) * p.ldo + n] = __float2half_rn(apply_epilogue(v[i], p.epi, done.m_lo + m, n));
+        }
+      }
+    }
+    if (!more) break;
+    buf ^= 1;  // the next pass writes the other half, so one barrier per pass is enough
+  }
+}
+
+template <int BITS, int ZMODE, int SRC>
+int launch_inst(const Params& pp, int warps, int grid, cudaStream_t stream) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)grid, 1, 1);
+  cfg.blockDim = dim3((unsigned)warps * 32, 1, 1);
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  // always a programmatic dependent: before its wait the kernel only prefetches, unless the host
+  // switched launch overlap on
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  if (pp.indptr) {
+    if (warps == 8) RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, true, 8>, pp));
+    else RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, true, 4>, pp));
+  } else {
+    if (warps == 8) RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, false, 8>, pp));
+    else RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, false, 4>, pp));
+  }
+  return 0;
+}
+
+template <int BITS>
+int launch_bits(const Params& pp, int zmode, int src, int warps, int grid, cudaStream_t stream) {
+  const bool general = zmode == kZeroGeneral;
+  if (src == kChannel)
+    return general ? launch_inst<BITS, kZeroGeneral, kChannel>(pp, warps, grid, stream)
+                   : launch_inst<BITS, kZeroConstInt, kChannel>(pp, warps, grid, stream);
+  if (src == kHalf)
+    return general ? launch_inst<BITS, kZeroGeneral, kHalf>(pp, warps, grid, stream)
+                   : launch_inst<BITS, kZeroConstInt, kHalf>(pp, warps, grid, stream);
+  if constexpr (BITS == 4) {
+    if (src == kRow32)
+      return general ? launch_inst<BITS, kZeroGeneral, kRow32>(pp, warps, grid, stream)
+                     : launch_inst<BITS, kZeroConstInt, kRow32>(pp, warps, grid, stream);
+  }
+  return general ? launch_inst<BITS, kZeroGeneral, kGeneral>(pp, warps, grid, stream)
+                 : launch_inst<BITS, kZeroConstInt, kGeneral>(pp, warps, grid, stream);
+}
+
+#endif  // __CUDACC__
+
+}  // namespace rk
+
+// Host entry.  Ungrouped: 1 <= p.m <= 8.  Grouped (indptr != nullptr): p.m = total rows, at most 32.
+int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const int64_t* indptr, int has_prev,
+                int num_experts, int64_t w_expert_bytes, int64_t s_expert_stride, cudaStream_t stream);
+
+}  // namespace rb200

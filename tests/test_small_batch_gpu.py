@@ -1,0 +1,59 @@
+"""The small-batch decode kernel (m <= 8, and expert layers of at most 32 rows) where its split can go
+wrong: k slices without a chunk, short last chunks and row tiles, odd row-block counts, the four-warp
+form of wide weights, scale sources, and experts with more rows than one pass holds."""
+import numpy as np
+import pytest
+import torch
+
+from relax_b200 import ops, synth
+from tests.test_gemv_gpu import _check_status
+from tests.util import assert_close, to_dev, u32_to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("m", [1, 8])
+@pytest.mark.parametrize("k,n,group,asym", [(64, 16, 32, False), (704, 48, 32, True), (2304, 1040, 32, False),
+                                            (2304, 400, 128, True), (1920, 144, 96, True), (256, 29056, 32, False),
+                                            (512, 28688, 256, True)])
+def test_int4_split(oracle, m, k, n, group, asym):
+    case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, group, asymmetric=asym)
+    pre = ops.preprocess_weight_q4f16(u32_to_dev(case.w))
+    z = to_dev(case.zeros) if asym else None
+    out = ops.gemm_fp16_q4f16(to_dev(case.x), pre, to_dev(case.scales), z, group_size=group)
+    _check_status()
+    C = oracle.C()
+    assert_close(out.cpu().numpy(), C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, case.zeros, 7.0, group))))
+
+
+@pytest.mark.parametrize("k,n,group", [(32, 16, -1), (288, 80, -1), (1056, 272, 32), (1152, 144, 64), (128, 28704, -1)])
+def test_int8_split(oracle, k, n, group):
+    m = 5
+    rs = np.random.RandomState(k + n)
+    x = rs.randn(m, k).astype(np.float16)
+    packed = rs.randint(-127, 128, size=(k, n)).astype(np.int8)
+    scales = rs.uniform(1e-4, 1e-3, size=(n,) if group < 0 else (k // group, n)).astype(np.float16)
+    out = ops.gemm_fp16_ft(to_dev(x), ops.preprocess_weight_ft(to_dev(packed), False), to_dev(scales), 8, group_size=group)
+    _check_status()
+    C = oracle.C()
+    assert_close(out.cpu().numpy(), C.epilogue(C.matmul_f32(x, C.decode_ft_kn(packed, scales, 8, group), False)))
+
+
+@pytest.mark.parametrize("rows", [[0, 9, 0, 23], [32, 0, 0, 0], [1, 1, 1, 1], [0, 0, 0, 0]])
+@pytest.mark.parametrize("bits,k,n", [(4, 384, 144), (8, 320, 16), (4, 128, 7168)])
+def test_experts(oracle, rows, bits, k, n):
+    rs = np.random.RandomState(sum(rows) + n)
+    x = rs.randn(32, k).astype(np.float16)
+    w = rs.randint(-128, 128, size=(4, k, n // 2 if bits == 4 else n)).astype(np.int8)
+    s = rs.uniform(0.001, 0.01, size=(4, k // 64, n)).astype(np.float16)
+    indptr = np.cumsum(rows).astype(np.int64)
+    out = torch.full((32, n), -7.0, dtype=torch.float16, device="cuda")
+    ops.moe_gemm_ft(to_dev(x), ops.preprocess_weight_ft(to_dev(w), bits == 4), to_dev(s), torch.from_numpy(indptr).cuda(), out=out)
+    _check_status()
+    C = oracle.C()
+    total = int(indptr[-1])
+    got = out.cpu().numpy()
+    assert np.all(got[total:] == -7.0)  # rows of no expert stay as they are
+    if total:
+        wq = np.stack([C.decode_ft_kn(w[e], s[e], bits, 64).T for e in range(4)])
+        assert_close(got[:total], C.epilogue(C.group_gemm_f32(x[:total], np.ascontiguousarray(wq), indptr)))
