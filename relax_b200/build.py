@@ -16,6 +16,8 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 _SRC = os.path.join(_PKG, "csrc")
 _OBJ = os.path.join(_PKG, "build")
 LIB_PATH = os.path.join(_PKG, "librelax_b200.so")
+_HOST_SRC = os.path.join(_PKG, "csrc_host", "torch_host.cc")
+HOST_PATH = os.path.join(_PKG, "_torch_host.so")
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -46,7 +48,32 @@ def _stale(src: str, obj: str, headers_mtime: float) -> bool:
     return os.path.getmtime(src) > t or headers_mtime > t
 
 
+def build_host(force: bool = False) -> str:
+    """The Python entry points in native code (``_torch_host.so``), against the installed torch."""
+    headers = glob.glob(os.path.join(_PKG, "..", "include", "*.h"))
+    if not force and not _stale(_HOST_SRC, HOST_PATH, max([os.path.getmtime(h) for h in headers] + [0.0])):
+        return HOST_PATH
+    import sysconfig
+
+    import torch
+    base = os.path.dirname(torch.__file__)
+    cuda = os.path.dirname(os.path.dirname(_nvcc()))
+    cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
+    cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+    for inc in (os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
+                os.path.join(cuda, "include"), sysconfig.get_paths()["include"]):
+        cmd.append("-I" + inc)
+    cmd += [_HOST_SRC, "-o", HOST_PATH, "-L" + os.path.join(base, "lib"), "-lc10", "-lc10_cuda", "-ltorch_cpu",
+            "-ltorch_cuda", "-ltorch_python"]
+    r = subprocess.run(cmd, capture_output=True, text=True)
+    if r.returncode != 0:
+        raise RuntimeError("host module: %s\n%s\n%s" % (" ".join(cmd), r.stdout, r.stderr))
+    return HOST_PATH
+
+
 def build(force: bool = False, verbose: bool = False) -> str:
+    build_host(force)
     os.makedirs(_OBJ, exist_ok=True)
     headers = glob.glob(os.path.join(_SRC, "*.h")) + glob.glob(os.path.join(_SRC, "*.cuh")) + \
         glob.glob(os.path.join(_PKG, "..", "include", "*.h"))

@@ -238,7 +238,13 @@ template <int BITS, bool PER_ROW>
 int launch_slices(const void* a, void* packed, void* scales, int64_t n, int64_t k, int slice, int group, int slices,
                   size_t smem, cudaStream_t stream) {
   auto kern = encode_slices_kernel<BITS, PER_ROW>;
-  RB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+  static thread_local int configured_device = -1;
+  int dev = 0;
+  RB200_CUDA(cudaGetDevice(&dev));
+  if (configured_device != dev) {
+    RB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
+    configured_device = dev;
+  }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = dim3((unsigned)(n / kRows), (unsigned)slices, 1);
   cfg.blockDim = dim3(256, 1, 1);

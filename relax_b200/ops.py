@@ -6,6 +6,7 @@ from typing import Optional
 
 import torch
 
+from ._host import native
 from .packed_func import get_global_func
 
 LAYOUT_FT_KN = 0
@@ -29,18 +30,7 @@ def gemm_fp16_ft(x, w_pre, scales, weight_bits: int, bias=None, residual=None,
                  group_size: int = -1, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``act(x @ decode(w) + bias)`` (optionally combined with a residual) for FT-layout weights:
     the call python/tvm/contrib/cutlass/gemm_operation.py:441-458 emits."""
-    k = x.shape[-1]
-    n = w_pre.shape[-1] * (2 if weight_bits == 4 else 1)
-    m = x.numel() // k
-    if out is None:
-        out = torch.empty(*x.shape[:-1], n // 2 if activation == "swiglu" else n, dtype=torch.float16, device=x.device)
-    bias_stride = 0
-    if bias is not None and bias.numel() == m * n and m > 1:
-        bias_stride = n
-    name = "cutlass.ft_gemm_fp16_int4" if weight_bits == 4 else "cutlass.ft_gemm_fp16_int8"
-    get_global_func(name)(x, w_pre, scales, bias, residual, activation, binary_op, unary_op, m, n, k,
-                          int(group_size if group_size > 0 else k), bias_stride, out)
-    return out
+    return native.gemm_ft(x, w_pre, scales, weight_bits, bias, residual, activation, binary_op, unary_op, group_size, out)
 
 
 def gemm_fp16_q4f16(x, w_pre, scales, zeros=None, bias=None, residual=None,
@@ -49,13 +39,8 @@ def gemm_fp16_q4f16(x, w_pre, scales, zeros=None, bias=None, residual=None,
                     out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Decode + matmul for q4f16_1-layout weights (tests/python/dlight/test_gpu_gemv.py:193-206),
     fp32 accumulation, fp16 output."""
-    n = w_pre.shape[0] // (2 if activation == "swiglu" else 1)
-    if out is None:
-        out = torch.empty(*x.shape[:-1], n, dtype=torch.float16, device=x.device)
-    get_global_func("relax_b200.gemm_fp16_q4f16")(x, w_pre, scales, zeros, bias, residual, activation,
-                                                  binary_op, unary_op, int(group_size),
-                                                  float(zero_const), out)
-    return out
+    return native.gemm_q4(x, w_pre, scales, zeros, bias, residual, activation, binary_op, unary_op, group_size,
+                          zero_const, out)
 
 
 def dequantize(w_pre, scales, n: int, k: int, weight_bits: int, layout: int, zeros=None,
@@ -72,10 +57,7 @@ def group_gemm_fp16(x, weight, indptr, workspace=None, out: Optional[torch.Tenso
     src/runtime/contrib/cutlass/fp16_group_gemm.cu:39-64 registers as
     ``cutlass.group_gemm_fp16_sm90`` (x fp16 [M, K], weight fp16 [E, N, K], indptr int64 [E] on
     the device)."""
-    if out is None:
-        out = torch.empty(x.shape[0], weight.shape[1], dtype=torch.float16, device=x.device)
-    get_global_func("cutlass.group_gemm_fp16_sm90")(x, weight, indptr, workspace, out)
-    return out
+    return native.group_fp16(x, weight, indptr, workspace, out)
 
 
 def moe_gemm_ft(x, w_pre, scales, indptr, zeros=None, out: Optional[torch.Tensor] = None,
@@ -84,27 +66,14 @@ def moe_gemm_ft(x, w_pre, scales, indptr, zeros=None, out: Optional[torch.Tensor
     [E, K, N] (int8) from :func:`preprocess_weight_ft`, ``scales`` fp16 [E, K/g, N] or [E, N].
     Expert-sharded layers: ``w_pre`` / ``scales`` hold experts ``first_expert ..`` only while
     ``indptr`` is the whole layer's table; rows of other experts are left untouched in ``out``."""
-    n = scales.shape[-1]
-    if out is None:
-        out = torch.empty(x.shape[0], n, dtype=torch.float16, device=x.device)
-    e_local = w_pre.shape[0]
-    if first_expert or e_local != indptr.shape[0]:
-        view = indptr[first_expert:first_expert + e_local]
-        get_global_func("cutlass.moe_gemm")(x, w_pre, scales, zeros, view, None, out, 1 if first_expert else 0)
-    else:
-        get_global_func("cutlass.moe_gemm")(x, w_pre, scales, zeros, indptr, None, out)
-    return out
+    return native.moe_ft(x, w_pre, scales, indptr, zeros, out, first_expert)
 
 
 def moe_gemm_q4f16(x, w_pre, scales, indptr, zeros=None, group_size: int = 32, zero_const: float = 7.0,
                    out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """Grouped decode-matmul over q4f16_1-layout experts: ``w_pre`` [E, N, K/8] words from
     :func:`preprocess_weight_q4f16`, ``scales`` fp16 [E, N, K/g]."""
-    if out is None:
-        out = torch.empty(x.shape[0], w_pre.shape[1], dtype=torch.float16, device=x.device)
-    get_global_func("relax_b200.moe_gemm_q4f16")(x, w_pre, scales, zeros, indptr, int(group_size),
-                                                 float(zero_const), out)
-    return out
+    return native.moe_q4(x, w_pre, scales, indptr, zeros, group_size, zero_const, out)
 
 
 def gptq_act_order(g_idx: torch.Tensor, groups: int) -> torch.Tensor:
@@ -119,9 +88,7 @@ def gptq_act_order(g_idx: torch.Tensor, groups: int) -> torch.Tensor:
 
 def gather_columns(x: torch.Tensor, perm: torch.Tensor) -> torch.Tensor:
     """``x[..., perm]`` for fp16 ``x`` (the activation side of an act-order weight)."""
-    out = torch.empty_like(x)
-    get_global_func("relax_b200.gather_columns")(x.contiguous(), perm, out)
-    return out
+    return native.gather_columns(x, perm)
 
 
 def preprocess_weight_autogptq(qweight: torch.Tensor, perm: Optional[torch.Tensor] = None) -> torch.Tensor:
@@ -151,39 +118,18 @@ def gemm_fp16_autogptq(x, w_pre, scales, zeros, bias=None, g_idx=None, perm=None
     :func:`unpack_zeros_autogptq`.  With groups in order along k (``g_idx = k // group_size``)
     nothing else is needed.  For an act-order weight pass the ``perm`` that ``w_pre`` was repacked
     with: ``x`` is gathered through it first.  A reordered ``g_idx`` without ``perm`` is rejected."""
-    k, n = w_pre.shape[0] * 8, w_pre.shape[1]
-    if perm is not None:
-        x = gather_columns(x, perm)
-    elif g_idx is not None:
-        expect = torch.arange(k, device=g_idx.device) // (k // scales.shape[0])
+    if perm is None and g_idx is not None:
+        expect = torch.arange(w_pre.shape[0] * 8, device=g_idx.device) // (w_pre.shape[0] * 8 // scales.shape[0])
         if not torch.equal(g_idx.to(torch.int64), expect):
             raise ValueError("g_idx reorders the groups: repack the weight with gptq_act_order's perm and pass perm")
-    if out is None:
-        out = torch.empty(*x.shape[:-1], n, dtype=torch.float16, device=x.device)
-    get_global_func("relax_b200.gemm_fp16_autogptq")(x, w_pre, scales, zeros, bias, out)
-    return out
+    return native.gemm_gptq(x, w_pre, scales, zeros, bias, perm, out)
 
 
 def encode_ft(y: torch.Tensor, weight_bits: int, group_size: int = -1):
     """The reference tests' quantiser on the GPU (tests/python/relax/test_codegen_cutlass.py:1391-1457,
     :1630-1676, :2043-2109): ``y`` fp16 [N, K] -> ``(packed int8 [K, N/2] | [K, N], scales fp16 [N] |
     [K/group, N])``, ready for :func:`preprocess_weight_ft`."""
-    import ctypes
-    from . import _lib
-    n, k = y.shape
-    per_row = group_size <= 0 or group_size >= k
-    packed = torch.empty(k, n // 2 if weight_bits == 4 else n, dtype=torch.int8, device=y.device)
-    scales = torch.empty((n,) if per_row else (k // group_size, n), dtype=torch.float16, device=y.device)
-    y = y.contiguous()
-    _lib.check(_lib.load().rb200_encode_ft(ctypes.c_void_p(y.data_ptr()), ctypes.c_void_p(packed.data_ptr()),
-                                           ctypes.c_void_p(scales.data_ptr()), n, k, int(weight_bits),
-                                           int(group_size), ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
-    return packed, scales
-
-
-def _ptr(t):
-    import ctypes
-    return ctypes.c_void_p(t.data_ptr())
+    return native.encode_ft(y, weight_bits, group_size)
 
 
 def moe_route(logits: torch.Tensor, top_k: int, out=None, workspace: Optional[torch.Tensor] = None):
@@ -192,27 +138,7 @@ def moe_route(logits: torch.Tensor, top_k: int, out=None, workspace: Optional[to
     of the grouped matmul (src/runtime/contrib/cutlass/fp16_group_gemm.cu:39-64).  ``out`` (the same
     four tensors) and ``workspace`` (uint8, :func:`moe_route_workspace_bytes`) make the call
     allocation-free, e.g. for CUDA-graph capture; ``logits`` must then be contiguous fp32."""
-    import ctypes
-    from . import _lib
-    lib = _lib.load()
-    t, e = logits.shape
-    r = t * top_k
-    dev = logits.device
-    if out is None:
-        out = (torch.empty(e, dtype=torch.int64, device=dev), torch.empty(r, dtype=torch.int32, device=dev),
-               torch.empty(r, dtype=torch.float32, device=dev), torch.empty(r, dtype=torch.int32, device=dev))
-    indptr, token_of_row, gate_of_row, row_of_flat = out
-    nbytes = lib.rb200_moe_route_workspace_bytes(t, top_k)
-    if workspace is None:
-        workspace = torch.empty(nbytes, dtype=torch.uint8, device=dev)
-    elif workspace.numel() < nbytes:
-        raise ValueError("routing workspace holds %d bytes, %d needed" % (workspace.numel(), nbytes))
-    if logits.dtype != torch.float32 or not logits.is_contiguous():
-        logits = logits.contiguous().float()
-    _lib.check(lib.rb200_moe_route(_ptr(logits), t, e, top_k, _ptr(indptr), _ptr(token_of_row), _ptr(gate_of_row),
-                                   _ptr(row_of_flat), _ptr(workspace), workspace.numel(),
-                                   ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
-    return indptr, token_of_row, gate_of_row, row_of_flat
+    return native.moe_route(logits, top_k, out, workspace)
 
 
 def moe_route_workspace_bytes(tokens: int, top_k: int) -> int:
@@ -222,28 +148,13 @@ def moe_route_workspace_bytes(tokens: int, top_k: int) -> int:
 
 def moe_gather(x: torch.Tensor, token_of_row: torch.Tensor, out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[r] = x[token_of_row[r]]``: the rows of x in the grouped matmul's order."""
-    import ctypes
-    from . import _lib
-    if out is None:
-        out = torch.empty(token_of_row.numel(), x.shape[1], dtype=torch.float16, device=x.device)
-    x = x.contiguous()
-    _lib.check(_lib.load().rb200_moe_gather(_ptr(x), _ptr(token_of_row), _ptr(out), token_of_row.numel(), x.shape[1],
-                                            ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
-    return out
+    return native.moe_gather(x, token_of_row, out)
 
 
 def moe_combine(y: torch.Tensor, row_of_flat: torch.Tensor, gate_of_row: torch.Tensor, top_k: int,
                 out: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``out[t] = sum over the token's top_k rows of gate * y[row]`` (fp32 sum, one rounding)."""
-    import ctypes
-    from . import _lib
-    tokens = row_of_flat.numel() // top_k
-    if out is None:
-        out = torch.empty(tokens, y.shape[1], dtype=torch.float16, device=y.device)
-    y = y.contiguous()
-    _lib.check(_lib.load().rb200_moe_combine(_ptr(y), _ptr(row_of_flat), _ptr(gate_of_row), _ptr(out), tokens, top_k,
-                                             y.shape[1], ctypes.c_void_p(torch.cuda.current_stream().cuda_stream)))
-    return out
+    return native.moe_combine(y, row_of_flat, gate_of_row, top_k, out)
 
 
 def preprocess_weight_gate_up(packed_weight: torch.Tensor, layout: int = LAYOUT_Q4_NK, is_int4: bool = True) -> torch.Tensor:

@@ -12,7 +12,7 @@ only; nothing here computes.
 from __future__ import annotations
 
 from dataclasses import dataclass
-from functools import reduce
+from functools import lru_cache, reduce
 from typing import Dict, Optional, Sequence
 
 BASE_PATTERNS = (
@@ -118,31 +118,33 @@ def call_arguments(name: str, lhs_shape, w_shape, scales_shape, out_shape, bias_
             "attrs": PATTERN_TABLE[name]}
 
 
+@lru_cache(maxsize=1024)
+def _call_plan(name: str, x_shape, x_dtype, w_shape, w_dtype, s_shape, s_dtype, bias_shape, residual: bool):
+    """The checks and scalar arguments of one pattern call, by shapes and types alone:
+    (weight_bits, activation, binary_op, unary_op, group_size)."""
+    a = PATTERN_TABLE[name]
+    if a.bias != (bias_shape is not None):
+        raise ValueError("%s %s a bias" % (name, "takes" if a.bias else "does not take"))
+    if a.residual != residual:
+        raise ValueError("%s %s a residual" % (name, "takes" if a.residual else "does not take"))
+    n = w_shape[-1] * 2 if s_shape[-1] == w_shape[-1] * 2 else w_shape[-1]
+    out_shape = tuple(x_shape[:-1]) + (n,)
+    ok = check_decode_matmul(tuple(x_shape), str(x_dtype).replace("torch.", ""), tuple(w_shape),
+                             str(w_dtype).replace("torch.", ""), tuple(s_shape), str(s_dtype).replace("torch.", ""),
+                             out_shape, "float16", None if bias_shape is None else tuple(bias_shape))
+    if not ok:
+        raise ValueError("%s: the reference's pattern check rejects these shapes / dtypes" % name)
+    c = call_arguments(name, tuple(x_shape), tuple(w_shape), tuple(s_shape), out_shape,
+                       None if bias_shape is None else tuple(bias_shape))
+    return c["weight_bits"], a.activation, a.binary_op, a.unary_op, c["group_size"]
+
+
 def run_pattern(name: str, x, w_pre, scales, bias=None, residual=None, out=None):
     """Calls the registered operator for one pattern instance (tensors: torch, CUDA) the way the
     reference's generated host code does: ``cutlass.ft_gemm_fp16_int{4,8}`` with the pattern's
     activation / binary op / unary op names."""
-    import torch
-
-    from .packed_func import get_global_func
-    a = PATTERN_TABLE[name]
-    if a.bias != (bias is not None):
-        raise ValueError("%s %s a bias" % (name, "takes" if a.bias else "does not take"))
-    if a.residual != (residual is not None):
-        raise ValueError("%s %s a residual" % (name, "takes" if a.residual else "does not take"))
-    n = w_pre.shape[-1] * 2 if scales.shape[-1] == w_pre.shape[-1] * 2 else w_pre.shape[-1]
-    out_shape = tuple(x.shape[:-1]) + (n,)
-    ok = check_decode_matmul(tuple(x.shape), str(x.dtype).replace("torch.", ""), tuple(w_pre.shape),
-                             str(w_pre.dtype).replace("torch.", ""), tuple(scales.shape),
-                             str(scales.dtype).replace("torch.", ""), out_shape, "float16",
-                             None if bias is None else tuple(bias.shape))
-    if not ok:
-        raise ValueError("%s: the reference's pattern check rejects these shapes / dtypes" % name)
-    c = call_arguments(name, tuple(x.shape), tuple(w_pre.shape), tuple(scales.shape), out_shape,
-                       None if bias is None else tuple(bias.shape))
-    if out is None:
-        out = torch.empty(out_shape, dtype=torch.float16, device=x.device)
-    fn = get_global_func("cutlass.ft_gemm_fp16_int4" if c["weight_bits"] == 4 else "cutlass.ft_gemm_fp16_int8")
-    fn(x, w_pre, scales, bias, residual, a.activation, a.binary_op, a.unary_op, c["m"], c["n"], c["k"],
-       c["group_size"] if c["group_size"] > 0 else c["k"], c["bias_stride"], out)
-    return out
+    from ._host import native
+    bits, activation, binary_op, unary_op, group = _call_plan(
+        name, x.shape, x.dtype, w_pre.shape, w_pre.dtype, scales.shape, scales.dtype,
+        None if bias is None else bias.shape, residual is not None)
+    return native.gemm_ft(x, w_pre, scales, bits, bias, residual, activation, binary_op, unary_op, group, out)
