@@ -10,6 +10,7 @@
 #include "gemv.h"
 #include "gemv_cluster.cuh"
 #include "umma_gemm.cuh"
+#include "umma_sk.cuh"
 #include "gemv_rk.cuh"
 #include "gemv_sk.cuh"
 #include "gemm_tc.h"
@@ -33,8 +34,6 @@ void set_last_error(const char* fmt, ...) {
 // ---------------------------------------------------------------- per-device scratch
 namespace {
 constexpr int kMaxDevices = 64;
-// split-k flags of the stream-k decode kernel: inside the ticket area of the scratch block
-constexpr size_t kSkFlagOffset = 49152, kSkFlagCount = 16384;
 DeviceScratch g_scratch[kMaxDevices];
 std::mutex g_scratch_mutex;
 }  // namespace
@@ -88,7 +87,8 @@ DeviceScratch* device_scratch(size_t min_partial_bytes, size_t min_counter_ints)
   if (counters < min_counter_ints) counters = min_counter_ints;
   const size_t header = 256;
   const size_t counter_bytes = ((counters * sizeof(int) + 255) / 256) * 256;
-  s.bytes = header + counter_bytes + partial;
+  const size_t vacant = (size_t)s.sm_count * 128 * 256 * sizeof(float);  // one 128 x 256 fp32 tile per SM
+  s.bytes = header + counter_bytes + partial + vacant;
   cudaError_t e = cudaMalloc(&s.base, s.bytes);
   if (e != cudaSuccess) {
     set_last_error("cudaMalloc(%zu) for library scratch failed: %s", s.bytes, cudaGetErrorString(e));
@@ -101,6 +101,9 @@ DeviceScratch* device_scratch(size_t min_partial_bytes, size_t min_counter_ints)
   s.counter_ints = counters;
   s.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(s.base) + header + counter_bytes);
   s.partial_bytes = partial;
+  s.vacant_words = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(s.partials) + partial);
+  s.vacant_bytes = vacant;
+  cudaMemset(s.vacant_words, 0xff, vacant);
   return &s;
 }
 
@@ -258,6 +261,7 @@ int rb200_check_async_error(void* stream, int* status_out) {
     if (v != 0) {
       // a wait that gave up may have left split-k flags and tickets behind: back to rest
       RB200_CUDA(cudaMemset(sc->base, 0, (size_t)(reinterpret_cast<uint8_t*>(sc->partials) - static_cast<uint8_t*>(sc->base))));
+      RB200_CUDA(cudaMemset(sc->vacant_words, 0xff, sc->vacant_bytes));
       st = v;
     }
   }
@@ -427,8 +431,13 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
     // against stream-k: k = n = 4096 3.9 / 8.1 us, n 22016 13.9 / 19.1, k 11008 x n 4096 8.0 / 13.4.
     if (p.m <= rk::kMaxBatch && !ar)
       return gemv_rk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
+    unsigned* flags = reinterpret_cast<unsigned*>(sc->counters) + kSkFlagOffset;
+    if (!ar) {
+      const int rc = umma_sk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, sc->vacant_words, sc->vacant_bytes, nullptr,
+                                 0, 1, 0, 0, stream);
+      if (rc <= 0) return rc;
+    }
     if (p.k % 64 == 0) {
-      unsigned* flags = reinterpret_cast<unsigned*>(sc->counters) + kSkFlagOffset;
       return gemv_sk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, sc->partials, sc->partial_bytes, flags,
                          kSkFlagCount, ar, stream);
     }
@@ -622,6 +631,10 @@ int rb200_group_gemm(const rb200_group_gemm_desc* d, void* stream_v) {
     return gemv_rk_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0, (int)d->num_experts,
                        w_expert_bytes, d->scale_stride_e, static_cast<cudaStream_t>(stream_v));
   }
+  if (packed)
+    return umma_sk_run(p, d->weight_bits, zmode, sc->sm_count, sc->vacant_words, sc->vacant_bytes, d->indptr,
+                       d->indptr_has_prev ? 1 : 0, (int)d->num_experts, w_expert_bytes, d->scale_stride_e,
+                       static_cast<cudaStream_t>(stream_v));
   return umma_group_gemm_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0,
                              (int)d->num_experts, w_expert_bytes,
                              packed ? d->scale_stride_e : 0, static_cast<cudaStream_t>(stream_v));

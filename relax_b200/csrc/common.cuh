@@ -33,6 +33,9 @@ void set_last_error(const char* fmt, ...);
     }                                                                                     \
   } while (0)
 
+// Split-k flags of the stream-k decode kernel: inside the ticket area of the scratch block, zero at rest.
+constexpr size_t kSkFlagOffset = 49152, kSkFlagCount = 16384;
+
 // Per-device library-owned state (scratch for split-K partials, tile counters, status word).
 struct DeviceScratch {
   void* base = nullptr;     // one cudaMalloc: [status word | counters | partials]
@@ -42,6 +45,8 @@ struct DeviceScratch {
   size_t counter_ints = 0;
   float* partials = nullptr;
   size_t partial_bytes = 0;
+  uint32_t* vacant_words = nullptr;  // hand-over words of the medium-batch kernel, all bits set at rest
+  size_t vacant_bytes = 0;
   int sm_count = 0;
 };
 // Returns the current device's scratch, allocating it on first use (never inside a capture:

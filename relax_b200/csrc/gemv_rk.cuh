@@ -1,6 +1,6 @@
-// Decode-path kernel for at most eight batch rows: row blocks per CTA, k split over its warps.
+// Decode-path kernel for at most sixteen batch rows: row blocks per CTA, k split over its warps.
 //
-//   out[m, n] = epilogue(sum_k x[m, k] * wq[n, k]),  m <= 8 (the n of one m16n8k16 MMA)
+//   out[m, n] = epilogue(sum_k x[m, k] * wq[n, k]),  m <= 8 or 16 (one or two m16n8k16 MMAs wide)
 //
 // Bound: HBM (the packed weight once) and, close behind, instruction issue: the exact two-rounding
 // decode is 52 of the 61 instructions a 512-byte tile needs (4 MMAs, 3 loads, 2 scale selects).
@@ -35,7 +35,8 @@ namespace rb200 {
 namespace rk {
 
 constexpr int kRows = 2;         // row blocks of one pass: activations fetched once serve both
-constexpr int kMaxBatch = 8;
+constexpr int kMaxBatch = 16;   // two m-tiles of eight rows
+constexpr int kEntryRows = 8;   // grouped form: batch rows of one entry
 constexpr int kLeadChunks = 2;   // chunks between an L2 prefetch and the load
 constexpr int kMaxEntries = 96;  // grouped form: (expert, eight batch rows) pairs; 64 experts, 32 rows in all
 
@@ -84,19 +85,20 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
-template <int kXV>
+template <int kXV, int MT>
 struct XHalf {
-  uint4 v[2][kXV];
+  uint4 v[2][MT][kXV];
 };
 
 // kWarps: warps per CTA = k slices of a row block (16 warps per SM either way)
-template <int BITS, int ZMODE, int SRC, bool GROUPED, int kWarps>
+// MT: m-tiles of eight batch rows (MMA n)
+template <int BITS, int ZMODE, int SRC, bool GROUPED, int kWarps, int MT>
 __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const Params pp) {
   constexpr int kFrag = BITS == 4 ? 64 : 32;
   constexpr int kLaneK = kFrag / 4;
   constexpr int kXV = BITS == 4 ? 2 : 1;  // 16-byte pieces of x per lane and tile
   constexpr bool kZ = ZMODE == kZeroGeneral;
-  __shared__ __align__(16) float4 red[2][kWarps][kRows][32];
+  __shared__ __align__(16) float4 red[2][kWarps][kRows * MT][32];
   __shared__ int s_entries, s_m_lo[kMaxEntries], s_m_n[kMaxEntries], s_expert[kMaxEntries];
   const GemvParams& p = pp.g;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -117,7 +119,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
           r0 = (e || pp.has_prev) ? (int)pp.indptr[e - 1] : 0;
           r1 = min((int)pp.indptr[e], p.m);  // never past the rows x / out hold
         }
-        const int mine = r1 > r0 ? (r1 - r0 + kMaxBatch - 1) / kMaxBatch : 0;
+        const int mine = r1 > r0 ? (r1 - r0 + kEntryRows - 1) / kEntryRows : 0;
         int incl = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
@@ -127,8 +129,8 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
         for (int i = 0; i < mine; ++i) {
           const int slot = n_e + incl - mine + i;
           if (slot < kMaxEntries) {
-            s_m_lo[slot] = r0 + i * kMaxBatch;
-            s_m_n[slot] = min(kMaxBatch, r1 - r0 - i * kMaxBatch);
+            s_m_lo[slot] = r0 + i * kEntryRows;
+            s_m_n[slot] = min(kEntryRows, r1 - r0 - i * kEntryRows);
             s_expert[slot] = e;
           }
         }
@@ -284,45 +286,49 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 
   int buf = 0;
   for (;;) {
-    float acc[kRows][2][4];
+    constexpr int kChains = MT == 1 ? 2 : 1;  // independent MMA chains (two m-tiles are two already)
+    float acc[kRows][MT][kChains][4];
 #pragma unroll
     for (int r = 0; r < kRows; ++r)
 #pragma unroll
-      for (int c = 0; c < 4; ++c) acc[r][0][c] = acc[r][1][c] = 0.0f;
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int i = 0; i < kChains; ++i)
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[r][mt][i][c] = 0.0f;
     // lanes of absent batch rows fetch row 0: their columns of the result are never stored
     const __half* x0 = p.x + (q.m_lo + (g < q.m_n ? g : 0)) * (unsigned)p.ldx + t * kLaneK;
+    const unsigned x_next = MT > 1 && g + 8 < q.m_n ? 8u * (unsigned)p.ldx : 0u;  // elements to the second m-tile's row
 
     auto mma_tile = [&](int r, const uint4& wv, uint32_t s_g, uint32_t s_g8, uint32_t z_g, uint32_t z_g8,
-                        const uint4 (&xv)[kXV]) {
-      uint32_t a[4];
-      if (BITS == 4) {
-        decode_int4_word<ZMODE>(wv.x, zc, s_g, s_g8, z_g, z_g8, a);
-        mma_16816(acc[r][0], a, xv[0].x, xv[0].y);
-        decode_int4_word<ZMODE>(wv.y, zc, s_g, s_g8, z_g, z_g8, a);
-        mma_16816(acc[r][1], a, xv[0].z, xv[0].w);
-        decode_int4_word<ZMODE>(wv.z, zc, s_g, s_g8, z_g, z_g8, a);
-        mma_16816(acc[r][0], a, xv[kXV - 1].x, xv[kXV - 1].y);
-        decode_int4_word<ZMODE>(wv.w, zc, s_g, s_g8, z_g, z_g8, a);
-        mma_16816(acc[r][1], a, xv[kXV - 1].z, xv[kXV - 1].w);
-      } else {
-        decode_int8_pair<ZMODE>(wv.x, wv.y, zc, s_g, s_g8, z_g, z_g8, a);
-        mma_16816(acc[r][0], a, xv[0].x, xv[0].y);
-        decode_int8_pair<ZMODE>(wv.z, wv.w, zc, s_g, s_g8, z_g, z_g8, a);
-        mma_16816(acc[r][1], a, xv[0].z, xv[0].w);
+                        const uint4 (&xv)[MT][kXV]) {
+      const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+      for (int j = 0; j < 2 * kXV; ++j) {  // MMAs of the tile: four int4 words, two int8 word pairs
+        uint32_t a[4];
+        if (BITS == 4) decode_int4_word<ZMODE>(ww[j], zc, s_g, s_g8, z_g, z_g8, a);
+        else decode_int8_pair<ZMODE>(ww[2 * (j & 1)], ww[2 * (j & 1) + 1], zc, s_g, s_g8, z_g, z_g8, a);
+#pragma unroll
+        for (int mt = 0; mt < MT; ++mt) {
+          const uint4& x = xv[mt][j >> 1];
+          mma_16816(acc[r][mt][j % kChains], a, (j & 1) ? x.z : x.x, (j & 1) ? x.w : x.y);
+        }
       }
     };
     const __half* xp = x0 + c0 * (kFrag * 4);
     // activations of either half: int8 fetches them half a chunk ahead, int4 has no registers to spare
     // for that and fetches them where they are used
     constexpr bool kXAhead = BITS == 8;
-    XHalf<kXV> xa, xb;
-    auto load_x = [&](XHalf<kXV>& xv, int half) {
+    XHalf<kXV, MT> xa, xb;
+    auto load_x = [&](XHalf<kXV, MT>& xv, int half) {
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int i = 0; i < kXV; ++i) xv.v[j][i] = ld_nc_v4(xp + (half * 2 + j) * kFrag + i * 8);
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int i = 0; i < kXV; ++i) xv.v[j][mt][i] = ld_nc_v4(xp + mt * x_next + (half * 2 + j) * kFrag + i * 8);
     };
-    auto half_step = [&](auto set_tag, auto rn_tag, const XHalf<kXV>& xv) {
+    auto half_step = [&](auto set_tag, auto rn_tag, const XHalf<kXV, MT>& xv) {
       constexpr int S = decltype(set_tag)::value, RN = decltype(rn_tag)::value;
 #pragma unroll
       for (int j = 0; j < 2; ++j)
@@ -395,9 +401,11 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 
     if (warp == kWarps - 1) {  // tiles of a short last chunk
       for (int kb = full_chunks * 4; kb < KB; ++kb) {
-        uint4 xt[kXV];
+        uint4 xt[MT][kXV];
 #pragma unroll
-        for (int i = 0; i < kXV; ++i) xt[i] = ld_nc_v4(x0 + kb * kFrag + i * 8);
+        for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+          for (int i = 0; i < kXV; ++i) xt[mt][i] = ld_nc_v4(x0 + mt * x_next + kb * kFrag + i * 8);
         const unsigned k = (unsigned)(kb * kFrag + t * kLaneK);
         const unsigned grp = SRC == kChannel ? 0u : (pp.group_shift >= 0 ? k >> pp.group_shift : k / (unsigned)p.group);
 #pragma unroll
@@ -424,13 +432,18 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
       start_pass(q);
     }
 
-    // the eight k slices meet in warp order
+    // the k slices meet in warp order
 #pragma unroll
     for (int r = 0; r < kRows; ++r)
-      red[buf][warp][r][lane] = make_float4(acc[r][0][0] + acc[r][1][0], acc[r][0][1] + acc[r][1][1],
-                                            acc[r][0][2] + acc[r][1][2], acc[r][0][3] + acc[r][1][3]);
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        float f[4];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) f[c] = acc[r][mt][0][c] + (kChains == 2 ? acc[r][mt][kChains - 1][c] : 0.0f);
+        red[buf][warp][r * MT + mt][lane] = make_float4(f[0], f[1], f[2], f[3]);
+      }
     __syncthreads();
-    if (warp < done.rn) {
+    if (warp < done.rn * MT) {
       float v[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
       for (int i = 0; i < kWarps; ++i) {
@@ -440,19 +453,19 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
         v[2] += f.z;
         v[3] += f.w;
       }
-      const int nb = done.nb0 + warp;
+      const int nb = done.nb0 + warp / MT, m8 = (warp % MT) * 8 + t * 2;
       if (p.epi.act == kActSwiglu) {
         // rows g / g + 8 of the block are gate_f / up_f of f = 8 nb + g (interleaved repack)
 #pragma unroll
         for (int cc = 0; cc < 2; ++cc) {
-          const int m = t * 2 + cc;
+          const int m = m8 + cc;
           if (m < done.m_n)
             p.out[(int64_t)(done.m_lo + m) * p.ldo + nb * 8 + g] = __float2half_rn(silu_mul(v[cc], v[cc + 2]));
         }
       } else {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          const int m = t * 2 + (i & 1);
+          const int m = m8 + (i & 1);
           const int64_t n = (int64_t)nb * 16 + g + (i >> 1) * 8;
           if (m < done.m_n)
             p.out[(int64_t)(done.m_lo + m) * p.ldo + n] = __float2half_rn(apply_epilogue(v[i], p.epi, done.m_lo + m, n));
@@ -477,13 +490,18 @@ int launch_inst(const Params& pp, int warps, int grid, cudaStream_t stream) {
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+#define RB200_RK(GR, W, M) RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, GR, W, M>, pp))
   if (pp.indptr) {
-    if (warps == 8) RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, true, 8>, pp));
-    else RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, true, 4>, pp));
+    if (warps == 8) RB200_RK(true, 8, 1);
+    else RB200_RK(true, 4, 1);
+  } else if (pp.g.m <= 8) {
+    if (warps == 8) RB200_RK(false, 8, 1);
+    else RB200_RK(false, 4, 1);
   } else {
-    if (warps == 8) RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, false, 8>, pp));
-    else RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, false, 4>, pp));
+    if (warps == 8) RB200_RK(false, 8, 2);
+    else RB200_RK(false, 4, 2);
   }
+#undef RB200_RK
   return 0;
 }
 
@@ -509,7 +527,7 @@ int launch_bits(const Params& pp, int zmode, int src, int warps, int grid, cudaS
 
 }  // namespace rk
 
-// Host entry.  Ungrouped: 1 <= p.m <= 8.  Grouped (indptr != nullptr): p.m = total rows, at most 32.
+// Host entry.  Ungrouped: 1 <= p.m <= 16.  Grouped (indptr != nullptr): p.m = total rows, at most 32.
 int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const int64_t* indptr, int has_prev,
                 int num_experts, int64_t w_expert_bytes, int64_t s_expert_stride, cudaStream_t stream);
 
