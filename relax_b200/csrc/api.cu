@@ -10,7 +10,7 @@
 #include "gemv.h"
 #include "gemv_cluster.cuh"
 #include "umma_gemm.cuh"
-#include "umma_sk.cuh"
+#include "umma_tile.cuh"
 #include "gemv_rk.cuh"
 #include "gemv_sk.cuh"
 #include "gemm_tc.h"
@@ -433,7 +433,7 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
       return gemv_rk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
     unsigned* flags = reinterpret_cast<unsigned*>(sc->counters) + kSkFlagOffset;
     if (!ar) {
-      const int rc = umma_sk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, sc->vacant_words, sc->vacant_bytes, nullptr,
+      const int rc = umma_run(p, d->weight_bits, zero_mode(d), sc->sm_count, sc->vacant_words, sc->vacant_bytes, nullptr,
                                  0, 1, 0, 0, stream);
       if (rc <= 0) return rc;
     }
@@ -632,7 +632,7 @@ int rb200_group_gemm(const rb200_group_gemm_desc* d, void* stream_v) {
                        w_expert_bytes, d->scale_stride_e, static_cast<cudaStream_t>(stream_v));
   }
   if (packed)
-    return umma_sk_run(p, d->weight_bits, zmode, sc->sm_count, sc->vacant_words, sc->vacant_bytes, d->indptr,
+    return umma_run(p, d->weight_bits, zmode, sc->sm_count, sc->vacant_words, sc->vacant_bytes, d->indptr,
                        d->indptr_has_prev ? 1 : 0, (int)d->num_experts, w_expert_bytes, d->scale_stride_e,
                        static_cast<cudaStream_t>(stream_v));
   return umma_group_gemm_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0,

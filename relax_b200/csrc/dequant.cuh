@@ -72,6 +72,11 @@ __device__ __forceinline__ uint32_t h2_sub(uint32_t a, uint32_t b) {
   asm("sub.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
+__device__ __forceinline__ uint32_t h2_add(uint32_t a, uint32_t b) {
+  uint32_t r;
+  asm("add.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
 __device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
   uint32_t r;
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
@@ -107,6 +112,10 @@ __device__ __forceinline__ uint32_t f2_to_h2(float lo, float hi) {
 // (row, group), subtracted with its own rounding exactly as the reference's fp16 TIR does.
 enum ZeroMode : int { kZeroConstInt = 0, kZeroGeneral = 1 };
 
+// kZeroExact: the form the kernels switch to when their zero points allow it (zero_offset_lo / _hi): the
+// offset zero point replaces the constant of kZeroConstInt, one operation per pair instead of two.
+constexpr int kZeroExact = 2;
+
 struct ZeroConsts {
   uint32_t sub_lo;   // f16x2(1024 + z)            (kZeroConstInt)  | f16x2(1024)  (kZeroGeneral)
   uint32_t add_hi;   // f16x2(-(64 + z))           (kZeroConstInt)  | f16x2(-64)   (kZeroGeneral)
@@ -117,6 +126,22 @@ __device__ __forceinline__ ZeroConsts make_zero_consts(int zmode, float zconst) 
   c.sub_lo = f2_to_h2(1024.0f + z, 1024.0f + z);
   c.add_hi = f2_to_h2(-(64.0f + z), -(64.0f + z));
   return c;
+}
+
+// f16x2(1024 + z) and f16x2(-(64 + z)) when that sum is exact, which integer zero points always are:
+// (1024 + u) - (1024 + z) is then u - z rounded once, the same as f16(u) - z.  `exact` keeps its value or
+// becomes false.
+__device__ __forceinline__ uint32_t zero_offset_lo(uint32_t z2, bool& exact) {
+  constexpr uint32_t k1024 = 0x64006400u;
+  const uint32_t o = h2_add(z2, k1024);
+  exact = exact && h2_sub(o, k1024) == z2;
+  return o;
+}
+__device__ __forceinline__ uint32_t zero_offset_hi(uint32_t z2, bool& exact) {
+  constexpr uint32_t k64 = 0x54005400u;
+  const uint32_t o = h2_add(z2, k64);
+  exact = exact && h2_sub(o, k64) == z2;
+  return o ^ 0x80008000u;
 }
 
 // One int4 word -> A fragment registers of one m16n8k16 MMA:

@@ -7,7 +7,7 @@
 #include <cstring>
 
 #include "umma_gemm.cuh"
-#include "umma_sk.cuh"
+#include "umma_tile.cuh"
 
 namespace rb200 {
 
@@ -34,10 +34,7 @@ int gemm_tc_launch(const rb200_gemm_desc* d, const Epilogue& epi, int group, int
     p.k = (int)d->k;
     p.group = group;
     p.zero_const = d->zero_const;
-    int rc = 1;
-    if (p.m > us::kMaxNb) rc = umma_gemm_run(p, d->weight_bits, zmode, sc->sm_count, stream);
-    if (rc > 0)
-      rc = umma_sk_run(p, d->weight_bits, zmode, sc->sm_count, sc->vacant_words, sc->vacant_bytes, nullptr, 0, 1, 0, 0, stream);
+    const int rc = umma_run(p, d->weight_bits, zmode, sc->sm_count, sc->vacant_words, sc->vacant_bytes, nullptr, 0, 1, 0, 0, stream);
     if (rc <= 0) return rc;
   }
   rb200_gemm_desc s = *d;

@@ -1,0 +1,8 @@
+#include "umma_pair.cuh"
+namespace rb200 {
+namespace up {
+int launch_i8(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream) {
+  return launch_bits<8>(pp, l, tx, stream);
+}
+}  // namespace up
+}  // namespace rb200

@@ -1,0 +1,181 @@
+// Host side of the tensor-core kernels over packed weights: coverage test, tile and pipeline plan, choice
+// between the one-CTA form (umma_sk) and CTA pairs (umma_pair), launch.
+#include "umma_pair.cuh"
+#include "umma_sk.cuh"
+
+#include <cmath>
+#include <cstring>
+
+#include "tensormap.h"
+
+namespace rb200 {
+
+namespace {
+using namespace us;
+
+int x_map(CUtensorMap* tx, const GemvParams& p, int rows) {
+  return make_tensor_map_2d(tx, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, (unsigned long long)p.k, (unsigned long long)p.m,
+                            (unsigned long long)p.ldx * 2, kKBlock, (unsigned)rows, CU_TENSOR_MAP_SWIZZLE_128B);
+}
+
+// Batch tiles of the pair kernel: of the splits of m into equal tiles of at most 256 rows, the one that the
+// clock counts below say is done first.  Per 64-k block the tensor pipe takes 2 nb clocks and the decode
+// of a CTA's 128 rows about 320, whichever is longer, so wide tiles win (2048 rows as 8 x 256 against
+// 11 x 192, whose drains overlap the next tile: 662 / 828 us for int8 k 8192 x n 28672) - unless there
+// are too few of them for the pairs: a tile cut over c more pairs costs its owner about 1600 clocks per
+// two parts and 48 columns (a trip to L2 each).
+int pair_m_tiles(long long n_tiles, int m, int k_blocks, int pairs) {
+  int best = 0;
+  double best_clk = 0.0;
+  const int least = (m + kMaxNb - 1) / kMaxNb;
+  for (int t = least; t <= least + 8; ++t) {
+    const int nb = ((m + t - 1) / t + 31) / 32 * 32;
+    if (t > least && nb < 64) break;
+    const long long items = n_tiles * t;
+    const double tiles = (double)items / pairs;
+    double clk = tiles * k_blocks * (nb * 2 > 320 ? nb * 2 : 320) + (tiles > 1.0 ? tiles : 1.0) * nb / 48.0 * 600.0;
+    if (items % pairs) clk += std::ceil((tiles < 1.0 ? 1.0 / tiles : 1.0) / 2.0) * nb / 48.0 * 1600.0;
+    if (best == 0 || clk < best_clk) {
+      best = t;
+      best_clk = clk;
+    }
+  }
+  return best;
+}
+
+int run_pair(Params& pp, int bits, int zmode, int src, int sm_count, size_t vacant_bytes, cudaStream_t stream) {
+  const GemvParams& p = pp.g;
+  const long long n_tiles = (p.n + 2 * kTileRows - 1) / (2 * kTileRows);
+  if (!pp.indptr) {
+    pp.m_tiles = pair_m_tiles(n_tiles, p.m, p.k / kKBlock, sm_count / 2);
+    pp.nb = (p.m + pp.m_tiles - 1) / pp.m_tiles;
+  }
+  pp.nb = (pp.nb + 31) / 32 * 32;
+  // tensor memory: two accumulators of up to 192 columns or one of 256, then A slots of 32 columns
+  pp.tmem_cols = 512;
+  pp.nd = pp.nb <= 192 ? 2 : 1;
+  pp.d_stride = pp.nb <= 128 ? 128 : (pp.nb <= 192 ? 192 : 256);
+  pp.a_base = pp.nd * pp.d_stride;
+  pp.na = (pp.tmem_cols - pp.a_base) / 32;
+  if (pp.na > kMaxA) pp.na = kMaxA;
+  const size_t budget = (size_t)227 * 1024;
+  pp.x_stages = kMaxStages;
+  pp.w_stages = kMaxStages;
+  while (pp.w_stages > 4 && up::smem_bytes(pp.nb, pp.x_stages, pp.w_stages) > budget) --pp.w_stages;
+  up::Launch l;
+  memset(&l, 0, sizeof(l));
+  l.zmode = zmode;
+  l.src = src;
+  l.smem = up::smem_bytes(pp.nb, pp.x_stages, pp.w_stages);
+  RB200_CHECK(l.smem <= budget, "pair kernel: %zu bytes of shared memory for %d batch rows", l.smem, pp.nb);
+  // most items a launch can have (grouped: every expert full tiles plus one ragged tile)
+  const long long items = pp.indptr ? n_tiles * ((long long)p.m / pp.nb + pp.num_experts) : n_tiles * pp.m_tiles;
+  RB200_CHECK(items < (1ll << 30), "too many tiles (n=%d, m=%d)", p.n, p.m);
+  l.most_pairs = items * pp.cpt;
+  RB200_CHECK((size_t)sm_count * pp.nb * kTileRows * sizeof(float) <= vacant_bytes, "split-k scratch too small for %d SMs", sm_count);
+  CUtensorMap tx;
+  if (x_map(&tx, p, pp.nb / 2) != 0) return -1;
+  return bits == 4 ? up::launch_i4(pp, l, tx, stream) : up::launch_i8(pp, l, tx, stream);
+}
+
+int run_single(Params& pp, int bits, int zmode, int src, int sm_count, size_t vacant_bytes, cudaStream_t stream) {
+  const GemvParams& p = pp.g;
+  if (!pp.indptr) {
+    pp.m_tiles = (p.m + kSmallNb - 1) / kSmallNb;
+    pp.nb = (p.m + pp.m_tiles - 1) / pp.m_tiles;
+  }
+  pp.nb = (pp.nb + 15) / 16 * 16;
+  // tensor memory: two accumulators, then A slots
+  pp.tmem_cols = 256;
+  pp.d_stride = pp.nb <= 32 ? 32 : 64;
+  pp.nd = 2;
+  pp.a_base = pp.nd * pp.d_stride;
+  const int own = bits == 4 ? 2 : 1;  // blocks per A slot (kOwn of the kernel)
+  pp.na = (pp.tmem_cols - pp.a_base) / (32 * own);
+  if (pp.na > kMaxA) pp.na = kMaxA;
+  // rings: x stages first (one 64-k block each), then as many weight stages as fit
+  const size_t budget = (size_t)(228 * 1024) / 2 - 1024;
+  pp.x_stages = 4;
+  pp.w_stages = kMaxStages;
+  while (pp.w_stages > 3 && smem_bytes(pp.nb, pp.x_stages, pp.w_stages) > budget) --pp.w_stages;
+  while (pp.x_stages < kMaxStages && smem_bytes(pp.nb, pp.x_stages + 1, pp.w_stages) <= budget) ++pp.x_stages;
+  Launch l;
+  memset(&l, 0, sizeof(l));
+  l.zmode = zmode;
+  l.src = src;
+  l.smem = smem_bytes(pp.nb, pp.x_stages, pp.w_stages);
+  RB200_CHECK(l.smem <= budget, "medium-batch kernel: %zu bytes of shared memory for %d batch rows", l.smem, pp.nb);
+  const long long n_tiles = (p.n + kTileRows - 1) / kTileRows;
+  const long long items = pp.indptr ? n_tiles * ((long long)p.m / pp.nb + pp.num_experts) : n_tiles * pp.m_tiles;
+  const long long units = items * pp.cpt;
+  long long grid = (long long)sm_count * 2;
+  // a tile cut into many short ranges spends its time in the hand-over: at least three chunks per CTA
+  // before a second CTA per SM
+  if (units < 3 * grid) grid = sm_count;
+  if (grid > units) grid = units;
+  RB200_CHECK(units * grid < (1ll << 31), "problem too large for the 32-bit work split (n=%d, k=%d, m=%d)", p.n, p.k, p.m);
+  l.grid = (int)grid;
+  RB200_CHECK((size_t)grid * pp.nb * kTileRows * sizeof(float) <= vacant_bytes, "split-k scratch too small for a grid of %d", l.grid);
+  CUtensorMap tx;
+  if (x_map(&tx, p, pp.nb) != 0) return -1;
+  return bits == 4 ? launch_i4(pp, l, tx, stream) : launch_i8(pp, l, tx, stream);
+}
+}  // namespace
+
+int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, uint32_t* vacant_words, size_t vacant_bytes,
+             const int64_t* indptr, int has_prev, int num_experts, int64_t w_expert_bytes,
+             int64_t s_expert_stride, cudaStream_t stream) {
+  const bool grouped = indptr != nullptr;
+  const int64_t per_expert_scales = p.group > 0 ? (int64_t)p.n * p.s_n + (int64_t)(p.k / p.group) * p.s_g : (int64_t)p.n * p.s_n;
+  const bool covered = p.n % 16 == 0 && p.k % kKBlock == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && p.ldx % 8 == 0 &&
+                       (reinterpret_cast<uintptr_t>(p.out) & 15u) == 0 && p.ldo % 8 == 0 && p.s_n < (1ll << 31) &&
+                       p.s_g < (1ll << 31) && per_expert_scales < (1ll << 40);
+  if (!covered) {
+    RB200_CHECK(!grouped, "grouped GEMM needs n %% 16 == 0, k %% 64 == 0 and 16-byte aligned x / out rows (n=%d, k=%d)", p.n, p.k);
+    return 1;
+  }
+  RB200_CHECK(!grouped || (num_experts >= 1 && num_experts <= kMaxExperts), "num_experts=%d outside [1, %d]", num_experts,
+              kMaxExperts);
+  Params pp;
+  memset(&pp, 0, sizeof(pp));
+  pp.g = p;
+  pp.indptr = indptr;
+  pp.has_prev = has_prev;
+  pp.num_experts = num_experts;
+  pp.w_expert_bytes = w_expert_bytes;
+  pp.s_expert_stride = s_expert_stride;
+  pp.s_n = (int)p.s_n;
+  pp.s_g = (int)p.s_g;
+  pp.early = launch_overlap_enabled() ? 1 : 0;
+  pp.wait_limit_ms = wait_limit_ms();
+
+  pp.partial = vacant_words;
+  const int lane_run = bits == 4 ? 16 : 8;
+  int src;
+  if (p.group <= 0 || p.group >= p.k) {
+    src = kChannel;
+  } else {
+    RB200_CHECK(p.group % lane_run == 0 && p.k % p.group == 0, "group_size=%d must divide k=%d and be a multiple of %d", p.group,
+                p.k, lane_run);
+    src = p.group % kKBlock == 0 ? kOne : (p.group == 32 ? kTwo : kAny);
+    const uintptr_t addr = reinterpret_cast<uintptr_t>(p.s) | reinterpret_cast<uintptr_t>(p.z);
+    pp.s_vec = p.s_g == 1 && p.s_n % 2 == 0 && (addr & 3u) == 0 && s_expert_stride % 2 == 0;
+  }
+
+  const int frag = bits == 4 ? 64 : 32;
+  pp.cpt = (p.k / frag + 3) / 4;
+  if (grouped) {
+    // The split of the rows over the experts is known on the device only: the tile is an even share plus
+    // three standard deviations of a uniform routing wide (an expert above it takes a second tile).
+    const double even = (double)p.m / num_experts;
+    int nb = (int)(even + 3.0 * std::sqrt(even)) + 1;
+    if (nb > p.m) nb = p.m;
+    pp.nb = nb > kMaxNb ? kMaxNb : nb;
+    pp.m_tiles = 1;
+  }
+  const bool single = (grouped ? pp.nb : p.m) <= kSmallNb;
+  return single ? run_single(pp, bits, zmode, src, sm_count, vacant_bytes, stream)
+                : run_pair(pp, bits, zmode, src, sm_count, vacant_bytes, stream);
+}
+
+}  // namespace rb200
