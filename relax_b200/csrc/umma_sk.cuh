@@ -223,7 +223,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
       const Item it = get_item(w.item);
       const uint8_t* w_e = p.w + it.e * pp.w_expert_bytes;
       for (int c = w.c0; c < w.c1; ++c) {
-        if (!mbar_wait_parked(&w_empty[ws], ph, p.status)) {
+        if (!mbar_wait_asleep(&w_empty[ws], ph, p.status, kNap)) {
           ok = false;
           break;
         }
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
       const int m0 = get_item(w.item).m0;
       const int kb_end = min(w.c1 * kBlkPerChunk, p.k / kKBlock);
       for (int kb = w.c0 * kBlkPerChunk; kb < kb_end; ++kb) {
-        if (!mbar_wait_parked(&x_empty[xs], ph, p.status)) {
+        if (!mbar_wait_asleep(&x_empty[xs], ph, p.status, kNap)) {
           ok = false;
           break;
         }
@@ -369,7 +369,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
       for (int c = w.c0; c < w.c1; ++c) {
         feed.advance();
         if (c + 1 < w.c1) fetch(c + 1);
-        if (!mbar_wait_parked(&w_full[ws], wph, p.status)) {
+        if (!mbar_wait_asleep(&w_full[ws], wph, p.status, kNap)) {
           ok = false;
           break;
         }
@@ -393,7 +393,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
             if (i > 0 && b >= nblk) break;
             decode_own<BITS, ZMODE>(pp, feed, i, kb, blk, off, zc, regs);
             if (i == 0) {  // the first block is decoded before the slot has to be free
-              ok = mbar_wait_parked(&a_empty[ab], aph, p.status);
+              ok = mbar_wait_asleep(&a_empty[ab], aph, p.status, kNap);
               if (!ok) break;
               tc_fence_after();
             }
@@ -421,7 +421,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
       }
       if (!ok) break;
       // ---------------------------------------------------------- this piece's accumulator
-      if (!mbar_wait_parked(&d_full[db], dph, p.status)) {
+      if (!mbar_wait_asleep(&d_full[db], dph, p.status, kNap)) {
         ok = false;
         break;
       }

@@ -31,7 +31,7 @@ int pair_m_tiles(long long n_tiles, int m, int k_blocks, int pairs) {
   for (int t = least; t <= least + 8; ++t) {
     const int nb = ((m + t - 1) / t + 31) / 32 * 32;
     if (t > least && nb < 64) break;
-    const long long items = n_tiles * t;
+    const long long items = n_tiles * ((m + nb - 1) / nb);
     const double tiles = (double)items / pairs;
     double clk = tiles * k_blocks * (nb * 2 > 320 ? nb * 2 : 320) + (tiles > 1.0 ? tiles : 1.0) * nb / 48.0 * 600.0;
     if (items % pairs) clk += std::ceil((tiles < 1.0 ? 1.0 / tiles : 1.0) / 2.0) * nb / 48.0 * 1600.0;
@@ -51,17 +51,19 @@ int run_pair(Params& pp, int bits, int zmode, int src, int sm_count, size_t vaca
     pp.nb = (p.m + pp.m_tiles - 1) / pp.m_tiles;
   }
   pp.nb = (pp.nb + 31) / 32 * 32;
-  // tensor memory: two accumulators of up to 192 columns or one of 256, then A slots of 32 columns
+  if (!pp.indptr) pp.m_tiles = (p.m + pp.nb - 1) / pp.nb;  // no tile without rows (an MMA of width 0 is illegal)
+  // tensor memory: two accumulators of up to 128 columns or one of 256, then A slots of 64 columns
   pp.tmem_cols = 512;
-  pp.nd = pp.nb <= 192 ? 2 : 1;
+  pp.nd = pp.nb <= 128 ? 2 : 1;
   pp.d_stride = pp.nb <= 128 ? 128 : (pp.nb <= 192 ? 192 : 256);
   pp.a_base = pp.nd * pp.d_stride;
-  pp.na = (pp.tmem_cols - pp.a_base) / 32;
+  pp.na = (pp.tmem_cols - pp.a_base) / 64;
   if (pp.na > kMaxA) pp.na = kMaxA;
   const size_t budget = (size_t)227 * 1024;
   pp.x_stages = kMaxStages;
   pp.w_stages = kMaxStages;
   while (pp.w_stages > 4 && up::smem_bytes(pp.nb, pp.x_stages, pp.w_stages) > budget) --pp.w_stages;
+  while (pp.x_stages > 2 && up::smem_bytes(pp.nb, pp.x_stages, pp.w_stages) > budget) --pp.x_stages;
   up::Launch l;
   memset(&l, 0, sizeof(l));
   l.zmode = zmode;
@@ -73,8 +75,14 @@ int run_pair(Params& pp, int bits, int zmode, int src, int sm_count, size_t vaca
   RB200_CHECK(items < (1ll << 30), "too many tiles (n=%d, m=%d)", p.n, p.m);
   l.most_pairs = items * pp.cpt;
   RB200_CHECK((size_t)sm_count * pp.nb * kTileRows * sizeof(float) <= vacant_bytes, "split-k scratch too small for %d SMs", sm_count);
-  CUtensorMap tx;
-  if (x_map(&tx, p, pp.nb / 2) != 0) return -1;
+  CUtensorMap tx;  // x as [64-k block][row][64 k]
+  {
+    const unsigned long long dims[3] = {64ull, (unsigned long long)p.m, (unsigned long long)(p.k / 64)};
+    const unsigned long long strides[2] = {(unsigned long long)p.ldx * 2ull, 128ull};
+    const unsigned box[3] = {64u, (unsigned)(pp.nb / 2), 2u};
+    if (make_tensor_map(&tx, p.x, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 3, dims, strides, box, CU_TENSOR_MAP_SWIZZLE_128B) != 0)
+      return -1;
+  }
   return bits == 4 ? up::launch_i4(pp, l, tx, stream) : up::launch_i8(pp, l, tx, stream);
 }
 
@@ -85,6 +93,7 @@ int run_single(Params& pp, int bits, int zmode, int src, int sm_count, size_t va
     pp.nb = (p.m + pp.m_tiles - 1) / pp.m_tiles;
   }
   pp.nb = (pp.nb + 15) / 16 * 16;
+  if (!pp.indptr) pp.m_tiles = (p.m + pp.nb - 1) / pp.nb;
   // tensor memory: two accumulators, then A slots
   pp.tmem_cols = 256;
   pp.d_stride = pp.nb <= 32 ? 32 : 64;
