@@ -480,8 +480,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       auto fetch = [&](int c, unsigned before) {
         const int j = own_step(before);
         if (j * kStepBlk >= kBlkPerChunk) return;
-#pragma unroll
-        for (int i = 0; i < kStepBlk; ++i) feed.fetch(pp, i, min(c * kBlkPerChunk + j * kStepBlk + i, k_blocks - 1));
+        feed.fetch_two(pp, c * kBlkPerChunk + j * kStepBlk, k_blocks);
       };
       int ws = 0, ab0 = 0;
       uint32_t wph = 0, aph0 = 1;
@@ -509,19 +508,14 @@ __global__ void __launch_bounds__(kThreads, 1)
             const uint8_t* blk = w_ring + (size_t)ws * kWBytes + bl * (nft * 512) + j * (kStepBlk * kTilesPerBlk * 512);
             const int kb = c * kBlkPerChunk + j * kStepBlk;
             const uint32_t a_taddr = lane_taddr | (tmem + (uint32_t)(pp.a_base + ab * (kStepBlk * 32)));
+            ok = mbar_wait_parked(&a_empty[ab], aph, p.status);
+            if (!ok) break;
+            tc_fence_after();
 #pragma unroll
             for (int i = 0; i < kStepBlk; ++i) {
               if (i > 0 && j * kStepBlk + i >= nblk) break;
-              uint32_t regs[32];
-              decode_own<BITS, ZMODE>(pp, feed, i, kb + i, blk + i * (kTilesPerBlk * 512), off, zc, regs);
-              if (i == 0) {  // the first block is decoded before the slot has to be free
-                ok = mbar_wait_parked(&a_empty[ab], aph, p.status);
-                if (!ok) break;
-                tc_fence_after();
-              }
-              tc_st32(a_taddr + (uint32_t)(i * 32), regs);
+              decode_own<BITS, ZMODE>(pp, feed, i, kb + i, blk + i * (kTilesPerBlk * 512), off, zc, a_taddr + (uint32_t)(i * 32));
             }
-            if (!ok) break;
             tc_wait_st();
             tc_fence_before();
             __syncwarp();

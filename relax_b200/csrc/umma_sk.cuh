@@ -223,7 +223,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
       const Item it = get_item(w.item);
       const uint8_t* w_e = p.w + it.e * pp.w_expert_bytes;
       for (int c = w.c0; c < w.c1; ++c) {
-        if (!mbar_wait_asleep(&w_empty[ws], ph, p.status, kNap)) {
+        if (!mbar_wait_parked(&w_empty[ws], ph, p.status)) {
           ok = false;
           break;
         }
@@ -310,7 +310,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
       const int m0 = get_item(w.item).m0;
       const int kb_end = min(w.c1 * kBlkPerChunk, p.k / kKBlock);
       for (int kb = w.c0 * kBlkPerChunk; kb < kb_end; ++kb) {
-        if (!mbar_wait_asleep(&x_empty[xs], ph, p.status, kNap)) {
+        if (!mbar_wait_parked(&x_empty[xs], ph, p.status)) {
           ok = false;
           break;
         }
@@ -344,8 +344,9 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
     ScaleFeed<BITS, ZMODE, SRC, kOwn> feed;
     feed.init(pp, hi);
     auto fetch = [&](int c) {
-#pragma unroll
-      for (int i = 0; i < kOwn; ++i) feed.fetch(pp, i, min(c * kBlkPerChunk + grp * kOwn + i, k_blocks - 1));
+      const int kb = c * kBlkPerChunk + grp * kOwn;
+      if (kOwn == 2) feed.fetch_two(pp, kb, k_blocks);
+      else feed.fetch(pp, 0, min(kb, k_blocks - 1));
     };
 
     bool ok = true;
@@ -369,7 +370,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
       for (int c = w.c0; c < w.c1; ++c) {
         feed.advance();
         if (c + 1 < w.c1) fetch(c + 1);
-        if (!mbar_wait_asleep(&w_full[ws], wph, p.status, kNap)) {
+        if (!mbar_wait_parked(&w_full[ws], wph, p.status)) {
           ok = false;
           break;
         }
@@ -384,29 +385,21 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
             aph ^= 1u;
           }
           const uint32_t a_taddr = lane_taddr | (tmem + (uint32_t)(pp.a_base + ab * (kOwn * 32)));
+          ok = mbar_wait_parked(&a_empty[ab], aph, p.status);
+          if (!ok) break;
+          tc_fence_after();
 #pragma unroll
           for (int i = 0; i < kOwn; ++i) {
             const int b = first + i;
-            uint32_t regs[32];
-            const uint8_t* blk = blk0 + b * (kTilesPerBlk * 512);
-            const int kb = c * kBlkPerChunk + b;
             if (i > 0 && b >= nblk) break;
-            decode_own<BITS, ZMODE>(pp, feed, i, kb, blk, off, zc, regs);
-            if (i == 0) {  // the first block is decoded before the slot has to be free
-              ok = mbar_wait_asleep(&a_empty[ab], aph, p.status, kNap);
-              if (!ok) break;
-              tc_fence_after();
-            }
-            tc_st32(a_taddr + (uint32_t)(i * 32), regs);
+            decode_own<BITS, ZMODE>(pp, feed, i, c * kBlkPerChunk + b, blk0 + b * (kTilesPerBlk * 512), off, zc,
+                                    a_taddr + (uint32_t)(i * 32));
           }
-          if (ok) {
-            tc_wait_st();
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&a_full[ab]);
-          }
+          tc_wait_st();
+          tc_fence_before();
+          __syncwarp();
+          if (lane == 0) mbar_arrive(&a_full[ab]);
         }
-        if (!ok) break;
         __syncwarp();
         if (lane == 0) mbar_arrive(&w_empty[ws]);
         if (++ws == w_stages) {
@@ -421,7 +414,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
       }
       if (!ok) break;
       // ---------------------------------------------------------- this piece's accumulator
-      if (!mbar_wait_asleep(&d_full[db], dph, p.status, kNap)) {
+      if (!mbar_wait_parked(&d_full[db], dph, p.status)) {
         ok = false;
         break;
       }

@@ -4,6 +4,7 @@
 #include "umma_sk.cuh"
 
 #include <cmath>
+#include <cstdlib>
 #include <cstring>
 
 #include "tensormap.h"
@@ -121,6 +122,9 @@ int run_single(Params& pp, int bits, int zmode, int src, int sm_count, size_t va
   // a tile cut into many short ranges spends its time in the hand-over: at least three chunks per CTA
   // before a second CTA per SM
   if (units < 3 * grid) grid = sm_count;
+  if (getenv("US_S")) grid = n_tiles * pp.m_tiles * atoi(getenv("US_S"));
+  if (getenv("US_G")) grid = atoi(getenv("US_G"));
+  if (grid > 2 * sm_count) grid = 2 * sm_count;
   if (grid > units) grid = units;
   RB200_CHECK(units * grid < (1ll << 31), "problem too large for the 32-bit work split (n=%d, k=%d, m=%d)", p.n, p.k, p.m);
   l.grid = (int)grid;
@@ -168,7 +172,11 @@ int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, uint32_t* v
                 p.k, lane_run);
     src = p.group % kKBlock == 0 ? kOne : (p.group == 32 ? kTwo : kAny);
     const uintptr_t addr = reinterpret_cast<uintptr_t>(p.s) | reinterpret_cast<uintptr_t>(p.z);
-    pp.s_vec = p.s_g == 1 && p.s_n % 2 == 0 && (addr & 3u) == 0 && s_expert_stride % 2 == 0;
+    auto words_of = [&](int halves) {
+      return p.s_g == 1 && p.s_n % halves == 0 && (addr & (uintptr_t)(2 * halves - 1)) == 0 && s_expert_stride % halves == 0;
+    };
+    // (a k of an odd number of 64-k blocks would read past its row: word by word)
+    pp.s_vec = words_of(4) && p.k % 128 == 0 ? 2 : (words_of(2) ? 1 : 0);
   }
 
   const int frag = bits == 4 ? 64 : 32;

@@ -38,7 +38,8 @@ struct Params {
   int x_stages, w_stages;
   int nd, d_stride, a_base, na, tmem_cols;  // accumulators and A slots in tensor memory
   int s_n, s_g;                // scale strides in elements
-  int s_vec;                   // kTwo: the two groups of a block are one aligned 32-bit word
+  int s_vec;                   // kTwo: the two groups of a block are one aligned 32-bit word (1), those of two
+                               // adjacent blocks one 64-bit word (2)
   int early;                   // weights / scales were not written by the previous kernel
   const int64_t* indptr;       // grouped form: end rows (device), else nullptr
   int has_prev, num_experts;
@@ -54,7 +55,7 @@ using ug::make_b_desc;
 using ug::tc_fence_after;
 using ug::tc_fence_before;
 using ug::tc_ld16;
-using ug::tc_st32;
+using ug::tc_st8;
 using ug::tc_wait_st;
 
 struct Tables {
@@ -119,12 +120,14 @@ __device__ __forceinline__ bool add_parts(float (&v)[16], uint4* part, int secon
   return true;
 }
 
-// One 64-k block of this thread's weight row -> 32 packed fp16 pairs in k order.  `blk`: this thread's
-// row block inside the stage, `off`: its unit offsets, HI: rows g + 8 of the 16-row block.
-// s / z: f16x2 scale and zero point of (tile, lane run): index ti * 4 + t for int8, t for int4.
+// One 64-k block of this thread's weight row -> 32 columns of tensor memory at `taddr`, packed fp16 pairs
+// in k order.  `blk`: this thread's row block inside the stage, `off`: its unit offsets, HI: rows g + 8 of
+// the 16-row block.  s / z: f16x2 scale and zero point of (tile, lane run): index ti * 4 + t for int8, t
+// for int4.  Stored eight columns at a time while the next eight are decoded: a store holds on to its
+// registers for 150 to 340 clocks, which one store of all 32 per block exposed in full.
 template <int BITS, int ZMODE, int HI, class SFn, class ZFn>
 __device__ __forceinline__ void decode_block(const uint8_t* blk, const uint32_t (&off)[4], const ZeroConsts& zc, SFn s_of, ZFn z_of,
-                                             uint32_t (&regs)[32]) {
+                                             uint32_t taddr) {
   if constexpr (BITS == 4) {
     constexpr uint32_t kMagic = 0x64006400u, kSixteenth = 0x2C002C00u;
     constexpr uint32_t kMask = HI ? 0x00f000f0u : 0x000f000fu;
@@ -133,6 +136,7 @@ __device__ __forceinline__ void decode_block(const uint8_t* blk, const uint32_t 
       const uint4 u = *reinterpret_cast<const uint4*>(blk + off[t]);
       const uint32_t s2 = s_of(t), z2 = z_of(t);
       const uint32_t ww[4] = {u.x, u.y, u.z, u.w};
+      uint32_t regs[8];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
         uint32_t e0 = and_or(ww[j], kMask, kMagic), e1 = and_or(ww[j] >> 8, kMask, kMagic);
@@ -147,29 +151,35 @@ __device__ __forceinline__ void decode_block(const uint8_t* blk, const uint32_t 
           e0 = h2_sub(e0, z2);
           e1 = h2_sub(e1, z2);
         }
-        regs[8 * t + 2 * j] = h2_mul(e0, s2);
-        regs[8 * t + 2 * j + 1] = h2_mul(e1, s2);
+        regs[2 * j] = h2_mul(e0, s2);
+        regs[2 * j + 1] = h2_mul(e1, s2);
       }
+      tc_st8(taddr + (uint32_t)(8 * t), regs);
     }
   } else {
     constexpr uint32_t kMagicBytes = 0x64646464u;
 #pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int ti = i >> 2, t = i & 3;
-      const uint4 u = *reinterpret_cast<const uint4*>(blk + ti * 512 + off[t]);
-      const uint32_t s2 = s_of(i), z2 = z_of(i);
-      const uint32_t ww[2] = {HI ? u.y : u.x, HI ? u.w : u.z};
+    for (int h = 0; h < 4; ++h) {
+      uint32_t regs[8];
 #pragma unroll
-      for (int j = 0; j < 2; ++j) {
-        uint32_t e0 = h2_sub(prmt(ww[j], kMagicBytes, 0x4140u), ZMODE == kZeroExact ? z2 : zc.sub_lo);
-        uint32_t e1 = h2_sub(prmt(ww[j], kMagicBytes, 0x4342u), ZMODE == kZeroExact ? z2 : zc.sub_lo);
-        if (ZMODE == kZeroGeneral) {
-          e0 = h2_sub(e0, z2);
-          e1 = h2_sub(e1, z2);
+      for (int o = 0; o < 2; ++o) {
+        const int i = 2 * h + o, ti = i >> 2, t = i & 3;
+        const uint4 u = *reinterpret_cast<const uint4*>(blk + ti * 512 + off[t]);
+        const uint32_t s2 = s_of(i), z2 = z_of(i);
+        const uint32_t ww[2] = {HI ? u.y : u.x, HI ? u.w : u.z};
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          uint32_t e0 = h2_sub(prmt(ww[j], kMagicBytes, 0x4140u), ZMODE == kZeroExact ? z2 : zc.sub_lo);
+          uint32_t e1 = h2_sub(prmt(ww[j], kMagicBytes, 0x4342u), ZMODE == kZeroExact ? z2 : zc.sub_lo);
+          if (ZMODE == kZeroGeneral) {
+            e0 = h2_sub(e0, z2);
+            e1 = h2_sub(e1, z2);
+          }
+          regs[4 * o + 2 * j] = h2_mul(e0, s2);
+          regs[4 * o + 2 * j + 1] = h2_mul(e1, s2);
         }
-        regs[16 * ti + 4 * t + 2 * j] = h2_mul(e0, s2);
-        regs[16 * ti + 4 * t + 2 * j + 1] = h2_mul(e1, s2);
       }
+      tc_st8(taddr + (uint32_t)(8 * h), regs);
     }
   }
 }
@@ -177,17 +187,17 @@ __device__ __forceinline__ void decode_block(const uint8_t* blk, const uint32_t 
 // The same with the scales and zero points of `feed`'s own block i (64-k block kb).
 template <int BITS, int ZMODE, class Feed>
 __device__ __forceinline__ void decode_own(const Params& pp, const Feed& feed, int i, int kb, const uint8_t* blk,
-                                           const uint32_t (&off)[4], const ZeroConsts& zc, uint32_t (&regs)[32]) {
+                                           const uint32_t (&off)[4], const ZeroConsts& zc, uint32_t taddr) {
   auto s_of = [&](int t) { return feed.scale(pp, i, kb, t); };
   if (ZMODE == kZeroGeneral && !feed.block_exact(i)) {
     auto z_of = [&](int t) { return feed.zero(pp, i, kb, t); };
-    if (feed.hi) decode_block<BITS, ZMODE, 1>(blk, off, zc, s_of, z_of, regs);
-    else decode_block<BITS, ZMODE, 0>(blk, off, zc, s_of, z_of, regs);
+    if (feed.hi) decode_block<BITS, ZMODE, 1>(blk, off, zc, s_of, z_of, taddr);
+    else decode_block<BITS, ZMODE, 0>(blk, off, zc, s_of, z_of, taddr);
   } else {
     constexpr int kMode = ZMODE == kZeroGeneral ? kZeroExact : ZMODE;
     auto z_of = [&](int t) { return ZMODE == kZeroGeneral ? feed.zero_exact(i, t) : 0u; };
-    if (feed.hi) decode_block<BITS, kMode, 1>(blk, off, zc, s_of, z_of, regs);
-    else decode_block<BITS, kMode, 0>(blk, off, zc, s_of, z_of, regs);
+    if (feed.hi) decode_block<BITS, kMode, 1>(blk, off, zc, s_of, z_of, taddr);
+    else decode_block<BITS, kMode, 0>(blk, off, zc, s_of, z_of, taddr);
   }
 }
 
@@ -242,6 +252,23 @@ struct ScaleFeed {
       sn[i] = ld_nc_u16(sp + o) | (ld_nc_u16(sp + o + pp.s_g) << 16);
       if (has_zeros) zn[i] = ld_nc_u16(zp + o) | (ld_nc_u16(zp + o + pp.s_g) << 16);
     }
+  }
+  // own blocks 0, 1 of the next chunk are the adjacent 64-k blocks kb, kb + 1 (kb even): their four group-32
+  // scales are one 8-byte load when the rows allow it
+  __device__ __forceinline__ void fetch_two(const Params& pp, int kb, int k_blocks) {
+    if (SRC == kTwo && pp.s_vec == 2) {
+      const uint2 s = __ldg(reinterpret_cast<const uint2*>(sp + kb * 2));
+      sn[0] = s.x;
+      sn[OWN - 1] = s.y;
+      if (has_zeros) {
+        const uint2 z = __ldg(reinterpret_cast<const uint2*>(zp + kb * 2));
+        zn[0] = z.x;
+        zn[OWN - 1] = z.y;
+      }
+      return;
+    }
+#pragma unroll
+    for (int i = 0; i < OWN; ++i) fetch(pp, i, min(kb + i, k_blocks - 1));
   }
   __device__ __forceinline__ void advance() {
 #pragma unroll
