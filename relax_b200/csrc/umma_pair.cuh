@@ -441,7 +441,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         const unsigned hi_u = (unsigned)w.item * (unsigned)cpt + (unsigned)cpt - 1u;
         last = 2 * (int)((((unsigned long long)hi_u + 1u) * takers - 1u) / total) + (int)rank;
       }
-      return drain_store(pp, dt, me, last, 2, e_stage + grp * kStageBytes, parity, group_sync);
+      return drain_store<true>(pp, dt, me, last, 2, e_stage + grp * kStageBytes, parity, group_sync);
     };
 
     int db = 0;

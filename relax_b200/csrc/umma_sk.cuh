@@ -435,7 +435,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
           const unsigned hi_u = (unsigned)w.item * (unsigned)cpt + (unsigned)cpt - 1u;
           last = (int)(((hi_u + 1u) * ctas - 1u) / total);
         }
-        ok = drain_store(pp, dt, me, last, 1, e_stage + grp * kStageBytes, step, group_sync);
+        ok = drain_store<false>(pp, dt, me, last, 1, e_stage + grp * kStageBytes, step, group_sync);
         if (!ok) break;
       }
       tc_fence_before();

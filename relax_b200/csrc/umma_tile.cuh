@@ -80,8 +80,10 @@ __device__ __forceinline__ bool arrived(const uint4& v) {
 }
 // v += the 16 columns of one contributor and, when `second` is not zero, of the one `second` words of
 // 16 bytes further on, in that order; leaves the words vacant.  False when the wait ran out.
+template <bool TWO>
 __device__ __forceinline__ bool add_parts(float (&v)[16], uint4* part, int second, unsigned limit_ms, int* status) {
   uint4 a[4], b[4];
+  if (!TWO) second = 0;
   unsigned long long t0 = 0ull;
   for (;;) {
     bool all = true;
@@ -335,8 +337,8 @@ __device__ __forceinline__ void drain_publish(const Params& pp, const DrainTile&
 }
 
 // epilogue and store; parts of slots me + slot_step, me + 2 slot_step, ... last are added first (fixed
-// order).  `sync`: barrier of the group, false when its wait ran out.
-template <class Sync>
+// order; TWO: two at a time, for 16 registers more).  `sync`: barrier of the group, false when its wait ran out.
+template <bool TWO, class Sync>
 __device__ __forceinline__ bool drain_store(const Params& pp, const DrainTile& t, int me, int last, int slot_step, uint8_t* stage,
                                             unsigned& parity, Sync sync) {
   const GemvParams& p = pp.g;
@@ -345,8 +347,8 @@ __device__ __forceinline__ bool drain_store(const Params& pp, const DrainTile& t
     float v[16];
     tc_ld16(t.d + (uint32_t)c0, v);
     bool ok = true;
-    for (int c = me + slot_step; c <= last && ok; c += 2 * slot_step)
-      ok = add_parts(v, reinterpret_cast<uint4*>(pp.partial) + ((size_t)c * (pp.nb / 4) + c0 / 4) * kTileRows + t.gj,
+    for (int c = me + slot_step; c <= last && ok; c += (TWO ? 2 : 1) * slot_step)
+      ok = add_parts<TWO>(v, reinterpret_cast<uint4*>(pp.partial) + ((size_t)c * (pp.nb / 4) + c0 / 4) * kTileRows + t.gj,
                      c + slot_step <= last ? slot_step * (pp.nb / 4) * kTileRows : 0, pp.wait_limit_ms, p.status);
     if (!__all_sync(0xffffffffu, ok)) return false;
     const int mrow0 = t.m0 + c0;
