@@ -197,6 +197,22 @@ __device__ __forceinline__ void decode_int8_pair(uint32_t w_g, uint32_t w_g8, co
   a[3] = h2_mul(h23, s_g8);
 }
 
+// The same fragments with the bare codes as fp16 subnormals, u * 2^-24 (rows g + 8 of int4: u * 2^-20):
+// a masked code is that number already, exactly, and the tensor cores take subnormals at full rate.
+__device__ __forceinline__ void codes_int4_word(uint32_t w, uint32_t (&a)[4]) {
+  const uint32_t w2 = w >> 8;
+  a[0] = w & 0x000f000fu;
+  a[1] = w & 0x00f000f0u;
+  a[2] = w2 & 0x000f000fu;
+  a[3] = w2 & 0x00f000f0u;
+}
+__device__ __forceinline__ void codes_int8_pair(uint32_t w_g, uint32_t w_g8, uint32_t (&a)[4]) {
+  a[0] = prmt(w_g, 0u, 0x4140u);
+  a[1] = prmt(w_g8, 0u, 0x4140u);
+  a[2] = prmt(w_g, 0u, 0x4342u);
+  a[3] = prmt(w_g8, 0u, 0x4342u);
+}
+
 // ---------------------------------------------------------------- epilogue
 constexpr int kActSwiglu = 4;  // fused gated MLP: out = silu(gate) * up, see RB200_ACT_SWIGLU
 __device__ __forceinline__ float silu_mul(float gate, float up) { return gate / (1.0f + __expf(-gate)) * up; }

@@ -3,7 +3,8 @@
 //   out[m, n] = epilogue(sum_k x[m, k] * wq[n, k]),  m <= 8 or 16 (one or two m16n8k16 MMAs wide)
 //
 // Bound: HBM (the packed weight once) and, close behind, instruction issue: the exact two-rounding
-// decode is 52 of the 61 instructions a 512-byte tile needs (4 MMAs, 3 loads, 2 scale selects).
+// decode is 52 of the 61 instructions a 512-byte tile needs (4 MMAs, 3 loads, 2 scale selects), 20
+// where the codes go into the MMA undecoded.
 // So nothing else is in the loop: no shared memory, no barriers, no copies through the async
 // engine.  A warp reads fragment tiles with 128-bit loads that are whole 512-byte lines in the
 // fragment layout, straight into the registers the MMA takes them from, one chunk (four tiles)
@@ -46,7 +47,19 @@ enum ScaleSrc : int {
   kRow32 = 1,    // int4, group 32, [N, K/32]: the eight groups of a chunk are one 16-byte load
   kHalf = 2,     // groups of whole chunk halves (two tiles), any strides: one 16-bit load per row and half
   kGeneral = 3,  // any strides and group size: one 16-bit load per row and tile
+  kTile = 4,     // as kGeneral, groups of whole tiles
 };
+
+// Where the codes go into the MMA as they are and zero point and scale are applied to its fp32 sums
+// (kFold below), which also rounds less: a group has to be whole tiles, since an MMA's sum runs over a
+// quarter of a tile.  It costs an MMA per code word and m-tile for the activations' sums, shared by the
+// row blocks of a pass: 8 clocks of the sub-partition's MMA pipe against 16 of decoding.  Measured at
+// k 4096 x n 11008 int4, four rows: group 128 with zero points 12.9 -> 10.6 us, without 10.7 -> 10.2,
+// group 64 12.0 -> 11.6, channel 8.8 -> 8.0.  With two m-tiles the MMAs are the bound and the decode
+// stays (16 rows: group 128 12.8 us against 14.6, channel 10.7 against 12.4; int8 even).  Two groups in a
+// tile, four batch rows of one group beside the same rows of the other in the MMA's eight columns, was
+// no faster than the decode for group 32 (k 4096 x n 12288 9.1 against 8.9, k 11008 x n 4096 8.6 against 8.0).
+constexpr bool folds(int src, int m_tiles) { return src != kRow32 && src != kGeneral && m_tiles == 1; }
 
 struct Params {
   GemvParams g;
@@ -98,6 +111,8 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   constexpr int kLaneK = kFrag / 4;
   constexpr int kXV = BITS == 4 ? 2 : 1;  // 16-byte pieces of x per lane and tile
   constexpr bool kZ = ZMODE == kZeroGeneral;
+  constexpr bool kFold = folds(SRC, MT);
+  constexpr bool kFoldAll = kFold && SRC == kChannel;  // the sums run over all of k
   __shared__ __align__(16) float4 red[2][kWarps][kRows * MT][32];
   __shared__ int s_entries, s_m_lo[kMaxEntries], s_m_n[kMaxEntries], s_expert[kMaxEntries];
   const GemvParams& p = pp.g;
@@ -158,6 +173,13 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   const uint32_t half_sel = (t >> 1) ? 0x3232u : 0x1010u;
   const int unit16 = frag_unit_pos(lane) * 16;
   const bool has_zeros = kZ && p.z != nullptr;
+  // kFold: A operand of the products that sum the activations, in the codes' units: the zero point,
+  // negated, or one
+  constexpr float kUnitLo = 1.0f / (1 << 24), kUnitHi = BITS == 4 ? 16.0f * kUnitLo : kUnitLo;
+  const float z_unit = kZ ? 1.0f : -p.zero_const;
+  const uint32_t one_lo = h2_bcast(__float2half_rn(z_unit * kUnitLo)), one_hi = h2_bcast(__float2half_rn(z_unit * kUnitHi));
+  const float zconst = __half2float(__float2half_rn(p.zero_const));
+  const uint32_t ones[4] = {one_lo, one_hi, one_lo, one_hi};
 
   // this warp's whole chunks (four fragment tiles); the tiles of a short last chunk go to the last warp
   const int full_chunks = KB / 4;
@@ -205,7 +227,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
           sv[S][r][i] = ld_nc_v2(sp[r][i] + S * 4);
           if (has_zeros) zv[S][r][i] = ld_nc_v2(zp[r][i] + S * 4);
         }
-      } else if (SRC == kHalf || SRC == kGeneral) {
+      } else if (SRC == kHalf || SRC == kGeneral || SRC == kTile) {
 #pragma unroll
         for (int j = 0; j < (SRC == kHalf ? 1 : 2); ++j) {
           const unsigned k = (unsigned)((c * 4 + S * 2 + j) * kFrag + t * kLaneK);
@@ -286,16 +308,16 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 
   int buf = 0;
   for (;;) {
-    constexpr int kChains = MT == 1 ? 2 : 1;  // independent MMA chains (two m-tiles are two already)
-    float acc[kRows][MT][kChains][4];
+    constexpr int kChains = MT == 1 && (!kFold || kFoldAll) ? 2 : 1;  // independent MMA chains (two m-tiles are two already)
+    float acc[kRows][kChains][MT][4];
 #pragma unroll
     for (int r = 0; r < kRows; ++r)
 #pragma unroll
-      for (int mt = 0; mt < MT; ++mt)
+      for (int i = 0; i < kChains; ++i)
 #pragma unroll
-        for (int i = 0; i < kChains; ++i)
+        for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-          for (int c = 0; c < 4; ++c) acc[r][mt][i][c] = 0.0f;
+          for (int c = 0; c < 4; ++c) acc[r][i][mt][c] = 0.0f;
     // lanes of absent batch rows fetch row 0: their columns of the result are never stored
     const __half* x0 = p.x + (q.m_lo + (g < q.m_n ? g : 0)) * (unsigned)p.ldx + t * kLaneK;
     const unsigned x_next = MT > 1 && g + 8 < q.m_n ? 8u * (unsigned)p.ldx : 0u;  // elements to the second m-tile's row
@@ -311,10 +333,49 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt) {
           const uint4& x = xv[mt][j >> 1];
-          mma_16816(acc[r][mt][j % kChains], a, (j & 1) ? x.z : x.x, (j & 1) ? x.w : x.y);
+          mma_16816(acc[r][j % kChains][mt], a, (j & 1) ? x.z : x.x, (j & 1) ? x.w : x.y);
         }
       }
     };
+    // kFold: sum (u - z) x = sum u x - z sum x; `sums` gets the second sum, times `ones`
+    float sums[MT][4];
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int c = 0; c < 4; ++c) sums[mt][c] = 0.0f;
+    // (the chains of a step are independent of each other and issued in turn)
+    auto sum_step = [&](float (&d)[MT][4], const uint4 (&xv)[MT][kXV], int j, bool first) {
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        const uint4& x = xv[mt][j >> 1];
+        if (first && j == 0) mma_16816_first(d[mt], ones, x.x, x.y);
+        else mma_16816(d[mt], ones, (j & 1) ? x.z : x.x, (j & 1) ? x.w : x.y);
+      }
+    };
+    auto code_step = [&](float (&d)[MT][4], const uint4& wv, const uint4 (&xv)[MT][kXV], int j, bool first) {
+      const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+      uint32_t a[4];
+      if (BITS == 4) codes_int4_word(ww[j], a);
+      else codes_int8_pair(ww[2 * (j & 1)], ww[2 * (j & 1) + 1], a);
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        const uint4& x = xv[mt][j >> 1];
+        if (first && j == 0) mma_16816_first(d[mt], a, x.x, x.y);
+        else mma_16816(d[mt], a, (j & 1) ? x.z : x.x, (j & 1) ? x.w : x.y);
+      }
+    };
+    // acc += s * (d + sums), or s * (d - z * sums)
+    auto add_scaled = [&](int r, const float (&d)[MT][4], const float (&xs)[MT][4], float s_g, float s_g8, float z_g,
+                          float z_g8) {
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float v = kZ ? d[mt][c] - (c < 2 ? z_g : z_g8) * xs[mt][c] : d[mt][c] + xs[mt][c];
+          acc[r][0][mt][c] += (c < 2 ? s_g : s_g8) * v;
+        }
+    };
+    auto half_of = [](uint32_t v, int hi) { return __half2float(__ushort_as_half((unsigned short)(hi ? v >> 16 : v & 0xffffu))); };
     const __half* xp = x0 + c0 * (kFrag * 4);
     // activations of either half: int8 fetches them half a chunk ahead, int4 has no registers to spare
     // for that and fetches them where they are used
@@ -330,6 +391,45 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
     };
     auto half_step = [&](auto set_tag, auto rn_tag, const XHalf<kXV, MT>& xv) {
       constexpr int S = decltype(set_tag)::value, RN = decltype(rn_tag)::value;
+      if constexpr (kFoldAll) {
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+#pragma unroll
+          for (int i = 0; i < 2 * kXV; ++i) {
+            sum_step(sums, xv.v[j], i, false);
+#pragma unroll
+            for (int r = 0; r < RN; ++r) code_step(acc[r][i % kChains], w[S][r][j], xv.v[j], i, false);
+          }
+        }
+        return;
+      } else if constexpr (kFold) {
+        constexpr int kSpan = SRC == kHalf ? 2 : 1;  // tiles of a group (as far as the half goes)
+        float d[RN][MT][4];
+#pragma unroll
+        for (int j = 0; j < 2; ++j) {
+          const bool first = j % kSpan == 0;
+#pragma unroll
+          for (int i = 0; i < 2 * kXV; ++i) {
+            sum_step(sums, xv.v[j], i, first);
+#pragma unroll
+            for (int r = 0; r < RN; ++r) code_step(d[r], w[S][r][j], xv.v[j], i, first);
+          }
+          if ((j + 1) % kSpan != 0) continue;
+#pragma unroll
+          for (int r = 0; r < RN; ++r) {
+            float s_g, s_g8, z_g = zconst, z_g8 = zconst;
+            const int at = SRC == kHalf ? 0 : j;
+            s_g = half_of(sg[S][r][at], 0);
+            s_g8 = half_of(sg[S][r][at], 1);
+            if (has_zeros) {
+              z_g = half_of(zg[S][r][at], 0);
+              z_g8 = half_of(zg[S][r][at], 1);
+            }
+            add_scaled(r, d[r], sums, s_g, s_g8, z_g, z_g8);
+          }
+        }
+        return;
+      }
 #pragma unroll
       for (int j = 0; j < 2; ++j)
 #pragma unroll
@@ -407,17 +507,32 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 #pragma unroll
           for (int i = 0; i < kXV; ++i) xt[mt][i] = ld_nc_v4(x0 + mt * x_next + kb * kFrag + i * 8);
         const unsigned k = (unsigned)(kb * kFrag + t * kLaneK);
+        if (kFold)
+#pragma unroll
+          for (int i = 0; i < 2 * kXV; ++i) sum_step(sums, xt, i, !kFoldAll);
         const unsigned grp = SRC == kChannel ? 0u : (pp.group_shift >= 0 ? k >> pp.group_shift : k / (unsigned)p.group);
 #pragma unroll
         for (int r = 0; r < kRows; ++r) {
           if (r >= q.rn) break;
           const uint4 wt = ld_stream_v4(p.w + (grouped ? q.e * pp.w_expert_bytes : 0) +
                                         frag_tile_offset(q.nb0 + r, kb, NB, KB) + unit16);
+          if (kFoldAll) {
+#pragma unroll
+            for (int i = 0; i < 2 * kXV; ++i) code_step(acc[r][i % kChains], wt, xt, i, false);
+            continue;
+          }
           const int64_t o = (grouped ? q.e * pp.s_expert_stride : 0) + ((q.nb0 + r) * 16 + g) * pp.s_n +
                             grp * (unsigned)pp.s_g;
           const uint32_t a = ld_nc_u16(p.s + o), b = ld_nc_u16(p.s + o + row8);
           const uint32_t za = has_zeros ? ld_nc_u16(p.z + o) * 0x10001u : zconst_h2;
           const uint32_t zb = has_zeros ? ld_nc_u16(p.z + o + row8) * 0x10001u : zconst_h2;
+          if (kFold) {
+            float d[MT][4];
+#pragma unroll
+            for (int i = 0; i < 2 * kXV; ++i) code_step(d, wt, xt, i, true);
+            add_scaled(r, d, sums, half_of(a, 0), half_of(b, 0), half_of(za, 0), half_of(zb, 0));
+            continue;
+          }
           mma_tile(r, wt, a * 0x10001u, b * 0x10001u, za, zb, xt);
         }
       }
@@ -425,6 +540,12 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 
     // the next pass's first loads leave before this one's sums are put together
     const Pass done = q;
+    uint32_t done_s[kRows], done_z[kRows];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      done_s[r] = kFoldAll ? ch_s[r] : 0u;
+      done_z[r] = kFoldAll && has_zeros ? ch_z[r] : 0u;
+    }
     pos += (unsigned)q.rn;
     if (more) {
       if constexpr (kLead) q = q_next;
@@ -439,7 +560,13 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
       for (int mt = 0; mt < MT; ++mt) {
         float f[4];
 #pragma unroll
-        for (int c = 0; c < 4; ++c) f[c] = acc[r][mt][0][c] + (kChains == 2 ? acc[r][mt][kChains - 1][c] : 0.0f);
+        for (int c = 0; c < 4; ++c) {
+          f[c] = acc[r][0][mt][c] + (kChains == 2 ? acc[r][kChains - 1][mt][c] : 0.0f);
+          if (kFoldAll) {
+            const float z = has_zeros ? half_of(done_z[r], c >> 1) : zconst;
+            f[c] = half_of(done_s[r], c >> 1) * (kZ ? f[c] - z * sums[mt][c] : f[c] + sums[mt][c]);
+          }
+        }
         red[buf][warp][r * MT + mt][lane] = make_float4(f[0], f[1], f[2], f[3]);
       }
     __syncthreads();
@@ -452,6 +579,12 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
         v[1] += f.y;
         v[2] += f.z;
         v[3] += f.w;
+      }
+      if (kFold) {  // the codes' units
+        v[0] *= 1.0f / kUnitLo;
+        v[1] *= 1.0f / kUnitLo;
+        v[2] *= 1.0f / kUnitHi;
+        v[3] *= 1.0f / kUnitHi;
       }
       const int nb = done.nb0 + warp / MT, m8 = (warp % MT) * 8 + t * 2;
       if (p.epi.act == kActSwiglu) {
@@ -505,22 +638,26 @@ int launch_inst(const Params& pp, int warps, int grid, cudaStream_t stream) {
   return 0;
 }
 
+template <int BITS, int SRC>
+int launch_src(const Params& pp, int zmode, int warps, int grid, cudaStream_t stream) {
+  return zmode == kZeroGeneral ? launch_inst<BITS, kZeroGeneral, SRC>(pp, warps, grid, stream)
+                               : launch_inst<BITS, kZeroConstInt, SRC>(pp, warps, grid, stream);
+}
+
 template <int BITS>
 int launch_bits(const Params& pp, int zmode, int src, int warps, int grid, cudaStream_t stream) {
-  const bool general = zmode == kZeroGeneral;
-  if (src == kChannel)
-    return general ? launch_inst<BITS, kZeroGeneral, kChannel>(pp, warps, grid, stream)
-                   : launch_inst<BITS, kZeroConstInt, kChannel>(pp, warps, grid, stream);
-  if (src == kHalf)
-    return general ? launch_inst<BITS, kZeroGeneral, kHalf>(pp, warps, grid, stream)
-                   : launch_inst<BITS, kZeroConstInt, kHalf>(pp, warps, grid, stream);
-  if constexpr (BITS == 4) {
-    if (src == kRow32)
-      return general ? launch_inst<BITS, kZeroGeneral, kRow32>(pp, warps, grid, stream)
-                     : launch_inst<BITS, kZeroConstInt, kRow32>(pp, warps, grid, stream);
+  switch (src) {
+    case kChannel:
+      return launch_src<BITS, kChannel>(pp, zmode, warps, grid, stream);
+    case kHalf:
+      return launch_src<BITS, kHalf>(pp, zmode, warps, grid, stream);
+    case kTile:
+      return launch_src<BITS, kTile>(pp, zmode, warps, grid, stream);
   }
-  return general ? launch_inst<BITS, kZeroGeneral, kGeneral>(pp, warps, grid, stream)
-                 : launch_inst<BITS, kZeroConstInt, kGeneral>(pp, warps, grid, stream);
+  if constexpr (BITS == 4) {
+    if (src == kRow32) return launch_src<BITS, kRow32>(pp, zmode, warps, grid, stream);
+  }
+  return launch_src<BITS, kGeneral>(pp, zmode, warps, grid, stream);
 }
 
 #endif  // __CUDACC__

@@ -1,4 +1,4 @@
-"""The small-batch decode kernel (m <= 8, and expert layers of at most 32 rows) where its split can go
+"""The small-batch decode kernel (m <= 16, and expert layers of at most 32 rows) where its split can go
 wrong: k slices without a chunk, short last chunks and row tiles, odd row-block counts, the four-warp
 form of wide weights, scale sources, and experts with more rows than one pass holds."""
 import numpy as np
@@ -12,10 +12,10 @@ from tests.util import assert_close, to_dev, u32_to_dev
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("m", [1, 8])
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
 @pytest.mark.parametrize("k,n,group,asym", [(64, 16, 32, False), (704, 48, 32, True), (2304, 1040, 32, False),
                                             (2304, 400, 128, True), (1920, 144, 96, True), (256, 29056, 32, False),
-                                            (512, 28688, 256, True)])
+                                            (512, 28688, 256, True), (704, 144, 64, True), (960, 48, 192, False)])
 def test_int4_split(oracle, m, k, n, group, asym):
     case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, group, asymmetric=asym)
     pre = ops.preprocess_weight_q4f16(u32_to_dev(case.w))
@@ -26,9 +26,9 @@ def test_int4_split(oracle, m, k, n, group, asym):
     assert_close(out.cpu().numpy(), C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, case.zeros, 7.0, group))))
 
 
+@pytest.mark.parametrize("m", [5, 13])
 @pytest.mark.parametrize("k,n,group", [(32, 16, -1), (288, 80, -1), (1056, 272, 32), (1152, 144, 64), (128, 28704, -1)])
-def test_int8_split(oracle, k, n, group):
-    m = 5
+def test_int8_split(oracle, m, k, n, group):
     rs = np.random.RandomState(k + n)
     x = rs.randn(m, k).astype(np.float16)
     packed = rs.randint(-127, 128, size=(k, n)).astype(np.int8)
