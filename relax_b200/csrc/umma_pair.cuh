@@ -422,14 +422,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       return fine;
     };
     // this group's share of a finished accumulator
-    auto drain = [&](const Walk& w, const Item& it, int db, int share, int shares) -> bool {
+    auto drain = [&](const Walk& w, const Item& it, int db, int share, int shares, uint32_t s_row) -> bool {
       if (!waited) {
         griddep_wait();  // outputs and scratch may be in use by the previous kernel until it has ended
         waited = true;
       }
       if (it.n_tile * kTileRows >= p.n) return true;
       const DrainTile dt = {lane_taddr | (tmem + (uint32_t)(db * pp.d_stride)), share * 16, shares * 16, min(nb, it.m_end - it.m0),
-                            it.n_tile * kTileRows, it.m0, it.m_end, row, gj};
+                            it.n_tile * kTileRows, it.m0, it.m_end, row, gj, folds<ZMODE, SRC>() ? drain_scale<BITS>(s_row, hi) : 1.0f};
       const int me = (int)blockIdx.x;
       if (w.c0 > 0) {
         drain_publish(pp, dt, me);
@@ -441,19 +441,22 @@ __global__ void __launch_bounds__(kThreads, 1)
         const unsigned hi_u = (unsigned)w.item * (unsigned)cpt + (unsigned)cpt - 1u;
         last = 2 * (int)((((unsigned long long)hi_u + 1u) * takers - 1u) / total) + (int)rank;
       }
-      return drain_store<true>(pp, dt, me, last, 2, e_stage + grp * kStageBytes, parity, group_sync);
+      return drain_store<true, folds<ZMODE, SRC>()>(pp, dt, me, last, 2, e_stage + grp * kStageBytes, parity, group_sync);
     };
 
+    ScaleFeed<BITS, ZMODE, SRC, kStepBlk> feed;
+    feed.init(pp, hi);
     int db = 0;
     uint32_t dph = 0;
     Walk w;
     if (grp == 2) {
       for (bool have = begin(w); ok && have; have = next(w)) {
         const Item it = get_item(w.item);
+        feed.row(pp, it.e, it.n_tile * kTileRows + row);
         ok = mbar_wait_parked(&d_full[db], dph, p.status);
         if (!ok) break;
         tc_fence_after();
-        ok = drain(w, it, db, 0, all_drain || is_last(w) ? kDrainGroups : 1);
+        ok = drain(w, it, db, 0, all_drain || is_last(w) ? kDrainGroups : 1, feed.s_row);
         if (!ok) break;
         tc_fence_before();
         __syncwarp();
@@ -468,8 +471,6 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t off[4];
 #pragma unroll
       for (int t = 0; t < 4; ++t) off[t] = (uint32_t)(t * 128 + ((g + 2 * t) & 7) * 16);
-      ScaleFeed<BITS, ZMODE, SRC, kStepBlk> feed;
-      feed.init(pp, hi);
       unsigned q = 0;  // steps before the current chunk
       // the step of a chunk this group decodes, given the steps before it: of two steps one, of a
       // single step every other one
@@ -514,7 +515,7 @@ __global__ void __launch_bounds__(kThreads, 1)
 #pragma unroll
             for (int i = 0; i < kStepBlk; ++i) {
               if (i > 0 && j * kStepBlk + i >= nblk) break;
-              decode_own<BITS, ZMODE>(pp, feed, i, kb + i, blk + i * (kTilesPerBlk * 512), off, zc, a_taddr + (uint32_t)(i * 32));
+              decode_own<BITS, ZMODE, SRC>(pp, feed, i, kb + i, blk + i * (kTilesPerBlk * 512), off, zc, a_taddr + (uint32_t)(i * 32));
             }
             tc_wait_st();
             tc_fence_before();
@@ -540,7 +541,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ok = all_drain ? mbar_wait_parked(&d_full[db], dph, p.status) : mbar_wait_parked(d_last, 0, p.status);
           if (!ok) break;
           tc_fence_after();
-          ok = drain(w, it, db, grp + 1, kDrainGroups);
+          ok = drain(w, it, db, grp + 1, kDrainGroups, feed.s_row);
           if (!ok) break;
           tc_fence_before();
           __syncwarp();

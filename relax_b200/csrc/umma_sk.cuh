@@ -392,7 +392,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
           for (int i = 0; i < kOwn; ++i) {
             const int b = first + i;
             if (i > 0 && b >= nblk) break;
-            decode_own<BITS, ZMODE>(pp, feed, i, c * kBlkPerChunk + b, blk0 + b * (kTilesPerBlk * 512), off, zc,
+            decode_own<BITS, ZMODE, SRC>(pp, feed, i, c * kBlkPerChunk + b, blk0 + b * (kTilesPerBlk * 512), off, zc,
                                     a_taddr + (uint32_t)(i * 32));
           }
           tc_wait_st();
@@ -424,7 +424,8 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
         waited = true;
       }
       const DrainTile dt = {lane_taddr | (tmem + (uint32_t)(db * pp.d_stride)), grp * 16, kGroups * 16, min(nb, it.m_end - it.m0),
-                            it.n_tile * kTileRows, it.m0, it.m_end, row, gj};
+                            it.n_tile * kTileRows, it.m0, it.m_end, row, gj,
+                            folds<ZMODE, SRC>() ? drain_scale<BITS>(feed.s_row, hi) : 1.0f};
       const int me = (int)blockIdx.x;
       if (w.c0 > 0) {
         drain_publish(pp, dt, me);
@@ -435,7 +436,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
           const unsigned hi_u = (unsigned)w.item * (unsigned)cpt + (unsigned)cpt - 1u;
           last = (int)(((hi_u + 1u) * ctas - 1u) / total);
         }
-        ok = drain_store<false>(pp, dt, me, last, 1, e_stage + grp * kStageBytes, step, group_sync);
+        ok = drain_store<false, folds<ZMODE, SRC>()>(pp, dt, me, last, 1, e_stage + grp * kStageBytes, step, group_sync);
         if (!ok) break;
       }
       tc_fence_before();
