@@ -28,6 +28,7 @@ int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const in
     RB200_CHECK(p.group % (frag / 4) == 0 && p.k % p.group == 0,
                 "group_size=%d must divide k=%d and be a multiple of %d", p.group, p.k, frag / 4);
     src = p.group % (2 * frag) == 0 ? kHalf : (p.group % frag == 0 ? kTile : kGeneral);
+    pp.per = p.group / (src == kHalf ? 2 * frag : frag);
     if ((p.group & (p.group - 1)) == 0)
       for (pp.group_shift = 0; (1 << pp.group_shift) < p.group;) ++pp.group_shift;
     const uintptr_t addr = reinterpret_cast<uintptr_t>(p.s) | reinterpret_cast<uintptr_t>(p.z) |

@@ -65,6 +65,7 @@ struct Params {
   GemvParams g;
   int group_shift;         // log2 of the group size, or -1
   unsigned per_cta, extra; // ungrouped: row blocks per CTA, and how many CTAs take one more
+  int per;                 // kHalf / kTile: halves / tiles of a group
   int s_n, s_g;            // scale strides in elements
   int early;               // the host promises that weights were not written by the previous kernel
   const int64_t* indptr;   // grouped form: end rows per expert (device), else nullptr
@@ -216,9 +217,22 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   const uint8_t* wp = nullptr;                 // next chunk to load
   const __half *sp[kRows][2], *zp[kRows][2];   // scales of rows g, g + 8 (kRow32: of the next chunk)
   int stride = 0;                              // bytes from a chunk to the next
+  unsigned s_at = 0u;                          // kHalf, kTile: offset of the next group's scales, and what
+  int s_left = 0;                              // is left of that group
 
   auto load_set = [&](auto set_tag, auto rn_tag, int c) {
     constexpr int S = decltype(set_tag)::value, RN = decltype(rn_tag)::value;
+    unsigned at[2];  // offsets of the groups' scales
+    if (SRC == kHalf || SRC == kTile) {
+#pragma unroll
+      for (int j = 0; j < (SRC == kHalf ? 1 : 2); ++j) {
+        at[j] = s_at;
+        if (--s_left == 0) {
+          s_left = pp.per;
+          s_at += (unsigned)pp.s_g;
+        }
+      }
+    }
 #pragma unroll
     for (int r = 0; r < RN; ++r) {
       w[S][r][0] = ld_stream_v4(wp + r * 2048 + S * 1024);
@@ -232,9 +246,13 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
       } else if (SRC == kHalf || SRC == kGeneral || SRC == kTile) {
 #pragma unroll
         for (int j = 0; j < (SRC == kHalf ? 1 : 2); ++j) {
-          const unsigned k = (unsigned)((c * 4 + S * 2 + j) * kFrag + t * kLaneK);
-          const unsigned grp = pp.group_shift >= 0 ? k >> pp.group_shift : k / (unsigned)p.group;
-          const unsigned o = grp * (unsigned)pp.s_g;
+          unsigned o = 0u;
+          if (SRC != kGeneral) {
+            o = at[j];
+          } else {
+            const unsigned k = (unsigned)((c * 4 + S * 2 + j) * kFrag + t * kLaneK);
+            o = (pp.group_shift >= 0 ? k >> pp.group_shift : k / (unsigned)p.group) * (unsigned)pp.s_g;
+          }
           const uint32_t a = ld_nc_u16(sp[r][0] + o), b = ld_nc_u16(sp[r][1] + o);
           sg[S][r][j][0] = kFold ? a : a | (b << 16);
           sg[S][r][j][1] = b;
@@ -279,6 +297,11 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
         ch_s[r] = ld_nc_u16(sp[r][0]) | (ld_nc_u16(sp[r][1]) << 16);
         if (has_zeros) ch_z[r] = ld_nc_u16(zp[r][0]) | (ld_nc_u16(zp[r][1]) << 16);
       }
+    }
+    if (SRC == kHalf || SRC == kTile) {
+      const unsigned unit = (unsigned)c0 * (SRC == kHalf ? 2u : 4u), grp = unit / (unsigned)pp.per;
+      s_at = grp * (unsigned)pp.s_g;
+      s_left = pp.per - (int)(unit - grp * (unsigned)pp.per);
     }
     if (c0 < c1) {
       if (q.rn == 2) {
