@@ -9,7 +9,7 @@
 #include "dequant.cuh"
 #include "gemv.h"
 #include "gemv_cluster.cuh"
-#include "umma_gemm.cuh"
+#include "umma_gemm.h"
 #include "umma_tile.cuh"
 #include "gemv_rk.cuh"
 #include "gemv_sk.cuh"
@@ -424,11 +424,11 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
     p.k = (int)d->k;
     p.group = group;
     p.zero_const = d->zero_const;
-    // Which decode kernel: up to eight rows (one MMA wide) the small-batch kernel; above that the
-    // stream-k kernel whenever x can be fetched as TMA tiles of whole 64-k blocks (always for int4), and
-    // the cluster kernel - split-k partials meeting in distributed shared memory - for the remaining
-    // int8 shapes (k a multiple of 32 only).  Measured with launch overlap at one row, small-batch
-    // against stream-k: k = n = 4096 3.9 / 8.1 us, n 22016 13.9 / 19.1, k 11008 x n 4096 8.0 / 13.4.
+    // Which kernel: up to 16 rows (two MMAs wide) the small-batch kernel (one row, against the stream-k
+    // kernel: k = n = 4096 3.9 / 8.1 us, n 22016 13.9 / 19.1, k 11008 x n 4096 8.0 / 13.4); above that the
+    // tensor-core kernels.  What they do not cover - the fused all-reduce, x or out without 16-byte rows -
+    // runs on the stream-k kernel, and int8 with k a multiple of 32 only on the cluster kernel, whose
+    // split-k partials meet in distributed shared memory.
     if (p.m <= rk::kMaxBatch && !ar)
       return gemv_rk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
     unsigned* flags = reinterpret_cast<unsigned*>(sc->counters) + kSkFlagOffset;
@@ -635,9 +635,8 @@ int rb200_group_gemm(const rb200_group_gemm_desc* d, void* stream_v) {
     return umma_run(p, d->weight_bits, zmode, sc->sm_count, sc->vacant_words, sc->vacant_bytes, d->indptr,
                        d->indptr_has_prev ? 1 : 0, (int)d->num_experts, w_expert_bytes, d->scale_stride_e,
                        static_cast<cudaStream_t>(stream_v));
-  return umma_group_gemm_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0,
-                             (int)d->num_experts, w_expert_bytes,
-                             packed ? d->scale_stride_e : 0, static_cast<cudaStream_t>(stream_v));
+  return umma_group_gemm_run(p, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0, (int)d->num_experts, w_expert_bytes,
+                             static_cast<cudaStream_t>(stream_v));
 }
 
 int rb200_dequantize(const rb200_gemm_desc* d, void* wq_out, void* stream_v) {

@@ -143,21 +143,6 @@ __device__ __forceinline__ bool mbar_wait_parked(uint64_t* bar, uint32_t parity,
   return false;
 }
 
-// For roles that are ahead of the critical path: sleeps between polls.  The suspend-time hint above does
-// not keep a waiting warp off the issue slots - it was seen to poll every 50 clocks or so, two thirds of
-// all instructions of a tensor-core kernel with a dozen waiting warps, and their energy under the power
-// cap.  Bounded by the number of sleeps, two seconds' worth.
-__device__ __forceinline__ bool mbar_wait_asleep(uint64_t* bar, uint32_t parity, int* status, unsigned ns) {
-  if (mbar_try_wait(bar, parity)) return true;
-#pragma unroll 1
-  for (unsigned left = 2000000000u / ns; left > 0u; --left) {
-    __nanosleep(ns);
-    if (mbar_try_wait(bar, parity)) return true;
-  }
-  if (status) atomicExch(status, kStatusWaitTimeout);
-  return false;
-}
-
 // Same, for roles with slack (producer, MMA issuer): sleeps between polls so the waiting warp
 // does not take issue slots from the warps doing the arithmetic.
 __device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, int* status) {

@@ -1,12 +1,11 @@
-// m > 32: the tcgen05 prefill kernel (256-row batch tiles, weights decoded into tensor memory);
-// shapes it does not cover (n not a multiple of 128, k not a multiple of 64, unaligned x) run as
-// consecutive 32-row batch slices on the decode kernel, each a full pass over the packed weight.
+// m > 32: the tensor-core kernels over packed weights; what they do not cover (int8 with k not a multiple
+// of 64, x or out without 16-byte rows) runs as consecutive 32-row batch slices, each a full pass over the
+// packed weight.
 #include "gemm_tc.h"
 
 #include <cstdlib>
 #include <cstring>
 
-#include "umma_gemm.cuh"
 #include "umma_tile.cuh"
 
 namespace rb200 {

@@ -23,6 +23,7 @@ size_t cluster_stage_bytes(int bits, int mt, int zmode, int src) {
 
 int gemv_cluster_run(const GemvParams& p_in, int bits, int zmode, int sm_count, cudaStream_t stream) {
   using namespace gc;
+  RB200_CHECK(bits == 8 && p_in.m > 16 && p_in.m <= 32, "cluster kernel: int8, 17 to 32 rows (bits=%d, m=%d)", bits, p_in.m);
   const int frag = bits == 4 ? 64 : 32;
   const int chunk = frag * kBlocksPerChunk;
   const int lane_run = frag / 4;
@@ -98,7 +99,6 @@ int gemv_cluster_run(const GemvParams& p_in, int bits, int zmode, int sm_count, 
   l.stage_bytes = cluster_stage_bytes(bits, l.mt, zmode, l.src);
   l.fixed_bytes = (size_t)2 * kConsumerWarps * l.mt * 512;
 
-  if (bits == 4) return launch_cluster_i4(cp, l, ts, tz, stream);
   return launch_cluster_i8(cp, l, ts, tz, stream);
 }
 

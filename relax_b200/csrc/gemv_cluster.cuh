@@ -1,4 +1,5 @@
-// Decode-path kernel, cluster variant (the default for m <= 32).
+// Decode-path kernel, cluster variant: int8 weights, 17 to 32 rows, k a multiple of 32 only (whole 64-k
+// blocks run on the tensor-core kernels).
 //
 // Same streaming structure as gemv.cu - a producer warp fills a ring of shared-memory stages
 // with bulk async copies, eight consumer warps decode 128-bit fragment words in registers and
@@ -497,8 +498,6 @@ struct ClusterLaunch {
 };
 
 // implemented per bit width (two translation units, so they compile in parallel)
-int launch_cluster_i4(const ClusterParams& cp, const ClusterLaunch& l, const CUtensorMap& ts,
-                      const CUtensorMap& tz, cudaStream_t stream);
 int launch_cluster_i8(const ClusterParams& cp, const ClusterLaunch& l, const CUtensorMap& ts,
                       const CUtensorMap& tz, cudaStream_t stream);
 size_t cluster_stage_bytes(int bits, int mt, int zmode, int src);

@@ -98,7 +98,6 @@ int launch_gs(const ClusterParams& cp, const ClusterLaunch& l, const CUtensorMap
   RB200_CASE(128, kSrcGlobal);
   RB200_CASE(0, kSrcGlobal);
   RB200_CASE(-1, kSrcGlobal);
-  if (BITS == 4) RB200_CASE(32, kSrcSmemNK);
   RB200_CASE(32, kSrcSmemKN);
   RB200_CASE(64, kSrcSmemKN);
   RB200_CASE(128, kSrcSmemKN);
@@ -112,11 +111,7 @@ int launch_bits(const ClusterParams& cp, const ClusterLaunch& l, const CUtensorM
                 const CUtensorMap& tz, cudaStream_t stream) {
 #define RB200_MZ(M, Z) \
   if (l.mt == (M) && l.zmode == (Z)) return launch_gs<BITS, M, Z>(cp, l, ts, tz, stream)
-  RB200_MZ(1, kZeroConstInt);
-  RB200_MZ(2, kZeroConstInt);
   RB200_MZ(4, kZeroConstInt);
-  RB200_MZ(1, kZeroGeneral);
-  RB200_MZ(2, kZeroGeneral);
   RB200_MZ(4, kZeroGeneral);
 #undef RB200_MZ
   RB200_CHECK(false, "bad m-tile count %d / zero mode %d", l.mt, l.zmode);

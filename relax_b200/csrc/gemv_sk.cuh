@@ -1,12 +1,10 @@
-// Decode-path kernel for 9 to 32 batch rows, and for every row-parallel shard whose epilogue sums
-// over ranks: warp-MMA consumers on a stream-k split.
+// Decode-path kernel for every row-parallel shard of at most 32 rows whose epilogue sums over ranks, and for
+// the shapes of 17 to 32 rows that the tensor-core kernels do not cover: warp-MMA consumers on a stream-k
+// split.
 //
 // What measurements on B200 settled before this version was written:
 //  * mma.sync.m16n8k16 sustains one MMA per 8 clocks per SM sub-partition - a 16x16 weight
-//    fragment (128 packed bytes) per 2 clocks per SM, far above the HBM rate - while one
-//    tcgen05.mma (M = 128, K = 16) occupies the tensor pipe for 108 clocks whatever its N up to
-//    192: with the batch as N it caps the weight stream near 2.8 TB/s.  Small batches belong on
-//    the warp MMA; tcgen05 pays off from a batch of a hundred rows up.
+//    fragment (128 packed bytes) per 2 clocks per SM, far above the HBM rate.
 //  * the async copy engine is paid per contiguous segment, not per byte.  Hence the
 //    stage-contiguous fragment layout: one 16 KB bulk copy per stage.
 //  * a warp that issues a 16-byte cp.async stalls until the address is translated - more than a

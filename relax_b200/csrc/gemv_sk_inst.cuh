@@ -57,8 +57,8 @@ int launch_gs(const Params& pp, const Launch& l, const CUtensorMap& tx, const CU
     RB200_CHECK(false, "the fused all-reduce epilogue covers symmetric weights with group-32 scales (int4) or "
                 "per-channel scales; got group code %d, scale source %d, zero mode %d", l.group_code, l.src, ZMODE);
   }
-  // without that epilogue one m-tile belongs to the small-batch kernel
-  if constexpr (MT > 1) {
+  // without that epilogue up to two m-tiles belong to the small-batch kernel
+  if constexpr (MT == 4) {
 #define RB200_CASE(G, S) \
   if (l.group_code == (G) && l.src == (S)) return launch_inst<BITS, MT, ZMODE, G, S>(pp, l, tx, ts, tz, stream)
   RB200_CASE(32, kSrcGlobal);

@@ -22,8 +22,6 @@ constexpr uint32_t kVacant = 0xffffffffu;  // a NaN; sums that are NaN are publi
 constexpr int kMaxNb = 256;
 constexpr int kStageBytes = 16 * kTileRows * 4;  // per drain group: two 16 x 128 fp16 buffers, or one fp32
 
-constexpr unsigned kNap = 64;  // nanoseconds between polls of a role that is ahead
-
 enum ScaleSrc : int {
   kChannel = 0,  // one per row
   kOne = 1,      // groups of whole 64-k blocks
