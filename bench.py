@@ -754,7 +754,7 @@ def run_gpu(args):
             tpeak = float(json.load(open(os.path.join(ROOT, "MEASURED_PEAKS.json")))["bf16_tflops"])
         except Exception:
             tpeak = 1590.0
-        prefill = {"workload": "W4A16 group-128 asymmetric GEMM m=2048 k=4096 n=22016", "kernel": "umma_gemm_kernel",
+        prefill = {"workload": "W4A16 group-128 asymmetric GEMM m=2048 k=4096 n=22016", "kernel": "umma_pair_kernel",
                    "ms": pt, "tflops": tf, "peak_tflops": tpeak, "frac": tf / tpeak,
                    "l2": "x + packed weight + out = 152 MB per launch, larger than L2"}
         del pw, ps, pz, px, po
@@ -836,11 +836,11 @@ def run_gpu(args):
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": peak, "unit": "GB/s",
                          "frac": achieved / peak,
                          # DRAM bytes per launch: the ncu capture of the gate_up M=1 launch read + wrote
-                         # 50.84 MB for 50.78 MB of algorithmic bytes (x 1.0012); scaled to the mean launch
-                         "traffic": 1.0012 * sum(c for _, c in per_shape.values()) / len(per_shape),
-                         "traffic_source": "profiles/gemv_sk_kernel_gate_up_m1.md, scaled by algorithmic bytes",
+                         # 50.77 MB for 50.78 MB of algorithmic bytes (x 0.9998); scaled to the mean launch
+                         "traffic": 0.9998 * sum(c for _, c in per_shape.values()) / len(per_shape),
+                         "traffic_source": "profiles/gemv_rk_kernel_gate_up_m1.md, scaled by algorithmic bytes",
                          "peak_kind": peak_kind,
-                         "kernel": "gemv_sk_kernel",
+                         "kernel": "gemv_rk_kernel (M <= 16), umma_sk_kernel (M = 32)",
                          "per_shape_gbs": shape_gbs, "per_shape_us": shape_us},
             "cpu_baseline": cpu,
             "clocks": {"sm_mhz": clk["sm_mhz"], "sm_max_mhz": clk["sm_max_mhz"], "reasons": clk["reasons"]},

@@ -236,11 +236,11 @@ RB200_API int rb200_gemm_fp16_intx_noalloc(const rb200_gemm_desc* desc, void* st
  * (num_experts * n * k * bits / 8 bytes), scales / zeros addressed
  *   e * scale_stride_e + n_idx * scale_stride_n + (k_idx / group_size) * scale_stride_g
  * - an extension: the reference has no quantised grouped GEMM.
- * Needs n % 128 == 0, k % 64 == 0, 16-byte aligned x / out rows, num_experts <= 64.
+ * Needs n % 16 == 0 (dense weights: n % 128 == 0), k % 64 == 0, 16-byte aligned x / out rows,
+ * num_experts <= 64.
  * workspace is accepted for signature parity and not used (nothing is allocated per call).
- * Packed weights with at most 32 rows in all (decode-size batches) run as one launch of the
- * small-batch decode kernel, which reads every expert's row range from indptr on the device and
- * skips experts without rows; they then need only n % 16 == 0.
+ * One launch for all experts; their row ranges are read from indptr on the device and experts
+ * without rows cost nothing.
  */
 typedef struct rb200_group_gemm_desc {
   uint32_t struct_size;   /* sizeof(rb200_group_gemm_desc) */
