@@ -429,6 +429,15 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
     // tensor-core kernels.  What they do not cover - the fused all-reduce, x or out without 16-byte rows -
     // runs on the stream-k kernel, and int8 with k a multiple of 32 only on the cluster kernel, whose
     // split-k partials meet in distributed shared memory.
+    // One exception: zero points per group of 32 at nine to sixteen rows spill there (two m-tiles beside
+    // four words of scales and zero points), and from 48 Mi weights on the tensor-core kernel is ahead (16
+    // rows: k 4096 x n 12288 17.9 / 15.0 us, k 11008 x n 6144 27.1 / 19.6; below, k 4096 x n 8192 11.1 / 11.8).
+    if (p.m > 8 && p.m <= rk::kMaxBatch && !ar && p.group == 32 && zero_mode(d) == kZeroGeneral && d->weight_bits == 4 &&
+        (int64_t)p.n * p.k >= (48ll << 20)) {
+      const int rc = umma_run(p, d->weight_bits, zero_mode(d), sc->sm_count, sc->vacant_words, sc->vacant_bytes, nullptr,
+                              0, 1, 0, 0, stream);
+      if (rc <= 0) return rc;
+    }
     if (p.m <= rk::kMaxBatch && !ar)
       return gemv_rk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
     unsigned* flags = reinterpret_cast<unsigned*>(sc->counters) + kSkFlagOffset;

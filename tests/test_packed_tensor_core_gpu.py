@@ -35,6 +35,18 @@ def test_int4(oracle, m, k, n, group, zeros):
     assert_close(got, C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, case.zeros, 7.0, group))))
 
 
+@pytest.mark.parametrize("m", [9, 16])
+@pytest.mark.parametrize("n", [12272, 12304])
+def test_int4_few_rows(oracle, m, n):
+    """either side of the size from which up to 16 rows with zero points per group of 32 come here"""
+    k, group = 4096, 32
+    case = synth.q4_case(np.random.Generator(np.random.PCG64(m + n)), m, k, n, group, asymmetric=True)
+    pre, s, z, x = ops.preprocess_weight_q4f16(u32_to_dev(case.w)), to_dev(case.scales), to_dev(case.zeros), to_dev(case.x)
+    got = _twice(lambda: ops.gemm_fp16_q4f16(x, pre, s, z, group_size=group))
+    C = oracle.C()
+    assert_close(got, C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, case.zeros, 7.0, group))))
+
+
 @pytest.mark.parametrize("m", [17, 48, 64, 65, 128, 160, 256, 300])
 @pytest.mark.parametrize("bits,k,n,group", [(8, 320, 144, -1), (8, 1152, 528, 32), (8, 2112, 272, 64), (4, 4160, 400, -1)])
 def test_ft(oracle, m, bits, k, n, group):
