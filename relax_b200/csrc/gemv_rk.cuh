@@ -316,9 +316,12 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 
   // L2 prefetch: a lane asks for one of the 16 lines of either row block's chunk.  int8 tiles take a
   // third of the arithmetic of int4 tiles per byte, so there the loads need this lead to keep HBM
-  // busy (k 8192 x n 28672: 54 -> 38 us); for int4 it only cost instructions (14.8 against 13.7 us at
-  // k 4096 x n 22016).
-  constexpr bool kLead = BITS == 8;
+  // busy (k 8192 x n 28672: 54 -> 38 us).  For int4 it only costs instructions in one matmul (14.8 against
+  // 13.7 us at k 4096 x n 22016; folded, k 4096 x n 57344 group 128 29.6 against 28.7), but an expert
+  // layer's weights are many times that, and its passes jump between experts: eight experts, 16 rows,
+  // k 4096 x n 28672 102.9 -> 98.6 us, k 14336 x n 4096 58.2 -> 51.7, one scale per row 80.5 -> 78.0 (scales
+  // per tile 28.2 -> 29.8: not there).
+  constexpr bool kLead = BITS == 8 || (GROUPED && kFold && !kZ && SRC != kTile);
   const int ahead = min(kLeadChunks, c1 - c0);
   auto line_of = [&](const Pass& q, int c) -> const uint8_t* {
     const int st = min(8, NB - (q.nb0 & ~7)) * 4;
