@@ -197,20 +197,31 @@ __device__ __forceinline__ void decode_int8_pair(uint32_t w_g, uint32_t w_g8, co
   a[3] = h2_mul(h23, s_g8);
 }
 
-// The same fragments with the bare codes as fp16 subnormals, u * 2^-24 (rows g + 8 of int4: u * 2^-20):
-// a masked code is that number already, exactly, and the tensor cores take subnormals at full rate.
-__device__ __forceinline__ void codes_int4_word(uint32_t w, uint32_t (&a)[4]) {
+// The same fragments unscaled, u - z in the codes' units: a masked code is the fp16 subnormal u * 2^-24
+// (rows g + 8 of int4: u * 2^-20) already, the tensor cores take subnormals at full rate, and the difference
+// rounds as f16(u) - z does (exact wherever that is).  z_g, z_g8: f16x2 zero points in those units.
+__device__ __forceinline__ void codes_int4_word(uint32_t w, uint32_t z_g, uint32_t z_g8, uint32_t (&a)[4]) {
   const uint32_t w2 = w >> 8;
-  a[0] = w & 0x000f000fu;
-  a[1] = w & 0x00f000f0u;
-  a[2] = w2 & 0x000f000fu;
-  a[3] = w2 & 0x00f000f0u;
+  a[0] = h2_sub(w & 0x000f000fu, z_g);
+  a[1] = h2_sub(w & 0x00f000f0u, z_g8);
+  a[2] = h2_sub(w2 & 0x000f000fu, z_g);
+  a[3] = h2_sub(w2 & 0x00f000f0u, z_g8);
 }
-__device__ __forceinline__ void codes_int8_pair(uint32_t w_g, uint32_t w_g8, uint32_t (&a)[4]) {
-  a[0] = prmt(w_g, 0u, 0x4140u);
-  a[1] = prmt(w_g8, 0u, 0x4140u);
-  a[2] = prmt(w_g, 0u, 0x4342u);
-  a[3] = prmt(w_g8, 0u, 0x4342u);
+__device__ __forceinline__ void codes_int8_pair(uint32_t w_g, uint32_t w_g8, uint32_t z_g, uint32_t z_g8, uint32_t (&a)[4]) {
+  a[0] = h2_sub(prmt(w_g, 0u, 0x4140u), z_g);
+  a[1] = h2_sub(prmt(w_g8, 0u, 0x4140u), z_g8);
+  a[2] = h2_sub(prmt(w_g, 0u, 0x4342u), z_g);
+  a[3] = h2_sub(prmt(w_g8, 0u, 0x4342u), z_g8);
+}
+// Zero points of rows g (low half) and g + 8 in those units, and whether they fit (integers do): a
+// subnormal has no room for a fraction.
+template <int BITS>
+__device__ __forceinline__ uint32_t zero_in_codes(uint32_t z_pair, bool& fits) {
+  constexpr uint32_t kUnits = BITS == 4 ? 0x00100001u : 0x00010001u;  // f16x2(2^-24, 2^-20 | 2^-24)
+  constexpr uint32_t k4096 = 0x6c006c00u, kRest = BITS == 4 ? 0x5c006c00u : 0x6c006c00u;
+  const uint32_t z = h2_mul(z_pair, kUnits);
+  fits = h2_mul(h2_mul(z, k4096), kRest) == z_pair;
+  return z;
 }
 
 // ---------------------------------------------------------------- epilogue

@@ -3,8 +3,8 @@
 //   out[m, n] = epilogue(sum_k x[m, k] * wq[n, k]),  m <= 8 or 16 (one or two m16n8k16 MMAs wide)
 //
 // Bound: HBM (the packed weight once) and, close behind, instruction issue: the exact two-rounding
-// decode is 52 of the 61 instructions a 512-byte tile needs (4 MMAs, 3 loads, 2 scale selects), 20
-// where the codes go into the MMA undecoded.
+// decode is 52 of the 61 instructions a 512-byte tile needs (4 MMAs, 3 loads, 2 scale selects), 36
+// where the scale is left to the sums.
 // So nothing else is in the loop: no shared memory, no barriers, no copies through the async
 // engine.  A warp reads fragment tiles with 128-bit loads that are whole 512-byte lines in the
 // fragment layout, straight into the registers the MMA takes them from, one chunk (four tiles)
@@ -50,15 +50,17 @@ enum ScaleSrc : int {
   kTile = 4,     // as kGeneral, groups of whole tiles
 };
 
-// Where the codes go into the MMA as they are and zero point and scale are applied to its fp32 sums
-// (kFold below), which also rounds less: a group has to be whole tiles, since an MMA's sum runs over a
-// quarter of a tile.  It costs an MMA per code word and m-tile for the activations' sums, shared by the
-// row blocks of a pass: 8 clocks of the sub-partition's MMA pipe against 16 of decoding.  Measured at
-// k 4096 x n 11008 int4, four rows: group 128 with zero points 12.9 -> 10.6 us, without 10.7 -> 10.2,
-// group 64 12.0 -> 11.6, channel 8.8 -> 8.0.  With two m-tiles the MMAs are the bound and the decode
-// stays (16 rows: group 128 12.8 us against 14.6, channel 10.7 against 12.4; int8 even).  Two groups in a
-// tile, four batch rows of one group beside the same rows of the other in the MMA's eight columns, was
-// no faster than the decode for group 32 (k 4096 x n 12288 9.1 against 8.9, k 11008 x n 4096 8.6 against 8.0).
+// Where u - z goes into the MMA in the codes' units and the scale is applied to its fp32 sums (kFold below),
+// which also rounds less: a group has to be whole tiles, since an MMA's sum runs over a quarter of a tile.
+// The difference comes before the product, as in the decode: sums of u x and of z x kept apart cancel when
+// the activations have a mean (int8 per row, k 28672, mean 4: relative error 1.3e-3 against 2.1e-4 here and
+// 2.5e-4 with decoded weights) and turn an infinite activation into NaN.  Nine instructions per code word of
+// int4 instead of 13, or 17 with zero points.  Measured at k 4096 x n 11008 int4, four rows, decoded against
+// this: group 128 with zero points 12.9 / 10.3 us, without 10.7 / 9.3, group 64 12.0 / 10.1, one scale per row
+// 8.8 / 8.2.  Two m-tiles decode (measured only for the form that kept the sums apart, which was slower
+// there: 16 rows, group 128 12.8 / 14.6), and so does group 32: two groups in a tile, four batch rows of one
+// beside the same rows of the other in the MMA's eight columns, was no faster (k 4096 x n 12288 8.9 / 9.1,
+// k 11008 x n 4096 8.0 / 8.6).
 constexpr bool folds(int src, int m_tiles) { return src != kRow32 && src != kGeneral && m_tiles == 1; }
 
 struct Params {
@@ -174,13 +176,29 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   const uint32_t half_sel = (t >> 1) ? 0x3232u : 0x1010u;
   const int unit16 = frag_unit_pos(lane) * 16;
   const bool has_zeros = kZ && p.z != nullptr;
-  // kFold: A operand of the products that sum the activations, in the codes' units: the zero point,
-  // negated, or one
+  // kFold: the codes' units, and what the MMA's codes are reduced by (f16x2 of rows g, g + 8)
   constexpr float kUnitLo = 1.0f / (1 << 24), kUnitHi = BITS == 4 ? 16.0f * kUnitLo : kUnitLo;
-  const float z_unit = kZ ? 1.0f : -p.zero_const;
-  const uint32_t one_lo = h2_bcast(__float2half_rn(z_unit * kUnitLo)), one_hi = h2_bcast(__float2half_rn(z_unit * kUnitHi));
-  const float zconst = __half2float(__float2half_rn(p.zero_const));
-  const uint32_t ones[4] = {one_lo, one_hi, one_lo, one_hi};
+  struct Zeros {
+    uint32_t z[kRows];
+    bool codes;  // in the codes' units, for all lanes and row blocks; else the zero points as they are
+  };
+  auto zeros_of = [&](const uint32_t (&z2)[kRows]) {
+    Zeros z;
+    bool fit = true;
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+      bool f;
+      z.z[r] = zero_in_codes<BITS>(z2[r], f);
+      fit = fit && f;
+    }
+    z.codes = !kZ || __all_sync(0xffffffffu, fit);  // (kZeroConstInt: an integer)
+    if (kZ && !z.codes)
+#pragma unroll
+      for (int r = 0; r < kRows; ++r) z.z[r] = z2[r];
+    return z;
+  };
+  using CodeUnits = std::true_type;
+  using PlainUnits = std::false_type;
 
   // this warp's whole chunks (four fragment tiles); the tiles of a short last chunk go to the last warp
   const int full_chunks = KB / 4;
@@ -212,7 +230,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   uint2 sv[2][kRows][2], zv[2][kRows][2];      // kRow32: rows g, g + 8: the half's four groups
   // kHalf, kTile, kGeneral: per half or tile, rows g, g + 8; a word each where registers allow it (as
   // one word they are waited for soon after their loads: int4 k 4096 x n 57344, group 128 36.6 -> 35.0 us)
-  uint32_t sg[2][kRows][2][2], zg[2][kRows][2][2];
+  uint32_t sg[2][kRows][2][2], zg[2][kRows][2];
   uint32_t ch_s[kRows], ch_z[kRows];           // kChannel
   const uint8_t* wp = nullptr;                 // next chunk to load
   const __half *sp[kRows][2], *zp[kRows][2];   // scales of rows g, g + 8 (kRow32: of the next chunk)
@@ -258,8 +276,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
           sg[S][r][j][1] = b;
           if (has_zeros) {
             const uint32_t za = ld_nc_u16(zp[r][0] + o), zb = ld_nc_u16(zp[r][1] + o);
-            zg[S][r][j][0] = kFold ? za : za | (zb << 16);
-            zg[S][r][j][1] = zb;
+            zg[S][r][j] = za | (zb << 16);
           }
         }
       }
@@ -328,6 +345,10 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
     return p.w + (grouped ? q.e * pp.w_expert_bytes : 0) +
            (int64_t)((q.nb0 & ~7) * KB + c * st + (q.nb0 & 7) * 4) * 512 + lane * 128;
   };
+  uint32_t zconst_of[kRows];
+#pragma unroll
+  for (int r = 0; r < kRows; ++r) zconst_of[r] = zconst_h2;
+  const Zeros zeros_const = zeros_of(zconst_of);
   Pass q = get_pass(pos);
   if (!grouped && pp.early) start_pass(q);
   if (kLead || !pp.early) {
@@ -371,26 +392,19 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
         }
       }
     };
-    // kFold: sum (u - z) x = sum u x - z sum x; `sums` gets the second sum, times `ones`
-    float sums[MT][4];
-#pragma unroll
-    for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-      for (int c = 0; c < 4; ++c) sums[mt][c] = 0.0f;
-    // (the chains of a step are independent of each other and issued in turn)
-    auto sum_step = [&](float (&d)[MT][4], const uint4 (&xv)[MT][kXV], int j, bool first) {
-#pragma unroll
-      for (int mt = 0; mt < MT; ++mt) {
-        const uint4& x = xv[mt][j >> 1];
-        if (first && j == 0) mma_16816_first(d[mt], ones, x.x, x.y);
-        else mma_16816(d[mt], ones, (j & 1) ? x.z : x.x, (j & 1) ? x.w : x.y);
-      }
-    };
-    auto code_step = [&](float (&d)[MT][4], const uint4& wv, const uint4 (&xv)[MT][kXV], int j, bool first) {
+    // kFold: d (+)= (u - z) x
+    auto code_step = [&](auto units, float (&d)[MT][4], const uint4& wv, uint32_t z2, const uint4 (&xv)[MT][kXV], int j, bool first) {
       const uint32_t ww[4] = {wv.x, wv.y, wv.z, wv.w};
+      const uint32_t z_g = prmt(z2, z2, 0x1010u), z_g8 = prmt(z2, z2, 0x3232u);
       uint32_t a[4];
-      if (BITS == 4) codes_int4_word(ww[j], a);
-      else codes_int8_pair(ww[2 * (j & 1)], ww[2 * (j & 1) + 1], a);
+      if (units) {
+        if (BITS == 4) codes_int4_word(ww[j], z_g, z_g8, a);
+        else codes_int8_pair(ww[2 * (j & 1)], ww[2 * (j & 1) + 1], z_g, z_g8, a);
+      } else {
+        constexpr uint32_t kOne = 0x3c003c00u;
+        if (BITS == 4) decode_int4_word<ZMODE>(ww[j], zc, kOne, kOne, z_g, z_g8, a);
+        else decode_int8_pair<ZMODE>(ww[2 * (j & 1)], ww[2 * (j & 1) + 1], zc, kOne, kOne, z_g, z_g8, a);
+      }
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt) {
         const uint4& x = xv[mt][j >> 1];
@@ -398,16 +412,16 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
         else mma_16816(d[mt], a, (j & 1) ? x.z : x.x, (j & 1) ? x.w : x.y);
       }
     };
-    // acc += s * (d + sums), or s * (d - z * sums)
-    auto add_scaled = [&](int r, const float (&d)[MT][4], const float (&xs)[MT][4], float s_g, float s_g8, float z_g,
-                          float z_g8) {
+    // acc += s * d, in the codes' units
+    auto add_scaled = [&](auto units, int r, const float (&d)[MT][4], float s_g, float s_g8) {
+      if (!units) {
+        s_g *= kUnitLo;
+        s_g8 *= kUnitHi;
+      }
 #pragma unroll
       for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const float v = kZ ? d[mt][c] - (c < 2 ? z_g : z_g8) * xs[mt][c] : d[mt][c] + xs[mt][c];
-          acc[r][0][mt][c] += (c < 2 ? s_g : s_g8) * v;
-        }
+        for (int c = 0; c < 4; ++c) acc[r][0][mt][c] += (c < 2 ? s_g : s_g8) * d[mt][c];
     };
     auto half_of = [](uint32_t v, int hi) { return __half2float(__ushort_as_half((unsigned short)(hi ? v >> 16 : v & 0xffffu))); };
     const __half* xp = x0 + c0 * (kFrag * 4);
@@ -424,44 +438,46 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 #pragma unroll
           for (int i = 0; i < kXV; ++i) xv.v[j][mt][i] = ld_nc_v4(xp + mt * x_next + (half * 2 + j) * kFrag + i * 8);
     };
+    Zeros ch_zeros = zeros_const;  // kFoldAll
+    if (kFoldAll && has_zeros) ch_zeros = zeros_of(ch_z);
+    auto in_units = [&](const Zeros& z, auto&& f) {
+      if (!kZ || z.codes) f(CodeUnits{});
+      else f(PlainUnits{});
+    };
     auto half_step = [&](auto set_tag, auto rn_tag, const XHalf<kXV, MT>& xv) {
       constexpr int S = decltype(set_tag)::value, RN = decltype(rn_tag)::value;
       if constexpr (kFoldAll) {
+        in_units(ch_zeros, [&](auto units) {
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
+          for (int j = 0; j < 2; ++j)
 #pragma unroll
-          for (int i = 0; i < 2 * kXV; ++i) {
-            sum_step(sums, xv.v[j], i, false);
+            for (int i = 0; i < 2 * kXV; ++i)
 #pragma unroll
-            for (int r = 0; r < RN; ++r) code_step(acc[r][i % kChains], w[S][r][j], xv.v[j], i, false);
-          }
-        }
+              for (int r = 0; r < RN; ++r) code_step(units, acc[r][i % kChains], w[S][r][j], ch_zeros.z[r], xv.v[j], i, false);
+        });
         return;
       } else if constexpr (kFold) {
         constexpr int kSpan = SRC == kHalf ? 2 : 1;  // tiles of a group (as far as the half goes)
-        float d[RN][MT][4];
 #pragma unroll
-        for (int j = 0; j < 2; ++j) {
-          const bool first = j % kSpan == 0;
+        for (int part = 0; part < 2 / kSpan; ++part) {
+          Zeros z = zeros_const;
+          if (has_zeros) {
+            uint32_t z2[kRows];
 #pragma unroll
-          for (int i = 0; i < 2 * kXV; ++i) {
-            sum_step(sums, xv.v[j], i, first);
-#pragma unroll
-            for (int r = 0; r < RN; ++r) code_step(d[r], w[S][r][j], xv.v[j], i, first);
+            for (int r = 0; r < kRows; ++r) z2[r] = zg[S][r < RN ? r : 0][part];
+            z = zeros_of(z2);
           }
-          if ((j + 1) % kSpan != 0) continue;
+          in_units(z, [&](auto units) {
+            float d[RN][MT][4];
 #pragma unroll
-          for (int r = 0; r < RN; ++r) {
-            float s_g, s_g8, z_g = zconst, z_g8 = zconst;
-            const int at = SRC == kHalf ? 0 : j;
-            s_g = half_of(sg[S][r][at][0], 0);
-            s_g8 = half_of(sg[S][r][at][1], 0);
-            if (has_zeros) {
-              z_g = half_of(zg[S][r][at][0], 0);
-              z_g8 = half_of(zg[S][r][at][1], 0);
-            }
-            add_scaled(r, d[r], sums, s_g, s_g8, z_g, z_g8);
-          }
+            for (int j = part * kSpan; j < (part + 1) * kSpan; ++j)
+#pragma unroll
+              for (int i = 0; i < 2 * kXV; ++i)
+#pragma unroll
+                for (int r = 0; r < RN; ++r) code_step(units, d[r], w[S][r][j], z.z[r], xv.v[j], i, j == part * kSpan);
+#pragma unroll
+            for (int r = 0; r < RN; ++r) add_scaled(units, r, d[r], half_of(sg[S][r][part][0], 0), half_of(sg[S][r][part][1], 0));
+          });
         }
         return;
       }
@@ -484,7 +500,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
             s_g = prmt(a, a, 0x1010u);
             s_g8 = prmt(a, a, 0x3232u);
             if (has_zeros) {
-              const uint32_t b = SRC == kChannel ? ch_z[r] : zg[S][r][SRC == kHalf ? 0 : j][0];
+              const uint32_t b = SRC == kChannel ? ch_z[r] : zg[S][r][SRC == kHalf ? 0 : j];
               z_g = prmt(b, b, 0x1010u);
               z_g8 = prmt(b, b, 0x3232u);
             }
@@ -542,9 +558,6 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 #pragma unroll
           for (int i = 0; i < kXV; ++i) xt[mt][i] = ld_nc_v4(x0 + mt * x_next + kb * kFrag + i * 8);
         const unsigned k = (unsigned)(kb * kFrag + t * kLaneK);
-        if (kFold)
-#pragma unroll
-          for (int i = 0; i < 2 * kXV; ++i) sum_step(sums, xt, i, !kFoldAll);
         const unsigned grp = SRC == kChannel ? 0u : (pp.group_shift >= 0 ? k >> pp.group_shift : k / (unsigned)p.group);
 #pragma unroll
         for (int r = 0; r < kRows; ++r) {
@@ -552,8 +565,10 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
           const uint4 wt = ld_stream_v4(p.w + (grouped ? q.e * pp.w_expert_bytes : 0) +
                                         frag_tile_offset(q.nb0 + r, kb, NB, KB) + unit16);
           if (kFoldAll) {
+            in_units(ch_zeros, [&](auto units) {
 #pragma unroll
-            for (int i = 0; i < 2 * kXV; ++i) code_step(acc[r][i % kChains], wt, xt, i, false);
+              for (int i = 0; i < 2 * kXV; ++i) code_step(units, acc[r][i % kChains], wt, ch_zeros.z[r], xt, i, false);
+            });
             continue;
           }
           const int64_t o = (grouped ? q.e * pp.s_expert_stride : 0) + ((q.nb0 + r) * 16 + g) * pp.s_n +
@@ -562,10 +577,16 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
           const uint32_t za = has_zeros ? ld_nc_u16(p.z + o) * 0x10001u : zconst_h2;
           const uint32_t zb = has_zeros ? ld_nc_u16(p.z + o + row8) * 0x10001u : zconst_h2;
           if (kFold) {
-            float d[MT][4];
+            uint32_t z2[kRows];
 #pragma unroll
-            for (int i = 0; i < 2 * kXV; ++i) code_step(d, wt, xt, i, true);
-            add_scaled(r, d, sums, half_of(a, 0), half_of(b, 0), half_of(za, 0), half_of(zb, 0));
+            for (int i = 0; i < kRows; ++i) z2[i] = prmt(za, zb, 0x5410u);
+            const Zeros z = zeros_of(z2);
+            in_units(z, [&](auto units) {
+              float d[MT][4];
+#pragma unroll
+              for (int i = 0; i < 2 * kXV; ++i) code_step(units, d, wt, z.z[0], xt, i, true);
+              add_scaled(units, r, d, half_of(a, 0), half_of(b, 0));
+            });
             continue;
           }
           mma_tile(r, wt, a * 0x10001u, b * 0x10001u, za, zb, xt);
@@ -575,12 +596,14 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 
     // the next pass's first loads leave before this one's sums are put together
     const Pass done = q;
-    uint32_t done_s[kRows], done_z[kRows];
+    float done_s[kRows][2];  // kFoldAll: scales of the sums
 #pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      done_s[r] = kFoldAll ? ch_s[r] : 0u;
-      done_z[r] = kFoldAll && has_zeros ? ch_z[r] : 0u;
-    }
+    for (int r = 0; r < kRows; ++r)
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        done_s[r][i] = kFoldAll ? half_of(ch_s[r], i) : 1.0f;
+        if (kFoldAll && kZ && !ch_zeros.codes) done_s[r][i] *= i ? kUnitHi : kUnitLo;
+      }
     pos += (unsigned)q.rn;
     if (more) {
       if constexpr (kLead) q = q_next;
@@ -597,10 +620,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           f[c] = acc[r][0][mt][c] + (kChains == 2 ? acc[r][kChains - 1][mt][c] : 0.0f);
-          if (kFoldAll) {
-            const float z = has_zeros ? half_of(done_z[r], c >> 1) : zconst;
-            f[c] = half_of(done_s[r], c >> 1) * (kZ ? f[c] - z * sums[mt][c] : f[c] + sums[mt][c]);
-          }
+          if (kFoldAll) f[c] *= done_s[r][c >> 1];
         }
         red[buf][warp][r * MT + mt][lane] = make_float4(f[0], f[1], f[2], f[3]);
       }

@@ -57,3 +57,63 @@ def test_experts(oracle, rows, bits, k, n):
     if total:
         wq = np.stack([C.decode_ft_kn(w[e], s[e], bits, 64).T for e in range(4)])
         assert_close(got[:total], C.epilogue(C.group_gemm_f32(x[:total], np.ascontiguousarray(wq), indptr)))
+
+
+def _forms():
+    yield "ft4_row", 4, -1, None
+    yield "ft8_row", 8, -1, None
+    yield "ft8_64", 8, 64, None
+    yield "q4_row_zeros", 4, -1, "int"
+    yield "q4_128_zeros", 4, 128, "int"
+    yield "q4_64_rounded_zeros", 4, 64, "any"
+    yield "q4_32", 4, 32, None
+
+
+def _call(oracle, name, bits, group, zeros, x, n, seed):
+    """One call on random codes; returns (result, decoded weights [n, k] in fp64)."""
+    k = x.shape[1]
+    rs = np.random.RandomState(seed)
+    C = oracle.C()
+    if name.startswith("ft"):
+        w = rs.randint(-128, 128, size=(k, n * bits // 8)).astype(np.int8)
+        s = rs.uniform(1e-4, 1e-3, size=(n,) if group < 0 else (k // group, n)).astype(np.float16)
+        out = ops.gemm_fp16_ft(to_dev(x), ops.preprocess_weight_ft(to_dev(w), bits == 4), to_dev(s), bits, group_size=group)
+        wq = C.decode_ft_kn(w, s, bits, group).T
+    else:
+        group = k if group < 0 else group
+        case = synth.q4_case(np.random.Generator(np.random.PCG64(seed)), 1, k, n, group, asymmetric=zeros is not None)
+        if zeros == "any":
+            case.zeros[:, ::2] = np.float16(7.3)
+        z = None if zeros is None else to_dev(case.zeros)
+        out = ops.gemm_fp16_q4f16(to_dev(x), ops.preprocess_weight_q4f16(u32_to_dev(case.w)), to_dev(case.scales), z, group_size=group)
+        wq = C.decode_q4_nk(case.w, case.scales, case.zeros, 7.0, group)
+    _check_status()
+    return out.cpu().numpy().astype(np.float64), wq.astype(np.float64)
+
+
+@pytest.mark.parametrize("m", [1, 8, 9])
+@pytest.mark.parametrize("form", list(_forms()), ids=lambda f: f[0])
+def test_activations_with_an_offset(oracle, form, m):
+    """Activations far from zero mean over a long k: the zero point has to leave the codes before they are
+    summed, or the sums of codes and of zero points cancel.  Bound: a weight that is not rounded to fp16
+    differs from the decoded one by at most 2^-11, 2.8e-4 in the mean square, the output's rounding is
+    another 2.8e-4, and fp32 sums of k / 128 MMAs add 3e-5: 4e-4 in the 2-norm, and 1e-3 asked."""
+    k, n = 28672, 64
+    x = (np.abs(np.random.RandomState(m).randn(m, k)) + 4.0).astype(np.float16)
+    got, wq = _call(oracle, *form, x, n, 11)
+    exp = x.astype(np.float64) @ wq.T
+    assert np.linalg.norm(got - exp) <= 1e-3 * np.linalg.norm(exp)
+
+
+@pytest.mark.parametrize("m", [1, 8, 9])
+@pytest.mark.parametrize("form", list(_forms()), ids=lambda f: f[0])
+def test_infinite_activation(oracle, form, m):
+    """One infinite activation: infinite results with the sign of its weight, NaN where that weight is zero."""
+    k, n = 1024, 256
+    x = np.random.RandomState(m).randn(m, k).astype(np.float16)
+    x[0, 517] = np.inf
+    got, wq = _call(oracle, *form, x, n, 12)
+    with np.errstate(invalid="ignore"):
+        exp = x.astype(np.float64) @ wq.T
+    assert np.array_equal(np.isnan(got), np.isnan(exp))
+    assert np.array_equal(np.isposinf(got), np.isposinf(exp)) and np.array_equal(np.isneginf(got), np.isneginf(exp))
