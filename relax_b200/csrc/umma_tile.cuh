@@ -8,6 +8,7 @@
 #include "dequant.cuh"
 #include "gemv.h"
 #include "umma_common.cuh"
+#include "umma_index.h"
 
 namespace rb200 {
 namespace us {
@@ -296,11 +297,12 @@ struct ScaleFeed {
   // scales are one 8-byte load when the rows allow it
   __device__ __forceinline__ void fetch_two(const Params& pp, int kb, int k_blocks) {
     if (SRC == kTwo && pp.s_vec == 2) {
-      const uint2 s = __ldg(reinterpret_cast<const uint2*>(sp + kb * 2));
+      const int at = pair_in_row(kb, k_blocks) * 2;
+      const uint2 s = __ldg(reinterpret_cast<const uint2*>(sp + at));
       sn[0] = s.x;
       sn[OWN - 1] = s.y;
       if (has_zeros) {
-        const uint2 z = __ldg(reinterpret_cast<const uint2*>(zp + kb * 2));
+        const uint2 z = __ldg(reinterpret_cast<const uint2*>(zp + at));
         zn[0] = z.x;
         zn[OWN - 1] = z.y;
       }

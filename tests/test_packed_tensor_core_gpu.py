@@ -1,7 +1,7 @@
 """The tensor-core kernels over packed weights (17 to 64 rows: one CTA per tile; above: CTA pairs) where
 their tiles and splits can go wrong: rows around 32-row steps, tile widths and the border between the two
-kernels, row counts that are no multiple of a 128- or 256-row tile, an odd number of 64-k blocks, every
-scale source and zero-point form, and experts with more rows than a tile.  Each launch is repeated into a
+kernels, row counts that are no multiple of a 128- or 256-row tile, an odd number of 64-k blocks and a last
+chunk of two, every scale source and zero-point form, and experts with more rows than a tile.  Each launch is repeated into a
 new output and has to repeat itself bit for bit: the hand-over words are back at rest."""
 import numpy as np
 import pytest
@@ -23,7 +23,8 @@ def _twice(run):
 
 @pytest.mark.parametrize("m", [17, 32, 33, 64, 65, 96, 97, 129, 192, 255, 257])
 @pytest.mark.parametrize("k,n,group,zeros", [(704, 144, 32, None), (2304, 400, 96, "int"), (4160, 16, 64, None),
-                                             (1024, 272, 128, "any"), (1024, 1040, 32, "int")])
+                                             (1024, 272, 128, "any"), (1024, 1040, 32, "int"),
+                                             (384, 144, 32, "int"), (1408, 272, 32, None)])
 def test_int4(oracle, m, k, n, group, zeros):
     case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, group, asymmetric=zeros is not None)
     if zeros == "any":
