@@ -87,9 +87,13 @@ __device__ __forceinline__ uint4 ld_stream_v4(const void* p) {
                : "l"(p));
   return v;
 }
-__device__ __forceinline__ uint4 ld_nc_v4(const void* p) {
+// Activations: not .nc, which is for memory that nothing writes while the kernel runs.  This kernel may be
+// resident before they are written - by the kernel it waits for, or, behind two small grids, while the one
+// before that still reads the same buffer on this SM.  Weights, scales and zero points are written by kernels
+// that let no dependent start early.
+__device__ __forceinline__ uint4 ld_x_v4(const void* p) {
   uint4 v;
-  asm volatile("ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(p));
   return v;
 }
 __device__ __forceinline__ uint2 ld_nc_v2(const void* p) {
@@ -361,6 +365,25 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   if (!grouped) griddep_wait();
   if (grouped || !pp.early) start_pass(q);
 
+  // lanes of absent batch rows fetch row 0: their columns of the result are never stored
+  auto x_of = [&](const Pass& q) { return p.x + (q.m_lo + (g < q.m_n ? g : 0)) * (unsigned)p.ldx + t * kLaneK; };
+  // elements to the second m-tile's row
+  auto x_next_of = [&](const Pass& q) { return MT > 1 && g + 8 < q.m_n ? 8u * (unsigned)p.ldx : 0u; };
+  auto load_x_at = [&](XHalf<kXV, MT>& xv, const __half* at, unsigned x_next) {
+#pragma unroll
+    for (int j = 0; j < 2; ++j)
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int i = 0; i < kXV; ++i) xv.v[j][mt][i] = ld_x_v4(at + mt * x_next + j * kFrag + i * 8);
+  };
+  // int8, one scale per row: the first x of a pass leaves with its first weights (unlike read-only loads they
+  // are not moved ahead of the barrier and the stores of the pass before: k 8192 x n 28672, eight rows,
+  // 40.9 -> 38.0 us; the other forms have no registers for it)
+  constexpr bool kXEarly = BITS == 8 && SRC == kChannel;
+  XHalf<kXV, MT> x_first;
+  if (kXEarly && c0 < c1) load_x_at(x_first, x_of(q) + c0 * (kFrag * 4), x_next_of(q));
+
   int buf = 0;
   for (;;) {
     constexpr int kChains = MT == 1 && (!kFold || kFoldAll) ? 2 : 1;  // independent MMA chains (two m-tiles are two already)
@@ -373,9 +396,8 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
           for (int c = 0; c < 4; ++c) acc[r][i][mt][c] = 0.0f;
-    // lanes of absent batch rows fetch row 0: their columns of the result are never stored
-    const __half* x0 = p.x + (q.m_lo + (g < q.m_n ? g : 0)) * (unsigned)p.ldx + t * kLaneK;
-    const unsigned x_next = MT > 1 && g + 8 < q.m_n ? 8u * (unsigned)p.ldx : 0u;  // elements to the second m-tile's row
+    const __half* x0 = x_of(q);
+    const unsigned x_next = x_next_of(q);
 
     auto mma_tile = [&](int r, const uint4& wv, uint32_t s_g, uint32_t s_g8, uint32_t z_g, uint32_t z_g8,
                         const uint4 (&xv)[MT][kXV]) {
@@ -429,15 +451,9 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
     // registers and gains (scales of a half without zero points: k 4096 x n 57344 35.0 -> 33.9 us; one per
     // row 24.5 -> 25.2), else where they are used
     constexpr bool kXAhead = BITS == 8 || (kFold && SRC == kHalf && !kZ);
-    XHalf<kXV, MT> xa, xb;
-    auto load_x = [&](XHalf<kXV, MT>& xv, int half) {
-#pragma unroll
-      for (int j = 0; j < 2; ++j)
-#pragma unroll
-        for (int mt = 0; mt < MT; ++mt)
-#pragma unroll
-          for (int i = 0; i < kXV; ++i) xv.v[j][mt][i] = ld_nc_v4(xp + mt * x_next + (half * 2 + j) * kFrag + i * 8);
-    };
+    XHalf<kXV, MT> x_here, xb;
+    XHalf<kXV, MT>& xa = kXEarly ? x_first : x_here;
+    auto load_x = [&](XHalf<kXV, MT>& xv, int half) { load_x_at(xv, xp + half * (2 * kFrag), x_next); };
     Zeros ch_zeros = zeros_const;  // kFoldAll
     if (kFoldAll && has_zeros) ch_zeros = zeros_of(ch_z);
     auto in_units = [&](const Zeros& z, auto&& f) {
@@ -535,7 +551,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
         if (again) load_set(I0{}, rn_tag, c + 1);
         if (kXAhead) {
           if (again) xp += kFrag * 4;
-          load_x(xa, 0);
+          if (!kXEarly || again) load_x(xa, 0);
         } else {
           load_x(xb, 1);
           xp += kFrag * 4;
@@ -545,7 +561,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
       }
     };
     if (c0 < c1) {
-      if (kXAhead) load_x(xa, 0);
+      if (kXAhead && !kXEarly) load_x(xa, 0);
       if (q.rn == 2) all_chunks(I2{});
       else all_chunks(I1{});
     }
@@ -556,7 +572,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
 #pragma unroll
         for (int mt = 0; mt < MT; ++mt)
 #pragma unroll
-          for (int i = 0; i < kXV; ++i) xt[mt][i] = ld_nc_v4(x0 + mt * x_next + kb * kFrag + i * 8);
+          for (int i = 0; i < kXV; ++i) xt[mt][i] = ld_x_v4(x0 + mt * x_next + kb * kFrag + i * 8);
         const unsigned k = (unsigned)(kb * kFrag + t * kLaneK);
         const unsigned grp = SRC == kChannel ? 0u : (pp.group_shift >= 0 ? k >> pp.group_shift : k / (unsigned)p.group);
 #pragma unroll
@@ -609,6 +625,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
       if constexpr (kLead) q = q_next;
       else q = get_pass(pos);
       start_pass(q);
+      if (kXEarly && c0 < c1) load_x_at(x_first, x_of(q) + c0 * (kFrag * 4), x_next_of(q));
     }
 
     // the k slices meet in warp order

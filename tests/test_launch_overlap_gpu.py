@@ -49,3 +49,47 @@ def test_dependent_chain_is_bit_identical(m):
         assert torch.equal(out, ref)
     finally:
         relax_b200.set_launch_overlap(False)
+
+
+@pytest.mark.parametrize("overlap", [False, True])
+@pytest.mark.parametrize("m", [1, 8, 16, 24])
+def test_buffers_written_while_a_later_launch_is_resident(m, overlap):
+    """Two buffers in turn, small grids: launch i reads the one that launch i - 1 wrote and launch i - 2 read,
+    and may be resident since before that write."""
+    g = np.random.Generator(np.random.PCG64(50 + m))
+    k = n = 512
+    layers = []
+    for i in range(24):
+        c = synth.q4_case(g, 1, k, n, (32, 128, 512)[i % 3])
+        scales = (c.scales * 0.72).astype(np.float16)  # results keep the size of their inputs
+        layers.append((ops.preprocess_weight_q4f16(u32_to_dev(c.w)), to_dev(scales), c.group))
+    x = to_dev(g.standard_normal((m, k), dtype=np.float32).astype(np.float16))
+    ref = [x]
+    for pre, sc, group in layers:
+        ref.append(ops.gemm_fp16_q4f16(ref[-1], pre, sc, group_size=group))
+        torch.cuda.synchronize()
+    assert torch.isfinite(ref[-1]).all() and ref[-1].abs().max() > 0
+    bufs = [x.clone(), torch.empty_like(x)]
+
+    def chain():
+        bufs[0].copy_(x)
+        for i, (pre, sc, group) in enumerate(layers):
+            ops.gemm_fp16_q4f16(bufs[i % 2], pre, sc, group_size=group, out=bufs[(i + 1) % 2])
+
+    before = relax_b200.get_launch_overlap()
+    relax_b200.set_launch_overlap(overlap)
+    try:
+        for _ in range(3):
+            chain()
+        torch.cuda.synchronize()
+        assert torch.equal(bufs[0], ref[-1]) and torch.equal(bufs[1], ref[-2])
+        graph = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graph):
+            chain()
+        for _ in range(20):
+            graph.replay()
+        torch.cuda.synchronize()
+        _check_status()
+        assert torch.equal(bufs[0], ref[-1]) and torch.equal(bufs[1], ref[-2])
+    finally:
+        relax_b200.set_launch_overlap(before)
