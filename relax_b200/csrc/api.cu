@@ -49,6 +49,18 @@ int sm_count_current() {
   return v;
 }
 
+// Fills device memory and waits for it, on a stream of its own: an ordinary fill is queued on the legacy
+// stream, which the callers' streams (created non-blocking, as torch's are) do not wait for.
+int fill_now(void* p, int byte, size_t bytes) {
+  cudaStream_t s = nullptr;
+  RB200_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+  cudaError_t e = cudaMemsetAsync(p, byte, bytes, s);
+  if (e == cudaSuccess) e = cudaStreamSynchronize(s);
+  cudaStreamDestroy(s);
+  RB200_CUDA(e);
+  return 0;
+}
+
 // The current device's scratch if it has been created, else nullptr: never allocates.
 DeviceScratch* device_scratch_if_any() {
   int dev = 0;
@@ -95,7 +107,6 @@ DeviceScratch* device_scratch(size_t min_partial_bytes, size_t min_counter_ints)
     s.base = nullptr;
     return nullptr;
   }
-  cudaMemset(s.base, 0, header + counter_bytes);
   s.status = static_cast<int*>(s.base);
   s.counters = reinterpret_cast<int*>(static_cast<uint8_t*>(s.base) + header);
   s.counter_ints = counters;
@@ -103,7 +114,11 @@ DeviceScratch* device_scratch(size_t min_partial_bytes, size_t min_counter_ints)
   s.partial_bytes = partial;
   s.vacant_words = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(s.partials) + partial);
   s.vacant_bytes = vacant;
-  cudaMemset(s.vacant_words, 0xff, vacant);
+  if (fill_now(s.base, 0, header + counter_bytes) != 0 || fill_now(s.vacant_words, 0xff, vacant) != 0) {
+    cudaFree(s.base);
+    s.base = nullptr;
+    return nullptr;
+  }
   return &s;
 }
 
@@ -260,8 +275,9 @@ int rb200_check_async_error(void* stream, int* status_out) {
     RB200_CUDA(cudaMemcpy(&v, sc->status, sizeof(int), cudaMemcpyDeviceToHost));
     if (v != 0) {
       // a wait that gave up may have left split-k flags and tickets behind: back to rest
-      RB200_CUDA(cudaMemset(sc->base, 0, (size_t)(reinterpret_cast<uint8_t*>(sc->partials) - static_cast<uint8_t*>(sc->base))));
-      RB200_CUDA(cudaMemset(sc->vacant_words, 0xff, sc->vacant_bytes));
+      if (fill_now(sc->base, 0, (size_t)(reinterpret_cast<uint8_t*>(sc->partials) - static_cast<uint8_t*>(sc->base))) != 0 ||
+          fill_now(sc->vacant_words, 0xff, sc->vacant_bytes) != 0)
+        return -1;
       st = v;
     }
   }

@@ -54,6 +54,8 @@ struct DeviceScratch {
 DeviceScratch* device_scratch(size_t min_partial_bytes, size_t min_counter_ints);
 // The current device's scratch if some earlier call created it, else nullptr; never allocates.
 DeviceScratch* device_scratch_if_any();
+// Sets device memory to a byte value; it is set when this returns, for every stream.
+int fill_now(void* p, int byte, size_t bytes);
 // Status word of the no-alloc entry point's static array on the current device (0 when that
 // entry has not been used on it); reads and clears it without allocating anything.
 int noalloc_read_status(int* status_out);
