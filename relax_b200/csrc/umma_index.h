@@ -14,7 +14,7 @@ namespace us {
 // its blocks of every chunk of four, and the last chunk may hold two only: kb == k_blocks there, and the
 // scales belong to no block, so the row's last pair stands in (past it lies the next row, or nothing).
 // kb and k_blocks are even.
-RB200_HD int pair_in_row(int kb, int k_blocks) { return kb < k_blocks ? kb : k_blocks - 2; }
+RB200_HD int pair_in_row(int kb, int k_blocks) { return kb < k_blocks - 2 ? kb : k_blocks - 2; }
 
 }  // namespace us
 }  // namespace rb200
