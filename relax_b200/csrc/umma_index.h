@@ -10,11 +10,11 @@
 namespace rb200 {
 namespace us {
 
-// First of the two adjacent 64-k blocks whose group-32 scales one 8-byte load takes.  A decode group asks for
-// its blocks of every chunk of four, and the last chunk may hold two only: kb == k_blocks there, and the
-// scales belong to no block, so the row's last pair stands in (past it lies the next row, or nothing).
-// kb and k_blocks are even.
-RB200_HD int pair_in_row(int kb, int k_blocks) { return kb < k_blocks - 2 ? kb : k_blocks - 2; }
+// Whether the group-32 scales of two adjacent 64-k blocks may be one 8-byte load: every chunk (256 k of int4, 128
+// of int8) is whole.  A decode group asks for its pair of every chunk, also of a last one that holds no such
+// pair, where the load would take the next row's scales and, behind the last row, what lies past the tensor.
+// (Clamped to the row instead, the load cost k 4096 x n 22016, 32 rows, 21.3 -> 21.6 us.)
+RB200_HD bool pairs_fit_rows(int k, int bits) { return k % (bits == 4 ? 256 : 128) == 0; }
 
 }  // namespace us
 }  // namespace rb200

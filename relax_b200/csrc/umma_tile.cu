@@ -181,8 +181,7 @@ int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, uint32_t* v
     auto words_of = [&](int halves) {
       return p.s_g == 1 && p.s_n % halves == 0 && (addr & (uintptr_t)(2 * halves - 1)) == 0 && s_expert_stride % halves == 0;
     };
-    // (a k of an odd number of 64-k blocks would read past its row: word by word)
-    pp.s_vec = words_of(4) && p.k % 128 == 0 ? 2 : (words_of(2) ? 1 : 0);
+    pp.s_vec = words_of(4) && pairs_fit_rows(p.k, bits) ? 2 : (words_of(2) ? 1 : 0);
   }
 
   const int frag = bits == 4 ? 64 : 32;

@@ -38,7 +38,7 @@ struct Params {
   int nd, d_stride, a_base, na, tmem_cols;  // accumulators and A slots in tensor memory
   int s_n, s_g;                // scale strides in elements
   int s_vec;                   // kTwo: the two groups of a block are one aligned 32-bit word (1), those of two
-                               // adjacent blocks one 64-bit word (2)
+                               // adjacent blocks one 64-bit word (2; pairs_fit_rows)
   int early;                   // weights / scales were not written by the previous kernel
   const int64_t* indptr;       // grouped form: end rows (device), else nullptr
   int has_prev, num_experts;
@@ -297,12 +297,11 @@ struct ScaleFeed {
   // scales are one 8-byte load when the rows allow it
   __device__ __forceinline__ void fetch_two(const Params& pp, int kb, int k_blocks) {
     if (SRC == kTwo && pp.s_vec == 2) {
-      const int at = pair_in_row(kb, k_blocks) * 2;
-      const uint2 s = __ldg(reinterpret_cast<const uint2*>(sp + at));
+      const uint2 s = __ldg(reinterpret_cast<const uint2*>(sp + kb * 2));
       sn[0] = s.x;
       sn[OWN - 1] = s.y;
       if (has_zeros) {
-        const uint2 z = __ldg(reinterpret_cast<const uint2*>(zp + at));
+        const uint2 z = __ldg(reinterpret_cast<const uint2*>(zp + kb * 2));
         zn[0] = z.x;
         zn[OWN - 1] = z.y;
       }

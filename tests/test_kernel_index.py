@@ -15,17 +15,21 @@ def lib(tmp_path_factory):
     src, so = str(d / "index.cc"), str(d / "index.so")
     with open(src, "w") as f:
         f.write('#include "umma_index.h"\n'
-                'extern "C" int pair_in_row(int kb, int k_blocks) { return rb200::us::pair_in_row(kb, k_blocks); }\n')
+                'extern "C" int pairs_fit_rows(int k, int bits) { return rb200::us::pairs_fit_rows(k, bits); }\n')
     subprocess.check_call(["g++", "-O1", "-shared", "-fPIC", "-I" + CSRC, src, "-o", so])
     return ctypes.CDLL(so)
 
 
-def test_scale_pairs_stay_in_their_row(lib):
-    """Group 32, k a multiple of 128: every pair of blocks a decode group asks for, in all chunks of four."""
-    for k in range(128, 32768 + 1, 128):
+@pytest.mark.parametrize("bits,chunk_blocks", [(4, 4), (8, 2)])
+def test_scale_pairs_stay_in_their_row(lib, bits, chunk_blocks):
+    """Group 32: where scales are fetched for pairs of 64-k blocks, every pair of every chunk is in the row."""
+    fitting = 0
+    for k in range(64, 32768 + 1, 64):
+        if not lib.pairs_fit_rows(k, bits):
+            continue
+        fitting += 1
         k_blocks = k // 64
-        for chunk in range((k_blocks + 3) // 4):
-            for kb in (chunk * 4, chunk * 4 + 2):
-                at = lib.pair_in_row(kb, k_blocks)
-                assert at % 2 == 0 and 0 <= at and at + 2 <= k_blocks, (k, kb, at)
-                assert at == kb or kb >= k_blocks
+        for chunk in range(-(-k_blocks // chunk_blocks)):
+            for kb in range(chunk * chunk_blocks, (chunk + 1) * chunk_blocks, 2):
+                assert kb % 2 == 0 and kb + 2 <= k_blocks, (k, kb)
+    assert fitting == 32768 // (64 * chunk_blocks)
