@@ -14,6 +14,7 @@
 #include "gemv_rk.cuh"
 #include "gemv_sk.cuh"
 #include "gemm_tc.h"
+#include "handover.h"
 #include "preprocess.h"
 
 namespace rb200 {
@@ -99,8 +100,7 @@ DeviceScratch* device_scratch(size_t min_partial_bytes, size_t min_counter_ints)
   if (counters < min_counter_ints) counters = min_counter_ints;
   const size_t header = 256;
   const size_t counter_bytes = ((counters * sizeof(int) + 255) / 256) * 256;
-  const size_t vacant = (size_t)s.sm_count * 128 * 256 * sizeof(float);  // one 128 x 256 fp32 tile per SM
-  s.bytes = header + counter_bytes + partial + vacant;
+  s.bytes = header + counter_bytes + partial;
   cudaError_t e = cudaMalloc(&s.base, s.bytes);
   if (e != cudaSuccess) {
     set_last_error("cudaMalloc(%zu) for library scratch failed: %s", s.bytes, cudaGetErrorString(e));
@@ -112,9 +112,7 @@ DeviceScratch* device_scratch(size_t min_partial_bytes, size_t min_counter_ints)
   s.counter_ints = counters;
   s.partials = reinterpret_cast<float*>(static_cast<uint8_t*>(s.base) + header + counter_bytes);
   s.partial_bytes = partial;
-  s.vacant_words = reinterpret_cast<uint32_t*>(reinterpret_cast<uint8_t*>(s.partials) + partial);
-  s.vacant_bytes = vacant;
-  if (fill_now(s.base, 0, header + counter_bytes) != 0 || fill_now(s.vacant_words, 0xff, vacant) != 0) {
+  if (fill_now(s.base, 0, header + counter_bytes) != 0) {
     cudaFree(s.base);
     s.base = nullptr;
     return nullptr;
@@ -275,8 +273,10 @@ int rb200_check_async_error(void* stream, int* status_out) {
     RB200_CUDA(cudaMemcpy(&v, sc->status, sizeof(int), cudaMemcpyDeviceToHost));
     if (v != 0) {
       // a wait that gave up may have left split-k flags and tickets behind: back to rest
+      // (which launch it was the status does not say: all of them have ended before anything is reset)
+      RB200_CUDA(cudaDeviceSynchronize());
       if (fill_now(sc->base, 0, (size_t)(reinterpret_cast<uint8_t*>(sc->partials) - static_cast<uint8_t*>(sc->base))) != 0 ||
-          fill_now(sc->vacant_words, 0xff, sc->vacant_bytes) != 0)
+          handover_reset() != 0)
         return -1;
       st = v;
     }
@@ -450,16 +450,14 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
     // rows: k 4096 x n 12288 17.9 / 15.0 us, k 11008 x n 6144 27.1 / 19.6; below, k 4096 x n 8192 11.1 / 11.8).
     if (p.m > 8 && p.m <= rk::kMaxBatch && !ar && p.group == 32 && zero_mode(d) == kZeroGeneral && d->weight_bits == 4 &&
         (int64_t)p.n * p.k >= (48ll << 20)) {
-      const int rc = umma_run(p, d->weight_bits, zero_mode(d), sc->sm_count, sc->vacant_words, sc->vacant_bytes, nullptr,
-                              0, 1, 0, 0, stream);
+      const int rc = umma_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
       if (rc <= 0) return rc;
     }
     if (p.m <= rk::kMaxBatch && !ar)
       return gemv_rk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
     unsigned* flags = reinterpret_cast<unsigned*>(sc->counters) + kSkFlagOffset;
     if (!ar) {
-      const int rc = umma_run(p, d->weight_bits, zero_mode(d), sc->sm_count, sc->vacant_words, sc->vacant_bytes, nullptr,
-                                 0, 1, 0, 0, stream);
+      const int rc = umma_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
       if (rc <= 0) return rc;
     }
     if (p.k % 64 == 0) {
@@ -657,9 +655,8 @@ int rb200_group_gemm(const rb200_group_gemm_desc* d, void* stream_v) {
                        w_expert_bytes, d->scale_stride_e, static_cast<cudaStream_t>(stream_v));
   }
   if (packed)
-    return umma_run(p, d->weight_bits, zmode, sc->sm_count, sc->vacant_words, sc->vacant_bytes, d->indptr,
-                       d->indptr_has_prev ? 1 : 0, (int)d->num_experts, w_expert_bytes, d->scale_stride_e,
-                       static_cast<cudaStream_t>(stream_v));
+    return umma_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0, (int)d->num_experts,
+                    w_expert_bytes, d->scale_stride_e, static_cast<cudaStream_t>(stream_v));
   return umma_group_gemm_run(p, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0, (int)d->num_experts, w_expert_bytes,
                              static_cast<cudaStream_t>(stream_v));
 }

@@ -45,8 +45,6 @@ struct DeviceScratch {
   size_t counter_ints = 0;
   float* partials = nullptr;
   size_t partial_bytes = 0;
-  uint32_t* vacant_words = nullptr;  // hand-over words of the medium-batch kernel, all bits set at rest
-  size_t vacant_bytes = 0;
   int sm_count = 0;
 };
 // Returns the current device's scratch, allocating it on first use (never inside a capture:

@@ -33,7 +33,7 @@ int gemm_tc_launch(const rb200_gemm_desc* d, const Epilogue& epi, int group, int
     p.k = (int)d->k;
     p.group = group;
     p.zero_const = d->zero_const;
-    const int rc = umma_run(p, d->weight_bits, zmode, sc->sm_count, sc->vacant_words, sc->vacant_bytes, nullptr, 0, 1, 0, 0, stream);
+    const int rc = umma_run(p, d->weight_bits, zmode, sc->sm_count, nullptr, 0, 1, 0, 0, stream);
     if (rc <= 0) return rc;
   }
   rb200_gemm_desc s = *d;

@@ -198,7 +198,8 @@ __global__ void __launch_bounds__(kThreads, 1)
   const unsigned items = grouped ? (unsigned)tt.base[pp.num_experts] : (unsigned)(n_tiles * pp.m_tiles);
   // the first `split` items are shared out in equal runs of chunks, the others in whole waves
   const unsigned waves = items / pairs, rem = items - waves * pairs;
-  const unsigned split = rem == 0 ? 0u : (waves >= 1 ? pairs + rem : rem);
+  // (none of them where there are no words to hand over a part of a tile)
+  const unsigned split = rem == 0 || !pp.partial ? 0u : (waves >= 1 ? pairs + rem : rem);
   const unsigned total = split * (unsigned)cpt;
   const unsigned takers = min(pairs, total);  // pairs with a run
   const unsigned u_begin = pair < takers ? (unsigned)((unsigned long long)pair * total / takers) : 0u;

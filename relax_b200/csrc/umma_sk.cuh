@@ -153,10 +153,12 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   const int NB = p.n / 16, KT = p.k / kFragK, cpt = pp.cpt;
   const unsigned items = grouped ? (unsigned)tt.base[pp.num_experts] : (unsigned)(n_tiles * pp.m_tiles);
   const unsigned total = items * (unsigned)cpt;  // total * grid fits 31 bits (checked by the host)
+  // what the cuts fall between: chunks, or tiles where there are no words to hand over a part of one
+  const unsigned step = pp.partial ? 1u : (unsigned)cpt, units = pp.partial ? total : items;
   // (experts without rows can leave fewer units than CTAs: the surplus CTAs stay out of the split)
-  const unsigned ctas = min(gridDim.x, total);
-  const unsigned u_begin = blockIdx.x < ctas ? blockIdx.x * total / ctas : 0u;
-  const unsigned u_end = blockIdx.x < ctas ? (blockIdx.x + 1) * total / ctas : 0u;
+  const unsigned ctas = min(gridDim.x, units);
+  const unsigned u_begin = blockIdx.x < ctas ? blockIdx.x * units / ctas * step : 0u;
+  const unsigned u_end = blockIdx.x < ctas ? (blockIdx.x + 1) * units / ctas * step : 0u;
 
   auto get_item = [&](int item) {
     Item it;

@@ -6,6 +6,7 @@
 #include <cmath>
 #include <cstring>
 
+#include "handover.h"
 #include "tensormap.h"
 
 namespace rb200 {
@@ -43,7 +44,7 @@ int pair_m_tiles(long long n_tiles, int m, int k_blocks, int pairs) {
   return best;
 }
 
-int run_pair(Params& pp, int bits, int zmode, int src, int sm_count, size_t vacant_bytes, cudaStream_t stream) {
+int run_pair(Params& pp, int bits, int zmode, int src, int sm_count, cudaStream_t stream) {
   const GemvParams& p = pp.g;
   const long long n_tiles = (p.n + 2 * kTileRows - 1) / (2 * kTileRows);
   if (!pp.indptr) {
@@ -74,7 +75,7 @@ int run_pair(Params& pp, int bits, int zmode, int src, int sm_count, size_t vaca
   const long long items = pp.indptr ? n_tiles * ((long long)p.m / pp.nb + pp.num_experts) : n_tiles * pp.m_tiles;
   RB200_CHECK(items < (1ll << 30), "too many tiles (n=%d, m=%d)", p.n, p.m);
   l.most_pairs = items * pp.cpt;
-  RB200_CHECK((size_t)sm_count * pp.nb * kTileRows * sizeof(float) <= vacant_bytes, "split-k scratch too small for %d SMs", sm_count);
+  pp.partial = handover_words(stream, sm_count, (size_t)sm_count * pp.nb * kTileRows * sizeof(float));
   CUtensorMap tx;  // x as [64-k block][row][64 k]
   {
     const unsigned long long dims[3] = {64ull, (unsigned long long)p.m, (unsigned long long)(p.k / 64)};
@@ -86,7 +87,7 @@ int run_pair(Params& pp, int bits, int zmode, int src, int sm_count, size_t vaca
   return bits == 4 ? up::launch_i4(pp, l, tx, stream) : up::launch_i8(pp, l, tx, stream);
 }
 
-int run_single(Params& pp, int bits, int zmode, int src, int sm_count, size_t vacant_bytes, cudaStream_t stream) {
+int run_single(Params& pp, int bits, int zmode, int src, int sm_count, cudaStream_t stream) {
   const GemvParams& p = pp.g;
   if (!pp.indptr) {
     pp.m_tiles = (p.m + kSmallNb - 1) / kSmallNb;
@@ -133,17 +134,17 @@ int run_single(Params& pp, int bits, int zmode, int src, int sm_count, size_t va
   }
   if (grid > units) grid = units;
   RB200_CHECK(units * grid < (1ll << 31), "problem too large for the 32-bit work split (n=%d, k=%d, m=%d)", p.n, p.k, p.m);
+  // (one CTA per tile cuts none)
+  if (pp.indptr || grid != items) pp.partial = handover_words(stream, sm_count, (size_t)grid * pp.nb * kTileRows * sizeof(float));
   l.grid = (int)grid;
-  RB200_CHECK((size_t)grid * pp.nb * kTileRows * sizeof(float) <= vacant_bytes, "split-k scratch too small for a grid of %d", l.grid);
   CUtensorMap tx;
   if (x_map(&tx, p, pp.nb) != 0) return -1;
   return bits == 4 ? launch_i4(pp, l, tx, stream) : launch_i8(pp, l, tx, stream);
 }
 }  // namespace
 
-int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, uint32_t* vacant_words, size_t vacant_bytes,
-             const int64_t* indptr, int has_prev, int num_experts, int64_t w_expert_bytes,
-             int64_t s_expert_stride, cudaStream_t stream) {
+int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, const int64_t* indptr, int has_prev, int num_experts,
+             int64_t w_expert_bytes, int64_t s_expert_stride, cudaStream_t stream) {
   const bool grouped = indptr != nullptr;
   const int64_t per_expert_scales = p.group > 0 ? (int64_t)p.n * p.s_n + (int64_t)(p.k / p.group) * p.s_g : (int64_t)p.n * p.s_n;
   const bool covered = p.n % 16 == 0 && p.k % kKBlock == 0 && (reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && p.ldx % 8 == 0 &&
@@ -168,7 +169,6 @@ int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, uint32_t* v
   pp.early = launch_overlap_enabled() ? 1 : 0;
   pp.wait_limit_ms = wait_limit_ms();
 
-  pp.partial = vacant_words;
   const int lane_run = bits == 4 ? 16 : 8;
   int src;
   if (p.group <= 0 || p.group >= p.k) {
@@ -196,8 +196,7 @@ int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, uint32_t* v
     pp.m_tiles = 1;
   }
   const bool single = (grouped ? pp.nb : p.m) <= kSmallNb;
-  return single ? run_single(pp, bits, zmode, src, sm_count, vacant_bytes, stream)
-                : run_pair(pp, bits, zmode, src, sm_count, vacant_bytes, stream);
+  return single ? run_single(pp, bits, zmode, src, sm_count, stream) : run_pair(pp, bits, zmode, src, sm_count, stream);
 }
 
 }  // namespace rb200

@@ -43,7 +43,7 @@ struct Params {
   const int64_t* indptr;       // grouped form: end rows (device), else nullptr
   int has_prev, num_experts;
   int64_t w_expert_bytes, s_expert_stride;
-  uint32_t* partial;           // [grid][nb / 4][128][4] fp32 words, kVacant at rest
+  uint32_t* partial;           // [grid][nb / 4][128][4] fp32 words, kVacant at rest; nullptr: no tile is cut
   unsigned wait_limit_ms;
 };
 
@@ -441,8 +441,7 @@ __device__ __forceinline__ bool drain_store(const Params& pp, const DrainTile& t
 // Host entry of the tensor-core kernels over packed weights: 1 when the problem is outside their coverage
 // (ungrouped only), 0 on launch, -1 on error.  Grouped (indptr != nullptr): p.m = total rows; shapes
 // outside the coverage are errors.
-int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, uint32_t* vacant_words, size_t vacant_bytes,
-             const int64_t* indptr, int has_prev, int num_experts, int64_t w_expert_bytes, int64_t s_expert_stride,
-             cudaStream_t stream);
+int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, const int64_t* indptr, int has_prev, int num_experts,
+             int64_t w_expert_bytes, int64_t s_expert_stride, cudaStream_t stream);
 
 }  // namespace rb200
