@@ -166,7 +166,8 @@ int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, const int64
   pp.s_expert_stride = s_expert_stride;
   pp.s_n = (int)p.s_n;
   pp.s_g = (int)p.s_g;
-  pp.early = launch_overlap_enabled() ? 1 : 0;
+  // (what the switch promises about weights it promises for decode batches only)
+  pp.early = launch_overlap_enabled() && !grouped && p.m <= 32 ? 1 : 0;
   pp.wait_limit_ms = wait_limit_ms();
 
   const int lane_run = bits == 4 ? 16 : 8;

@@ -93,3 +93,32 @@ def test_buffers_written_while_a_later_launch_is_resident(m, overlap):
         assert torch.equal(bufs[0], ref[-1]) and torch.equal(bufs[1], ref[-2])
     finally:
         relax_b200.set_launch_overlap(before)
+
+
+@pytest.mark.parametrize("m", [48, 160])
+def test_prefill_reads_weights_written_just_before(m):
+    """With overlap on, a batch above 32 rows is still ordered behind the kernel that writes its weights."""
+    g = np.random.Generator(np.random.PCG64(m))
+    k, n = 4096, 4096
+    cases = [synth.q4_case(g, 1, k, n, 32) for _ in range(2)]
+    src = [u32_to_dev(c.w) for c in cases]
+    scales = [to_dev(c.scales) for c in cases]
+    x = to_dev(g.standard_normal((m, k), dtype=np.float32).astype(np.float16))
+    ref = [ops.gemm_fp16_q4f16(x, ops.preprocess_weight_q4f16(w), s).clone() for w, s in zip(src, scales)]
+    sc = torch.empty_like(scales[0])
+    outs = [torch.empty_like(r) for r in ref]
+    torch.cuda.synchronize()
+    relax_b200.set_launch_overlap(True)
+    try:
+        for rep in range(20):
+            for i in (0, 1):
+                sc.copy_(scales[i])
+                pre = ops.preprocess_weight_q4f16(src[i])  # the block the call before last gave back
+                ops.gemm_fp16_q4f16(x, pre, sc, out=outs[i])
+                del pre
+        torch.cuda.synchronize()
+        _check_status()
+    finally:
+        relax_b200.set_launch_overlap(False)
+    for o, r in zip(outs, ref):
+        assert torch.equal(o, r)
