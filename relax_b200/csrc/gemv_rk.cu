@@ -12,7 +12,6 @@ int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const in
   RB200_CHECK((reinterpret_cast<uintptr_t>(p.x) & 15u) == 0 && p.ldx % 8 == 0,
               "x must be 16-byte aligned with a row pitch that is a multiple of 8 elements");
   RB200_CHECK(p.m >= 1 && p.m <= (indptr ? 32 : kMaxBatch), "small-batch kernel: m=%d out of range", p.m);
-  RB200_CHECK(num_experts <= 64, "num_experts=%d above 64", num_experts);
   Params pp;
   memset(&pp, 0, sizeof(pp));
   pp.g = p;
@@ -48,7 +47,9 @@ int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const in
   const int warps = blocks >= (long long)sm_count * 12 ? 4 : 8;
   long long grid = (long long)sm_count * (16 / warps);
   if (grid > blocks) grid = blocks;
-  RB200_CHECK(blocks * grid < (1ll << 31), "too many row blocks for the small-batch kernel (n=%d)", p.n);
+  // the kernel numbers row blocks entry by entry: an expert may have several, and most have none
+  const long long numbered = indptr ? (long long)(p.n / 16) * kMaxEntries : blocks;
+  RB200_CHECK(numbered * grid < (1ll << 32), "too many row blocks for the small-batch kernel (n=%d)", p.n);
   pp.per_cta = (unsigned)(blocks / grid);
   pp.extra = (unsigned)(blocks % grid);
   return bits == 4 ? launch_i4(pp, zmode, src, warps, (int)grid, stream) : launch_i8(pp, zmode, src, warps, (int)grid, stream);

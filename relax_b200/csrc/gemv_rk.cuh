@@ -39,7 +39,7 @@ constexpr int kRows = 2;         // row blocks of one pass: activations fetched 
 constexpr int kMaxBatch = 16;   // two m-tiles of eight rows
 constexpr int kEntryRows = 8;   // grouped form: batch rows of one entry
 constexpr int kLeadChunks = 2;   // chunks between an L2 prefetch and the load
-constexpr int kMaxEntries = 96;  // grouped form: (expert, eight batch rows) pairs; 64 experts, 32 rows in all
+constexpr int kMaxEntries = 32;  // grouped form: (expert, eight batch rows) pairs that 32 rows in all can make
 
 // where a lane gets its scales / zero points from
 enum ScaleSrc : int {

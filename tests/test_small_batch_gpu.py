@@ -59,6 +59,22 @@ def test_experts(oracle, rows, bits, k, n):
         assert_close(got[:total], C.epilogue(C.group_gemm_f32(x[:total], np.ascontiguousarray(wq), indptr)))
 
 
+@pytest.mark.parametrize("experts,rows", [(128, 32), (160, 9), (65, 1)])
+def test_many_experts(oracle, experts, rows):
+    """More experts than rows by far: their number is not limited where the rows are few."""
+    rs = np.random.RandomState(experts + rows)
+    k, n = 128, 48
+    x = rs.randn(rows, k).astype(np.float16)
+    w = rs.randint(-128, 128, size=(experts, k, n // 2)).astype(np.int8)
+    s = rs.uniform(0.001, 0.01, size=(experts, k // 64, n)).astype(np.float16)
+    indptr = np.cumsum(np.bincount(rs.randint(0, experts, size=rows), minlength=experts)).astype(np.int64)
+    out = ops.moe_gemm_ft(to_dev(x), ops.preprocess_weight_ft(to_dev(w), True), to_dev(s), torch.from_numpy(indptr).cuda())
+    _check_status()
+    C = oracle.C()
+    wq = np.stack([C.decode_ft_kn(w[e], s[e], 4, 64).T for e in range(experts)])
+    assert_close(out.cpu().numpy(), C.epilogue(C.group_gemm_f32(x, np.ascontiguousarray(wq), indptr)))
+
+
 def _forms():
     yield "ft4_row", 4, -1, None
     yield "ft8_row", 8, -1, None
