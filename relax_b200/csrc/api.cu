@@ -443,7 +443,8 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
     // Which kernel: up to 16 rows (two MMAs wide) the small-batch kernel (one row, against the stream-k
     // kernel: k = n = 4096 3.9 / 8.1 us, n 22016 13.9 / 19.1, k 11008 x n 4096 8.0 / 13.4); above that the
     // tensor-core kernels.  What they do not cover - the fused all-reduce, x or out without 16-byte rows -
-    // runs on the stream-k kernel, and int8 with k a multiple of 32 only on the cluster kernel, whose
+    // runs on the stream-k kernel (small batches whose strides need more than 31 bits on the tensor-core kernels
+    // too), and int8 with k a multiple of 32 only on the cluster kernel, whose
     // split-k partials meet in distributed shared memory.
     // One exception: zero points per group of 32 at nine to sixteen rows spill there (two m-tiles beside
     // four words of scales and zero points), and from 48 Mi weights on the tensor-core kernel is ahead (16
@@ -453,8 +454,10 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
       const int rc = umma_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
       if (rc <= 0) return rc;
     }
-    if (p.m <= rk::kMaxBatch && !ar)
-      return gemv_rk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
+    if (p.m <= rk::kMaxBatch && !ar) {
+      const int rc = gemv_rk_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
+      if (rc <= 0) return rc;
+    }
     unsigned* flags = reinterpret_cast<unsigned*>(sc->counters) + kSkFlagOffset;
     if (!ar) {
       const int rc = umma_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);
@@ -651,8 +654,9 @@ int rb200_group_gemm(const rb200_group_gemm_desc* d, void* stream_v) {
   if (packed && d->total_rows <= 32 && d->k % 64 == 0 && d->n % 16 == 0 && aligned16(d->x) && aligned16(d->out)) {
     // Decode-size batch: one launch of the small-batch kernel streams the weights of every expert
     // that has rows (eight experts of k 4096 x n 14336, 16 rows: 75 us; one launch per expert 150 us).
-    return gemv_rk_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0, (int)d->num_experts,
-                       w_expert_bytes, d->scale_stride_e, static_cast<cudaStream_t>(stream_v));
+    const int rc = gemv_rk_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0,
+                               (int)d->num_experts, w_expert_bytes, d->scale_stride_e, static_cast<cudaStream_t>(stream_v));
+    if (rc <= 0) return rc;
   }
   if (packed)
     return umma_run(p, d->weight_bits, zmode, sc->sm_count, d->indptr, d->indptr_has_prev ? 1 : 0, (int)d->num_experts,

@@ -35,9 +35,10 @@ int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const in
     // whole 16-byte runs of eight group scales per chunk of 256 k
     if (bits == 4 && p.group == 32 && p.s_g == 1 && p.s_n % 8 == 0 && p.k % 256 == 0 && (addr & 15u) == 0) src = kRow32;
   }
-  RB200_CHECK(p.s_n < (1ll << 31) && p.s_g < (1ll << 31) && (p.n + 16) * p.s_n + (p.k / frag) * 4 * p.s_g < (1ll << 31) &&
-                  p.ldx * p.m < (1ll << 31),
-              "strides too large for the small-batch kernel (n=%d, k=%d)", p.n, p.k);
+  // 32-bit offsets of scales and activations
+  if (p.s_n >= (1ll << 31) || p.s_g >= (1ll << 31) || (p.n + 16) * p.s_n + (p.k / frag) * 4 * p.s_g >= (1ll << 31) ||
+      p.ldx * p.m >= (1ll << 31))
+    return 1;
   pp.s_n = (int)p.s_n;
   pp.s_g = (int)p.s_g;
   const long long blocks = (long long)(p.n / 16) * (indptr ? num_experts : 1);

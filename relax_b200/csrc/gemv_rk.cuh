@@ -736,7 +736,8 @@ int launch_bits(const Params& pp, int zmode, int src, int warps, int grid, cudaS
 
 }  // namespace rk
 
-// Host entry.  Ungrouped: 1 <= p.m <= 16.  Grouped (indptr != nullptr): p.m = total rows, at most 32.
+// Host entry: 1 when offsets of scales or activations need more than 31 bits, 0 on launch, -1 on error.
+// Ungrouped: 1 <= p.m <= 16.  Grouped (indptr != nullptr): p.m = total rows, at most 32.
 int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const int64_t* indptr, int has_prev,
                 int num_experts, int64_t w_expert_bytes, int64_t s_expert_stride, cudaStream_t stream);
 

@@ -89,3 +89,24 @@ def test_unknown_op_codes_are_rejected(oracle):
         setattr(d, field, 11)
         assert lib.rb200_gemm_fp16_intx(ctypes.byref(d), None) == -1
         assert b"unknown" in lib.rb200_last_error()
+
+
+@pytest.mark.parametrize("m", [1, 12])
+def test_scale_strides_beyond_31_bits(oracle, m):
+    """A small batch whose scales are rows of a table of more than 2^31 elements."""
+    k, n, group, stride = 128, 32, 32, 1 << 26
+    case = synth.q4_case(np.random.Generator(np.random.PCG64(m)), m, k, n, group)
+    table = torch.empty(n * stride, dtype=torch.float16, device="cuda")
+    rows = table.as_strided((n, k // group), (stride, 1))
+    rows.copy_(to_dev(case.scales))
+    x, out = to_dev(case.x), torch.empty(m, n, dtype=torch.float16, device="cuda")
+    pre = ops.preprocess_weight_q4f16(u32_to_dev(case.w))
+    d = _lib.GemmDesc(struct_size=ctypes.sizeof(_lib.GemmDesc), weight_bits=4, x=x.data_ptr(), w=pre.data_ptr(),
+                      scales=rows.data_ptr(), out=out.data_ptr(), m=m, n=n, k=k, group_size=group, scale_stride_n=stride,
+                      scale_stride_g=1, zero_const=7.0)
+    torch.cuda.synchronize()
+    _lib.check(_lib.load().rb200_gemm_fp16_intx(ctypes.byref(d), None))
+    torch.cuda.synchronize()
+    _check_status()
+    C = oracle.C()
+    assert_close(out.cpu().numpy(), C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, None, 7.0, group))))
