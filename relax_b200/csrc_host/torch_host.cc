@@ -18,6 +18,7 @@
 #include <c10/cuda/CUDAFunctions.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
+#include <torch/csrc/Exceptions.h>
 #include <torch/csrc/autograd/python_variable.h>
 
 #include "../../include/relax_b200_packed.h"
@@ -226,13 +227,9 @@ struct Out {
     PyErr_Format(PyExc_TypeError, "%s expects %d arguments, got %zd", __func__, (N), nargs);  \
     return nullptr;                                                                           \
   }
-#define GUARD_BEGIN try {
-#define GUARD_END                                          \
-  }                                                        \
-  catch (const std::exception& e) {                        \
-    PyErr_SetString(PyExc_RuntimeError, e.what());         \
-    return nullptr;                                        \
-  }
+// C++ exceptions become the Python ones that torch itself raises (torch.OutOfMemoryError among them)
+#define GUARD_BEGIN HANDLE_TH_ERRORS
+#define GUARD_END END_HANDLE_TH_ERRORS
 
 RB200FunctionHandle as_handle(PyObject* o) { return PyLong_AsVoidPtr(o); }
 
