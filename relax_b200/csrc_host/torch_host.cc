@@ -187,8 +187,16 @@ const at::Tensor* as_tensor(PyObject* o, const char* what) {
   }
   return &THPVariable_Unpack(o);
 }
+// what int() takes: a group size may come as the quotient k / groups
 bool as_int(PyObject* o, int64_t* out) {
-  *out = PyLong_AsLongLong(o);
+  if (!PyLong_Check(o)) {
+    PyObject* i = PyNumber_Long(o);
+    if (!i) return false;
+    *out = PyLong_AsLongLong(i);
+    Py_DECREF(i);
+  } else {
+    *out = PyLong_AsLongLong(o);
+  }
   return !(*out == -1 && PyErr_Occurred());
 }
 bool as_real(PyObject* o, double* out) {

@@ -3,7 +3,21 @@ raise.  CPU tensors go as far as the library's own checks."""
 import pytest
 import torch
 
+import relax_b200
 from relax_b200 import ops
+
+
+@pytest.mark.parametrize("group", [32, 32.0, "32", torch.tensor(32)])
+def test_integer_arguments_take_what_int_takes(group):
+    x, w, s = torch.zeros(1, 64).half(), torch.zeros(16, 8, dtype=torch.int32), torch.zeros(16, 2).half()
+    with pytest.raises(relax_b200.RB200Error, match="CUDA device"):
+        ops.gemm_fp16_q4f16(x, w, s, group_size=group)
+
+
+def test_integer_arguments_refuse_the_rest():
+    x, w, s = torch.zeros(1, 64).half(), torch.zeros(16, 8, dtype=torch.int32), torch.zeros(16, 2).half()
+    with pytest.raises(TypeError):
+        ops.gemm_fp16_q4f16(x, w, s, group_size=[32])
 
 
 @pytest.mark.gpu
