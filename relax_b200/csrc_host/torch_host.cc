@@ -266,6 +266,16 @@ PyObject* call(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   GUARD_END
 }
 
+// check(*args): raises for what no global function takes
+PyObject* check(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
+  GUARD_BEGIN
+  Frame fr;
+  for (Py_ssize_t i = 0; i < nargs; ++i)
+    if (!fr.object(a[i])) return nullptr;
+  Py_RETURN_NONE;
+  GUARD_END
+}
+
 // call_like(handle, tensor, *args): destination-passing function whose result is a new tensor like the first
 PyObject* call_like(PyObject*, PyObject* const* a, Py_ssize_t nargs) {
   GUARD_BEGIN
@@ -597,7 +607,7 @@ PyObject* init(PyObject*, PyObject* args) {
 #define FAST(NAME) {#NAME, reinterpret_cast<PyCFunction>(reinterpret_cast<void (*)()>(NAME)), METH_FASTCALL, nullptr}
 PyMethodDef methods[] = {
     {"init", init, METH_VARARGS, nullptr},
-    FAST(call),      FAST(call_like), FAST(gemm_ft),    FAST(gemm_q4),    FAST(gemm_gptq),   FAST(gather_columns),
+    FAST(call),      FAST(check),     FAST(call_like), FAST(gemm_ft),    FAST(gemm_q4),    FAST(gemm_gptq),   FAST(gather_columns),
     FAST(moe_ft),    FAST(moe_q4),    FAST(group_fp16), FAST(moe_route),  FAST(moe_gather),  FAST(moe_combine),
     FAST(encode_ft), {nullptr, nullptr, 0, nullptr}};
 PyModuleDef module = {PyModuleDef_HEAD_INIT, "_torch_host", nullptr, -1, methods, nullptr, nullptr, nullptr, nullptr};

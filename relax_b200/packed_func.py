@@ -40,6 +40,7 @@ class PackedFunc:
 
     def bind(self, *args: Any) -> BoundCall:
         """The call with these tensors and scalars, to be repeated."""
+        native.check(*args)
         return BoundCall(self.handle, args)
 
     def __call__(self, *args: Any):

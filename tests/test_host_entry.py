@@ -20,6 +20,16 @@ def test_integer_arguments_refuse_the_rest():
         ops.gemm_fp16_q4f16(x, w, s, group_size=[32])
 
 
+def test_bind_refuses_what_a_call_refuses():
+    f = relax_b200.get_global_func("relax_b200.gather_columns")
+    x = torch.zeros(1, 64).half()
+    with pytest.raises(TypeError):
+        f.bind(x, [0], x)
+    with pytest.raises(KeyError):
+        f.bind(x, torch.zeros(64, dtype=torch.complex64), x)
+    f.bind(x, None, x)
+
+
 @pytest.mark.gpu
 def test_out_of_memory():
     x = torch.empty(1, 64, dtype=torch.float16, device="cuda").expand(1 << 30, 64)
