@@ -12,6 +12,7 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <ATen/Context.h>
 #include <ATen/cuda/EmptyTensor.h>
 #include <ATen/ops/empty.h>
 #include <ATen/ops/empty_like.h>
@@ -78,8 +79,8 @@ bool any_device() {
   return have;
 }
 
-// The library's stream on this thread becomes torch's current stream of the device the tensors are
-// on, and that device current, for the lifetime of the object.
+// The library's stream on this thread becomes torch's current stream of the device the tensors are on (and
+// stays it until the next call), and that device current for the lifetime of the object.
 struct OnStream {
   c10::cuda::OptionalCUDAGuard guard;
   explicit OnStream(int device) {
@@ -205,7 +206,9 @@ bool as_real(PyObject* o, double* out) {
 }
 
 at::Tensor empty_on(c10::IntArrayRef sizes, c10::ScalarType dtype, const at::Tensor& like) {
-  if (like.is_cuda()) return at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt);
+  // (under deterministic algorithms torch.empty may fill its result: rows of no expert are then NaN)
+  if (like.is_cuda() && !at::globalContext().deterministicAlgorithms())
+    return at::detail::empty_cuda(sizes, dtype, like.device(), std::nullopt);
   return at::empty(sizes, at::TensorOptions().dtype(dtype).device(like.device()));
 }
 // x's leading extents followed by n

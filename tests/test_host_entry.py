@@ -37,3 +37,18 @@ def test_out_of_memory():
     with pytest.raises(torch.OutOfMemoryError):
         ops.gemm_fp16_q4f16(x, w, None)
     torch.empty(16, device="cuda")
+
+
+@pytest.mark.gpu
+def test_results_are_filled_under_deterministic_algorithms():
+    """Rows of no expert are left as torch.empty made them, which is NaN under deterministic algorithms."""
+    w = ops.preprocess_weight_ft(torch.zeros(2, 64, 16, dtype=torch.int8, device="cuda"), False)
+    x, s = torch.zeros(40, 64, device="cuda").half(), torch.ones(2, 16, device="cuda").half()
+    indptr = torch.tensor([3, 5], device="cuda")
+    torch.use_deterministic_algorithms(True)
+    try:
+        for rows in (20, 40):
+            out = ops.moe_gemm_ft(x[:rows], w, s, indptr)
+            assert torch.isfinite(out[:5]).all() and torch.isnan(out[5:]).all()
+    finally:
+        torch.use_deterministic_algorithms(False)
