@@ -18,6 +18,7 @@ _OBJ = os.path.join(_PKG, "build")
 LIB_PATH = os.path.join(_PKG, "librelax_b200.so")
 _HOST_SRC = os.path.join(_PKG, "csrc_host", "torch_host.cc")
 HOST_PATH = os.path.join(_PKG, "_torch_host.so")
+_HOST_ABI = os.path.join(_OBJ, "torch_host.abi")  # what HOST_PATH was built for
 
 NVCC_FLAGS = [
     "-gencode", "arch=compute_100a,code=sm_100a", "-lineinfo", "-O3", "-std=c++17",
@@ -48,10 +49,25 @@ def _stale(src: str, obj: str, headers_mtime: float) -> bool:
     return os.path.getmtime(src) > t or headers_mtime > t
 
 
+def host_abi() -> str:
+    """What a binary of the host module depends on beside its sources."""
+    import sysconfig
+
+    import torch
+    return "torch %s, %s, C++11 ABI %d" % (torch.__version__, sysconfig.get_config_var("SOABI"),
+                                           int(torch._C._GLIBCXX_USE_CXX11_ABI))
+
+
 def build_host(force: bool = False) -> str:
-    """The Python entry points in native code (``_torch_host.so``), against the installed torch."""
+    """The Python entry points in native code (``_torch_host.so``), against the installed torch: rebuilt when
+    a source is newer, and for another torch or Python than it was built with."""
     headers = glob.glob(os.path.join(_PKG, "..", "include", "*.h"))
-    if not force and not _stale(_HOST_SRC, HOST_PATH, max([os.path.getmtime(h) for h in headers] + [0.0])):
+    built_for = None
+    if os.path.exists(_HOST_ABI):
+        with open(_HOST_ABI) as f:
+            built_for = f.read()
+    if not force and built_for == host_abi() and \
+            not _stale(_HOST_SRC, HOST_PATH, max([os.path.getmtime(h) for h in headers] + [0.0])):
         return HOST_PATH
     import sysconfig
 
@@ -60,7 +76,8 @@ def build_host(force: bool = False) -> str:
     cuda = os.path.dirname(os.path.dirname(_nvcc()))
     cxx = "/usr/bin/g++" if os.path.exists("/usr/bin/g++") else "g++"
     cmd = [cxx, "-O2", "-std=c++17", "-fPIC", "-shared", "-fvisibility=hidden",
-           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI)]
+           "-D_GLIBCXX_USE_CXX11_ABI=%d" % int(torch._C._GLIBCXX_USE_CXX11_ABI),
+           '-DRB200_BUILT_FOR="%s"' % host_abi()]
     for inc in (os.path.join(base, "include"), os.path.join(base, "include", "torch", "csrc", "api", "include"),
                 os.path.join(cuda, "include"), sysconfig.get_paths()["include"]):
         cmd.append("-I" + inc)
@@ -69,6 +86,9 @@ def build_host(force: bool = False) -> str:
     r = subprocess.run(cmd, capture_output=True, text=True)
     if r.returncode != 0:
         raise RuntimeError("host module: %s\n%s\n%s" % (" ".join(cmd), r.stdout, r.stderr))
+    os.makedirs(_OBJ, exist_ok=True)
+    with open(_HOST_ABI, "w") as f:
+        f.write(host_abi())
     return HOST_PATH
 
 

@@ -617,4 +617,8 @@ PyModuleDef module = {PyModuleDef_HEAD_INIT, "_torch_host", nullptr, -1, methods
 
 }  // namespace
 
-PyMODINIT_FUNC PyInit__torch_host(void) { return PyModule_Create(&module); }
+PyMODINIT_FUNC PyInit__torch_host(void) {
+  PyObject* m = PyModule_Create(&module);
+  if (m && PyModule_AddStringConstant(m, "built_for", RB200_BUILT_FOR) != 0) Py_CLEAR(m);
+  return m;
+}

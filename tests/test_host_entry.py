@@ -30,6 +30,27 @@ def test_bind_refuses_what_a_call_refuses():
     f.bind(x, None, x)
 
 
+def test_host_module_is_rebuilt_for_another_torch(tmp_path, monkeypatch):
+    from relax_b200 import _host, build
+    abi, commands = tmp_path / "torch_host.abi", []
+
+    def run(cmd, **kw):
+        commands.append(cmd)
+        return type("Result", (), {"returncode": 0})()
+
+    monkeypatch.setattr(build, "_HOST_ABI", str(abi))
+    monkeypatch.setattr(build.subprocess, "run", run)
+    abi.write_text(build.host_abi())
+    build.build_host()
+    assert not commands
+    abi.write_text(build.host_abi().replace("torch ", "torch 1"))
+    build.build_host()
+    assert len(commands) == 1 and abi.read_text() == build.host_abi()
+    _host.check_abi(_host.native.built_for, build.host_abi())
+    with pytest.raises(RuntimeError, match="rebuild"):
+        _host.check_abi("torch 1.0", build.host_abi())
+
+
 @pytest.mark.gpu
 def test_out_of_memory():
     x = torch.empty(1, 64, dtype=torch.float16, device="cuda").expand(1 << 30, 64)
