@@ -93,8 +93,6 @@ DeviceScratch* device_scratch(size_t min_partial_bytes, size_t min_counter_ints)
   s.sm_count = prop.multiProcessorCount;
   // generous defaults so ordinary use never grows: partials for 2 CTAs/SM at m <= 32
   size_t partial = (size_t)s.sm_count * 2 * 2 * 8 * 4 * 128 * sizeof(float);
-  // and for the split-k form of the prefill kernel: one 128 x 256 fp32 partial tile per SM
-  if (partial < (size_t)s.sm_count * 128 * 256 * sizeof(float)) partial = (size_t)s.sm_count * 128 * 256 * sizeof(float);
   if (partial < min_partial_bytes) partial = min_partial_bytes;
   size_t counters = 1u << 16;
   if (counters < min_counter_ints) counters = min_counter_ints;
@@ -442,7 +440,7 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
     p.zero_const = d->zero_const;
     // Which kernel: up to 16 rows (two MMAs wide) the small-batch kernel (one row, against the stream-k
     // kernel: k = n = 4096 3.9 / 8.1 us, n 22016 13.9 / 19.1, k 11008 x n 4096 8.0 / 13.4); above that the
-    // tensor-core kernels.  What they do not cover - the fused all-reduce, x or out without 16-byte rows -
+    // tensor-core kernels.  What they do not cover - the fused all-reduce, out without 16-byte rows -
     // runs on the stream-k kernel (small batches whose strides need more than 31 bits on the tensor-core kernels
     // too), and int8 with k a multiple of 32 only on the cluster kernel, whose
     // split-k partials meet in distributed shared memory.

@@ -1,5 +1,5 @@
 // m > 32: the tensor-core kernels over packed weights; what they do not cover (int8 with k not a multiple
-// of 64, x or out without 16-byte rows) runs as consecutive 32-row batch slices, each a full pass over the
+// of 64, out without 16-byte rows) runs as consecutive 32-row batch slices, each a full pass over the
 // packed weight.
 #include "gemm_tc.h"
 

@@ -13,7 +13,7 @@
 //   everything is handed over in steps of two 64-k blocks: with one block a step the barriers, commits and
 //   tensor-memory store waits of a step took longer than its MMAs (int8, m 256, k 8192 x n 57344: 191 us
 //   without any arithmetic, 118 us without arithmetic, stores and three of the four MMAs);
-//   accumulators: two of up to 192 columns, so that one drains while the next tile runs, or one of 256.
+//   accumulators: two of up to 128 columns, so that one drains while the next tile runs, or one of up to 256.
 //
 //   warp 0        packed weights, one 16 KB bulk copy per chunk (128 rows x 256 | 128 k)
 //   warp 1        MMA issue (rank 0)
