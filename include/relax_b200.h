@@ -41,7 +41,7 @@ RB200_API void* rb200_get_stream(void);
  * array of rb200_gemm_fp16_intx_noalloc.  Synchronises the given stream.  0 = no error recorded,
  * 1 = a wait ran out (the kernel skipped its remaining work and left outputs unwritten).
  * Allocates nothing: a status word that no call has created yet reads as 0.  After a non-zero
- * status the split-k flags and tickets of the scratch block are put back at rest.
+ * status it synchronises the device and puts the split-k flags, tickets and hand-over words back at rest.
  * Replaces nothing in the reference, whose kernels spin without a bound
  * (3rdparty/tensorrt_llm/custom_allreduce_kernels.cu:94-113) and whose collectives abort the
  * process on error (src/runtime/disco/nccl/nccl_context.h:50-56).
@@ -58,12 +58,14 @@ RB200_API int rb200_set_wait_limit_ms(unsigned limit_ms);
 
 /*
  * Launch overlap for serving loops (process-wide switch, default off; no counterpart in the
- * reference, whose generated host code launches every kernel fully stream-ordered).  When on,
- * the decode-path matmul kernels (m <= 32) are launched as programmatic dependents: a kernel may
- * become resident and start streaming its WEIGHT, SCALE and ZERO-POINT tensors while the previous
- * kernel on the stream is still finishing; it reads x / bias / residual and writes out / scratch
- * only after that kernel has completed, so activations stay ordered as before.
- * Contract when on: the weight, scale and zero-point tensors passed to a matmul call were not
+ * reference, whose generated host code launches every kernel fully stream-ordered).  Matmul kernels
+ * over packed weights are always programmatic dependents: a kernel may become resident while the
+ * previous kernel on the stream is still finishing, but until that has completed it only asks for
+ * weights to be brought into L2, so it stays ordered in everything it reads and writes.  When on,
+ * calls of at most 32 rows (not the grouped form) also read their WEIGHT, SCALE and ZERO-POINT
+ * tensors before that; x / bias / residual are read and out / scratch written only after it, so
+ * activations stay ordered as before.
+ * Contract when on: the weight, scale and zero-point tensors passed to such a call were not
  * written by the kernel immediately before it on the same stream (repack weights ahead of time,
  * or synchronise once after preprocessing).  Works inside CUDA-graph capture.
  */
@@ -237,7 +239,7 @@ RB200_API int rb200_gemm_fp16_intx_noalloc(const rb200_gemm_desc* desc, void* st
  *   e * scale_stride_e + n_idx * scale_stride_n + (k_idx / group_size) * scale_stride_g
  * - an extension: the reference has no quantised grouped GEMM.
  * Needs n % 16 == 0 (dense weights: n % 128 == 0), k % 64 == 0, 16-byte aligned x / out rows,
- * num_experts <= 64.
+ * num_experts <= 64 (any number for packed weights with total_rows <= 32).
  * workspace is accepted for signature parity and not used (nothing is allocated per call).
  * One launch for all experts; their row ranges are read from indptr on the device and experts
  * without rows cost nothing.
