@@ -9,15 +9,19 @@
 //
 // Bound: HBM, the fp16 weight read once.  A CTA keeps 32 rows x a slice of k in shared memory
 // between the two passes over it (absmax, quantise); with one scale per row the slices of a row
-// are the CTAs of one cluster, which exchange their maxima through distributed shared memory.
-// Quantising multiplies by the reciprocal scale and rounds by an addition, seven instructions
-// per value; a value whose product lies within the error bound of a rounding boundary is divided
-// instead, so that every code is the one the division gives.  Measured, fp16 11008 x 4096: int4 55 us
-// (2.1 TB/s), int8 in groups of 64 50 us; 230 us with a division and two global reads per value.
-// The source is read from memory once; what bounds the rest has not been profiled (the instructions above are
-// some 12 us of issue at that size, the bytes 17).
-#include <cooperative_groups.h>
-
+// are the CTAs of one cluster, which push their maxima into one another's shared memory: one cluster
+// barrier between the passes, and none that a CTA has to leave behind.
+// Quantising is four instructions per value (widen, multiply into the rounding constant, shift-add into
+// the packed word; half of a clamp).  The division of the definition is not needed: with a scale made
+// from an fp16 absmax, a / scale is either a tie exactly or more than 1.2e-4 away from one, so a
+// reciprocal that is four units too large rounds every tie away from zero and nothing else differently.
+// That was checked for all (absmax, value) pairs of fp16 and both widths, 2e9 of them, against the
+// division; the test repeats it for a sample.  Infinite maxima and NaN take the division.
+// The CTAs are persistent: three slices in shared memory, one being quantised, one whose maxima travel, one on
+// its way from memory.  Measured, fp16 11008 x 4096 (90 MB): one scale per row 31 us, int8 in groups of 64
+// 35 us; 45 / 55 us with a CTA per slice and a cluster barrier (its loads, its exchange and its arithmetic
+// one after the other, 37 us of it before the first code), and 53 / 50 us with a test for ties per value as well.
+// Loading and exchanging alone take 21 us, the codes 6, their stores (16 bytes of a k at a time) 6.
 #include "../../include/relax_b200.h"
 #include "common.cuh"
 
@@ -26,6 +30,8 @@ namespace {
 
 constexpr int kRows = 32;     // n per CTA
 constexpr int kMaxSpan = 512;  // k per pass through shared memory
+constexpr int kMaxCluster = 16;
+constexpr int kBufs = 3;       // slices of a CTA in shared memory: quantised, maxima being exchanged, on its way
 
 // code of one value by the definition: round_half_away(a / scale), clamped
 template <int BITS>
@@ -34,134 +40,320 @@ __device__ __noinline__ int encode_exact(float a, float scale) {
   return (int)fminf(fmaxf(roundf(__fdiv_rn(a, scale)), qlo), qhi);
 }
 
+constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer in the low mantissa bits
+
+// Reciprocal of a scale, four units too large (ties go away from zero, see above), and the largest value
+// that is worth looking at: fp16(7 | 127 scales), as two halves, so that no code leaves its range upwards.
+template <int BITS>
+__device__ __forceinline__ float2 quantiser(float scale) {
+  const float inv = __uint_as_float(__float_as_uint(__fdiv_rn(1.0f, scale)) + 4u);
+  const unsigned cap = __half_as_ushort(__float2half_rn((BITS == 4 ? 7.0f : 127.0f) * scale));
+  return make_float2(inv, __uint_as_float(cap * 0x10001u));
+}
+// what the packed sums of a word hold beside the codes: the bits of kMagic less the codes' bias, at every position
+template <int BITS>
+constexpr uint32_t rounding_sum() {
+  uint32_t sum = 0u;
+  for (int i = 0; i < 32 / BITS; ++i) sum = (sum << BITS) + 0x4b400000u - (1u << (BITS - 1));
+  return sum;
+}
+
+__device__ __forceinline__ __half2 abs_max(uint4 v) {  // drops NaN operands, as fmaxf does
+  const __half2* h = reinterpret_cast<const __half2*>(&v);
+  return __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+}
+__device__ __forceinline__ __half2 abs_max_nan(uint4 v) {  // 0x7fff for a NaN
+  const __half2* h = reinterpret_cast<const __half2*>(&v);
+  return __hmax2_nan(__hmax2_nan(__habs2(h[0]), __habs2(h[1])), __hmax2_nan(__habs2(h[2]), __habs2(h[3])));
+}
+__device__ __forceinline__ unsigned larger_bits(__half2 m) {  // non-negative: bits order as values
+  const unsigned u = *reinterpret_cast<const unsigned*>(&m);
+  return max(u & 0xffffu, u >> 16);
+}
+
+// 16-byte unit `u` of row r in shared memory: the rows of different packed words lie on different banks, since
+// the lanes of a quarter-warp read one word's rows each, at the same few k.
+template <int BITS>
+__device__ __forceinline__ int unit_at(int r, int u) {
+  return u ^ (BITS == 4 ? ((r >> 3) & 3) << 1 : (r >> 2) & 7);
+}
+
+// Bounded wait for the maxima other CTAs of the cluster push; a wait that ran out is reported.
+__device__ __forceinline__ void wait_pushed(uint64_t* bar, uint32_t phase, int* status) {
+#pragma unroll 1
+  for (int i = 0; i < 200000; ++i) {
+    uint32_t ok;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2, 10000;\n\t"
+        "selp.u32 %0, 1, 0, p;\n\t}"
+        : "=r"(ok)
+        : "r"(smem_u32(bar)), "r"(phase)
+        : "memory");
+    if (ok) return;
+  }
+  if (status) atomicExch(status, kStatusWaitTimeout);
+}
+
 // Rows in tiles of 32, k in slices that fit shared memory; needs n % 32 == 0, 16-byte rows and
 // groups of whole 16-byte vectors (the kernel below covers the rest).
-// PER_ROW: gridDim.y slices of a row form one cluster.  Otherwise a slice holds whole groups.
-template <int BITS, bool PER_ROW>
-__global__ void __launch_bounds__(256, 4) encode_slices_kernel(const __half* __restrict__ A, int8_t* __restrict__ packed,
-                                                            __half* __restrict__ scales, int64_t N, int64_t K, int slice,
-                                                            int group) {
-  namespace cg = cooperative_groups;
-  extern __shared__ __align__(16) uint8_t enc_smem[];
-  __half* tile = reinterpret_cast<__half*>(enc_smem);                             // [32][slice]
-  unsigned* amax = reinterpret_cast<unsigned*>(enc_smem + (size_t)kRows * slice * 2);  // [32][groups] fp16 bits
+// PER_ROW: the slices of a row form one cluster (rank = slice), the clusters share out the row tiles.
+// Otherwise a slice holds whole groups and the CTAs share out the (row tile, slice) pairs.
+template <int BITS, bool PER_ROW, int kThreads>
+__global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
+    encode_slices_kernel(const __half* __restrict__ A, int8_t* __restrict__ packed, __half* __restrict__ scales, int64_t N, int64_t K,
+                         int slice, int slices, int group, int* status) {
+  constexpr int kWarps = kThreads / 32, kOwnRows = kRows / kWarps;
+  constexpr unsigned kInf = 0x7c00u;
+  extern __shared__ __align__(128) uint8_t enc_smem[];
+  __shared__ unsigned row_max[kBufs][PER_ROW ? kMaxCluster : 1][kRows];  // PER_ROW: bits of a slice's maximum | NaN << 15
+  __shared__ __align__(8) uint64_t max_bar[kBufs];                      // counts the bytes of the maxima
+  const int units = (slice + 63) / 64 * 8;                           // 16-byte units of a row
   const int groups = PER_ROW ? 1 : slice / group;
-  float* s_scale = reinterpret_cast<float*>(amax + kRows * groups);               // [groups][32]
-  float* s_inv = s_scale + kRows * groups;                                        // [groups][32]
-  const int64_t n0 = (int64_t)blockIdx.x * kRows, k0 = (int64_t)blockIdx.y * slice;
-  const int span = (int)min((int64_t)slice, K - k0);
+  uint4* ring = reinterpret_cast<uint4*>(enc_smem);                                          // [kBufs][32][units]
+  float2* quant = reinterpret_cast<float2*>(enc_smem + (size_t)kBufs * kRows * units * 16);  // [groups][33]: reciprocal, clamp
+  float* s_scale = reinterpret_cast<float*>(quant + (kRows + 1) * groups);                   // [groups][32]
+  unsigned* amax = reinterpret_cast<unsigned*>(s_scale + kRows * groups);                    // [32][groups] fp16 bits
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float mul = BITS == 4 ? 0.125f : 0.0078125f;
-
-  for (int i = tid; i < kRows * groups; i += 256) amax[i] = 0u;
-  __syncthreads();
-  // pass 1: rows warp, warp + 8, ... of the slice into shared memory, absolute maxima on the way
-  const __half* src = A + (n0 + warp) * K + k0;
-  __half2 mx[kRows / 8];
-#pragma unroll
-  for (int i = 0; i < kRows / 8; ++i) mx[i] = __half2half2(__ushort_as_half(0));
-#pragma unroll 2
-  for (int c = lane * 8; c < span; c += 256) {
-    uint4 v[kRows / 8];
-#pragma unroll
-    for (int i = 0; i < kRows / 8; ++i) v[i] = __ldg(reinterpret_cast<const uint4*>(src + (int64_t)i * 8 * K + c));
-#pragma unroll
-    for (int i = 0; i < kRows / 8; ++i) {
-      const int r = warp + 8 * i;
-      *reinterpret_cast<uint4*>(tile + (size_t)r * slice + c) = v[i];
-      const __half2* h = reinterpret_cast<const __half2*>(&v[i]);
-      // __hmax2 drops a NaN operand, as fmaxf does
-      const __half2 m = __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
-      if (PER_ROW) {
-        mx[i] = __hmax2(mx[i], m);
-      } else {
-        const __half hm = __hmax(__hmax(__low2half(m), __high2half(m)), __ushort_as_half(0));
-        atomicMax(&amax[r * groups + c / group], (unsigned)__half_as_ushort(hm));  // non-negative: bits order as values
-      }
-    }
-  }
+  const unsigned n_tiles = (unsigned)(N / kRows);
+  unsigned rank = 0u, ranks = 1u;
   if (PER_ROW) {
-#pragma unroll
-    for (int i = 0; i < kRows / 8; ++i) {
-      unsigned m = max((unsigned)__half_as_ushort(__low2half(mx[i])), (unsigned)__half_as_ushort(__high2half(mx[i])));
-      m = __reduce_max_sync(0xffffffffu, m);
-      if (lane == 0) amax[warp + 8 * i] = m;
+    asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+    asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    if (tid == 0) {
+      for (int i = 0; i < kBufs; ++i) {
+        mbar_init(&max_bar[i], 1);
+        mbar_arrive_expect_tx(&max_bar[i], ranks * kRows * 4);
+      }
+      mbar_fence_init();
     }
-    cg::cluster_group cl = cg::this_cluster();
-    cl.sync();
-    if (tid < kRows) {
-      unsigned m = 0u;
-      for (unsigned c = 0; c < cl.num_blocks(); ++c) m = max(m, *cl.map_shared_rank(amax + tid, c));
-      const float sc = fmaxf(__half2float(__ushort_as_half((unsigned short)m)), 1e-4f) * mul;
-      s_scale[tid] = sc;
-      s_inv[tid] = __fdiv_rn(1.0f, sc);
-      if (blockIdx.y == 0) scales[n0 + tid] = __float2half_rn(sc);
-    }
-    cl.sync();  // no CTA leaves while its maxima are being read
+    asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every CTA's barriers exist
   } else {
-    __syncthreads();
-    for (int i = tid; i < kRows * (span / group); i += 256) {
-      const int r = i % kRows, g = i / kRows;
-      const float sc = fmaxf(__half2float(__ushort_as_half((unsigned short)amax[r * groups + g])), 1e-4f) * mul;
-      s_scale[g * kRows + r] = sc;
-      s_inv[g * kRows + r] = __fdiv_rn(1.0f, sc);
-      scales[(k0 / group + g) * N + n0 + r] = __float2half_rn(sc);
-    }
+    for (int i = tid; i < kRows * groups; i += kThreads) amax[i] = 0u;
     __syncthreads();
   }
+  // this CTA's items
+  const unsigned first = blockIdx.x / ranks, step = gridDim.x / ranks, items = PER_ROW ? n_tiles : n_tiles * (unsigned)slices;
+  auto tile_of = [&](unsigned item) { return PER_ROW ? item : item % n_tiles; };
+  auto slice_of = [&](unsigned item) { return PER_ROW ? rank : item / n_tiles; };
+  auto span_of = [&](unsigned item) { return (int)min((int64_t)slice, K - (int64_t)slice_of(item) * slice); };
+  auto row_of = [&](int i) { return warp + kWarps * i; };  // rows this warp loads and takes the maxima of
+  auto load = [&](unsigned item, int buf) {                // a lane's vectors of them; the lane reads them back itself
+    const __half* src = A + ((int64_t)tile_of(item) * kRows + warp) * K + (int64_t)slice_of(item) * slice;
+    const int span = span_of(item);
+    uint4* dst = ring + (size_t)buf * kRows * units;
+    for (int u = lane; u * 8 < span; u += 32)
+#pragma unroll
+      for (int i = 0; i < kOwnRows; ++i)
+        asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(dst + row_of(i) * units + unit_at<BITS>(row_of(i), u))),
+                     "l"(src + (int64_t)i * kWarps * K + u * 8)
+                     : "memory");
+  };
+  auto commit = [] { asm volatile("cp.async.commit_group;" ::: "memory"); };
 
-  // pass 2: a thread takes two neighbouring k of all 32 rows and writes their packed bytes
-  constexpr float kMagic = 12582912.0f;  // 1.5 * 2^23: adding it rounds to an integer in the low mantissa bits
-  constexpr float kTop = kMagic + (BITS == 4 ? 7.0f : 127.0f);
-  // |a * rn(1/s) - a/s| and the division's own rounding are 2^-24 relative each: at most 2^-20 (int4)
-  // or 2^-16 (int8) in total; a product closer than that to k + 1/2 is settled by the division
-  constexpr float kSafe = 0.5f - (BITS == 4 ? 2e-6f : 2e-5f);
-  for (int c = tid * 2; c < span; c += 512) {
-    const int g = PER_ROW ? 0 : c / group;
-    const float* sc = s_scale + g * kRows;
-    const float* inv = s_inv + g * kRows;
-    uint32_t lo[BITS], hi[BITS];  // 32 codes of k and of k + 1: BITS words each
-    constexpr int kPer = 32 / BITS;
-    constexpr uint32_t mask = BITS == 4 ? 15u : 255u;
-    unsigned doubtful = 0u;       // words with a value near a rounding boundary
+  // maxima of a slice's rows, pushed to every CTA of the cluster: asynchronous stores that count on the
+  // receiver's barrier, since a release of cluster scope would wait for the packed bytes on their way to memory.
+  // A CTA may be two items ahead of another (only one warp waits for the maxima of an item before it pushes
+  // the next), so there are as many places for them as buffers.
+  auto push_maxima = [&](unsigned item, int buf) {
+    const int span = span_of(item);
+    const uint4* t = ring + (size_t)buf * kRows * units;
+    unsigned own[kOwnRows], any = 0u;
+    __half2 mx[kOwnRows];
 #pragma unroll
-    for (int w = 0; w < BITS; ++w) {
-      uint32_t x = 0u, y = 0u;
-      bool near = false;
+    for (int i = 0; i < kOwnRows; ++i) mx[i] = __half2half2(__ushort_as_half(0));
+    for (int u = lane; u * 8 < span; u += 32)
 #pragma unroll
-      for (int i = kPer - 1; i >= 0; --i) {
-        const int r = w * kPer + i;
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(tile + (size_t)r * slice + c));
-        const float iv = inv[r];
-        const float t0 = fmaf(a.x, iv, kMagic), t1 = fmaf(a.y, iv, kMagic);
-        near |= !(fabsf(fmaf(a.x, iv, kMagic - t0)) < kSafe) | !(fabsf(fmaf(a.y, iv, kMagic - t1)) < kSafe);
-        x = (x << BITS) | (__float_as_uint(fminf(t0, kTop)) & mask);
-        y = (y << BITS) | (__float_as_uint(fminf(t1, kTop)) & mask);
-      }
-      lo[w] = x;
-      hi[w] = y;
-      doubtful |= (near ? 1u : 0u) << w;
+      for (int i = 0; i < kOwnRows; ++i) mx[i] = __hmax2_nan(mx[i], abs_max_nan(t[row_of(i) * units + unit_at<BITS>(row_of(i), u)]));
+#pragma unroll
+    for (int i = 0; i < kOwnRows; ++i) {
+      own[i] = __reduce_max_sync(0xffffffffu, larger_bits(mx[i]));
+      any = max(any, own[i]);
     }
-    const int64_t pitch = N * BITS / 8;
-    int8_t* d = packed + (k0 + c) * pitch + n0 * BITS / 8;
-#pragma unroll
-    for (int q = 0; q < BITS / 4; ++q) {
-      *reinterpret_cast<uint4*>(d + q * 16) = make_uint4(lo[4 * q], lo[4 * q + 1], lo[4 * q + 2], lo[4 * q + 3]);
-      *reinterpret_cast<uint4*>(d + pitch + q * 16) = make_uint4(hi[4 * q], hi[4 * q + 1], hi[4 * q + 2], hi[4 * q + 3]);
-    }
-    while (doubtful) {  // rare: those words again, by division
-      const int w = __ffs(doubtful) - 1;
-      doubtful &= doubtful - 1u;
-      uint32_t x = 0u, y = 0u;
+    if (any > kInf) {  // without the NaNs
 #pragma unroll 1
-      for (int i = kPer - 1; i >= 0; --i) {
-        const int r = w * kPer + i;
-        const float2 a = __half22float2(*reinterpret_cast<const __half2*>(tile + (size_t)r * slice + c));
-        x = (x << BITS) | ((uint32_t)encode_exact<BITS>(a.x, sc[r]) & mask);
-        y = (y << BITS) | ((uint32_t)encode_exact<BITS>(a.y, sc[r]) & mask);
+      for (int i = 0; i < kOwnRows; ++i) {
+        unsigned m = 0u;
+        for (int u = lane; u * 8 < span; u += 32) m = max(m, larger_bits(abs_max(t[row_of(i) * units + unit_at<BITS>(row_of(i), u)])));
+        m = __reduce_max_sync(0xffffffffu, m) | 0x8000u;
+#pragma unroll
+        for (int j = 0; j < kOwnRows; ++j)
+          if (j == i) own[j] = m;
       }
-      reinterpret_cast<uint32_t*>(d)[w] = x;
-      reinterpret_cast<uint32_t*>(d + pitch)[w] = y;
+    }
+    for (unsigned at = (unsigned)lane; at < kOwnRows * ranks; at += 32) {  // (row, receiver) pairs
+      const unsigned i = at / ranks, to = at - i * ranks;
+      unsigned v = own[0];
+#pragma unroll
+      for (int j = 1; j < kOwnRows; ++j)
+        if (i == (unsigned)j) v = own[j];
+      uint32_t dst, bar;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&row_max[buf][rank][warp + kWarps * i])), "r"(to));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_u32(&max_bar[buf])), "r"(to));
+      asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(dst), "r"(v), "r"(bar) : "memory");
+    }
+  };
+  // maxima of the slice's groups
+  const int seg = PER_ROW ? 1 : group / 8;  // vectors of a group
+  const bool fold_seg = seg <= 32 && (seg & (seg - 1)) == 0;
+  const int seg_shift = 31 - __clz(seg);
+  auto group_of = [&](int u) { return fold_seg ? u >> seg_shift : u / seg; };
+  auto group_maxima = [&](unsigned item, int buf) -> bool {
+    const int span = span_of(item);
+    const uint4* t = ring + (size_t)buf * kRows * units;
+    bool special = false;
+    for (int u0 = 0; u0 * 8 < span; u0 += 32) {
+      const int u = u0 + lane;
+      const bool in = u * 8 < span;
+      const int g = in ? group_of(u) : 0;
+      uint4 v[kOwnRows];
+      __half2 m[kOwnRows / 2];  // of two rows
+#pragma unroll
+      for (int i = 0; i < kOwnRows; ++i) v[i] = in ? t[row_of(i) * units + unit_at<BITS>(row_of(i), u)] : make_uint4(0u, 0u, 0u, 0u);
+      bool nan = false;
+#pragma unroll
+      for (int i = 0; i < kOwnRows / 2; ++i) {
+        const __half2 a = abs_max_nan(v[2 * i]), b = abs_max_nan(v[2 * i + 1]);
+        m[i] = __hmax2_nan(__lows2half2(a, b), __highs2half2(a, b));
+        nan |= __hisnan(__low2half(m[i])) | __hisnan(__high2half(m[i]));
+      }
+      if (nan) {
+        special = true;
+#pragma unroll
+        for (int i = 0; i < kOwnRows / 2; ++i) {
+          const __half2 a = abs_max(v[2 * i]), b = abs_max(v[2 * i + 1]);
+          m[i] = __hmax2(__hmax2(__lows2half2(a, b), __highs2half2(a, b)), __half2half2(__ushort_as_half(0)));
+        }
+      }
+      __syncwarp();
+      if (fold_seg)  // the lanes of a group are neighbours
+        for (int o = seg >> 1; o > 0; o >>= 1)
+#pragma unroll
+          for (int i = 0; i < kOwnRows / 2; ++i) m[i] = __hmax2(m[i], __shfl_xor_sync(0xffffffffu, m[i], o));
+      if (in && (!fold_seg || (lane & (seg - 1)) == 0)) {
+#pragma unroll
+        for (int i = 0; i < kOwnRows; ++i) {
+          const unsigned b = __half_as_ushort(i & 1 ? __high2half(m[i / 2]) : __low2half(m[i / 2]));
+          if (fold_seg) amax[row_of(i) * groups + g] = b;
+          else atomicMax(&amax[row_of(i) * groups + g], b);
+        }
+      }
+    }
+    return special;
+  };
+  // scale of (group g, row r) of an item from the bits of its maximum; true where the division has to do it
+  auto set_scale = [&](unsigned item, int g, int r, unsigned m) -> bool {
+    const float sc = fmaxf(__half2float(__ushort_as_half((unsigned short)m)), 1e-4f) * mul;
+    s_scale[g * kRows + r] = sc;
+    quant[g * (kRows + 1) + r + (r >> 4)] = quantiser<BITS>(sc);
+    const int64_t n = (int64_t)tile_of(item) * kRows + r;
+    if (!PER_ROW) scales[((int64_t)slice_of(item) * groups + g) * N + n] = __float2half_rn(sc);
+    else if (rank == 0) scales[n] = __float2half_rn(sc);
+    return m >= kInf;
+  };
+
+  // a thread makes one packed word each of eight neighbouring k; the words of a k are made by neighbouring lanes
+  const int word = tid % BITS, r0 = word * (32 / BITS);
+  auto quantise = [&](unsigned item, int buf, bool special) {
+    constexpr int kPer = 32 / BITS;             // codes of a word
+    constexpr uint32_t kSum = rounding_sum<BITS>(), kSigns = BITS == 4 ? 0x88888888u : 0x80808080u;
+    const int64_t pitch = N * BITS / 8;
+    const int span = span_of(item);
+    const uint4* t = ring + ((size_t)buf * kRows + r0) * units;
+    int8_t* d = packed + (int64_t)tile_of(item) * (kRows * BITS / 8) + word * 4 +
+                ((int64_t)slice_of(item) * slice + tid / BITS * 8) * pitch;
+    for (int u = tid / BITS; u * 8 < span; u += kThreads / BITS, d += (kThreads / BITS * 8) * pitch) {
+      const int g = PER_ROW ? 0 : group_of(u);
+      const uint4* col = t + unit_at<BITS>(r0, u);
+      uint32_t x[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) x[j] = 0u;
+      if (special) {
+#pragma unroll 1
+        for (int j = 0; j < 8; ++j) {
+          uint32_t y = 0u;
+#pragma unroll 1
+          for (int i = kPer - 1; i >= 0; --i)
+            y = (y << BITS) | ((uint32_t)encode_exact<BITS>(__half2float(reinterpret_cast<const __half*>(col + (size_t)i * units)[j]),
+                                                            s_scale[g * kRows + r0 + i]) & ((1u << BITS) - 1u));
+#pragma unroll
+          for (int k = 0; k < 8; ++k)
+            if (k == j) x[k] = y;
+        }
+      } else {
+        // sums of (rounding constant + code) << position; the constants come off at the end
+        const float2* qz = quant + g * (kRows + 1) + r0 + (r0 >> 4);
+#pragma unroll
+        for (int i = kPer - 1; i >= 0; --i) {
+          const uint4 raw = col[(size_t)i * units];
+          const float2 q = qz[i];
+          const __half2 cap = *reinterpret_cast<const __half2*>(&q.y);
+          const __half2* h = reinterpret_cast<const __half2*>(&raw);
+#pragma unroll
+          for (int j = 0; j < 4; ++j) {
+            const float2 a = __half22float2(__hmin2(h[j], cap));
+            x[2 * j] = (x[2 * j] << BITS) + __float_as_uint(fmaf(a.x, q.x, kMagic));
+            x[2 * j + 1] = (x[2 * j + 1] << BITS) + __float_as_uint(fmaf(a.y, q.x, kMagic));
+          }
+        }
+#pragma unroll
+        for (int j = 0; j < 8; ++j) x[j] = (x[j] - kSum) ^ kSigns;
+      }
+#pragma unroll
+      for (int j = 0; j < 8; ++j) *reinterpret_cast<uint32_t*>(d + j * pitch) = x[j];
+    }
+  };
+
+  for (int i = 0; i < kBufs; ++i) {
+    if (first + i * step < items) load(first + i * step, i);
+    commit();
+  }
+  if (PER_ROW) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+  int buf = 0;
+  uint32_t phase = 0u;
+  if (PER_ROW && first < items) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 1) : "memory");
+    push_maxima(first, 0);
+  }
+  for (unsigned item = first; item < items; item += step) {
+    bool special = false;
+    if (PER_ROW) {
+      // the next item's maxima are on their way through the cluster while this one is quantised
+      const int next = buf + 1 == kBufs ? 0 : buf + 1;
+      asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 2) : "memory");
+      if (warp == 0) {
+        wait_pushed(&max_bar[buf], phase, status);
+        unsigned m = 0u;
+        for (unsigned c = 0; c < ranks; ++c) {
+          const unsigned b = row_max[buf][c][lane];
+          m = max(m, b & 0x7fffu);
+          special |= b >= 0x8000u;
+        }
+        special |= set_scale(item, 0, lane, m);
+        __syncwarp();
+        // for the item kBufs further on: no CTA pushes that one before this warp has pushed the next
+        if (lane == 0) mbar_arrive_expect_tx(&max_bar[buf], ranks * kRows * 4);
+      }
+      if (item + step < items) push_maxima(item + step, next);
+    } else {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 1) : "memory");
+      special = group_maxima(item, buf);
+      __syncthreads();
+      for (int i = tid; i < kRows * (span_of(item) / group); i += kThreads) {
+        const int r = i % kRows, g = i / kRows;
+        special |= set_scale(item, g, r, amax[r * groups + g]);
+        amax[r * groups + g] = 0u;
+      }
+    }
+    special = __syncthreads_or(special);
+    quantise(item, buf, special);
+    __syncthreads();  // the buffer is free
+    if (item + kBufs * step < items) load(item + kBufs * step, buf);
+    commit();
+    if (++buf == kBufs) {
+      buf = 0;
+      phase ^= 1u;
     }
   }
 }
@@ -235,32 +427,54 @@ __global__ void __launch_bounds__(256) encode_ft_kernel(const __half* __restrict
   }
 }
 
-template <int BITS, bool PER_ROW>
-int launch_slices(const void* a, void* packed, void* scales, int64_t n, int64_t k, int slice, int group, int slices,
-                  size_t smem, cudaStream_t stream) {
-  auto kern = encode_slices_kernel<BITS, PER_ROW>;
-  static thread_local int configured_device = -1;
+size_t slices_smem(int64_t slice, int64_t groups) {
+  return (size_t)kBufs * kRows * ((slice + 63) / 64 * 128) + (size_t)groups * ((kRows + 1) * 8 + kRows * 8);
+}
+
+template <int BITS, bool PER_ROW, int kThreads>
+int launch_threads(const void* a, void* packed, void* scales, int64_t n, int64_t k, int slice, int group, int slices,
+                   size_t smem, cudaStream_t stream) {
+  auto kern = encode_slices_kernel<BITS, PER_ROW, kThreads>;
+  static thread_local int configured_device = -1, fit = 0, fit_slices = 0;
+  static thread_local size_t fit_smem = 0;
   int dev = 0;
   RB200_CUDA(cudaGetDevice(&dev));
-  if (configured_device != dev) {
-    RB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 227 * 1024));
-    configured_device = dev;
-  }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3((unsigned)(n / kRows), (unsigned)slices, 1);
-  cfg.blockDim = dim3(256, 1, 1);
+  cfg.blockDim = dim3(kThreads, 1, 1);
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
+  const unsigned ranks = PER_ROW ? (unsigned)slices : 1u;
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 1;
-  attr[0].val.clusterDim.y = PER_ROW ? (unsigned)slices : 1u;
+  attr[0].val.clusterDim.x = ranks;
+  attr[0].val.clusterDim.y = 1;
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
+  if (configured_device != dev || fit_smem != smem || fit_slices != (int)ranks) {  // clusters that run at the same time
+    RB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
+    RB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+    cfg.gridDim = dim3(ranks * (unsigned)sm_count_current(), 1, 1);
+    RB200_CUDA(cudaOccupancyMaxActiveClusters(&fit, kern, &cfg));
+    if (fit < 1) return 1;
+    configured_device = dev;
+    fit_smem = smem;
+    fit_slices = (int)ranks;
+  }
+  const int64_t items = n / kRows * (PER_ROW ? 1 : slices);
+  cfg.gridDim = dim3((unsigned)(items < fit ? items : fit) * ranks, 1, 1);
+  const DeviceScratch* scratch = device_scratch_if_any();
   RB200_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<const __half*>(a), static_cast<int8_t*>(packed),
-                                static_cast<__half*>(scales), n, k, slice, group));
+                                static_cast<__half*>(scales), n, k, slice, slices, group, scratch ? scratch->status : nullptr));
   return 0;
+}
+
+// two CTAs per SM where a slice is at most 512 k (100 KB of shared memory), else one: sixteen warps either way
+template <int BITS, bool PER_ROW>
+int launch_slices(const void* a, void* packed, void* scales, int64_t n, int64_t k, int slice, int group, int slices,
+                  size_t smem, cudaStream_t stream) {
+  return slice <= 512 ? launch_threads<BITS, PER_ROW, 256>(a, packed, scales, n, k, slice, group, slices, smem, stream)
+                      : launch_threads<BITS, PER_ROW, 512>(a, packed, scales, n, k, slice, group, slices, smem, stream);
 }
 
 }  // namespace
@@ -280,24 +494,27 @@ extern "C" int rb200_encode_ft(const void* a, void* packed, void* scales, int64_
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool aligned = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(packed)) & 15u) == 0;
   if (aligned && n % kRows == 0 && k % 8 == 0 && n / kRows < (1ll << 31)) {
-    // slice of k per CTA: 32 rows x 1024 k are 64 KB, two or three CTAs per SM.  One scale per row:
-    // the slices of a row are a cluster of at most eight CTAs, so long rows take longer slices.
+    // slice of k per CTA: 32 rows x 512 k are 32 KB.  One scale per row: the slices of a row are a cluster, of
+    // eight CTAs up to 8192 k and sixteen above (three buffers of longer slices would not fit)
+    int rc = 1;
     if (per_row) {
       int64_t c = 1;
       while (c < 8 && k > c * 512) c *= 2;
+      if (k > 8192) c = kMaxCluster;
       const int64_t slice = ((k + c - 1) / c + 7) / 8 * 8;
-      const size_t smem = (size_t)kRows * slice * 2 + kRows * 12;
+      const size_t smem = slices_smem(slice, 1);
       if (smem <= 200 * 1024 && (c - 1) * slice < k)
-        return weight_bits == 4 ? launch_slices<4, true>(a, packed, scales, n, k, (int)slice, 0, (int)c, smem, s)
-                                : launch_slices<8, true>(a, packed, scales, n, k, (int)slice, 0, (int)c, smem, s);
+        rc = weight_bits == 4 ? launch_slices<4, true>(a, packed, scales, n, k, (int)slice, 0, (int)c, smem, s)
+                              : launch_slices<8, true>(a, packed, scales, n, k, (int)slice, 0, (int)c, smem, s);
     } else if (group % 8 == 0 && group <= 1024) {
       const int64_t slice = (group > 512 ? 1024 : 512) / group * group;
-      const size_t smem = (size_t)kRows * slice * 2 + kRows * (slice / group) * 12;
+      const size_t smem = slices_smem(slice, slice / group);
       const int64_t c = (k + slice - 1) / slice;
-      if (c <= 65535)
-        return weight_bits == 4 ? launch_slices<4, false>(a, packed, scales, n, k, (int)slice, (int)group, (int)c, smem, s)
-                                : launch_slices<8, false>(a, packed, scales, n, k, (int)slice, (int)group, (int)c, smem, s);
+      if (n / kRows * c < (1ll << 31))
+        rc = weight_bits == 4 ? launch_slices<4, false>(a, packed, scales, n, k, (int)slice, (int)group, (int)c, smem, s)
+                              : launch_slices<8, false>(a, packed, scales, n, k, (int)slice, (int)group, (int)c, smem, s);
     }
+    if (rc <= 0) return rc;
   }
   dim3 grid((unsigned)((n + kRows - 1) / kRows), (unsigned)(k / group), 1);
   if (weight_bits == 4)

@@ -36,3 +36,56 @@ def test_reference_flow_entirely_on_gpu():
     out = ops.gemm_fp16_ft(to_dev(x), pre, scales, 4, bias=to_dev(bias))
     ref = np.dot(x.astype(np.float32), y.astype(np.float32).T) + bias.astype(np.float32)
     np.testing.assert_allclose(out.cpu().numpy().astype(np.float32), ref, rtol=1e-2, atol=1e-2)
+
+
+@pytest.mark.parametrize("bits,group", [(4, -1), (8, -1), (4, 64), (8, 64), (8, 24), (4, 512), (8, 768)])
+@pytest.mark.parametrize("k", [768, 4608, 12288])
+def test_encode_of_long_rows_ties_and_special_values(oracle, bits, group, k):
+    """Slices of 128 and 256 threads, one and several per cluster, groups folded over lanes or not: values on
+    and next to rounding boundaries, at the top of the range, infinities and NaN.  Rows in tiles of 32 take
+    the kernel with the nudged reciprocal, the two odd rows at the end the one that divides."""
+    if group > 0 and k % group:
+        pytest.skip("groups must divide k")
+    n = 96
+    rs = np.random.RandomState(bits + k)
+    y = rs.normal(0, 0.02, size=(n, k)).astype(np.float16)
+    g = k if group <= 0 else group
+    for r in range(n):  # ties: (2 c + 1) / 2 scales of every group's own maximum, and their neighbours
+        m = np.abs(y[r].reshape(-1, g)).max(axis=1, keepdims=True).astype(np.float32)
+        c = rs.randint(0, 2 ** (bits - 1), size=(k // g, g // 4))
+        t = ((2 * c + 1) * m / 2 ** bits).astype(np.float16)
+        t = (t.view(np.uint16) + rs.randint(-1, 2, size=t.shape)).astype(np.uint16).view(np.float16)
+        y[r].reshape(-1, g)[:, 1:1 + g // 4] = np.where(np.abs(t) <= m, t, 0) * rs.choice([-1, 1], size=t.shape)
+    y[3, :] = 0
+    y[5, :] = (y[5] * 2e-3).astype(np.float16)  # below the floor of the scale
+    packed, scales = ops.encode_ft(to_dev(y), bits, group)
+    exp_packed, exp_scales = oracle.np_encode_ft(y, bits, group)
+    assert np.array_equal(scales.cpu().numpy().view(np.uint16), exp_scales.view(np.uint16))
+    assert np.array_equal(packed.cpu().numpy(), exp_packed)
+    y[7, k - 3] = np.inf
+    y[8, 5] = -np.inf
+    y[40, 17] = np.nan
+    y[41, :] = np.nan
+    both = np.concatenate([y, y[:2]])
+    want_packed, want_scales = ops.encode_ft(to_dev(both), bits, group)
+    packed, scales = ops.encode_ft(to_dev(y), bits, group)
+    cols = n // 2 if bits == 4 else n
+    assert torch.equal(scales.view(torch.int16), want_scales[..., :n].contiguous().view(torch.int16))
+    assert torch.equal(packed, want_packed[:, :cols])
+
+
+@pytest.mark.parametrize("bits,group", [(4, -1), (8, -1), (8, 64), (4, 24)])
+@pytest.mark.parametrize("n,k", [(32 * 701, 1056), (32 * 131, 4104)])
+def test_encode_with_several_tiles_per_cta(oracle, bits, group, n, k):
+    """More row tiles than run at once: every buffer and every place for the maxima is used again, several
+    times over, with row maxima that differ from tile to tile."""
+    if group > 0 and k % group:
+        k = k // group * group
+    rs = np.random.RandomState(bits)
+    y = (rs.standard_normal((n, k)).astype(np.float32) * rs.uniform(0.001, 0.2, size=(n, 1)).astype(np.float32)).astype(np.float16)
+    exp_packed, exp_scales = oracle.np_encode_ft(y, bits, group)
+    w = to_dev(y)
+    for _ in range(3):
+        packed, scales = ops.encode_ft(w, bits, group)
+        assert np.array_equal(scales.cpu().numpy().view(np.uint16), exp_scales.view(np.uint16))
+        assert np.array_equal(packed.cpu().numpy(), exp_packed)
