@@ -186,6 +186,29 @@ __device__ __forceinline__ void griddep_launch_dependents() {
 }
 __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
+// A short kernel of a chain: launched as a programmatic dependent, so that its launch is over when the kernel
+// before it ends.  It waits before its first access and only then lets its own dependents start: what a
+// dependent reads ahead of its wait was then written at least one whole kernel earlier.  Its loads must not be
+// .nc ones (no const __restrict__), since it is resident while the kernel before it still writes.
+__device__ __forceinline__ void griddep_chain() {
+  griddep_wait();
+  griddep_launch_dependents();
+}
+template <class... P, class... A>
+cudaError_t launch_dependent(void (*kernel)(P...), dim3 grid, unsigned threads, size_t smem, cudaStream_t stream, A... args) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
 __device__ __forceinline__ uint32_t ld_nc_u16(const __half* p) {
   unsigned short v;
   asm volatile("ld.global.nc.u16 %0, [%1];" : "=h"(v) : "l"(p));

@@ -118,3 +118,35 @@ def test_expert_layer_with_caller_buffers_replays_from_a_graph():
         torch.cuda.synchronize()
         assert torch.equal(out, exp)
     _check_status()
+
+
+@pytest.mark.parametrize("tokens,experts,top_k", [(1, 1, 1), (33, 3, 3), (31, 9, 4), (1000, 9, 2), (1024, 16, 4), (1025, 16, 4), (7, 17, 4), (64, 16, 5)])
+def test_route_in_one_cta_and_in_several_kernels(oracle, tokens, experts, top_k):
+    """Both sides of what the one-CTA kernel takes (1024 tokens, 16 experts, 4 choices)."""
+    g = np.random.Generator(np.random.PCG64(7 * tokens + experts))
+    logits = np.round(g.standard_normal((tokens, experts), dtype=np.float32) * 2) / 2  # many ties
+    indptr, token_of_row, gate_of_row, row_of_flat = ops.moe_route(to_dev(logits), top_k)
+    e_indptr, e_tok, e_gate, e_rof = oracle.np_moe_route(logits, top_k)
+    assert np.array_equal(indptr.cpu().numpy(), e_indptr)
+    assert np.array_equal(token_of_row.cpu().numpy(), e_tok)
+    assert np.array_equal(row_of_flat.cpu().numpy(), e_rof)
+    np.testing.assert_allclose(gate_of_row.cpu().numpy(), e_gate, rtol=2e-6, atol=1e-8)
+
+
+@pytest.mark.parametrize("experts,top_k", [(8, 2), (5, 4), (16, 4)])
+def test_route_is_the_same_for_few_and_many_tokens(experts, top_k):
+    """The same logits, infinities and NaN among them, as 1024 tokens (one CTA) and with one more (several
+    kernels): the same choices, and gates bit for bit."""
+    g = np.random.Generator(np.random.PCG64(experts))
+    logits = g.standard_normal((1025, experts), dtype=np.float32)
+    logits[3, 1] = np.inf
+    logits[4, 2] = -np.inf
+    logits[5, :] = -np.inf
+    logits[6, 0] = np.nan
+    logits[7, 4] = np.nan
+    many, few = ops.moe_route(to_dev(logits), top_k), ops.moe_route(to_dev(logits[:1024]), top_k)
+    rof_m, rof_f = many[3].cpu().numpy()[:1024 * top_k], few[3].cpu().numpy()
+    experts_of = lambda indptr, rows: np.searchsorted(indptr.cpu().numpy(), rows, side="right")
+    assert np.array_equal(experts_of(many[0], rof_m), experts_of(few[0], rof_f))
+    assert np.array_equal(many[2].cpu().numpy()[rof_m].view(np.int32), few[2].cpu().numpy()[rof_f].view(np.int32))
+    assert np.array_equal(few[1].cpu().numpy()[rof_f], np.repeat(np.arange(1024), top_k))
