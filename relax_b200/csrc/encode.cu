@@ -305,6 +305,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
     }
   };
 
+  griddep_wait();  // a programmatic dependent that lets none start early: its outputs are weights
   for (int i = 0; i < kBufs; ++i) {
     if (first + i * step < items) load(first + i * step, i);
     commit();
@@ -444,7 +445,7 @@ int launch_threads(const void* a, void* packed, void* scales, int64_t n, int64_t
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
   const unsigned ranks = PER_ROW ? (unsigned)slices : 1u;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = ranks;
   attr[0].val.clusterDim.y = 1;
@@ -463,6 +464,9 @@ int launch_threads(const void* a, void* packed, void* scales, int64_t n, int64_t
   }
   const int64_t items = n / kRows * (PER_ROW ? 1 : slices);
   cfg.gridDim = dim3((unsigned)(items < fit ? items : fit) * ranks, 1, 1);
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.numAttrs = 2;
   const DeviceScratch* scratch = device_scratch_if_any();
   RB200_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<const __half*>(a), static_cast<int8_t*>(packed),
                                 static_cast<__half*>(scales), n, k, slice, slices, group, scratch ? scratch->status : nullptr));

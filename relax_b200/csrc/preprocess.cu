@@ -29,12 +29,21 @@ __device__ __forceinline__ uint32_t load_code(const uint8_t* src, int64_t n, int
 // AutoGPTQ zero points: zq uint32 [G, N/8] (nibble j of word (g, n/8) = column 8*(n/8) + j) ->
 // fp16 [G, N] holding f16(zq) + f16(1), the value the decode subtracts
 // (tests/python/dlight/test_gpu_gemv.py:648).
-__global__ void unpack_zeros_autogptq_kernel(const uint32_t* __restrict__ zq, __half* __restrict__ out, int64_t total,
-                                             int64_t N) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t g = i / N, n = i % N;
-    const uint32_t q = (zq[g * (N / 8) + (n >> 3)] >> ((n & 7) * 4)) & 15u;
-    out[i] = __hadd(__int2half_rn((int)q), __float2half_rn(1.0f));
+// A thread per word: its eight columns are neighbours, 16 bytes where the output allows (with the
+// repack, k 4096 x n 11008: 16.2 -> 11.0 us; a thread per column with two 64-bit divisions before).
+__global__ void __launch_bounds__(256) unpack_zeros_autogptq_kernel(const uint32_t* zq, __half* out, int64_t words, bool vec) {
+  griddep_chain();
+  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < words; i += (int64_t)gridDim.x * blockDim.x) {
+    const uint32_t q = zq[i];
+    __half v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = __hadd(__int2half_rn((int)((q >> (4 * j)) & 15u)), __float2half_rn(1.0f));
+    if (vec) {
+      *reinterpret_cast<uint4*>(out + i * 8) = *reinterpret_cast<const uint4*>(v);
+    } else {
+#pragma unroll
+      for (int j = 0; j < 8; ++j) out[i * 8 + j] = v[j];
+    }
   }
 }
 
@@ -138,7 +147,7 @@ __device__ __forceinline__ void transpose_bytes4(uint32_t a, uint32_t b, uint32_
 // Measured, k 8192 x n 28672, source + destination bytes: q4f16_1 45 us (5.2 TB/s), AutoGPTQ 54 us,
 // FT int4 46 us (5.1 TB/s; 3.6 before), FT int8 90 us (5.2 TB/s).
 template <int BITS, int LAYOUT, bool GATE_UP>
-__global__ void __launch_bounds__(128) repack_stage_kernel(const uint8_t* __restrict__ src, uint8_t* __restrict__ dst,
+__global__ void __launch_bounds__(128) repack_stage_kernel(const uint8_t* src, uint8_t* dst,
                                                            int64_t K, int64_t N, uint32_t tiles, uint32_t chunks,
                                                            uint32_t total) {
   constexpr int kFrag = BITS == 4 ? 64 : 32;
@@ -148,6 +157,7 @@ __global__ void __launch_bounds__(128) repack_stage_kernel(const uint8_t* __rest
   const int t = tid & 3, b = (tid >> 2) & 7, kbl = tid >> 5;
   const int64_t KB = K / kFrag, NB = N / 16;
   const int64_t expert_bytes = K * N * BITS / 8;
+  griddep_wait();  // a programmatic dependent (of the quantiser, when a model is loaded) that lets none start early
   for (uint32_t st = blockIdx.x; st < total; st += gridDim.x) {
     // neighbours in flight share the source's contiguous axis: n for [K, N] layouts, k for [N, K]
     uint32_t e, tile, chunk;
@@ -179,10 +189,10 @@ __global__ void __launch_bounds__(128) repack_stage_kernel(const uint8_t* __rest
 #pragma unroll
         for (int i = 0; i < 16; ++i) {
           if (GATE_UP) {
-            v[i].x = __ldg(reinterpret_cast<const uint32_t*>(q + i * pitch + n_lo / 2));
-            v[i].y = __ldg(reinterpret_cast<const uint32_t*>(q + i * pitch + n_hi / 2));
+            v[i].x = *(reinterpret_cast<const uint32_t*>(q + i * pitch + n_lo / 2));
+            v[i].y = *(reinterpret_cast<const uint32_t*>(q + i * pitch + n_hi / 2));
           } else {
-            v[i] = __ldg(reinterpret_cast<const uint2*>(q + i * pitch + n_lo / 2));
+            v[i] = *(reinterpret_cast<const uint2*>(q + i * pitch + n_lo / 2));
           }
         }
         uint32_t w[4][8];
@@ -214,11 +224,11 @@ __global__ void __launch_bounds__(128) repack_stage_kernel(const uint8_t* __rest
 #pragma unroll
         for (int i = 0; i < 8; ++i) {
           if (GATE_UP) {
-            const uint2 lo = __ldg(reinterpret_cast<const uint2*>(q + i * N + n_lo));
-            const uint2 hi = __ldg(reinterpret_cast<const uint2*>(q + i * N + n_hi));
+            const uint2 lo = *(reinterpret_cast<const uint2*>(q + i * N + n_lo));
+            const uint2 hi = *(reinterpret_cast<const uint2*>(q + i * N + n_hi));
             v[i] = make_uint4(lo.x, lo.y, hi.x, hi.y);
           } else {
-            v[i] = __ldg(reinterpret_cast<const uint4*>(q + i * N + n_lo));
+            v[i] = *(reinterpret_cast<const uint4*>(q + i * N + n_lo));
           }
         }
         uint32_t w[4][8];  // word 2j + r8 of the unit of row g
@@ -245,8 +255,8 @@ __global__ void __launch_bounds__(128) repack_stage_kernel(const uint8_t* __rest
           const int64_t pitch = K / 2;
 #pragma unroll
           for (int g = 0; g < 8; ++g) {
-            const uint2 a = __ldg(reinterpret_cast<const uint2*>(q + (n_lo + g) * pitch));
-            const uint2 c = __ldg(reinterpret_cast<const uint2*>(q + (n_hi + g) * pitch));
+            const uint2 a = *(reinterpret_cast<const uint2*>(q + (n_lo + g) * pitch));
+            const uint2 c = *(reinterpret_cast<const uint2*>(q + (n_hi + g) * pitch));
             lo[0][g] = a.x, lo[1][g] = a.y, hi[0][g] = c.x, hi[1][g] = c.y;
           }
         } else {  // [K/8, N]
@@ -255,8 +265,8 @@ __global__ void __launch_bounds__(128) repack_stage_kernel(const uint8_t* __rest
           for (int h = 0; h < 2; ++h)
 #pragma unroll
             for (int g4 = 0; g4 < 8; g4 += 4) {
-              const uint4 a = __ldg(reinterpret_cast<const uint4*>(q + (h * N + n_lo + g4) * 4));
-              const uint4 c = __ldg(reinterpret_cast<const uint4*>(q + (h * N + n_hi + g4) * 4));
+              const uint4 a = *(reinterpret_cast<const uint4*>(q + (h * N + n_lo + g4) * 4));
+              const uint4 c = *(reinterpret_cast<const uint4*>(q + (h * N + n_hi + g4) * 4));
               lo[h][g4] = a.x, lo[h][g4 + 1] = a.y, lo[h][g4 + 2] = a.z, lo[h][g4 + 3] = a.w;
               hi[h][g4] = c.x, hi[h][g4 + 1] = c.y, hi[h][g4 + 2] = c.z, hi[h][g4 + 3] = c.w;
             }
@@ -315,13 +325,53 @@ __global__ void gptq_act_order_kernel(const int32_t* __restrict__ g_idx, int K, 
   }
 }
 
-// out[m, j] = x[m, perm[j]] over fp16
-__global__ void gather_columns_kernel(const __half* __restrict__ x, const int32_t* __restrict__ perm,
-                                      __half* __restrict__ out, int64_t M, int64_t K, int64_t ldx, int64_t ldo) {
-  const int64_t total = M * K;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < total; i += (int64_t)gridDim.x * blockDim.x) {
-    const int64_t m = i / K, j = i % K;
-    out[m * ldo + j] = x[m * ldx + perm[j]];
+// out[m, j] = x[m, perm[j]] over fp16.  A thread takes VEC neighbouring j of every gridDim.y-th row; eight where
+// the rows of `out` and perm are 16-byte aligned.
+template <int VEC>
+__global__ void __launch_bounds__(128) gather_columns_kernel(const __half* x, const int32_t* perm, __half* out, int64_t M, int64_t K,
+                                                             int64_t ldx, int64_t ldo) {
+  griddep_chain();
+  const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
+  if (j >= K) return;
+  int32_t from[VEC];
+  if (VEC == 8) {
+    *reinterpret_cast<int4*>(from) = *reinterpret_cast<const int4*>(perm + j);
+    *reinterpret_cast<int4*>(from + 4) = *reinterpret_cast<const int4*>(perm + j + 4);
+  } else {
+    from[0] = perm[j];
+  }
+  for (int64_t m = blockIdx.y; m < M; m += gridDim.y) {
+    __align__(16) __half v[VEC];
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) v[i] = x[m * ldx + from[i]];
+    if (VEC == 8) *reinterpret_cast<uint4*>(out + m * ldo + j) = *reinterpret_cast<const uint4*>(v);
+    else out[m * ldo + j] = v[0];
+  }
+}
+
+// The same with `rows` rows at a time in shared memory: whole lines in and out, and the indices read once for them.
+__global__ void __launch_bounds__(256) gather_columns_staged_kernel(const __half* x, const int32_t* perm, __half* out, int64_t M,
+                                                                    int K, int64_t ldx, int64_t ldo, int rows) {
+  extern __shared__ __align__(16) uint4 staged[];  // [rows][K / 8]
+  const __half* h = reinterpret_cast<const __half*>(staged);
+  const int vecs = K / 8;
+  griddep_chain();
+  for (int64_t m0 = (int64_t)blockIdx.x * rows; m0 < M; m0 += (int64_t)gridDim.x * rows) {
+    const int n = (int)min((int64_t)rows, M - m0);
+    for (int r = 0; r < n; ++r)
+      for (int c = threadIdx.x; c < vecs; c += 256) staged[r * vecs + c] = reinterpret_cast<const uint4*>(x + (m0 + r) * ldx)[c];
+    __syncthreads();
+    for (int c = threadIdx.x; c < vecs; c += 256) {
+      const int4 a = reinterpret_cast<const int4*>(perm)[2 * c], b = reinterpret_cast<const int4*>(perm)[2 * c + 1];
+      const int from[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
+      for (int r = 0; r < n; ++r) {
+        __align__(16) __half v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = h[r * K + from[i]];
+        reinterpret_cast<uint4*>(out + (m0 + r) * ldo)[c] = *reinterpret_cast<const uint4*>(v);
+      }
+    }
+    __syncthreads();
   }
 }
 
@@ -358,19 +408,14 @@ int preprocess_launch(const void* src, void* dst, int64_t experts, int64_t k, in
     const uint32_t stages = (uint32_t)(experts * tiles * chunks);
     uint32_t grid = (uint32_t)sm_count_current() * 12;
     if (grid > stages) grid = stages;
-#define RB200_RS(B, L)                                                                                              \
-  do {                                                                                                              \
-    if (interleave)                                                                                                 \
-      repack_stage_kernel<B, L, true><<<grid, 128, 0, stream>>>(s, d, k, n, (uint32_t)tiles, (uint32_t)chunks, stages); \
-    else                                                                                                            \
-      repack_stage_kernel<B, L, false><<<grid, 128, 0, stream>>>(s, d, k, n, (uint32_t)tiles, (uint32_t)chunks, stages); \
-  } while (0)
+#define RB200_RS(B, L)                                                                                           \
+  RB200_CUDA(launch_dependent(interleave ? repack_stage_kernel<B, L, true> : repack_stage_kernel<B, L, false>, dim3(grid), 128, 0, \
+                              stream, s, d, k, n, (uint32_t)tiles, (uint32_t)chunks, stages))
     if (bits == 8) RB200_RS(8, 0);
     else if (layout == 0) RB200_RS(4, 0);
     else if (layout == 1) RB200_RS(4, 1);
     else RB200_RS(4, 2);
 #undef RB200_RS
-    RB200_CUDA(cudaGetLastError());
     return 0;
   }
   // a k permutation (act-order) or an unaligned source: code by code
@@ -407,24 +452,47 @@ int gptq_act_order_launch(const int32_t* g_idx, int64_t k, int64_t groups, int32
 
 int gather_columns_launch(const void* x, const int32_t* perm, void* out, int64_t m, int64_t k, int64_t ldx,
                           int64_t ldo, cudaStream_t stream) {
-  const int64_t total = m * k;
-  if (total == 0) return 0;
-  int64_t blocks = (total + 255) / 256;
-  if (blocks > (int64_t)sm_count_current() * 16) blocks = (int64_t)sm_count_current() * 16;
-  gather_columns_kernel<<<(int)blocks, 256, 0, stream>>>(static_cast<const __half*>(x), perm, static_cast<__half*>(out),
-                                                        m, k, ldx, ldo);
-  RB200_CUDA(cudaGetLastError());
+  if (m * k == 0) return 0;
+  const bool vec = k % 8 == 0 && ldo % 8 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(perm)) & 15u) == 0;
+  // From 65 rows on through shared memory, where the rows can be read 16 bytes at a time; below, the direct form's
+  // single trip to memory is shorter.  Measured (graph of launches; element by
+  // element with 64-bit divisions before): k 4096, 16 rows 1.48 us (2.00), 256 rows 2.4 (5.4), 2048 rows 11.1 (25.4);
+  // k 14336, 32 rows 2.6 direct, 3.8 staged (4.0), 64 rows 4.6 / 3.9 (5.7), 2048 rows 41 (105).
+  constexpr int64_t kStaged = 96 * 1024;
+  if (vec && m > 64 && ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && k * 2 <= kStaged) {
+    static thread_local int configured_device = -1;
+    int dev = 0;
+    RB200_CUDA(cudaGetDevice(&dev));
+    if (configured_device != dev) {
+      RB200_CUDA(cudaFuncSetAttribute(gather_columns_staged_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kStaged));
+      configured_device = dev;
+    }
+    int64_t rows = kStaged / (k * 2);
+    if (rows > 4) rows = 4;
+    while (rows > 1 && (m + rows - 1) / rows < sm_count_current() * 2) --rows;
+    const int64_t need = (m + rows - 1) / rows, most = (int64_t)sm_count_current() * 8;
+    RB200_CUDA(launch_dependent(gather_columns_staged_kernel, dim3((unsigned)(need < most ? need : most)), 256, (size_t)(rows * k * 2),
+                                stream, static_cast<const __half*>(x), perm, static_cast<__half*>(out), m, (int)k, ldx, ldo, (int)rows));
+    return 0;
+  }
+  const int64_t columns = (k / (vec ? 8 : 1) + 127) / 128;
+  RB200_CHECK(columns < (1ll << 31), "k=%lld is too large", (long long)k);
+  // rows that a thread does one after the other share its indices: no more CTAs than fill the device a few times
+  int64_t rows = (int64_t)sm_count_current() * 16 / columns + 1;
+  if (rows > m) rows = m;
+  if (rows > 65535) rows = 65535;
+  RB200_CUDA(launch_dependent(vec ? gather_columns_kernel<8> : gather_columns_kernel<1>, dim3((unsigned)columns, (unsigned)rows), 128, 0,
+                              stream, static_cast<const __half*>(x), perm, static_cast<__half*>(out), m, k, ldx, ldo));
   return 0;
 }
 
 int unpack_zeros_autogptq_launch(const void* zq, void* out, int64_t groups, int64_t n, cudaStream_t stream) {
-  const int64_t total = groups * n;
-  if (total == 0) return 0;
-  int64_t blocks = (total + 255) / 256;
+  const int64_t words = groups * (n / 8);
+  if (words == 0) return 0;
+  int64_t blocks = (words + 255) / 256;
   if (blocks > (int64_t)sm_count_current() * 16) blocks = (int64_t)sm_count_current() * 16;
-  unpack_zeros_autogptq_kernel<<<(int)blocks, 256, 0, stream>>>(static_cast<const uint32_t*>(zq),
-                                                               static_cast<__half*>(out), total, n);
-  RB200_CUDA(cudaGetLastError());
+  RB200_CUDA(launch_dependent(unpack_zeros_autogptq_kernel, dim3((unsigned)blocks), 256, 0, stream, static_cast<const uint32_t*>(zq),
+                              static_cast<__half*>(out), words, (reinterpret_cast<uintptr_t>(out) & 15u) == 0));
   return 0;
 }
 

@@ -108,3 +108,14 @@ def test_act_order_uneven_groups_are_rejected():
     g_idx = np.zeros(256, dtype=np.int32)  # every row in group 0 of 2
     with pytest.raises(RuntimeError):
         ops.gptq_act_order(torch.from_numpy(g_idx).cuda(), 2)
+
+
+@pytest.mark.parametrize("m,k", [(1, 8), (3, 1004), (64, 4096), (65, 4096), (300, 1032), (700, 14336), (70, 49160)])
+def test_gather_columns_forms(m, k):
+    """One column and eight columns per thread, through shared memory with one row and several at a time, and a
+    row that does not fit there."""
+    x = torch.randn(m, k, device="cuda").half()
+    perm = torch.randperm(k, device="cuda").int()
+    assert torch.equal(ops.gather_columns(x, perm), x[:, perm.long()])
+    wide = torch.randn(m * k + 1, device="cuda").half()[1:].view(m, k)  # two bytes off a 16-byte boundary
+    assert torch.equal(ops.gather_columns(wide, perm), wide[:, perm.long()])
