@@ -18,10 +18,14 @@
 //   warp 0        packed weights, one 16 KB bulk copy per chunk (128 rows x 256 | 128 k)
 //   warp 1        MMA issue (rank 0)
 //   warp 2        x: one TMA tile [nb/2 rows x 128 k] per step, completing on rank 0's barrier
-//   warps 4-11    two groups of four warps decode alternate steps
-//   warps 12-15   drain: epilogue, one rounding, transpose through shared memory, whole-line stores.
-//                 The decode groups help where they would only wait: with a single accumulator, and on
-//                 the last tile.
+//   warps 4-15    three groups of four warps.  With two accumulators two of them decode alternate steps and
+//                 the third drains: epilogue, one rounding, transpose through shared memory, whole-line
+//                 stores (the others help it with the last tile).  With a single accumulator there is nothing
+//                 to drain while a tile is made, so all three decode in turn and then drain in shares.
+//                 (Measured with two decoding: the MMA waited 148 000 of 425 000 clocks for A at 2048 rows of
+//                 int4, k 4096 x n 22016, group 128; 75 000 with three.  An expert layer of 1024 rows, int4,
+//                 hidden 4096, ffn 14336, eight experts: 317 -> 272 us with this and scales that are not waited
+//                 for where they are loaded; 500 rows of AutoGPTQ k 4096 x n 11008 65 -> 55.)
 //
 // Work split: whole waves of tiles go round robin over the pairs, neighbours sharing a weight tile in L2;
 // the remainder - between one and two waves - is cut into equal runs of (tile, chunk) units that the
@@ -142,11 +146,12 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t rank = cluster_rank();
   const unsigned pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const bool grouped = pp.indptr != nullptr;
-  const bool all_drain = pp.nd == 1;
+  const bool all_drain = pp.nd == 1;      // nothing to drain while a tile is made: all three groups decode, then drain
+  const int decoders = all_drain ? 3 : 2;  // groups
   if (tid == 0) {
     for (int s = 0; s < w_stages; ++s) {
       mbar_init(&w_full[s], 1);
-      mbar_init(&w_empty[s], 8);
+      mbar_init(&w_empty[s], 4 * decoders);
     }
     for (int s = 0; s < x_stages; ++s) {
       mbar_init(&x_full[s], 1);
@@ -450,14 +455,14 @@ __global__ void __launch_bounds__(kThreads, 1)
     int db = 0;
     uint32_t dph = 0;
     Walk w;
-    if (grp == 2) {
+    if (grp >= decoders) {
       for (bool have = begin(w); ok && have; have = next(w)) {
         const Item it = get_item(w.item);
         feed.row(pp, it.e, it.n_tile * kTileRows + row);
         ok = mbar_wait_parked(&d_full[db], dph, p.status);
         if (!ok) break;
         tc_fence_after();
-        ok = drain(w, it, db, 0, all_drain || is_last(w) ? kDrainGroups : 1, feed.s_row);
+        ok = drain(w, it, db, 0, is_last(w) ? kDrainGroups : 1, feed.s_row);
         if (!ok) break;
         tc_fence_before();
         __syncwarp();
@@ -472,29 +477,27 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t off[4];
 #pragma unroll
       for (int t = 0; t < 4; ++t) off[t] = (uint32_t)(t * 128 + ((g + 2 * t) & 7) * 16);
-      unsigned q = 0;  // steps before the current chunk
-      // the step of a chunk this group decodes, given the steps before it: of two steps one, of a
-      // single step every other one
-      auto own_step = [&](unsigned before) -> int {
-        const int j = (int)((before ^ (unsigned)grp) & 1u);
-        return j;
-      };
-      auto fetch = [&](int c, unsigned before) {
-        const int j = own_step(before);
-        if (j * kStepBlk >= kBlkPerChunk) return;
-        feed.fetch_two(pp, c * kBlkPerChunk + j * kStepBlk, k_blocks);
+      int turn = 0;  // group whose turn the first step of the current chunk is
+      // the groups take the steps in turn: this group's step of a chunk, given whose turn its first one is
+      auto own_step = [&](int turn) { return grp >= turn ? grp - turn : grp - turn + decoders; };
+      auto next_turn = [&](int turn, int steps) { return turn + steps >= decoders ? turn + steps - decoders : turn + steps; };
+      auto fetch = [&](int c, int turn) {
+        // (on every path, a group without a step in the chunk too: a load under a branch is waited for where the paths meet)
+        const int j = min(own_step(turn), kBlkPerChunk / kStepBlk - 1);
+        feed.fetch_two(pp, min(c * kBlkPerChunk + j * kStepBlk, (k_blocks - 1) & ~1), k_blocks);
       };
       int ws = 0, ab0 = 0;
       uint32_t wph = 0, aph0 = 1;
       for (bool have = begin(w); ok && have; have = next(w)) {
         const Item it = get_item(w.item);
         feed.row(pp, it.e, it.n_tile * kTileRows + row);
-        fetch(w.c0, q);
+        fetch(w.c0, turn);
         for (int c = w.c0; c < w.c1; ++c) {
           const int nft = min(4, KT - c * 4), nblk = nft / kTilesPerBlk, steps = (nblk + kStepBlk - 1) / kStepBlk;
-          const int j = own_step(q);
+          const int j = own_step(turn);
           feed.advance();
-          if (c + 1 < w.c1) fetch(c + 1, q + (unsigned)steps);
+          turn = next_turn(turn, steps);
+          fetch(min(c + 1, w.c1 - 1), turn);
           // (a group without a step in this chunk waits all the same: its arrival must not run ahead)
           if (!mbar_wait_parked(&w_full[ws], wph, p.status)) {
             ok = false;
@@ -529,7 +532,6 @@ __global__ void __launch_bounds__(kThreads, 1)
             ws = 0;
             wph ^= 1u;
           }
-          q += (unsigned)steps;
           ab0 += steps;
           if (ab0 >= pp.na) {
             ab0 -= pp.na;
@@ -542,7 +544,7 @@ __global__ void __launch_bounds__(kThreads, 1)
           ok = all_drain ? mbar_wait_parked(&d_full[db], dph, p.status) : mbar_wait_parked(d_last, 0, p.status);
           if (!ok) break;
           tc_fence_after();
-          ok = drain(w, it, db, grp + 1, kDrainGroups, feed.s_row);
+          ok = drain(w, it, db, grp == 2 ? 0 : grp + 1, kDrainGroups, feed.s_row);
           if (!ok) break;
           tc_fence_before();
           __syncwarp();

@@ -53,10 +53,12 @@ int run_pair(Params& pp, int bits, int zmode, int src, int sm_count, cudaStream_
   }
   pp.nb = (pp.nb + 31) / 32 * 32;
   if (!pp.indptr) pp.m_tiles = (p.m + pp.nb - 1) / pp.nb;  // no tile without rows (an MMA of width 0 is illegal)
-  // tensor memory: two accumulators of up to 128 columns or one of 256, then A slots of 64 columns
+  // tensor memory: two accumulators of up to 160 columns or one of 256, then A slots of 64 columns (at least three:
+  // int8 k 8192 x n 57344, 160 rows, two accumulators 139 us, one 142; int4 k 4096 x n 22016, group 32, 129 rows
+  // 35.0 / 36.7)
   pp.tmem_cols = 512;
-  pp.nd = pp.nb <= 128 ? 2 : 1;
-  pp.d_stride = pp.nb <= 128 ? 128 : (pp.nb <= 192 ? 192 : 256);
+  pp.nd = pp.nb <= 160 ? 2 : 1;
+  pp.d_stride = pp.nb <= 128 ? 128 : (pp.nb <= 160 ? 160 : (pp.nb <= 192 ? 192 : 256));
   pp.a_base = pp.nd * pp.d_stride;
   pp.na = (pp.tmem_cols - pp.a_base) / 64;
   if (pp.na > kMaxA) pp.na = kMaxA;
@@ -178,6 +180,10 @@ int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, const int64
     RB200_CHECK(p.group % lane_run == 0 && p.k % p.group == 0, "group_size=%d must divide k=%d and be a multiple of %d", p.group,
                 p.k, lane_run);
     src = p.group % kKBlock == 0 ? kOne : (p.group == 32 ? kTwo : kAny);
+    pp.blk_shift = -1;
+    const int blocks = p.group / kKBlock;
+    if (src == kOne && (blocks & (blocks - 1)) == 0)
+      for (pp.blk_shift = 0; (1 << pp.blk_shift) < blocks;) ++pp.blk_shift;
     const uintptr_t addr = reinterpret_cast<uintptr_t>(p.s) | reinterpret_cast<uintptr_t>(p.z);
     auto words_of = [&](int halves) {
       return p.s_g == 1 && p.s_n % halves == 0 && (addr & (uintptr_t)(2 * halves - 1)) == 0 && s_expert_stride % halves == 0;

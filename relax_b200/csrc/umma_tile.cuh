@@ -37,6 +37,7 @@ struct Params {
   int x_stages, w_stages;
   int nd, d_stride, a_base, na, tmem_cols;  // accumulators and A slots in tensor memory
   int s_n, s_g;                // scale strides in elements
+  int blk_shift;               // kOne: log2 of a group's 64-k blocks, or -1
   int s_vec;                   // kTwo: the two groups of a block are one aligned 32-bit word (1), those of two
                                // adjacent blocks one 64-bit word (2; pairs_fit_rows)
   int early;                   // weights / scales were not written by the previous kernel
@@ -270,7 +271,7 @@ struct ScaleFeed {
     sp = pp.g.s + o;
     zp = pp.g.z + o;
     if (SRC == kChannel) {
-      s_row = ld_nc_u16(sp) * 0x10001u;
+      s_row = ld_nc_u16(sp);  // doubled where it is used, not to wait for it here
       if (has_zeros) {
         z_row = ld_nc_u16(zp) * 0x10001u;
         row_exact = true;
@@ -281,9 +282,9 @@ struct ScaleFeed {
   // the i-th own block of the next chunk is 64-k block kb
   __device__ __forceinline__ void fetch(const Params& pp, int i, int kb) {
     if (SRC == kOne) {
-      const int64_t o = (int64_t)((unsigned)(kb * kKBlock) / (unsigned)pp.g.group) * pp.s_g;
-      sn[i] = ld_nc_u16(sp + o) * 0x10001u;
-      if (has_zeros) zn[i] = ld_nc_u16(zp + o) * 0x10001u;
+      const int64_t o = (int64_t)(pp.blk_shift >= 0 ? (unsigned)kb >> pp.blk_shift : (unsigned)(kb * kKBlock) / (unsigned)pp.g.group) * pp.s_g;
+      sn[i] = ld_nc_u16(sp + o);
+      if (has_zeros) zn[i] = ld_nc_u16(zp + o);
     } else if (SRC == kTwo && pp.s_vec) {
       sn[i] = __ldg(reinterpret_cast<const uint32_t*>(sp + kb * 2));
       if (has_zeros) zn[i] = __ldg(reinterpret_cast<const uint32_t*>(zp + kb * 2));
@@ -313,8 +314,10 @@ struct ScaleFeed {
   __device__ __forceinline__ void advance() {
 #pragma unroll
     for (int i = 0; i < OWN; ++i) {
-      sv[i] = sn[i];
-      zv[i] = zn[i];
+      // (kOne: doubled here and not where it is loaded, which would wait for the load there: an expert layer's
+      // matmul of 1024 rows, k 4096 x n 14336, group 128, spent 1400 of 2900 clocks a step on that)
+      sv[i] = SRC == kOne ? sn[i] * 0x10001u : sn[i];
+      zv[i] = SRC == kOne ? zn[i] * 0x10001u : zn[i];
       if (kZ && (SRC == kOne || SRC == kTwo) && has_zeros) {
         exact[i] = true;
         zo[i] = offset(zv[i], exact[i]);
@@ -331,7 +334,7 @@ struct ScaleFeed {
   }
   // run t (int8: fragment tile * 4 + lane run) of own block i = 64-k block kb
   __device__ __forceinline__ uint32_t scale(const Params& pp, int i, int kb, int t) const {
-    if (SRC == kChannel) return s_row;
+    if (SRC == kChannel) return prmt(s_row, s_row, 0x1010u);
     if (SRC == kOne) return sv[i];
     if (SRC == kTwo) return prmt(sv[i], sv[i], (BITS == 4 ? t >> 1 : t >> 2) ? 0x3232u : 0x1010u);
     const unsigned k = (unsigned)(kb * kKBlock + (BITS == 4 ? t * 16 : t * 8));
