@@ -371,7 +371,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
       fetch(w.c0);
       for (int c = w.c0; c < w.c1; ++c) {
         feed.advance();
-        fetch(c + (c + 1 < w.c1 ? 1 : 0));  // (on every path: a load under a branch is waited for where the paths meet)
+        if (c + 1 < w.c1) fetch(c + 1);
         if (!mbar_wait_parked(&w_full[ws], wph, p.status)) {
           ok = false;
           break;
