@@ -190,6 +190,8 @@ __device__ __forceinline__ void griddep_wait() { asm volatile("griddepcontrol.wa
 // before it ends.  It waits before its first access and only then lets its own dependents start: what a
 // dependent reads ahead of its wait was then written at least one whole kernel earlier.  Its loads must not be
 // .nc ones (no const __restrict__), since it is resident while the kernel before it still writes.
+// For kernels whose outputs are activations: what weights, scales or zero points are made by calls griddep_wait()
+// alone, since matmuls may read those ahead of their own wait.
 __device__ __forceinline__ void griddep_chain() {
   griddep_wait();
   griddep_launch_dependents();

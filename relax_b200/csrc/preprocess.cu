@@ -32,7 +32,7 @@ __device__ __forceinline__ uint32_t load_code(const uint8_t* src, int64_t n, int
 // A thread per word: its eight columns are neighbours, 16 bytes where the output allows (with the
 // repack, k 4096 x n 11008: 16.2 -> 11.0 us; a thread per column with two 64-bit divisions before).
 __global__ void __launch_bounds__(256) unpack_zeros_autogptq_kernel(const uint32_t* zq, __half* out, int64_t words, bool vec) {
-  griddep_chain();
+  griddep_wait();  // zero points are read like weights: no dependent may start before they are written
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < words; i += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t q = zq[i];
     __half v[8];
