@@ -35,7 +35,6 @@
 namespace rb200 {
 namespace rk {
 
-constexpr int kRows = 2;         // row blocks of one pass: activations fetched once serve both
 constexpr int kMaxBatch = 16;   // two m-tiles of eight rows
 constexpr int kEntryRows = 8;   // grouped form: batch rows of one entry
 constexpr int kLeadChunks = 2;   // chunks between an L2 prefetch and the load
@@ -62,6 +61,11 @@ enum ScaleSrc : int {
 // beside the same rows of the other in the MMA's eight columns, was no faster (k 4096 x n 12288 8.9 / 9.1,
 // k 11008 x n 4096 8.0 / 8.6).
 constexpr bool folds(int src, int m_tiles) { return src != kRow32 && src != kGeneral && m_tiles == 1; }
+
+// Row blocks of one pass: activations fetched once serve both.  With a scale and a zero point per group of 32 the two
+// need more registers than there are (384 to 640 bytes spilled), and one is faster (three layers of hidden 4096, ffn
+// 11008: one row 166 -> 149 us, eight 182 -> 157; k 4096 x n 22016, eight rows 24.0 -> 21.4).
+constexpr int pass_rows(int src, int zmode) { return src == kRow32 && zmode == kZeroGeneral ? 1 : 2; }
 
 struct Params {
   GemvParams g;
@@ -118,6 +122,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   constexpr int kLaneK = kFrag / 4;
   constexpr int kXV = BITS == 4 ? 2 : 1;  // 16-byte pieces of x per lane and tile
   constexpr bool kZ = ZMODE == kZeroGeneral;
+  constexpr int kRows = pass_rows(SRC, ZMODE);
   constexpr bool kFold = folds(SRC, MT);
   constexpr bool kFoldAll = kFold && SRC == kChannel;  // the sums run over all of k
   __shared__ __align__(16) float4 red[2][kWarps][kRows * MT][32];
@@ -330,13 +335,15 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
       s_left = pp.per - (int)(unit - grp * (unsigned)pp.per);
     }
     if (c0 < c1) {
-      if (q.rn == 2) {
-        load_set(I0{}, I2{}, c0);
-        load_set(I1{}, I2{}, c0);
-      } else {
-        load_set(I0{}, I1{}, c0);
-        load_set(I1{}, I1{}, c0);
+      if constexpr (kRows == 2) {
+        if (q.rn == 2) {
+          load_set(I0{}, I2{}, c0);
+          load_set(I1{}, I2{}, c0);
+          return;
+        }
       }
+      load_set(I0{}, I1{}, c0);
+      load_set(I1{}, I1{}, c0);
     }
   };
 
@@ -579,8 +586,12 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
     };
     if (c0 < c1) {
       if (kXAhead && !kXEarly) load_x(xa, 0);
-      if (q.rn == 2) all_chunks(I2{});
-      else all_chunks(I1{});
+      if constexpr (kRows == 2) {
+        if (q.rn == 2) all_chunks(I2{});
+        else all_chunks(I1{});
+      } else {
+        all_chunks(I1{});
+      }
     }
 
     if (warp == kWarps - 1) {  // tiles of a short last chunk
