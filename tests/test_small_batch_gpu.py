@@ -133,3 +133,14 @@ def test_infinite_activation(oracle, form, m):
         exp = x.astype(np.float64) @ wq.T
     assert np.array_equal(np.isnan(got), np.isnan(exp))
     assert np.array_equal(np.isposinf(got), np.isposinf(exp)) and np.array_equal(np.isneginf(got), np.isneginf(exp))
+
+
+@pytest.mark.parametrize("m", [1, 8, 9, 16])
+@pytest.mark.parametrize("k,n", [(256, 16), (2304, 400), (4096, 4752)])
+def test_group_32_with_zero_points(oracle, m, k, n):
+    """one row block per pass: a single one, a short last row tile, several passes per CTA"""
+    case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, 32, asymmetric=True)
+    pre, s, z, x = ops.preprocess_weight_q4f16(u32_to_dev(case.w)), to_dev(case.scales), to_dev(case.zeros), to_dev(case.x)
+    out = ops.gemm_fp16_q4f16(x, pre, s, z, group_size=32).cpu().numpy()
+    C = oracle.C()
+    assert_close(out, C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, case.zeros, 7.0, 32))))
