@@ -58,9 +58,11 @@ constexpr uint32_t rounding_sum() {
   return sum;
 }
 
-__device__ __forceinline__ __half2 abs_max(uint4 v) {  // drops NaN operands, as fmaxf does
+// without the NaNs: __hmax2 drops one NaN operand and gives NaN for two, hence the maximum with zero
+__device__ __forceinline__ __half2 abs_max(uint4 v) {
   const __half2* h = reinterpret_cast<const __half2*>(&v);
-  return __hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3])));
+  return __hmax2(__hmax2(__hmax2(__habs2(h[0]), __habs2(h[1])), __hmax2(__habs2(h[2]), __habs2(h[3]))),
+                 __half2half2(__ushort_as_half(0)));
 }
 __device__ __forceinline__ __half2 abs_max_nan(uint4 v) {  // 0x7fff for a NaN
   const __half2* h = reinterpret_cast<const __half2*>(&v);
@@ -223,7 +225,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
 #pragma unroll
         for (int i = 0; i < kOwnRows / 2; ++i) {
           const __half2 a = abs_max(v[2 * i]), b = abs_max(v[2 * i + 1]);
-          m[i] = __hmax2(__hmax2(__lows2half2(a, b), __highs2half2(a, b)), __half2half2(__ushort_as_half(0)));
+          m[i] = __hmax2(__lows2half2(a, b), __highs2half2(a, b));
         }
       }
       __syncwarp();

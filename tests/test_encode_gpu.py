@@ -89,3 +89,33 @@ def test_encode_with_several_tiles_per_cta(oracle, bits, group, n, k):
         packed, scales = ops.encode_ft(w, bits, group)
         assert np.array_equal(scales.cpu().numpy().view(np.uint16), exp_scales.view(np.uint16))
         assert np.array_equal(packed.cpu().numpy(), exp_packed)
+
+
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("k", [512, 4096, 12288])
+def test_row_maximum_without_the_nans(oracle, bits, k):
+    """One scale per row, one, eight and sixteen CTAs a cluster: whole vectors of NaN, and NaN at the even or the
+    odd places of one only, in the first, a middle and the last slice.  NaN is no maximum, in any pattern."""
+    n, finite = 64, np.random.RandomState(k + bits).normal(0, 0.02, size=(64, k)).astype(np.float16)
+    nan = np.zeros((n, k), dtype=bool)
+    for r, (at, places) in enumerate([(at, p) for at in (0, k // 2 // 8 * 8, k - 8)
+                                      for p in (slice(0, 8), slice(0, 8, 2), slice(1, 8, 2), slice(3, 4))]):
+        nan[2 * r, at:at + 8][places] = True
+    nan[25, :k // 2] = True
+    nan[27, 1::2] = True
+    y = finite.copy()
+    y[nan] = np.float16(np.nan)
+    y[4] = -y[4]  # NaN with the sign set
+    got, scales = ops.encode_ft(to_dev(y), bits)
+    want, want_scales = ops.encode_ft(to_dev(np.concatenate([y, y[:2]])), bits)  # the any-shape kernel
+    assert torch.equal(scales.view(torch.int16), want_scales[:n].view(torch.int16))
+    assert torch.equal(got, want[:, :n // 2 if bits == 4 else n])
+    finite[nan] = 0
+    finite[4] = -finite[4]
+    exp, exp_scales = oracle.np_encode_ft(finite, bits, -1)
+    assert np.array_equal(scales.cpu().numpy().view(np.uint16), exp_scales.view(np.uint16).reshape(-1))
+
+    def codes(p):  # [n, k]
+        p = p.view(np.uint8).T
+        return np.stack([p & 15, p >> 4], axis=1).reshape(n, k) if bits == 4 else p
+    assert np.array_equal(codes(got.cpu().numpy())[~nan], codes(exp)[~nan])
