@@ -37,8 +37,8 @@ RB200_API void* rb200_get_stream(void);
 
 /*
  * Reads (and clears) the device-side status words that bounded waits inside the kernels set
- * when they give up: the one in the library's per-device scratch block and the one in the static
- * array of rb200_gemm_fp16_intx_noalloc.  Synchronises the given stream.  0 = no error recorded,
+ * when they give up: the one in the library's per-device scratch block, the one in the static
+ * array of rb200_gemm_fp16_intx_noalloc and that of rb200_encode_ft.  Synchronises the given stream.  0 = no error recorded,
  * 1 = a wait ran out (the kernel skipped its remaining work and left outputs unwritten).
  * Allocates nothing: a status word that no call has created yet reads as 0.  After a non-zero
  * status it synchronises the device and puts the split-k flags, tickets and hand-over words back at rest.

@@ -260,9 +260,9 @@ int rb200_set_stream(void* stream) {
 void* rb200_get_stream(void) { return g_stream; }
 
 int rb200_check_async_error(void* stream, int* status_out) {
-  // Two status words can exist on a device: the one in the library's lazily allocated scratch
-  // block (every entry point but the no-alloc one) and the one in the no-alloc entry's static
-  // array.  Neither is created here: a host that only ever used the no-alloc entry must be
+  // Three status words can exist on a device: the one in the library's lazily allocated scratch
+  // block (every entry point but the next two), the one in the no-alloc entry's static array and
+  // the quantiser's.  None is created here: a host that only ever used the no-alloc entry must be
   // able to ask without triggering a device allocation.
   int st = 0;
   RB200_CUDA(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)));
@@ -279,9 +279,9 @@ int rb200_check_async_error(void* stream, int* status_out) {
       st = v;
     }
   }
-  int v2 = 0;
-  if (noalloc_read_status(&v2) != 0) return -1;
-  if (st == 0) st = v2;
+  int v2 = 0, v3 = 0;
+  if (noalloc_read_status(&v2) != 0 || encode_read_status(&v3) != 0) return -1;
+  if (st == 0) st = v2 != 0 ? v2 : v3;
   if (status_out) *status_out = st;
   return 0;
 }

@@ -57,6 +57,8 @@ int fill_now(void* p, int byte, size_t bytes);
 // Status word of the no-alloc entry point's static array on the current device (0 when that
 // entry has not been used on it); reads and clears it without allocating anything.
 int noalloc_read_status(int* status_out);
+// The same for the quantiser's waits.
+int encode_read_status(int* status_out);
 // Upper bound, in milliseconds, of the waits on flags written by other CTAs or other GPUs
 // (split-k fix-up, all-reduce); 0 = the default of about two seconds.  See rb200_set_wait_limit_ms.
 unsigned wait_limit_ms();

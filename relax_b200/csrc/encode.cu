@@ -22,6 +22,8 @@
 // 35 us; 45 / 55 us with a CTA per slice and a cluster barrier (its loads, its exchange and its arithmetic
 // one after the other, 37 us of it before the first code), and 53 / 50 us with a test for ties per value as well.
 // Loading and exchanging alone take 21 us, the codes 6, their stores (16 bytes of a k at a time) 6.
+#include <atomic>
+
 #include "../../include/relax_b200.h"
 #include "common.cuh"
 
@@ -80,8 +82,13 @@ __device__ __forceinline__ int unit_at(int r, int u) {
   return u ^ (BITS == 4 ? ((r >> 3) & 3) << 1 : (r >> 2) & 7);
 }
 
-// Bounded wait for the maxima other CTAs of the cluster push; a wait that ran out is reported.
-__device__ __forceinline__ void wait_pushed(uint64_t* bar, uint32_t phase, int* status) {
+// Status word of the kernel's waits, read and cleared by encode_read_status.  A word of its own: quantising is what a
+// process does first, before any call has made the library's scratch.
+__device__ int g_status;
+
+// Bounded wait (about two seconds) for the maxima other CTAs of the cluster push; false when it ran out.  (The lanes
+// of a warp wait each for itself: bringing them together first takes 3 % of the whole kernel.)
+__device__ __forceinline__ bool wait_pushed(uint64_t* bar, uint32_t phase) {
 #pragma unroll 1
   for (int i = 0; i < 200000; ++i) {
     uint32_t ok;
@@ -92,9 +99,9 @@ __device__ __forceinline__ void wait_pushed(uint64_t* bar, uint32_t phase, int* 
         : "=r"(ok)
         : "r"(smem_u32(bar)), "r"(phase)
         : "memory");
-    if (ok) return;
+    if (ok) return true;
   }
-  if (status) atomicExch(status, kStatusWaitTimeout);
+  return false;
 }
 
 // Rows in tiles of 32, k in slices that fit shared memory; needs n % 32 == 0, 16-byte rows and
@@ -104,12 +111,13 @@ __device__ __forceinline__ void wait_pushed(uint64_t* bar, uint32_t phase, int* 
 template <int BITS, bool PER_ROW, int kThreads>
 __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
     encode_slices_kernel(const __half* __restrict__ A, int8_t* __restrict__ packed, __half* __restrict__ scales, int64_t N, int64_t K,
-                         int slice, int slices, int group, int* status) {
+                         int slice, int slices, int group) {
   constexpr int kWarps = kThreads / 32, kOwnRows = kRows / kWarps;
   constexpr unsigned kInf = 0x7c00u;
   extern __shared__ __align__(128) uint8_t enc_smem[];
   __shared__ unsigned row_max[kBufs][PER_ROW ? kMaxCluster : 1][kRows];  // PER_ROW: bits of a slice's maximum | NaN << 15
   __shared__ __align__(8) uint64_t max_bar[kBufs];                      // counts the bytes of the maxima
+  __shared__ int gave_up;                                               // a wait for maxima ran out
   const int units = (slice + 63) / 64 * 8;                           // 16-byte units of a row
   const int groups = PER_ROW ? 1 : slice / group;
   uint4* ring = reinterpret_cast<uint4*>(enc_smem);                                          // [kBufs][32][units]
@@ -128,6 +136,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
         mbar_init(&max_bar[i], 1);
         mbar_arrive_expect_tx(&max_bar[i], ranks * kRows * 4);
       }
+      gave_up = 0;
       mbar_fence_init();
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every CTA's barriers exist
@@ -326,17 +335,22 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
       const int next = buf + 1 == kBufs ? 0 : buf + 1;
       asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 2) : "memory");
       if (warp == 0) {
-        wait_pushed(&max_bar[buf], phase, status);
-        unsigned m = 0u;
-        for (unsigned c = 0; c < ranks; ++c) {
-          const unsigned b = row_max[buf][c][lane];
-          m = max(m, b & 0x7fffu);
-          special |= b >= 0x8000u;
+        const bool fine = wait_pushed(&max_bar[buf], phase);
+        if (fine) {
+          unsigned m = 0u;
+          for (unsigned c = 0; c < ranks; ++c) {
+            const unsigned b = row_max[buf][c][lane];
+            m = max(m, b & 0x7fffu);
+            special |= b >= 0x8000u;
+          }
+          special |= set_scale(item, 0, lane, m);
+        } else {
+          gave_up = 1;
+          special = true;  // (gave_up is looked at only then)
         }
-        special |= set_scale(item, 0, lane, m);
         __syncwarp();
         // for the item kBufs further on: no CTA pushes that one before this warp has pushed the next
-        if (lane == 0) mbar_arrive_expect_tx(&max_bar[buf], ranks * kRows * 4);
+        if (lane == 0 && fine) mbar_arrive_expect_tx(&max_bar[buf], ranks * kRows * 4);
       }
       if (item + step < items) push_maxima(item + step, next);
     } else {
@@ -350,6 +364,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
       }
     }
     special = __syncthreads_or(special);
+    if (PER_ROW && special && gave_up) break;  // nothing more is written
     quantise(item, buf, special);
     __syncthreads();  // the buffer is free
     if (item + kBufs * step < items) load(item + kBufs * step, buf);
@@ -358,6 +373,13 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
       buf = 0;
       phase ^= 1u;
     }
+  }
+  if (PER_ROW && gave_up) {
+    // The other CTAs of the cluster have left, or meet here when their own waits run out (they miss what this one has
+    // not pushed), so that none is gone while another still stores into its shared memory.
+    if (tid == 0) atomicExch(&g_status, kStatusWaitTimeout);
+    asm volatile("cp.async.wait_all;" ::: "memory");
+    asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
   }
 }
 
@@ -430,6 +452,9 @@ __global__ void __launch_bounds__(256) encode_ft_kernel(const __half* __restrict
   }
 }
 
+constexpr int kMaxDevices = 64;
+std::atomic<bool> g_launched[kMaxDevices];  // devices whose status word a wait may have set
+
 size_t slices_smem(int64_t slice, int64_t groups) {
   return (size_t)kBufs * kRows * ((slice + 63) / 64 * 128) + (size_t)groups * ((kRows + 1) * 8 + kRows * 8);
 }
@@ -469,9 +494,9 @@ int launch_threads(const void* a, void* packed, void* scales, int64_t n, int64_t
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
-  const DeviceScratch* scratch = device_scratch_if_any();
   RB200_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<const __half*>(a), static_cast<int8_t*>(packed),
-                                static_cast<__half*>(scales), n, k, slice, slices, group, scratch ? scratch->status : nullptr));
+                                static_cast<__half*>(scales), n, k, slice, slices, group));
+  if (dev >= 0 && dev < kMaxDevices) g_launched[dev].store(true, std::memory_order_relaxed);
   return 0;
 }
 
@@ -484,6 +509,23 @@ int launch_slices(const void* a, void* packed, void* scales, int64_t n, int64_t 
 }
 
 }  // namespace
+
+// Status of the quantiser's waits on the current device, cleared when set; 0 where nothing was launched.
+int encode_read_status(int* status_out) {
+  *status_out = 0;
+  int dev = -1;
+  RB200_CUDA(cudaGetDevice(&dev));
+  if (dev < 0 || dev >= kMaxDevices || !g_launched[dev].load(std::memory_order_relaxed)) return 0;
+  int v = 0;
+  RB200_CUDA(cudaMemcpyFromSymbol(&v, g_status, sizeof(int)));
+  if (v != 0) {
+    const int zero = 0;
+    RB200_CUDA(cudaMemcpyToSymbol(g_status, &zero, sizeof(int)));
+  }
+  *status_out = v;
+  return 0;
+}
+
 }  // namespace rb200
 
 using namespace rb200;

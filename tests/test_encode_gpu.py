@@ -2,6 +2,10 @@
 (tests/python/relax/test_codegen_cutlass.py:1391-1457, :1630-1676, :2043-2109): codes and scales
 bit for bit, then the reference tests' whole flow - encode, preprocess, fused decode-matmul -
 against the unquantised product at the reference's tolerance."""
+import os
+import subprocess
+import sys
+
 import numpy as np
 import pytest
 import torch
@@ -10,6 +14,7 @@ from relax_b200 import ops
 from tests.util import to_dev
 
 pytestmark = pytest.mark.gpu
+ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
 
 @pytest.mark.parametrize("bits,group,n,k", [(4, -1, 128, 64), (8, -1, 128, 64), (8, 64, 128, 128), (4, 64, 96, 256),
@@ -119,3 +124,28 @@ def test_row_maximum_without_the_nans(oracle, bits, k):
         p = p.view(np.uint8).T
         return np.stack([p & 15, p >> 4], axis=1).reshape(n, k) if bits == 4 else p
     assert np.array_equal(codes(got.cpu().numpy())[~nan], codes(exp)[~nan])
+
+
+FIRST_CALL = """
+import ctypes
+import torch
+from relax_b200 import _lib, ops
+lib, st = _lib.load(), ctypes.c_int(-1)
+assert lib.rb200_check_async_error(None, ctypes.byref(st)) == 0 and st.value == 0  # before there is any status word
+w = torch.randn(1024, 4096, device="cuda").half()
+graph = torch.cuda.CUDAGraph()
+with torch.cuda.graph(graph):
+    packed, scales = ops.encode_ft(w, 4)
+graph.replay()
+torch.cuda.synchronize()
+assert lib.rb200_check_async_error(None, ctypes.byref(st)) == 0 and st.value == 0
+again, scales_again = ops.encode_ft(w, 4)
+assert torch.equal(packed, again) and torch.equal(scales, scales_again)
+assert lib.rb200_check_async_error(None, ctypes.byref(st)) == 0 and st.value == 0
+"""
+
+
+def test_quantising_is_the_first_call_of_a_process():
+    """Its waits report through a status word that needs no earlier call, here under capture."""
+    r = subprocess.run([sys.executable, "-c", FIRST_CALL], cwd=ROOT, capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0, r.stdout + r.stderr
