@@ -26,6 +26,7 @@
 
 #include "../../include/relax_b200.h"
 #include "common.cuh"
+#include "encode_plan.h"
 
 namespace rb200 {
 namespace {
@@ -463,8 +464,7 @@ template <int BITS, bool PER_ROW, int kThreads>
 int launch_threads(const void* a, void* packed, void* scales, int64_t n, int64_t k, int slice, int group, int slices,
                    size_t smem, cudaStream_t stream) {
   auto kern = encode_slices_kernel<BITS, PER_ROW, kThreads>;
-  static thread_local int configured_device = -1, fit = 0, fit_slices = 0;
-  static thread_local size_t fit_smem = 0;
+  static thread_local FitCache cache;
   int dev = 0;
   RB200_CUDA(cudaGetDevice(&dev));
   cudaLaunchConfig_t cfg = {};
@@ -479,16 +479,18 @@ int launch_threads(const void* a, void* packed, void* scales, int64_t n, int64_t
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  if (configured_device != dev || fit_smem != smem || fit_slices != (int)ranks) {  // clusters that run at the same time
-    RB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
-    RB200_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1));
+  const int fit = cache.get(dev, (int)ranks, smem, [&] {  // clusters that run at the same time
+    int clusters = 0;
     cfg.gridDim = dim3(ranks * (unsigned)sm_count_current(), 1, 1);
-    RB200_CUDA(cudaOccupancyMaxActiveClusters(&fit, kern, &cfg));
-    if (fit < 1) return 1;
-    configured_device = dev;
-    fit_smem = smem;
-    fit_slices = (int)ranks;
-  }
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+        cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
+      cudaGetLastError();  // the kernel for any shape takes it
+      return 0;
+    }
+    return clusters;
+  });
+  if (fit < 1) return 1;
   const int64_t items = n / kRows * (PER_ROW ? 1 : slices);
   cfg.gridDim = dim3((unsigned)(items < fit ? items : fit) * ranks, 1, 1);
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;

@@ -14,8 +14,11 @@ def lib(tmp_path_factory):
     d = tmp_path_factory.mktemp("index")
     src, so = str(d / "index.cc"), str(d / "index.so")
     with open(src, "w") as f:
-        f.write('#include "umma_index.h"\n'
-                'extern "C" int pairs_fit_rows(int k, int bits) { return rb200::us::pairs_fit_rows(k, bits); }\n')
+        f.write('#include "umma_index.h"\n#include "encode_plan.h"\n'
+                'extern "C" int pairs_fit_rows(int k, int bits) { return rb200::us::pairs_fit_rows(k, bits); }\n'
+                'static rb200::FitCache cache;\n'
+                'extern "C" int clusters_fit(int dev, int ranks, long smem, int answer, int* asked) {\n'
+                '  return cache.get(dev, ranks, smem, [&] { ++*asked; return answer; }); }\n')
     subprocess.check_call(["g++", "-O1", "-shared", "-fPIC", "-I" + CSRC, src, "-o", so])
     return ctypes.CDLL(so)
 
@@ -33,3 +36,17 @@ def test_scale_pairs_stay_in_their_row(lib, bits, chunk_blocks):
             for kb in range(chunk * chunk_blocks, (chunk + 1) * chunk_blocks, 2):
                 assert kb % 2 == 0 and kb + 2 <= k_blocks, (k, kb)
     assert fitting == 32768 // (64 * chunk_blocks)
+
+
+def test_a_cluster_that_does_not_fit_leaves_other_shapes_alone(lib):
+    """The answer for one launch shape is never given for another, in particular not a 0."""
+    asked = ctypes.c_int(0)
+
+    def fit(dev, ranks, smem, answer):
+        return lib.clusters_fit(dev, ranks, ctypes.c_long(smem), answer, ctypes.byref(asked))
+    shapes = [(0, 8, 99000), (0, 16, 99000), (0, 8, 200000), (1, 8, 99000)]
+    for answer, shape in enumerate(shapes):
+        assert fit(*shape, answer) == answer
+        assert fit(*shape, 77) == answer  # kept, a 0 too
+    assert fit(*shapes[0], 18) == 18 and fit(*shapes[1], 0) == 0 and fit(*shapes[0], 18) == 18
+    assert asked.value == 7
