@@ -31,10 +31,10 @@
 namespace rb200 {
 namespace {
 
-constexpr int kRows = 32;     // n per CTA
-constexpr int kMaxSpan = 512;  // k per pass through shared memory
-constexpr int kMaxCluster = 16;
-constexpr int kBufs = 3;       // slices of a CTA in shared memory: quantised, maxima being exchanged, on its way
+constexpr int kRows = kEncodeRows;  // n per CTA
+constexpr int kMaxSpan = 512;       // k per pass through shared memory
+constexpr int kMaxCluster = kEncodeMaxCluster;
+constexpr int kPlaces = 3;  // for maxima
 
 // code of one value by the definition: round_half_away(a / scale), clamped
 template <int BITS>
@@ -109,15 +109,17 @@ __device__ __forceinline__ bool wait_pushed(uint64_t* bar, uint32_t phase) {
 // groups of whole 16-byte vectors (the kernel below covers the rest).
 // PER_ROW: the slices of a row form one cluster (rank = slice), the clusters share out the row tiles.
 // Otherwise a slice holds whole groups and the CTAs share out the (row tile, slice) pairs.
-template <int BITS, bool PER_ROW, int kThreads>
+// kBufs: slices of a CTA in shared memory.  Three: quantised, maxima being exchanged, on its way.  Long rows have room
+// for two, and a slice's maxima then leave after the one before has been quantised, or for one.
+template <int BITS, bool PER_ROW, int kThreads, int kBufs>
 __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
     encode_slices_kernel(const __half* __restrict__ A, int8_t* __restrict__ packed, __half* __restrict__ scales, int64_t N, int64_t K,
                          int slice, int slices, int group) {
   constexpr int kWarps = kThreads / 32, kOwnRows = kRows / kWarps;
   constexpr unsigned kInf = 0x7c00u;
   extern __shared__ __align__(128) uint8_t enc_smem[];
-  __shared__ unsigned row_max[kBufs][PER_ROW ? kMaxCluster : 1][kRows];  // PER_ROW: bits of a slice's maximum | NaN << 15
-  __shared__ __align__(8) uint64_t max_bar[kBufs];                      // counts the bytes of the maxima
+  __shared__ unsigned row_max[kPlaces][PER_ROW ? kMaxCluster : 1][kRows];  // PER_ROW: bits of a slice's maximum | NaN << 15
+  __shared__ __align__(8) uint64_t max_bar[kPlaces];                    // counts the bytes of the maxima
   __shared__ int gave_up;                                               // a wait for maxima ran out
   const int units = (slice + 63) / 64 * 8;                           // 16-byte units of a row
   const int groups = PER_ROW ? 1 : slice / group;
@@ -133,7 +135,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
     asm("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
     asm("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
     if (tid == 0) {
-      for (int i = 0; i < kBufs; ++i) {
+      for (int i = 0; i < kPlaces; ++i) {
         mbar_init(&max_bar[i], 1);
         mbar_arrive_expect_tx(&max_bar[i], ranks * kRows * 4);
       }
@@ -167,8 +169,8 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
   // maxima of a slice's rows, pushed to every CTA of the cluster: asynchronous stores that count on the
   // receiver's barrier, since a release of cluster scope would wait for the packed bytes on their way to memory.
   // A CTA may be two items ahead of another (only one warp waits for the maxima of an item before it pushes
-  // the next), so there are as many places for them as buffers.
-  auto push_maxima = [&](unsigned item, int buf) {
+  // the next), so there are three places for them.
+  auto push_maxima = [&](unsigned item, int buf, int place) {
     const int span = span_of(item);
     const uint4* t = ring + (size_t)buf * kRows * units;
     unsigned own[kOwnRows], any = 0u;
@@ -201,8 +203,8 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
       for (int j = 1; j < kOwnRows; ++j)
         if (i == (unsigned)j) v = own[j];
       uint32_t dst, bar;
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&row_max[buf][rank][warp + kWarps * i])), "r"(to));
-      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_u32(&max_bar[buf])), "r"(to));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(smem_u32(&row_max[place][rank][warp + kWarps * i])), "r"(to));
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(bar) : "r"(smem_u32(&max_bar[place])), "r"(to));
       asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.u32 [%0], %1, [%2];" ::"r"(dst), "r"(v), "r"(bar) : "memory");
     }
   };
@@ -323,24 +325,24 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
     commit();
   }
   if (PER_ROW) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
-  int buf = 0;
+  int buf = 0, place = 0;
   uint32_t phase = 0u;
   if (PER_ROW && first < items) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 1) : "memory");
-    push_maxima(first, 0);
+    push_maxima(first, 0, 0);
   }
   for (unsigned item = first; item < items; item += step) {
     bool special = false;
+    const int next = buf + 1 == kBufs ? 0 : buf + 1, next_place = place + 1 == kPlaces ? 0 : place + 1;
     if (PER_ROW) {
       // the next item's maxima are on their way through the cluster while this one is quantised
-      const int next = buf + 1 == kBufs ? 0 : buf + 1;
-      asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 2) : "memory");
+      if (kBufs == 3) asm volatile("cp.async.wait_group 1;" ::: "memory");
       if (warp == 0) {
-        const bool fine = wait_pushed(&max_bar[buf], phase);
+        const bool fine = wait_pushed(&max_bar[place], phase);
         if (fine) {
           unsigned m = 0u;
           for (unsigned c = 0; c < ranks; ++c) {
-            const unsigned b = row_max[buf][c][lane];
+            const unsigned b = row_max[place][c][lane];
             m = max(m, b & 0x7fffu);
             special |= b >= 0x8000u;
           }
@@ -350,10 +352,10 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
           special = true;  // (gave_up is looked at only then)
         }
         __syncwarp();
-        // for the item kBufs further on: no CTA pushes that one before this warp has pushed the next
-        if (lane == 0 && fine) mbar_arrive_expect_tx(&max_bar[buf], ranks * kRows * 4);
+        // for the item kPlaces further on: no CTA pushes that one before this warp has pushed the next
+        if (lane == 0 && fine) mbar_arrive_expect_tx(&max_bar[place], ranks * kRows * 4);
       }
-      if (item + step < items) push_maxima(item + step, next);
+      if (kBufs == 3 && item + step < items) push_maxima(item + step, next, next_place);
     } else {
       asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 1) : "memory");
       special = group_maxima(item, buf);
@@ -370,10 +372,13 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
     __syncthreads();  // the buffer is free
     if (item + kBufs * step < items) load(item + kBufs * step, buf);
     commit();
-    if (++buf == kBufs) {
-      buf = 0;
-      phase ^= 1u;
+    if (PER_ROW && kBufs < 3) {
+      asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 1) : "memory");
+      if (item + step < items) push_maxima(item + step, next, next_place);
     }
+    buf = next;
+    place = next_place;
+    if (place == 0) phase ^= 1u;
   }
   if (PER_ROW && gave_up) {
     // The other CTAs of the cluster have left, or meet here when their own waits run out (they miss what this one has
@@ -456,22 +461,18 @@ __global__ void __launch_bounds__(256) encode_ft_kernel(const __half* __restrict
 constexpr int kMaxDevices = 64;
 std::atomic<bool> g_launched[kMaxDevices];  // devices whose status word a wait may have set
 
-size_t slices_smem(int64_t slice, int64_t groups) {
-  return (size_t)kBufs * kRows * ((slice + 63) / 64 * 128) + (size_t)groups * ((kRows + 1) * 8 + kRows * 8);
-}
-
-template <int BITS, bool PER_ROW, int kThreads>
-int launch_threads(const void* a, void* packed, void* scales, int64_t n, int64_t k, int slice, int group, int slices,
-                   size_t smem, cudaStream_t stream) {
-  auto kern = encode_slices_kernel<BITS, PER_ROW, kThreads>;
+template <int BITS, bool PER_ROW, int kThreads, int kBufs>
+int launch_slices(const void* a, void* packed, void* scales, int64_t n, int64_t k, int group, const EncodePlan& plan,
+                  cudaStream_t stream) {
+  auto kern = encode_slices_kernel<BITS, PER_ROW, kThreads, kBufs>;
   static thread_local FitCache cache;
   int dev = 0;
   RB200_CUDA(cudaGetDevice(&dev));
   cudaLaunchConfig_t cfg = {};
   cfg.blockDim = dim3(kThreads, 1, 1);
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = plan.smem;
   cfg.stream = stream;
-  const unsigned ranks = PER_ROW ? (unsigned)slices : 1u;
+  const unsigned ranks = PER_ROW ? (unsigned)plan.slices : 1u;
   cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeClusterDimension;
   attr[0].val.clusterDim.x = ranks;
@@ -479,10 +480,10 @@ int launch_threads(const void* a, void* packed, void* scales, int64_t n, int64_t
   attr[0].val.clusterDim.z = 1;
   cfg.attrs = attr;
   cfg.numAttrs = 1;
-  const int fit = cache.get(dev, (int)ranks, smem, [&] {  // clusters that run at the same time
+  const int fit = cache.get(dev, (int)ranks, plan.smem, [&] {  // clusters that run at the same time
     int clusters = 0;
     cfg.gridDim = dim3(ranks * (unsigned)sm_count_current(), 1, 1);
-    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024) != cudaSuccess ||
+    if (cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kEncodeSmem) != cudaSuccess ||
         cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
         cudaOccupancyMaxActiveClusters(&clusters, kern, &cfg) != cudaSuccess) {
       cudaGetLastError();  // the kernel for any shape takes it
@@ -491,23 +492,29 @@ int launch_threads(const void* a, void* packed, void* scales, int64_t n, int64_t
     return clusters;
   });
   if (fit < 1) return 1;
-  const int64_t items = n / kRows * (PER_ROW ? 1 : slices);
+  const int64_t items = n / kRows * (PER_ROW ? 1 : plan.slices);
   cfg.gridDim = dim3((unsigned)(items < fit ? items : fit) * ranks, 1, 1);
   attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   cfg.numAttrs = 2;
   RB200_CUDA(cudaLaunchKernelEx(&cfg, kern, static_cast<const __half*>(a), static_cast<int8_t*>(packed),
-                                static_cast<__half*>(scales), n, k, slice, slices, group));
+                                static_cast<__half*>(scales), n, k, plan.slice, plan.slices, group));
   if (dev >= 0 && dev < kMaxDevices) g_launched[dev].store(true, std::memory_order_relaxed);
   return 0;
 }
 
-// two CTAs per SM where a slice is at most 512 k (100 KB of shared memory), else one: sixteen warps either way
-template <int BITS, bool PER_ROW>
-int launch_slices(const void* a, void* packed, void* scales, int64_t n, int64_t k, int slice, int group, int slices,
-                  size_t smem, cudaStream_t stream) {
-  return slice <= 512 ? launch_threads<BITS, PER_ROW, 256>(a, packed, scales, n, k, slice, group, slices, smem, stream)
-                      : launch_threads<BITS, PER_ROW, 512>(a, packed, scales, n, k, slice, group, slices, smem, stream);
+template <int BITS>
+int launch_rows(const void* a, void* packed, void* scales, int64_t n, int64_t k, const EncodePlan& plan, cudaStream_t stream) {
+  if (plan.bufs == 2) return launch_slices<BITS, true, 512, 2>(a, packed, scales, n, k, 0, plan, stream);
+  if (plan.bufs == 1) return launch_slices<BITS, true, 512, 1>(a, packed, scales, n, k, 0, plan, stream);
+  return plan.threads == 256 ? launch_slices<BITS, true, 256, 3>(a, packed, scales, n, k, 0, plan, stream)
+                             : launch_slices<BITS, true, 512, 3>(a, packed, scales, n, k, 0, plan, stream);
+}
+template <int BITS>
+int launch_groups(const void* a, void* packed, void* scales, int64_t n, int64_t k, int group, const EncodePlan& plan,
+                  cudaStream_t stream) {
+  return plan.threads == 256 ? launch_slices<BITS, false, 256, 3>(a, packed, scales, n, k, group, plan, stream)
+                             : launch_slices<BITS, false, 512, 3>(a, packed, scales, n, k, group, plan, stream);
 }
 
 }  // namespace
@@ -544,25 +551,14 @@ extern "C" int rb200_encode_ft(const void* a, void* packed, void* scales, int64_
   cudaStream_t s = static_cast<cudaStream_t>(stream);
   const bool aligned = ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(packed)) & 15u) == 0;
   if (aligned && n % kRows == 0 && k % 8 == 0 && n / kRows < (1ll << 31)) {
-    // slice of k per CTA: 32 rows x 512 k are 32 KB.  One scale per row: the slices of a row are a cluster, of
-    // eight CTAs up to 8192 k and sixteen above (three buffers of longer slices would not fit)
     int rc = 1;
+    EncodePlan plan;
     if (per_row) {
-      int64_t c = 1;
-      while (c < 8 && k > c * 512) c *= 2;
-      if (k > 8192) c = kMaxCluster;
-      const int64_t slice = ((k + c - 1) / c + 7) / 8 * 8;
-      const size_t smem = slices_smem(slice, 1);
-      if (smem <= 200 * 1024 && (c - 1) * slice < k)
-        rc = weight_bits == 4 ? launch_slices<4, true>(a, packed, scales, n, k, (int)slice, 0, (int)c, smem, s)
-                              : launch_slices<8, true>(a, packed, scales, n, k, (int)slice, 0, (int)c, smem, s);
-    } else if (group % 8 == 0 && group <= 1024) {
-      const int64_t slice = (group > 512 ? 1024 : 512) / group * group;
-      const size_t smem = slices_smem(slice, slice / group);
-      const int64_t c = (k + slice - 1) / slice;
-      if (n / kRows * c < (1ll << 31))
-        rc = weight_bits == 4 ? launch_slices<4, false>(a, packed, scales, n, k, (int)slice, (int)group, (int)c, smem, s)
-                              : launch_slices<8, false>(a, packed, scales, n, k, (int)slice, (int)group, (int)c, smem, s);
+      if (plan_encode_rows(k, &plan))
+        rc = weight_bits == 4 ? launch_rows<4>(a, packed, scales, n, k, plan, s) : launch_rows<8>(a, packed, scales, n, k, plan, s);
+    } else if (group % 8 == 0 && plan_encode_groups(k, group, &plan) && n / kRows * plan.slices < (1ll << 31)) {
+      rc = weight_bits == 4 ? launch_groups<4>(a, packed, scales, n, k, (int)group, plan, s)
+                            : launch_groups<8>(a, packed, scales, n, k, (int)group, plan, s);
     }
     if (rc <= 0) return rc;
   }

@@ -126,6 +126,22 @@ def test_row_maximum_without_the_nans(oracle, bits, k):
     assert np.array_equal(codes(got.cpu().numpy())[~nan], codes(exp)[~nan])
 
 
+@pytest.mark.parametrize("bits", [4, 8])
+@pytest.mark.parametrize("n,k", [(32, 16384), (32, 16392), (32 * 40, 18944), (64, 24576), (64, 24584), (32 * 40, 28672),
+                                 (32, 50176), (32, 50184)])
+def test_encode_of_rows_beyond_three_buffers(oracle, bits, n, k):
+    """Two buffers or one a CTA, one and several row tiles a cluster, and the first length that is left to the
+    kernel for any shape."""
+    rs = np.random.RandomState(bits + k)
+    y = (rs.standard_normal((n, k)).astype(np.float32) * rs.uniform(0.001, 0.2, size=(n, 1)).astype(np.float32)).astype(np.float16)
+    exp_packed, exp_scales = oracle.np_encode_ft(y, bits, -1)
+    w = to_dev(y)
+    for _ in range(3):
+        packed, scales = ops.encode_ft(w, bits)
+        assert np.array_equal(scales.cpu().numpy().view(np.uint16), exp_scales.view(np.uint16))
+        assert np.array_equal(packed.cpu().numpy(), exp_packed)
+
+
 FIRST_CALL = """
 import ctypes
 import torch

@@ -18,7 +18,9 @@ def lib(tmp_path_factory):
                 'extern "C" int pairs_fit_rows(int k, int bits) { return rb200::us::pairs_fit_rows(k, bits); }\n'
                 'static rb200::FitCache cache;\n'
                 'extern "C" int clusters_fit(int dev, int ranks, long smem, int answer, int* asked) {\n'
-                '  return cache.get(dev, ranks, smem, [&] { ++*asked; return answer; }); }\n')
+                '  return cache.get(dev, ranks, smem, [&] { ++*asked; return answer; }); }\n'
+                'extern "C" int encode_rows(long k, int* out) { rb200::EncodePlan p; if (!rb200::plan_encode_rows(k, &p)) return 0;\n'
+                '  out[0] = p.slice, out[1] = p.slices, out[2] = p.bufs, out[3] = p.threads, out[4] = (int)p.smem; return 1; }\n')
     subprocess.check_call(["g++", "-O1", "-shared", "-fPIC", "-I" + CSRC, src, "-o", so])
     return ctypes.CDLL(so)
 
@@ -50,3 +52,20 @@ def test_a_cluster_that_does_not_fit_leaves_other_shapes_alone(lib):
         assert fit(*shape, 77) == answer  # kept, a 0 too
     assert fit(*shapes[0], 18) == 18 and fit(*shapes[1], 0) == 0 and fit(*shapes[0], 18) == 18
     assert asked.value == 7
+
+
+def test_rows_up_to_50176_are_read_once(lib):
+    """The quantiser's slices cover every row, none of them empty, in shared memory that a CTA can have; the kernel
+    that reads twice is left to rows beyond what one buffer of sixteen CTAs holds."""
+    out, most = (ctypes.c_int * 5)(), {1: 0, 2: 0, 3: 0}
+    for k in range(8, 60001, 8):
+        planned = lib.encode_rows(ctypes.c_long(k), out)
+        assert planned == (k <= 50176), k
+        if not planned:
+            continue
+        piece, pieces, bufs, threads, smem = out
+        assert piece % 8 == 0 and piece * pieces >= k > piece * (pieces - 1) and pieces <= 16, k
+        assert bufs * 32 * -(-piece // 64) * 128 < smem <= 200 * 1024, k
+        assert threads == 512 or (bufs == 3 and 2 * (smem + 8 * 1024) <= 228 * 1024), k
+        most[bufs] = max(most[bufs], k)
+    assert most == {3: 16384, 2: 24576, 1: 50176}
