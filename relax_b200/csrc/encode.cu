@@ -120,7 +120,6 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
   extern __shared__ __align__(128) uint8_t enc_smem[];
   __shared__ unsigned row_max[kPlaces][PER_ROW ? kMaxCluster : 1][kRows];  // PER_ROW: bits of a slice's maximum | NaN << 15
   __shared__ __align__(8) uint64_t max_bar[kPlaces];                    // counts the bytes of the maxima
-  __shared__ int gave_up;                                               // a wait for maxima ran out
   const int units = (slice + 63) / 64 * 8;                           // 16-byte units of a row
   const int groups = PER_ROW ? 1 : slice / group;
   uint4* ring = reinterpret_cast<uint4*>(enc_smem);                                          // [kBufs][32][units]
@@ -139,7 +138,6 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
         mbar_init(&max_bar[i], 1);
         mbar_arrive_expect_tx(&max_bar[i], ranks * kRows * 4);
       }
-      gave_up = 0;
       mbar_fence_init();
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every CTA's barriers exist
@@ -326,13 +324,15 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
   }
   if (PER_ROW) asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
   int buf = 0, place = 0;
+  bool gave_up = false;  // a wait for maxima ran out
   uint32_t phase = 0u;
   if (PER_ROW && first < items) {
     asm volatile("cp.async.wait_group %0;" ::"n"(kBufs - 1) : "memory");
     push_maxima(first, 0, 0);
   }
   for (unsigned item = first; item < items; item += step) {
-    bool special = false;
+    bool special = false;  // the division has to make the codes
+    bool lost = false;     // the wait for the item's maxima ran out
     const int next = buf + 1 == kBufs ? 0 : buf + 1, next_place = place + 1 == kPlaces ? 0 : place + 1;
     if (PER_ROW) {
       // the next item's maxima are on their way through the cluster while this one is quantised
@@ -348,8 +348,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
           }
           special |= set_scale(item, 0, lane, m);
         } else {
-          gave_up = 1;
-          special = true;  // (gave_up is looked at only then)
+          special = lost = true;
         }
         __syncwarp();
         // for the item kPlaces further on: no CTA pushes that one before this warp has pushed the next
@@ -367,7 +366,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
       }
     }
     special = __syncthreads_or(special);
-    if (PER_ROW && special && gave_up) break;  // nothing more is written
+    if (PER_ROW && special && (gave_up = __syncthreads_or(lost))) break;  // nothing more is written
     quantise(item, buf, special);
     __syncthreads();  // the buffer is free
     if (item + kBufs * step < items) load(item + kBufs * step, buf);
