@@ -125,7 +125,8 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
   uint4* ring = reinterpret_cast<uint4*>(enc_smem);                                          // [kBufs][32][units]
   float2* quant = reinterpret_cast<float2*>(enc_smem + (size_t)kBufs * kRows * units * 16);  // [groups][33]: reciprocal, clamp
   float* s_scale = reinterpret_cast<float*>(quant + (kRows + 1) * groups);                   // [groups][32]
-  unsigned* amax = reinterpret_cast<unsigned*>(s_scale + kRows * groups);                    // [32][groups] fp16 bits
+  unsigned* amax = reinterpret_cast<unsigned*>(s_scale + kRows * groups);                    // [32][amax_pitch] fp16 bits
+  const int amax_pitch = encode_amax_pitch(groups);
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const float mul = BITS == 4 ? 0.125f : 0.0078125f;
   const unsigned n_tiles = (unsigned)(N / kRows);
@@ -142,7 +143,7 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
     }
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");  // every CTA's barriers exist
   } else {
-    for (int i = tid; i < kRows * groups; i += kThreads) amax[i] = 0u;
+    for (int i = tid; i < kRows * amax_pitch; i += kThreads) amax[i] = 0u;
     __syncthreads();
   }
   // this CTA's items
@@ -247,8 +248,8 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
 #pragma unroll
         for (int i = 0; i < kOwnRows; ++i) {
           const unsigned b = __half_as_ushort(i & 1 ? __high2half(m[i / 2]) : __low2half(m[i / 2]));
-          if (fold_seg) amax[row_of(i) * groups + g] = b;
-          else atomicMax(&amax[row_of(i) * groups + g], b);
+          if (fold_seg) amax[row_of(i) * amax_pitch + g] = b;
+          else atomicMax(&amax[row_of(i) * amax_pitch + g], b);
         }
       }
     }
@@ -361,8 +362,8 @@ __global__ void __launch_bounds__(kThreads, kThreads == 256 ? 2 : 1)
       __syncthreads();
       for (int i = tid; i < kRows * (span_of(item) / group); i += kThreads) {
         const int r = i % kRows, g = i / kRows;
-        special |= set_scale(item, g, r, amax[r * groups + g]);
-        amax[r * groups + g] = 0u;
+        special |= set_scale(item, g, r, amax[r * amax_pitch + g]);
+        amax[r * amax_pitch + g] = 0u;
       }
     }
     special = __syncthreads_or(special);

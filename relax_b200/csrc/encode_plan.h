@@ -17,9 +17,19 @@ constexpr int kEncodeRows = 32;
 constexpr int kEncodeMaxCluster = 16;
 constexpr size_t kEncodeSmem = 200 * 1024;
 
+// Words from a row's group maxima to the next row's: odd, since a warp reads one group of all rows (fp16 11008 x 4096,
+// groups of 8, an even pitch: 84 us instead of 55; groups of 16 53 instead of 41).
+constexpr int encode_amax_pitch(int groups) { return groups | 1; }
+
 inline size_t encode_smem(int64_t slice, int64_t groups, int bufs) {
-  return (size_t)bufs * kEncodeRows * ((slice + 63) / 64 * 128) + (size_t)groups * ((kEncodeRows + 1) * 8 + kEncodeRows * 8);
+  return (size_t)bufs * kEncodeRows * ((slice + 63) / 64 * 128) + (size_t)groups * ((kEncodeRows + 1) * 8 + kEncodeRows * 4) +
+         (size_t)kEncodeRows * encode_amax_pitch((int)groups) * 4;
 }
+
+// Sixteen warps an SM: two CTAs of eight where two fit, else one of sixteen.  Two fit with slices of up to 512 k, but not
+// with groups of 8, whose scales bring the shared memory to 129 KB (fp16 11008 x 4096, groups of 8: int4 55 us, with one
+// CTA of eight warps 59; int8 55 / 64).  `places`: words for maxima; 1 KB of a CTA is the system's.
+inline int encode_threads(size_t smem, size_t places) { return 2 * (smem + places * 4 + 64 + 1024) <= 228 * 1024 ? 256 : 512; }
 
 // One scale per row (k % 8 == 0).  The slices of a row are a cluster, of eight CTAs up to 8192 k and sixteen above.
 // Three buffers hold slices of up to 1024 k; above, two (up to 24576 k) and then one are still several times faster
@@ -33,8 +43,7 @@ inline bool plan_encode_rows(int64_t k, EncodePlan* p) {
   while (bufs > 1 && encode_smem(slice, 1, bufs) > kEncodeSmem) --bufs;
   const size_t smem = encode_smem(slice, 1, bufs);
   if (smem > kEncodeSmem || (c - 1) * slice >= k) return false;
-  // two CTAs per SM where a slice is at most 512 k (100 KB of shared memory), else one: sixteen warps either way
-  *p = EncodePlan{(int)slice, (int)c, bufs, slice <= 512 ? 256 : 512, smem};
+  *p = EncodePlan{(int)slice, (int)c, bufs, bufs == 3 ? encode_threads(smem, 3 * kEncodeMaxCluster * kEncodeRows) : 512, smem};
   return true;
 }
 
@@ -43,7 +52,8 @@ inline bool plan_encode_groups(int64_t k, int64_t group, EncodePlan* p) {
   if (group > 1024) return false;
   const int64_t slice = (group > 512 ? 1024 : 512) / group * group, c = (k + slice - 1) / slice;
   if (c >= (1ll << 31)) return false;
-  *p = EncodePlan{(int)slice, (int)c, 3, slice <= 512 ? 256 : 512, encode_smem(slice, slice / group, 3)};
+  const size_t smem = encode_smem(slice, slice / group, 3);
+  *p = EncodePlan{(int)slice, (int)c, 3, encode_threads(smem, 3 * kEncodeRows), smem};
   return true;
 }
 

@@ -126,6 +126,13 @@ def test_row_maximum_without_the_nans(oracle, bits, k):
     assert np.array_equal(codes(got.cpu().numpy())[~nan], codes(exp)[~nan])
 
 
+@pytest.mark.parametrize("bits,group", [(4, 8), (8, 8), (4, 16), (8, 1024)])
+def test_encode_of_the_smallest_and_largest_groups(oracle, bits, group):
+    """Groups of 8 have the most scales in shared memory, one CTA of sixteen warps an SM."""
+    test_encode_of_long_rows_ties_and_special_values(oracle, bits, group, 4096)
+    test_encode_with_several_tiles_per_cta(oracle, bits, group, 32 * 131, 4096)
+
+
 @pytest.mark.parametrize("bits", [4, 8])
 @pytest.mark.parametrize("n,k", [(32, 16384), (32, 16392), (32 * 40, 18944), (64, 24576), (64, 24584), (32 * 40, 28672),
                                  (32, 50176), (32, 50184)])

@@ -20,6 +20,9 @@ def lib(tmp_path_factory):
                 'extern "C" int clusters_fit(int dev, int ranks, long smem, int answer, int* asked) {\n'
                 '  return cache.get(dev, ranks, smem, [&] { ++*asked; return answer; }); }\n'
                 'extern "C" int encode_rows(long k, int* out) { rb200::EncodePlan p; if (!rb200::plan_encode_rows(k, &p)) return 0;\n'
+                '  out[0] = p.slice, out[1] = p.slices, out[2] = p.bufs, out[3] = p.threads, out[4] = (int)p.smem; return 1; }\n'
+                'extern "C" int encode_groups(long k, long group, int* out) { rb200::EncodePlan p;\n'
+                '  if (!rb200::plan_encode_groups(k, group, &p)) return 0;\n'
                 '  out[0] = p.slice, out[1] = p.slices, out[2] = p.bufs, out[3] = p.threads, out[4] = (int)p.smem; return 1; }\n')
     subprocess.check_call(["g++", "-O1", "-shared", "-fPIC", "-I" + CSRC, src, "-o", so])
     return ctypes.CDLL(so)
@@ -66,6 +69,18 @@ def test_rows_up_to_50176_are_read_once(lib):
         piece, pieces, bufs, threads, smem = out
         assert piece % 8 == 0 and piece * pieces >= k > piece * (pieces - 1) and pieces <= 16, k
         assert bufs * 32 * -(-piece // 64) * 128 < smem <= 200 * 1024, k
-        assert threads == 512 or (bufs == 3 and 2 * (smem + 8 * 1024) <= 228 * 1024), k
+        assert threads == (256 if piece <= 512 else 512), k  # two CTAs an SM, or one
         most[bufs] = max(most[bufs], k)
     assert most == {3: 16384, 2: 24576, 1: 50176}
+
+
+@pytest.mark.parametrize("group", list(range(8, 1025, 8)))
+def test_groups_are_whole_in_a_slice_and_an_sm_has_sixteen_warps(lib, group):
+    out = (ctypes.c_int * 5)()
+    for k in (group * 2, group * 3, group * 130):
+        assert lib.encode_groups(ctypes.c_long(k), ctypes.c_long(group), out)
+        piece, pieces, bufs, threads, smem = out
+        assert bufs == 3 and piece % group == 0 and piece * pieces >= k > piece * (pieces - 1)
+        assert 3 * 32 * -(-piece // 64) * 128 < smem <= 200 * 1024
+        two = 2 * (smem + 1536) <= 228 * 1024
+        assert threads == (256 if two else 512) and (group == 8) == (piece <= 512 and not two)
