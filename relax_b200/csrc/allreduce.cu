@@ -147,7 +147,7 @@ __global__ void __launch_bounds__(kArThreads) allreduce_oneshot_kernel(const ArP
           acc[2 * i + 1] += f.y;
         }
       }
-      __half res[8];
+      __align__(16) __half res[8];
 #pragma unroll
       for (int i = 0; i < 8; ++i) res[i] = __float2half_rn(acc[i]);
       if (u * 8 + 8 <= p.count) {

@@ -35,7 +35,7 @@ __global__ void __launch_bounds__(256) unpack_zeros_autogptq_kernel(const uint32
   griddep_wait();  // zero points are read like weights: no dependent may start before they are written
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < words; i += (int64_t)gridDim.x * blockDim.x) {
     const uint32_t q = zq[i];
-    __half v[8];
+    __align__(16) __half v[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = __hadd(__int2half_rn((int)((q >> (4 * j)) & 15u)), __float2half_rn(1.0f));
     if (vec) {
@@ -333,7 +333,7 @@ __global__ void __launch_bounds__(128) gather_columns_kernel(const __half* x, co
   griddep_chain();
   const int64_t j = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * VEC;
   if (j >= K) return;
-  int32_t from[VEC];
+  __align__(16) int32_t from[VEC];
   if (VEC == 8) {
     *reinterpret_cast<int4*>(from) = *reinterpret_cast<const int4*>(perm + j);
     *reinterpret_cast<int4*>(from + 4) = *reinterpret_cast<const int4*>(perm + j + 4);

@@ -410,7 +410,7 @@ __device__ __forceinline__ bool drain_store(const Params& pp, const DrainTile& t
       if (m < t.m_end && t.n0 + q * 16 < p.n) {
         const float4* src = reinterpret_cast<const float4*>(st + mi * kTileRows + q * 16);
         const float4 g0 = src[0], g1 = src[1], u0 = src[2], u1 = src[3];
-        __half2 res[4];
+        __align__(16) __half2 res[4];
         res[0] = __floats2half2_rn(silu_mul(g0.x, u0.x), silu_mul(g0.y, u0.y));
         res[1] = __floats2half2_rn(silu_mul(g0.z, u0.z), silu_mul(g0.w, u0.w));
         res[2] = __floats2half2_rn(silu_mul(g1.x, u1.x), silu_mul(g1.y, u1.y));
