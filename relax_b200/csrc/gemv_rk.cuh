@@ -240,9 +240,19 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   // kHalf, kTile, kGeneral: per half or tile, rows g, g + 8; a word each where registers allow it (as
   // one word they are waited for soon after their loads: int4 k 4096 x n 57344, group 128 36.6 -> 35.0 us)
   uint32_t sg[2][kRows][2][2], zg[2][kRows][2];
-  uint32_t ch_s[kRows][2], ch_z[kRows][2];     // kChannel: rows g, g + 8, apart for the same reason: they are loaded
-                                               // before a pass's first weights (int4 k 4096 x n 22016, one row
-                                               // 11.5 -> 11.3 us, thirteen 17.4 -> 17.3)
+  // kChannel: rows g, g + 8.  They are loaded before a pass's first weights and, as one word, waited for there, so
+  // without zero points they are a word each (int4 k 4096 x n 22016, one row: 12.2 us as one word, 12.0 apart).  Beside
+  // zero points that is so for int4 at nine to sixteen rows only (k = n = 4096, sixteen rows 6.37 / 6.16); int8 spills
+  // 28 bytes there (k 4096 x n 22016, twelve rows 23.1 / 23.9; k 11008 x n 4096, sixteen 12.6 / 13.0), and at up to
+  // eight rows one word is as fast or faster (int4 k = n = 4096, one row 4.24 / 4.33, n 22016 13.7 / 13.8).
+  constexpr bool kApart = !kZ || (BITS == 4 && MT == 2);
+  uint32_t ch_s[kRows][2], ch_z[kRows][2];  // kApart: rows g, g + 8; else both in the first
+  // of row g (i = 0) or g + 8, twice; of both
+  auto ch_twice = [](const uint32_t (&v)[2], int i) {
+    const uint32_t w = kApart ? v[i] : v[0];
+    return prmt(w, w, kApart || i == 0 ? 0x1010u : 0x3232u);
+  };
+  auto ch_both = [](const uint32_t (&v)[2]) { return kApart ? prmt(v[0], v[1], 0x5410u) : v[0]; };
   const uint8_t* wp = nullptr;                 // next chunk to load
   const __half *sp[kRows][2], *zp[kRows][2];   // scales of rows g, g + 8 (kRow32: of the next chunk)
   int stride = 0;                              // bytes from a chunk to the next
@@ -322,10 +332,13 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
         zp[r][i] = p.z + o + i * row8;
       }
       if (SRC == kChannel) {
-#pragma unroll
-        for (int i = 0; i < 2; ++i) {
-          ch_s[r][i] = ld_nc_u16(sp[r][i]);
-          if (has_zeros) ch_z[r][i] = ld_nc_u16(zp[r][i]);
+        const uint32_t a = ld_nc_u16(sp[r][0]), b = ld_nc_u16(sp[r][1]);
+        ch_s[r][0] = kApart ? a : a | (b << 16);
+        ch_s[r][1] = b;
+        if (has_zeros) {
+          const uint32_t za = ld_nc_u16(zp[r][0]), zb = ld_nc_u16(zp[r][1]);
+          ch_z[r][0] = kApart ? za : za | (zb << 16);
+          ch_z[r][1] = zb;
         }
       }
     }
@@ -470,7 +483,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
     if (kFoldAll && has_zeros) {
       uint32_t z2[kRows];
 #pragma unroll
-      for (int r = 0; r < kRows; ++r) z2[r] = prmt(ch_z[r][0], ch_z[r][1], 0x5410u);
+      for (int r = 0; r < kRows; ++r) z2[r] = ch_both(ch_z[r]);
       ch_zeros = zeros_of(z2);
     }
     auto in_units = [&](const Zeros& z, auto&& f) {
@@ -529,11 +542,11 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
               z_g8 = prmt(zb, zb, half_sel);
             }
           } else if (SRC == kChannel) {
-            s_g = prmt(ch_s[r][0], ch_s[r][0], 0x1010u);
-            s_g8 = prmt(ch_s[r][1], ch_s[r][1], 0x1010u);
+            s_g = ch_twice(ch_s[r], 0);
+            s_g8 = ch_twice(ch_s[r], 1);
             if (has_zeros) {
-              z_g = prmt(ch_z[r][0], ch_z[r][0], 0x1010u);
-              z_g8 = prmt(ch_z[r][1], ch_z[r][1], 0x1010u);
+              z_g = ch_twice(ch_z[r], 0);
+              z_g8 = ch_twice(ch_z[r], 1);
             }
           } else {
             const uint32_t a = sg[S][r][SRC == kHalf ? 0 : j][0];
@@ -645,7 +658,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
     for (int r = 0; r < kRows; ++r)
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
-        done_s[r][i] = kFoldAll ? half_of(ch_s[r][i], 0) : 1.0f;
+        done_s[r][i] = !kFoldAll ? 1.0f : (kApart ? half_of(ch_s[r][i], 0) : half_of(ch_s[r][0], i));
         if (kFoldAll && kZ && !ch_zeros.codes) done_s[r][i] *= i ? kUnitHi : kUnitLo;
       }
     pos += (unsigned)q.rn;
