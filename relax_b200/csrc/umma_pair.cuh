@@ -450,7 +450,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       return drain_store<true, folds<ZMODE, SRC>()>(pp, dt, me, last, 2, e_stage + grp * kStageBytes, parity, group_sync);
     };
 
-    ScaleFeed<BITS, ZMODE, SRC, kStepBlk> feed;
+    ScaleFeed<BITS, ZMODE, SRC, kStepBlk, true> feed;
     feed.init(pp, hi);
     int db = 0;
     uint32_t dph = 0;

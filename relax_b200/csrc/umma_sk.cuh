@@ -343,7 +343,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
     bool waited = grouped || !pp.early;
 
     const int k_blocks = p.k / kKBlock;
-    ScaleFeed<BITS, ZMODE, SRC, kOwn> feed;
+    ScaleFeed<BITS, ZMODE, SRC, kOwn, BITS == 8> feed;
     feed.init(pp, hi);
     auto fetch = [&](int c) {
       const int kb = c * kBlkPerChunk + grp * kOwn;

@@ -242,12 +242,18 @@ __device__ __forceinline__ void decode_own(const Params& pp, const Feed& feed, i
 }
 
 // Scales and zero points of the blocks one group of warps decodes, fetched a chunk ahead.
-template <int BITS, int ZMODE, int SRC, int OWN>
+// APART: where a kTwo block's two groups are no word, they are put together when their chunk's turn comes and not
+// where they are loaded, which would wait for the loads there (int8 in groups of 32: k 8192 x n 8192, 256 rows 87 us
+// put together at the load, 53 apart, k 4096 x n 22016, 32 rows 33.6 / 28.4; int4 with scales [K/32, N], 128 rows,
+// k 4096 x n 22016 41.4 / 31.8).  Int4 on one CTA a tile has no registers for it, and would lose 2 % where the groups
+// are words (k 4096 x n 22016, 32 rows).
+template <int BITS, int ZMODE, int SRC, int OWN, bool APART>
 struct ScaleFeed {
   static constexpr bool kZ = ZMODE == kZeroGeneral;
   const __half *sp, *zp;
   uint32_t s_row, z_row;                        // kChannel
   uint32_t sv[OWN], zv[OWN], sn[OWN], zn[OWN];  // current chunk, next chunk
+  uint32_t sn2[OWN], zn2[OWN];                  // APART: the next chunk's second groups, 0 beside words
   uint32_t zconst_h2;
   bool has_zeros, hi;
   uint32_t zo[OWN], z_row_o;                    // offset zero points (kZeroExact; kCodes: in the codes' units) ...
@@ -261,6 +267,8 @@ struct ScaleFeed {
     row_exact = SRC != kAny;
     zconst_h2 = h2_bcast(__float2half_rn(pp.g.zero_const));
     has_zeros = kZ && pp.g.z != nullptr;
+#pragma unroll
+    for (int i = 0; i < OWN; ++i) sn2[i] = zn2[i] = 0u;
     s_row = 0u;
     z_row = zconst_h2;
     if (kZ) z_row_o = offset(zconst_h2, row_exact);
@@ -290,8 +298,14 @@ struct ScaleFeed {
       if (has_zeros) zn[i] = __ldg(reinterpret_cast<const uint32_t*>(zp + kb * 2));
     } else if (SRC == kTwo) {
       const int64_t o = (int64_t)(kb * 2) * pp.s_g;
-      sn[i] = ld_nc_u16(sp + o) | (ld_nc_u16(sp + o + pp.s_g) << 16);
-      if (has_zeros) zn[i] = ld_nc_u16(zp + o) | (ld_nc_u16(zp + o + pp.s_g) << 16);
+      const uint32_t a = ld_nc_u16(sp + o), b = ld_nc_u16(sp + o + pp.s_g);
+      sn[i] = APART ? a : a | (b << 16);
+      sn2[i] = b;
+      if (has_zeros) {
+        const uint32_t za = ld_nc_u16(zp + o), zb = ld_nc_u16(zp + o + pp.s_g);
+        zn[i] = APART ? za : za | (zb << 16);
+        zn2[i] = zb;
+      }
     }
   }
   // own blocks 0, 1 of the next chunk are the adjacent 64-k blocks kb, kb + 1 (kb even): their four group-32
@@ -316,8 +330,8 @@ struct ScaleFeed {
     for (int i = 0; i < OWN; ++i) {
       // (kOne: doubled here and not where it is loaded, which would wait for the load there: an expert layer's
       // matmul of 1024 rows, k 4096 x n 14336, group 128, spent 1400 of 2900 clocks a step on that)
-      sv[i] = SRC == kOne ? sn[i] * 0x10001u : sn[i];
-      zv[i] = SRC == kOne ? zn[i] * 0x10001u : zn[i];
+      sv[i] = SRC == kOne ? sn[i] * 0x10001u : (SRC == kTwo && APART ? sn[i] | (sn2[i] << 16) : sn[i]);
+      zv[i] = SRC == kOne ? zn[i] * 0x10001u : (SRC == kTwo && APART ? zn[i] | (zn2[i] << 16) : zn[i]);
       if (kZ && (SRC == kOne || SRC == kTwo) && has_zeros) {
         exact[i] = true;
         zo[i] = offset(zv[i], exact[i]);

@@ -8,6 +8,7 @@ import pytest
 import torch
 
 from relax_b200 import ops, synth
+from tests.test_autogptq_gpu import _case as gptq_case
 from tests.test_gemv_gpu import _check_status
 from tests.util import assert_close, bits16, to_dev, u32_to_dev
 
@@ -75,3 +76,16 @@ def test_experts(oracle, rows, bits, k, n, group):
     C = oracle.C()
     wq = np.stack([C.decode_ft_kn(w[e], s[e], bits, group).T for e in range(4)])
     assert_close(got, C.epilogue(C.group_gemm_f32(x, np.ascontiguousarray(wq), indptr)))
+
+
+@pytest.mark.parametrize("m", [24, 64, 65, 128, 176, 256])
+@pytest.mark.parametrize("k,n", [(1152, 528), (320, 144)])
+def test_int4_groups_of_32_by_columns(oracle, m, k, n):
+    """scales, and zero points, whose two groups of a 64-k block are no word: [K/32, N]"""
+    test_ft(oracle, m, 4, k, n, 32)
+    qweight, qzeros, scales, _, x, bias = gptq_case(m + k, m, k, n, 32)
+    pre, zeros = ops.preprocess_weight_autogptq(u32_to_dev(qweight)), ops.unpack_zeros_autogptq(u32_to_dev(qzeros))
+    xd, sd, bd = to_dev(x), to_dev(scales), to_dev(bias)
+    got = _twice(lambda: ops.gemm_fp16_autogptq(xd, pre, sd, zeros, bias=bd))
+    C = oracle.C()
+    assert_close(got, C.epilogue(C.matmul_f32(x, C.decode_autogptq(qweight, qzeros, scales, (np.arange(k) // 32).astype(np.uint32)), False), bias))
