@@ -251,7 +251,7 @@ template <int BITS, int ZMODE, int SRC, int OWN, bool APART>
 struct ScaleFeed {
   static constexpr bool kZ = ZMODE == kZeroGeneral;
   const __half *sp, *zp;
-  uint32_t s_row, z_row;                        // kChannel
+  uint32_t s_row, s_row2, z_row;                // kChannel (s_row2, int4: twice, for the current chunk)
   uint32_t sv[OWN], zv[OWN], sn[OWN], zn[OWN];  // current chunk, next chunk
   uint32_t sn2[OWN], zn2[OWN];                  // APART: the next chunk's second groups, 0 beside words
   uint32_t zconst_h2;
@@ -279,7 +279,9 @@ struct ScaleFeed {
     sp = pp.g.s + o;
     zp = pp.g.z + o;
     if (SRC == kChannel) {
-      s_row = ld_nc_u16(sp);  // doubled where it is used, not to wait for it here
+      // doubled for a chunk or where it is used, not to wait for it here (int4 with zero points, k 4096 x n 22016, 24
+      // rows: 22.6 us doubled at each use, 22.2 for a chunk; int8 has no register for it and loses 1 %)
+      s_row = ld_nc_u16(sp);
       if (has_zeros) {
         z_row = ld_nc_u16(zp) * 0x10001u;
         row_exact = true;
@@ -326,6 +328,7 @@ struct ScaleFeed {
     for (int i = 0; i < OWN; ++i) fetch(pp, i, min(kb + i, k_blocks - 1));
   }
   __device__ __forceinline__ void advance() {
+    if (SRC == kChannel && BITS == 4 && !folds<ZMODE, SRC>()) s_row2 = s_row * 0x10001u;
 #pragma unroll
     for (int i = 0; i < OWN; ++i) {
       // (kOne: doubled here and not where it is loaded, which would wait for the load there: an expert layer's
@@ -348,7 +351,7 @@ struct ScaleFeed {
   }
   // run t (int8: fragment tile * 4 + lane run) of own block i = 64-k block kb
   __device__ __forceinline__ uint32_t scale(const Params& pp, int i, int kb, int t) const {
-    if (SRC == kChannel) return prmt(s_row, s_row, 0x1010u);
+    if (SRC == kChannel) return BITS == 4 ? s_row2 : prmt(s_row, s_row, 0x1010u);
     if (SRC == kOne) return sv[i];
     if (SRC == kTwo) return prmt(sv[i], sv[i], (BITS == 4 ? t >> 1 : t >> 2) ? 0x3232u : 0x1010u);
     const unsigned k = (unsigned)(kb * kKBlock + (BITS == 4 ? t * 16 : t * 8));
