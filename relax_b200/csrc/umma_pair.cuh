@@ -13,7 +13,7 @@
 //   everything is handed over in steps of two 64-k blocks: with one block a step the barriers, commits and
 //   tensor-memory store waits of a step took longer than its MMAs (int8, m 256, k 8192 x n 57344: 191 us
 //   without any arithmetic, 118 us without arithmetic, stores and three of the four MMAs);
-//   accumulators: two of up to 128 columns, so that one drains while the next tile runs, or one of up to 256.
+//   accumulators: two of up to 160 columns, so that one drains while the next tile runs, or one of up to 256.
 //
 //   warp 0        packed weights, one 16 KB bulk copy per chunk (128 rows x 256 | 128 k)
 //   warp 1        MMA issue (rank 0)
@@ -21,11 +21,12 @@
 //   warps 4-15    three groups of four warps.  With two accumulators two of them decode alternate steps and
 //                 the third drains: epilogue, one rounding, transpose through shared memory, whole-line
 //                 stores (the others help it with the last tile).  With a single accumulator there is nothing
-//                 to drain while a tile is made, so all three decode in turn and then drain in shares.
-//                 (Measured with two decoding: the MMA waited 148 000 of 425 000 clocks for A at 2048 rows of
-//                 int4, k 4096 x n 22016, group 128; 75 000 with three.  An expert layer of 1024 rows, int4,
-//                 hidden 4096, ffn 14336, eight experts: 317 -> 272 us with this and scales that are not waited
-//                 for where they are loaded; 500 rows of AutoGPTQ k 4096 x n 11008 65 -> 55.)
+//                 to drain while a tile is made: all three decode in turn and then drain in shares, up to a tile
+//                 of 192 rows.  Above, a block's MMAs take longer than two groups take to decode it, and a third
+//                 only gets in their way (int8 per row, k 4096 x n 22016, 256 rows 53.7 us with three, 52.1 with
+//                 two; int4 group 32 47.9 / 46.6, group 64 with zero points 51.6 / 50.4).  At 192 and fewer three
+//                 are ahead by up to 3 % (int8 per row, k 28672 x n 8192, 192 rows 110.3 us with two, 108.3 with
+//                 three), and an expert layer's tiles, whose MMAs are narrower than the tile, gain most.
 //
 // Work split: whole waves of tiles go round robin over the pairs, neighbours sharing a weight tile in L2;
 // the remainder - between one and two waves - is cut into equal runs of (tile, chunk) units that the
@@ -146,8 +147,9 @@ __global__ void __launch_bounds__(kThreads, 1)
   const uint32_t rank = cluster_rank();
   const unsigned pair = blockIdx.x >> 1, pairs = gridDim.x >> 1;
   const bool grouped = pp.indptr != nullptr;
-  const bool all_drain = pp.nd == 1;      // nothing to drain while a tile is made: all three groups decode, then drain
-  const int decoders = all_drain ? 3 : 2;  // groups
+  const bool all_drain = pp.nd == 1;  // nothing to drain while a tile is made
+  // groups that decode (na >= 3 A slots: with fewer, three would meet in a slot's phase)
+  const int decoders = all_drain && nb <= 192 ? 3 : 2;
   if (tid == 0) {
     for (int s = 0; s < w_stages; ++s) {
       mbar_init(&w_full[s], 1);
@@ -407,7 +409,7 @@ __global__ void __launch_bounds__(kThreads, 1)
       }
     }
   } else if (warp >= 4) {
-    // ============================================================ decode (groups 0, 1) and drain (group 2)
+    // ============================================================ decode (groups 0, 1 or all three) and drain
     const int grp = (warp - 4) >> 2, w4 = warp & 3;
     const int hi = w4 & 1;
     const int bl = (w4 >> 1) * 4 + (lane >> 3), g = lane & 7;
@@ -462,7 +464,7 @@ __global__ void __launch_bounds__(kThreads, 1)
         ok = mbar_wait_parked(&d_full[db], dph, p.status);
         if (!ok) break;
         tc_fence_after();
-        ok = drain(w, it, db, 0, is_last(w) ? kDrainGroups : 1, feed.s_row);
+        ok = drain(w, it, db, 0, all_drain || is_last(w) ? kDrainGroups : 1, feed.s_row);
         if (!ok) break;
         tc_fence_before();
         __syncwarp();
@@ -477,13 +479,10 @@ __global__ void __launch_bounds__(kThreads, 1)
       uint32_t off[4];
 #pragma unroll
       for (int t = 0; t < 4; ++t) off[t] = (uint32_t)(t * 128 + ((g + 2 * t) & 7) * 16);
-      int turn = 0;  // group whose turn the first step of the current chunk is
-      // the groups take the steps in turn: this group's step of a chunk, given whose turn its first one is
-      auto own_step = [&](int turn) { return grp >= turn ? grp - turn : grp - turn + decoders; };
-      auto next_turn = [&](int turn, int steps) { return turn + steps >= decoders ? turn + steps - decoders : turn + steps; };
-      auto fetch = [&](int c, int turn) {
+      int own = grp;  // the groups take the steps in turn: this group's next one, counted from the current chunk's first
+      auto fetch = [&](int c, int own) {
         // (on every path, a group without a step in the chunk too: a load under a branch is waited for where the paths meet)
-        const int j = min(own_step(turn), kBlkPerChunk / kStepBlk - 1);
+        const int j = min(own, kBlkPerChunk / kStepBlk - 1);
         feed.fetch_two(pp, min(c * kBlkPerChunk + j * kStepBlk, (k_blocks - 1) & ~1), k_blocks);
       };
       int ws = 0, ab0 = 0;
@@ -491,13 +490,14 @@ __global__ void __launch_bounds__(kThreads, 1)
       for (bool have = begin(w); ok && have; have = next(w)) {
         const Item it = get_item(w.item);
         feed.row(pp, it.e, it.n_tile * kTileRows + row);
-        fetch(w.c0, turn);
+        fetch(w.c0, own);
         for (int c = w.c0; c < w.c1; ++c) {
           const int nft = min(4, KT - c * 4), nblk = nft / kTilesPerBlk, steps = (nblk + kStepBlk - 1) / kStepBlk;
-          const int j = own_step(turn);
+          const int j = own;
           feed.advance();
-          turn = next_turn(turn, steps);
-          fetch(min(c + 1, w.c1 - 1), turn);
+          own -= steps;
+          if (own < 0) own += decoders;
+          fetch(min(c + 1, w.c1 - 1), own);
           // (a group without a step in this chunk waits all the same: its arrival must not run ahead)
           if (!mbar_wait_parked(&w_full[ws], wph, p.status)) {
             ok = false;
