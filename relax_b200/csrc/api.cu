@@ -444,9 +444,12 @@ static int gemm_impl(const rb200_gemm_desc* d, const sk::ArCtx* ar, void* stream
     // runs on the stream-k kernel (small batches whose strides need more than 31 bits on the tensor-core kernels
     // too), and int8 with k a multiple of 32 only on the cluster kernel, whose
     // split-k partials meet in distributed shared memory.
-    // One exception: zero points per group of 32 at nine to sixteen rows spill there (two m-tiles beside
-    // four words of scales and zero points), and from 48 Mi weights on the tensor-core kernel is ahead (16
-    // rows: k 4096 x n 12288 17.9 / 15.0 us, k 11008 x n 6144 27.1 / 19.6; below, k 4096 x n 8192 11.1 / 11.8).
+    // One exception: zero points per group of 32 at nine to sixteen rows take the tensor-core kernel from 48 Mi
+    // weights on.  That line is from when the small-batch kernel took two row blocks a pass there and spilled; with
+    // one it is ahead below the line and, for some shapes, above it, as row blocks fit the CTAs (sixteen rows,
+    // small-batch / tensor-core kernel: k 4096 x n 8192 11.8 / 12.1 us, n 12288 17.0 / 17.4, n 22016 27.2 / 27.2,
+    // n 32768 38.1 / 35.8; k 14336 x n 4096 17.8 / 22.9; k 8192 x n 8192 20.4 / 22.3, n 28672 63.2 / 58.0;
+    // k 11008 x n 6144 25.4 / 22.7).
     if (p.m > 8 && p.m <= rk::kMaxBatch && !ar && p.group == 32 && zero_mode(d) == kZeroGeneral && d->weight_bits == 4 &&
         (int64_t)p.n * p.k >= (48ll << 20)) {
       const int rc = umma_run(p, d->weight_bits, zero_mode(d), sc->sm_count, nullptr, 0, 1, 0, 0, stream);

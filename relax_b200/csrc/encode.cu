@@ -18,10 +18,12 @@
 // That was checked for all (absmax, value) pairs of fp16 and both widths, 2e9 of them, against the
 // division; the test repeats it for a sample.  Infinite maxima and NaN take the division.
 // The CTAs are persistent: three slices in shared memory, one being quantised, one whose maxima travel, one on
-// its way from memory.  Measured, fp16 11008 x 4096 (90 MB): one scale per row 31 us, int8 in groups of 64
+// its way from memory; rows of more than 16384 k have room for two, of more than 24576 for one (encode_plan.h).
+// Measured, fp16 11008 x 4096 (90 MB): one scale per row 31 us, int8 in groups of 64
 // 35 us; 45 / 55 us with a CTA per slice and a cluster barrier (its loads, its exchange and its arithmetic
 // one after the other, 37 us of it before the first code), and 53 / 50 us with a test for ties per value as well.
 // Loading and exchanging alone take 21 us, the codes 6, their stores (16 bytes of a k at a time) 6.
+// 8192 x 16384 int4 99 us (2.7 TB/s of source), x 18944 134, x 24576 149, x 28672 218 (one buffer).
 #include <atomic>
 
 #include "../../include/relax_b200.h"

@@ -455,9 +455,11 @@ int gather_columns_launch(const void* x, const int32_t* perm, void* out, int64_t
   if (m * k == 0) return 0;
   const bool vec = k % 8 == 0 && ldo % 8 == 0 && ((reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(perm)) & 15u) == 0;
   // From 65 rows on through shared memory, where the rows can be read 16 bytes at a time; below, the direct form's
-  // single trip to memory is shorter.  Measured (graph of launches; element by
-  // element with 64-bit divisions before): k 4096, 16 rows 1.48 us (2.00), 256 rows 2.4 (5.4), 2048 rows 11.1 (25.4);
-  // k 14336, 32 rows 2.6 direct, 3.8 staged (4.0), 64 rows 4.6 / 3.9 (5.7), 2048 rows 41 (105).
+  // single trip to memory is shorter, as long as its CTAs run at once.  The line suits k 4096 (64 rows direct 1.8 us,
+  // 65 staged 2.0); longer rows would cross earlier: k 11008, 48 rows 2.6 direct, 64 rows 4.2, 65 staged 3.5; k 14336,
+  // 32 rows 2.7 direct, 48 rows 4.6, 65 staged 3.9.  Measured (graph of launches; element by element with 64-bit
+  // divisions before): k 4096, 16 rows 1.5 us (2.0), 512 rows 3.8 (7.9), 2048 rows 11.1 (25.4); k 14336, 512 rows
+  // 10.5 (26.9), 2048 rows 41 (105).
   constexpr int64_t kStaged = 96 * 1024;
   if (vec && m > 64 && ldx % 8 == 0 && (reinterpret_cast<uintptr_t>(x) & 15u) == 0 && k * 2 <= kStaged) {
     static thread_local int configured_device = -1;

@@ -21,7 +21,8 @@ int x_map(CUtensorMap* tx, const GemvParams& p, int rows) {
 
 // Batch tiles of the pair kernel: of the splits of m into equal tiles of at most 256 rows, the one that the
 // clock counts below say is done first.  Per 64-k block the tensor pipe takes 2 nb clocks and the decode
-// of a CTA's 128 rows about 320, whichever is longer, so wide tiles win (2048 rows as 8 x 256 against
+// of a CTA's 128 rows by two groups of warps about 320 (the counts know neither the third group of tiles of 161 to
+// 192 rows nor that two accumulators hide the drain up to 160), whichever is longer, so wide tiles win (2048 rows as 8 x 256 against
 // 11 x 192 with two accumulators of that width, a form no longer here: 662 / 828 us for int8 k 8192 x
 // n 28672) - unless there are too few of them for the pairs: a tile cut over c more pairs costs its owner about 1600 clocks per
 // two parts and 48 columns (a trip to L2 each).

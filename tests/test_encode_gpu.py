@@ -46,9 +46,9 @@ def test_reference_flow_entirely_on_gpu():
 @pytest.mark.parametrize("bits,group", [(4, -1), (8, -1), (4, 64), (8, 64), (8, 24), (4, 512), (8, 768)])
 @pytest.mark.parametrize("k", [768, 4608, 12288])
 def test_encode_of_long_rows_ties_and_special_values(oracle, bits, group, k):
-    """Slices of 128 and 256 threads, one and several per cluster, groups folded over lanes or not: values on
-    and next to rounding boundaries, at the top of the range, infinities and NaN.  Rows in tiles of 32 take
-    the kernel with the nudged reciprocal, the two odd rows at the end the one that divides."""
+    """CTAs of 256 and 512 threads, one and several per cluster, groups folded over lanes or not: values on
+    and next to rounding boundaries, at the top of the range, infinities and NaN.  n % 32 == 0 takes the
+    kernel with the nudged reciprocal; the same rows and two more take the one that divides."""
     if group > 0 and k % group:
         pytest.skip("groups must divide k")
     n = 96
