@@ -214,13 +214,20 @@ __device__ __forceinline__ void codes_int8_pair(uint32_t w_g, uint32_t w_g8, uin
   a[3] = h2_sub(prmt(w_g8, 0u, 0x4342u), z_g8);
 }
 // Zero points of rows g (low half) and g + 8 in those units, and whether they fit (integers do): a
-// subnormal has no room for a fraction.
+// subnormal has no room for a fraction.  misfit gets bits where they don't.
 template <int BITS>
-__device__ __forceinline__ uint32_t zero_in_codes(uint32_t z_pair, bool& fits) {
+__device__ __forceinline__ uint32_t zero_in_codes(uint32_t z_pair, uint32_t& misfit) {
   constexpr uint32_t kUnits = BITS == 4 ? 0x00100001u : 0x00010001u;  // f16x2(2^-24, 2^-20 | 2^-24)
   constexpr uint32_t k4096 = 0x6c006c00u, kRest = BITS == 4 ? 0x5c006c00u : 0x6c006c00u;
   const uint32_t z = h2_mul(z_pair, kUnits);
-  fits = h2_mul(h2_mul(z, k4096), kRest) == z_pair;
+  misfit |= h2_mul(h2_mul(z, k4096), kRest) ^ z_pair;
+  return z;
+}
+template <int BITS>
+__device__ __forceinline__ uint32_t zero_in_codes(uint32_t z_pair, bool& fits) {
+  uint32_t misfit = 0;
+  const uint32_t z = zero_in_codes<BITS>(z_pair, misfit);
+  fits = misfit == 0;
   return z;
 }
 

@@ -1,0 +1,73 @@
+// Host side of the int4 kernel for at most eight rows: which calls it takes, launch.
+#include "gemv_flat.cuh"
+
+namespace rb200 {
+namespace fl {
+
+int source(const rk::Params& pp, int bits, int zmode, int src) {
+  const GemvParams& p = pp.g;
+  const bool z = zmode == kZeroGeneral, tail = p.k % 256 != 0;
+  if (bits != 4 || p.m > 8 || (z && !p.z)) return -1;
+  const uintptr_t addr = reinterpret_cast<uintptr_t>(p.s) | reinterpret_cast<uintptr_t>(p.z);
+  const int64_t weights = (int64_t)p.n * p.k;
+  // Groups of 32: four columns of one row each beside another four.  (Eight rows stay where two row blocks
+  // share a load of x.)
+  if (p.group == 32 && p.s_g == 1 && p.s_n % 2 == 0 && (addr & 3u) == 0 && p.m <= 4)
+    return src == rk::kRow32 || tail ? rk::kRow32 : (z && p.k % 64 == 0 ? rk::kRow32 : -1);
+  if (src == rk::kGeneral || src == rk::kRow32) return -1;
+  if (!tail && p.s_g == 1 && p.group == 64 && p.s_n % 4 == 0 && (addr & 7u) == 0)
+    // k 2048 x n 4096 without zero points 2.77 / 2.85 us (here), k = n = 4096 4.44 / 3.93; eight rows 3.13 / 3.5, 4.94 / 4.7
+    return z || p.k >= 4096 ? kRow64 : -1;
+  if (!tail && p.s_g == 1 && p.group == 128 && p.s_n % 2 == 0 && (addr & 3u) == 0)
+    // eight rows: k 2048 x n 4096 with zero points 3.34 / 3.58, k = n = 4096 5.09 / 4.82, without 4.33 / 4.67
+    return p.m <= 4 || (z && p.k >= 4096) ? kRow128 : -1;
+  if (src == rk::kChannel) return tail && !z ? src : -1;  // whole chunks: k 8192 x n 28672 24.6 / 29
+  if (src == rk::kTile && z) return -1;                   // spills 450 bytes: k 4096 x n 11008, one row 11.1 / 12.1
+  if (tail) return src;
+  // scales one by one, whole chunks: k = n = 4096 without zero points 3.88 / 4.06, x n 11008 7.77 / 6.88, eight rows
+  // k 11008 x n 4096 8.28 / 8.59; groups of 64 with zero points k = n = 4096 5.34 / 5.81, x n 11008 11.0 / 10.4;
+  // groups of 128 with zero points k = n = 4096 4.83 / 4.31, 1024 x 1024 2.49 / 2.41
+  if (src == rk::kHalf && z) return src;
+  return p.m <= 4 && weights >= (32ll << 20) ? src : -1;
+}
+
+template <int Z, int SRC, bool kEither = true>
+int launch_tail(const Params& pp, int grid, cudaStream_t stream) {
+  const dim3 g((unsigned)grid);
+  if constexpr (kEither) {
+    if (pp.g.k % 256) {
+      RB200_CUDA(launch_dependent(gemv_flat_kernel<Z, SRC, true>, g, kWarps * 32, 0, stream, pp));
+      return 0;
+    }
+  }
+  RB200_CUDA(launch_dependent(gemv_flat_kernel<Z, SRC, false>, g, kWarps * 32, 0, stream, pp));
+  return 0;
+}
+template <int SRC, bool kEither = true>
+int launch_src(const Params& pp, int zmode, int grid, cudaStream_t stream) {
+  return zmode == kZeroGeneral ? launch_tail<kZeroGeneral, SRC, kEither>(pp, grid, stream)
+                               : launch_tail<kZeroConstInt, SRC, kEither>(pp, grid, stream);
+}
+
+int launch(const rk::Params& rp, int zmode, int src, int grid, cudaStream_t stream) {
+  Params pp;
+  static_cast<rk::Params&>(pp) = rp;
+  pp.s_last = pp.g.group > 0 ? (unsigned)(pp.g.k / pp.g.group - 1) * (unsigned)pp.s_g : 0u;
+  switch (src) {
+    case rk::kRow32:
+      return launch_src<rk::kRow32>(pp, zmode, grid, stream);
+    case kRow64:
+      return launch_src<kRow64, false>(pp, zmode, grid, stream);
+    case kRow128:
+      return launch_src<kRow128, false>(pp, zmode, grid, stream);
+    case rk::kHalf:
+      return launch_src<rk::kHalf>(pp, zmode, grid, stream);
+    case rk::kTile:
+      return launch_tail<kZeroConstInt, rk::kTile>(pp, grid, stream);
+  }
+  RB200_CUDA(launch_dependent(gemv_flat_kernel<kZeroConstInt, rk::kChannel, true>, dim3((unsigned)grid), kWarps * 32, 0, stream, pp));
+  return 0;
+}
+
+}  // namespace fl
+}  // namespace rb200

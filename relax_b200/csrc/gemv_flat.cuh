@@ -1,0 +1,486 @@
+// Decode-path kernel for at most eight batch rows of int4: one sequence of units per warp.
+//
+// The small-batch kernel of gemv_rk.cuh works through row blocks two at a time and starts each pair anew: its
+// loads are drained at a pass's end (two chunks of 256 k a warp at k 4096), the two-rounding decode of groups of
+// 32 takes 13 instructions a word, and a scale or zero point is a 16-bit load of its own.  Here a warp's work is
+// one sequence of units (row block, chunk), always two of them loaded ahead whatever row block they belong to,
+// and
+//   * sums of up to eight row blocks wait in shared memory, so that the warps of a CTA meet once;
+//   * u - z goes into the MMA in the codes' units and the scale is applied to the fp32 sums of a group (see
+//     folds() in gemv_rk.cuh), for groups of 32 too: an MMA's k slots reach over a whole tile, two groups, so
+//     the MMA's eight columns are up to four batch rows of the tile's first group beside the same rows of its
+//     second (a lane's x is zero where its k belong to the other group);
+//   * the groups of a chunk are one load of each row where they lie side by side ([N, K/g]);
+//   * a column without a batch row is never loaded (zeros stay in its registers): with the absent rows read as
+//     row 0 the loads of x took 70 % of what L1 passes on, now 20 %;
+//   * k may end within a chunk (k % 256 != 0): the last unit of a row block is shorter.
+// Zero points that are not integers do not fit the codes' units.  Row blocks that met one are computed again
+// before they are stored, by the decode without scales (again(), never reached with integers; inside the loop, or
+// called, it cost the kernels with zero points 300 to 700 bytes of spills).
+//
+// Bound: instruction issue and latency, then HBM.  Of 65 instructions a 512-byte tile needs 36 are the codes, 4
+// MMAs, 8 the scales; issue slots are half used and a warp mostly waits for its weights, but a third set of loads
+// in flight gave nothing, nor did L2 prefetches ahead of them, and with four warps a CTA instead of eight it was
+// up to 17 % slower.  Without the codes' arithmetic the loads alone would take 25 % less (k 4096 x n 22016).
+// Replacing the subtraction of z by z times the sums of x, kept in shared memory, needed 12 % fewer
+// instructions and was 5 to 15 % slower: the sums come before the first unit.
+//
+// Measured against the two-row-block kernel (graphs of launches over 300 MB of weights, launch overlap on; us):
+//                                   one row          four rows        eight rows
+//   group 32, k = n = 4096          4.19 / 3.83      4.57 / 3.97      (stays there)
+//   group 32, k 4096 x n 22016      14.6 / 12.2      15.4 / 12.3
+//   group 32, k 5504 x n 4096       8.2 / 5.1        8.5 / 5.2
+//   the same with zero points       9.1 / 5.5        9.4 / 5.6
+//   group 32 + z, k 4096 x n 22016  20.1 / 13.2      20.9 / 13.5
+//   group 64 + z, k 4096 x n 22016  23.4 / 13.5      24.3 / 14.0      24.8 / 15.1
+//   group 128 + z [K/g, N], x 11008 11.0 / 8.7       11.6 / 9.1       11.6 / 9.9
+#pragma once
+
+#include "gemv_rk.cuh"
+
+namespace rb200 {
+namespace fl {
+
+constexpr int kWarps = 8;  // k slices of a row block; two CTAs per SM
+
+// Beside rk::ScaleSrc: [N, K/g] with groups of 64 or 128, the groups of a chunk are one load of each row.
+constexpr int kRow64 = 5, kRow128 = 6;
+
+struct Params : rk::Params {
+  unsigned s_last;  // offset of the last group's scales
+};
+
+// Where this kernel takes its scales from for these operands, or -1: the kernel of gemv_rk.cuh.
+int source(const rk::Params& pp, int bits, int zmode, int src);
+int launch(const rk::Params& pp, int zmode, int src, int grid, cudaStream_t stream);
+
+#ifdef __CUDACC__
+
+// Loads that keep the register's value where they are switched off.
+__device__ __forceinline__ void ld_w_if(uint4& v, const void* p, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
+               "@q ld.global.nc.L1::no_allocate.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+               : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+               : "l"(p), "r"((int)on));
+}
+// (not .nc: see ld_x_v4 in gemv_rk.cuh)
+__device__ __forceinline__ void ld_x_if(uint4& v, const void* p, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
+               "@q ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+               : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+               : "l"(p), "r"((int)on));
+}
+__device__ __forceinline__ void ld_nc_if(uint4& v, const void* p, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %5, 0;\n\t"
+               "@q ld.global.nc.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+               : "+r"(v.x), "+r"(v.y), "+r"(v.z), "+r"(v.w)
+               : "l"(p), "r"((int)on));
+}
+__device__ __forceinline__ void ld_nc_if(uint2& v, const void* p, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %3, 0;\n\t@q ld.global.nc.v2.u32 {%0, %1}, [%2];\n\t}"
+               : "+r"(v.x), "+r"(v.y)
+               : "l"(p), "r"((int)on));
+}
+__device__ __forceinline__ void ld_nc_if(uint32_t& v, const void* p, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t@q ld.global.nc.u32 %0, [%1];\n\t}"
+               : "+r"(v)
+               : "l"(p), "r"((int)on));
+}
+// (straight into 32 bits: a conversion beside the load is waited for there)
+__device__ __forceinline__ void ld_nc16_if(uint32_t& v, const void* p, bool on) {
+  asm volatile("{\n\t.reg .pred q;\n\tsetp.ne.s32 q, %2, 0;\n\t@q ld.global.nc.u16 %0, [%1];\n\t}"
+               : "+r"(v)
+               : "l"(p), "r"((int)on));
+}
+__device__ __forceinline__ uint32_t word(const uint4& v, int i) { return i == 0 ? v.x : i == 1 ? v.y : i == 2 ? v.z : v.w; }
+__device__ __forceinline__ float half_lo(uint32_t v) { return __half2float(__ushort_as_half((unsigned short)v)); }
+__device__ __forceinline__ float2 halves(uint32_t v) { return __half22float2(*reinterpret_cast<const __half2*>(&v)); }
+
+constexpr float kUnitLo = 1.0f / (1 << 24), kUnitHi = 16.0f * kUnitLo;  // the codes' units, rows g and g + 8
+
+// A warp's sums of one row block once more, in the codes' units and the caller's columns: for zero points that are not
+// integers.  k blocks kb0 to kb1; x at kb0, read by the lanes that have a column.
+template <bool kPairs>
+__device__ __forceinline__ float4 again(const rk::Params& pp, const __half* x, bool mine, int nb, int kb0, int kb1) {
+  const GemvParams& p = pp.g;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int NB = p.n / 16, KB = p.k / 64;
+  const ZeroConsts zc = make_zero_consts(kZeroGeneral, 0.0f);
+  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+  for (int kb = kb0; kb < kb1; ++kb, x += 64) {
+    const uint4 w = rk::ld_stream_v4(p.w + frag_tile_offset(nb, kb, NB, KB) + frag_unit_pos(lane) * 16);
+    uint4 xv[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+    ld_x_if(xv[0], x, mine);
+    ld_x_if(xv[1], x + 8, mine);
+    const unsigned grp = (unsigned)(kb * 64) / (unsigned)p.group;
+    uint32_t z[2];
+    float d[4], s[2][2];
+#pragma unroll
+    for (int i = 0; i < 2; ++i) {
+      const int64_t o = (int64_t)(nb * 16 + g + 8 * i) * pp.s_n + (int64_t)grp * pp.s_g;
+      z[i] = ld_nc_u16(p.z + o + (kPairs ? t >> 1 : 0)) * 0x10001u;
+      s[i][0] = half_lo(ld_nc_u16(p.s + o));
+      s[i][1] = kPairs ? half_lo(ld_nc_u16(p.s + o + 1)) : s[i][0];
+    }
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      constexpr uint32_t kOne = 0x3c003c00u;
+      uint32_t a[4];
+      decode_int4_word<kZeroGeneral>(word(w, i), zc, kOne, kOne, z[0], z[1], a);
+      const uint4& xx = xv[i >> 1];
+      if (i == 0) mma_16816_first(d, a, xx.x, xx.y);
+      else mma_16816(d, a, (i & 1) ? xx.z : xx.x, (i & 1) ? xx.w : xx.y);
+    }
+#pragma unroll
+    for (int c = 0; c < 4; ++c) acc[c] += (c < 2 ? kUnitLo : kUnitHi) * s[c >> 1][c & 1] * d[c];
+  }
+  return make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+
+// kTail: k % 256 != 0
+template <int ZMODE, int SRC, bool kTail>
+__global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params pp) {
+  using namespace rk;
+  constexpr int kFrag = 64, kChunkK = 4 * kFrag;
+  constexpr bool kZ = ZMODE == kZeroGeneral;
+  constexpr bool kPairs = SRC == kRow32, kChan = SRC == kChannel, kRow = SRC == kRow64 || SRC == kRow128;
+  constexpr int kSpans = kChan ? 1 : SRC == kHalf || SRC == kRow128 ? 2 : 4, kSpan = 4 / kSpans;  // of a chunk; tiles of one
+  constexpr bool kWords = kPairs && (kZ || kTail);  // scales by words: lane t has tile t's (registers, alignment)
+  constexpr int kVals = kPairs ? 2 : 4;
+  __shared__ __align__(16) float red[kWarps][kWarps][32 * kVals];
+  const GemvParams& p = pp.g;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  const int g = lane >> 2, t = lane & 3;
+  const int NB = p.n / 16, KB = p.k / kFrag;
+
+  griddep_launch_dependents();
+  const int pos = (int)(blockIdx.x * pp.per_cta + min(blockIdx.x, pp.extra));
+  const int blocks = (int)(pp.per_cta + (blockIdx.x < pp.extra ? 1u : 0u));
+  const int chunks = (KB + 3) / 4, nkb_last = KB - (chunks - 1) * 4;
+  const int c0 = warp * chunks / kWarps, nc = (warp + 1) * chunks / kWarps - c0;
+  const bool ends_short = kTail && warp == kWarps - 1;  // (that warp has at least one chunk)
+  const int unit16 = frag_unit_pos(lane) * 16;
+  const int row8 = pp.s_n * 8;  // elements from row g's scale to row g + 8's
+
+  // ---- loads: two register sets, each loaded again as it is used up
+  uint4 w[2][4];
+  uint4 sq[2][2];                               // kRow32: the chunk's groups of rows g, g + 8
+  uint32_t sw[2][2], zw[2][2];                  // kRow32 by words: tile t's two groups of them
+  uint2 sr[2][2], zr[2][2];                     // kRow64, kRow128: the chunk's groups
+  uint32_t sg[2][kSpans][2], zg[2][kSpans][2];  // kHalf, kTile: one by one
+  const uint8_t* wp;
+  const __half *sp, *zp;
+  int stride, left, lnb, to_load;
+  unsigned s_at = 0, s_at0 = 0;  // kHalf, kTile: offset of the next group's scales, and what
+  int s_left = 0, s_left0 = 0;   // is left of that group
+  if (SRC == kHalf || SRC == kTile) {
+    const unsigned unit = (unsigned)c0 * (unsigned)kSpans;
+    const unsigned grp = pp.group_shift >= 0 ? (unsigned)(c0 * kChunkK) >> pp.group_shift : unit / (unsigned)pp.per;
+    s_at0 = grp * (unsigned)pp.s_g;
+    s_left0 = pp.per - (int)(unit - grp * (unsigned)pp.per);
+  }
+  auto aim = [&]() {  // at chunk c0 of row block lnb
+    const int nblk = min(8, NB - (lnb & ~7));
+    stride = nblk * 2048;
+    wp = p.w + (int64_t)((lnb & ~7) * KB + c0 * 4 * nblk + (lnb & 7) * (kTail && c0 == chunks - 1 ? nkb_last : 4)) * 512 + unit16;
+  };
+  auto start_at = [&](int block) {  // at the first unit of the CTA's block
+    lnb = pos + block;
+    to_load = (blocks - block) * nc;
+    left = nc;
+    aim();
+    const int o = (lnb * 16 + g) * pp.s_n + (kPairs ? c0 * 8 + (kWords ? 2 * t : 0) : kRow ? c0 * kSpans : 0);
+    sp = p.s + o;
+    zp = kZ ? p.z + o : nullptr;
+    s_at = s_at0;
+    s_left = s_left0;
+  };
+  start_at(0);
+  auto advance = [&]() {
+    constexpr int kStep = kPairs ? 8 : kRow ? kSpans : 0;  // scales of a chunk
+    --to_load;
+    wp += stride;
+    sp += kStep;
+    if (kZ) zp += kStep;
+    if (--left == 0) {
+      left = nc;
+      ++lnb;
+      aim();  // (as cheap as stepping from one block to the next, which needs a branch at a tile's end)
+      const int o = 16 * pp.s_n - nc * kStep;
+      sp += o;
+      if (kZ) zp += o;
+      s_at = s_at0;
+      s_left = s_left0;
+    } else if (kTail && ends_short && left == 1) {
+      wp -= (lnb & 7) * (4 - nkb_last) * 512;
+    }
+  };
+  auto load_w = [&](auto set, int j, bool on) {
+    constexpr int S = decltype(set)::value;
+    ld_w_if(w[S][j], wp + j * 512, on && (!kTail || !ends_short || left > 1 || j < nkb_last));
+  };
+  auto load_s = [&](auto set, bool on) {
+    constexpr int S = decltype(set)::value;
+    if (kPairs || kRow) {
+      const bool there = on && (!kTail || !ends_short || left > 1 || t < nkb_last);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        if (kWords) ld_nc_if(sw[S][i], sp + i * row8, there);
+        else if (kPairs) ld_nc_if(sq[S][i], sp + i * row8, on);
+        else if (SRC == kRow128) ld_nc_if(sr[S][i].x, sp + i * row8, on);
+        else ld_nc_if(sr[S][i], sp + i * row8, on);
+        if (!kZ) continue;
+        if (kWords) ld_nc_if(zw[S][i], zp + i * row8, there);
+        else if (SRC == kRow128) ld_nc_if(zr[S][i].x, zp + i * row8, on);
+        else ld_nc_if(zr[S][i], zp + i * row8, on);
+      }
+    } else if (!kChan) {
+#pragma unroll
+      for (int q = 0; q < kSpans; ++q) {
+        const unsigned o = kTail ? min(s_at, pp.s_last) : s_at;  // (behind the end of k the last group's once more)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          ld_nc16_if(sg[S][q][i], sp + o + i * row8, on);
+          if (kZ) ld_nc16_if(zg[S][q][i], zp + o + i * row8, on);
+        }
+        if (--s_left == 0) {
+          s_left = pp.per;
+          s_at += (unsigned)pp.s_g;
+        }
+      }
+    }
+  };
+  using I0 = std::integral_constant<int, 0>;
+  using I1 = std::integral_constant<int, 1>;
+  auto load = [&](auto set) {
+    const bool on = to_load > 0;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) load_w(set, j, on);
+    load_s(set, on);
+    advance();
+  };
+  auto clear = [&]() {
+#pragma unroll
+    for (int S = 0; S < 2; ++S) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) w[S][j] = make_uint4(0, 0, 0, 0);
+#pragma unroll
+      for (int i = 0; i < 2; ++i) {
+        sq[S][i] = make_uint4(0, 0, 0, 0);
+        sw[S][i] = zw[S][i] = 0;
+        sr[S][i] = zr[S][i] = make_uint2(0, 0);
+#pragma unroll
+        for (int q = 0; q < kSpans; ++q) sg[S][q][i] = zg[S][q][i] = 0;
+      }
+    }
+  };
+  clear();
+  // kChannel: the scales of the row block whose sums this warp puts together
+  uint32_t ch_s[2] = {0x3c00u, 0x3c00u};
+  auto load_channel = [&](int first, int count) {
+    if (kChan && warp < count) {
+      const __half* s = p.s + ((pos + first + warp) * 16 + g) * pp.s_n;
+#pragma unroll
+      for (int i = 0; i < 2; ++i) ld_nc16_if(ch_s[i], s + i * row8, true);
+    }
+  };
+  if (pp.early) {
+    load(I0{});
+    load(I1{});
+  } else if (lane < 16) {
+    // before the wait: a prefetch returns nothing to this kernel, so it is safe whatever the previous
+    // kernel still writes
+    const uint8_t* line = wp - unit16 + lane * 128;
+    for (int c = 0; c < min(2, min(nc, KB / 4 - c0)); ++c, line += stride) prefetch_l2(line);
+  }
+  griddep_wait();
+  if (!pp.early) {
+    load(I0{});
+    load(I1{});
+  }
+  int count = min(kWarps, blocks);
+  load_channel(0, count);
+
+  // ---- activations: each tile's are loaded for the next unit as it is used.  (No branch around the first
+  // loads, that costs 5 % of a small matmul: a warp without chunks has no column.)
+  const int m = kPairs ? g >> 1 : g;
+  const bool mine = m < p.m && nc > 0 && (!kPairs || (t >> 1) == (g & 1));
+  const __half* const x0 = p.x + (m < p.m ? m : 0) * (unsigned)p.ldx + t * 16 + c0 * kChunkK;
+  const __half* xp = x0;
+  uint4 x[4][2];
+  auto clear_x = [&]() {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) x[j][0] = x[j][1] = make_uint4(0, 0, 0, 0);
+  };
+  clear_x();
+  auto load_x = [&](int j, bool last) {
+    const bool there = mine && (!kTail || !ends_short || !last || j < nkb_last);
+#pragma unroll
+    for (int i = 0; i < 2; ++i) ld_x_if(x[j][i], xp + j * kFrag + i * 8, there);
+  };
+#pragma unroll
+  for (int j = 0; j < 4; ++j) load_x(j, nc == 1);
+
+  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  int done_left = nc;  // chunks of the row block that are to be done
+  uint32_t misfit = 0;  // not zero: a zero point was no integer
+  uint32_t z_g, z_g8;
+  auto set_zero = [&](uint32_t z2) {
+    const uint32_t z = zero_in_codes<4>(z2, misfit);
+    z_g = prmt(z, z, 0x1010u);
+    z_g8 = prmt(z, z, 0x3232u);
+  };
+  if (!kZ) set_zero(h2_bcast(__float2half_rn(p.zero_const)));
+  auto step = [&](auto set) {
+    constexpr int S = decltype(set)::value;
+    const bool on = to_load > 0;
+    if (kTail && ends_short && done_left == 1) {
+#pragma unroll
+      for (int j = 1; j < 4; ++j)
+        if (j >= nkb_last) x[j][0] = x[j][1] = make_uint4(0, 0, 0, 0);
+    }
+    xp = done_left == 1 ? x0 : xp + kChunkK;
+    const bool next_last = done_left == 2 || nc == 1;
+#pragma unroll
+    for (int q = 0; q < kSpans; ++q) {
+      if (kZ) {
+        if (kPairs) {
+          const uint32_t a = __shfl_sync(0xffffffffu, zw[S][0], q, 4), b = __shfl_sync(0xffffffffu, zw[S][1], q, 4);
+          set_zero(prmt(a, b, t >> 1 ? 0x7632u : 0x5410u));
+        } else if (kRow) {
+          const uint32_t a = q < 2 ? zr[S][0].x : zr[S][0].y, b = q < 2 ? zr[S][1].x : zr[S][1].y;
+          set_zero(prmt(a, b, q & 1 ? 0x7632u : 0x5410u));
+        } else {
+          set_zero(zg[S][q][0] | (zg[S][q][1] << 16));
+        }
+      }
+      float d[4];
+#pragma unroll
+      for (int j = q * kSpan; j < (q + 1) * kSpan; ++j) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          uint32_t a[4];
+          codes_int4_word(word(w[S][j], i), z_g, z_g8, a);
+          const uint4& xx = x[j][i >> 1];
+          const uint32_t b0 = (i & 1) ? xx.z : xx.x, b1 = (i & 1) ? xx.w : xx.y;
+          if (kChan) mma_16816(j & 1 ? acc2 : acc, a, b0, b1);
+          else if (i == 0 && j == q * kSpan) mma_16816_first(d, a, b0, b1);
+          else mma_16816(d, a, b0, b1);
+        }
+        load_w(set, j, on);
+        load_x(j, next_last);
+      }
+      if (!kChan) {
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const uint32_t one = kRow ? (q < 2 ? sr[S][i].x : sr[S][i].y) >> (q & 1 ? 16 : 0) : sg[S][q][i];
+          const float2 s = !kPairs ? make_float2(half_lo(one), half_lo(one))
+                                   : halves(kWords ? __shfl_sync(0xffffffffu, sw[S][i], q, 4) : word(sq[S][i], q));
+          acc[2 * i] += s.x * d[2 * i];
+          acc[2 * i + 1] += s.y * d[2 * i + 1];
+        }
+      }
+    }
+    load_s(set, on);
+    advance();
+  };
+
+  // the sums of a row block are kept until kWarps blocks are done, or all
+  int slot = 0, window = 0;
+  auto window_done = [&]() {
+    if (--done_left != 0) return false;
+    if (kChan) {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        acc[c] += acc2[c];
+        acc2[c] = 0.0f;
+      }
+    }
+    if (kPairs) *reinterpret_cast<float2*>(&red[slot][warp][lane * 2]) = make_float2(acc[0] + acc[1], acc[2] + acc[3]);
+    else *reinterpret_cast<float4*>(&red[slot][warp][lane * 4]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
+    acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
+    done_left = nc;
+    return ++slot == count;
+  };
+  // the k slices meet in warp order
+  auto put_together = [&]() {
+    if (warp >= count) return;
+    float v[kVals];
+#pragma unroll
+    for (int c = 0; c < kVals; ++c) v[c] = 0.0f;
+#pragma unroll
+    for (int i = 0; i < kWarps; ++i)
+#pragma unroll
+      for (int c = 0; c < kVals; ++c) v[c] += red[warp][i][lane * kVals + c];
+#pragma unroll
+    for (int c = 0; c < kVals; ++c) v[c] *= (c < kVals / 2 ? 1.0f / kUnitLo : 1.0f / kUnitHi) * half_lo(ch_s[c / (kVals / 2)]);
+    const int nb = pos + window + warp;
+#pragma unroll
+    for (int c = 0; c < kVals / 2; ++c) {
+      const int mm = t * (kVals / 2) + c;
+      if (mm >= p.m) continue;
+      const float lo = v[c], hi = v[c + kVals / 2];
+      if (p.epi.act == kActSwiglu) {
+        // rows g / g + 8 of the block are gate_f / up_f of f = 8 nb + g (interleaved repack)
+        p.out[(int64_t)mm * p.ldo + nb * 8 + g] = __float2half_rn(silu_mul(lo, hi));
+      } else {
+        const int64_t n = (int64_t)nb * 16 + g;
+        p.out[(int64_t)mm * p.ldo + n] = __float2half_rn(apply_epilogue(lo, p.epi, mm, n));
+        p.out[(int64_t)mm * p.ldo + n + 8] = __float2half_rn(apply_epilogue(hi, p.epi, mm, n + 8));
+      }
+    }
+  };
+  bool odd = false;  // which set is next
+  for (;;) {
+    if (nc == 0) {
+      for (int i = 0; i < count; ++i)
+#pragma unroll
+        for (int v = 0; v < kVals; ++v) red[i][warp][lane * kVals + v] = 0.0f;
+    } else {
+#pragma unroll 1
+      for (;;) {
+        if (!odd) {
+          step(I0{});
+          odd = true;
+          if (window_done()) break;
+        }
+        step(I1{});
+        odd = false;
+        if (window_done()) break;
+      }
+    }
+    if (kZ) {
+      if (__syncthreads_or(misfit != 0)) break;
+    } else {
+      __syncthreads();
+    }
+    put_together();
+    window += count;
+    if (window >= blocks) break;
+    count = min(kWarps, blocks - window);
+    load_channel(window, count);
+    slot = 0;
+    __syncthreads();
+  }
+  if (kZ) {
+    // left early: these row blocks and the rest once more
+    while (window < blocks) {
+      count = min(kWarps, blocks - window);
+      for (int i = 0; i < count; ++i) {
+        const float4 f = again<kPairs>(pp, x0, mine, pos + window + i, c0 * 4, min(KB, (c0 + nc) * 4));
+        if (kPairs) *reinterpret_cast<float2*>(&red[i][warp][lane * 2]) = make_float2(f.x + f.y, f.z + f.w);
+        else *reinterpret_cast<float4*>(&red[i][warp][lane * 4]) = f;
+      }
+      __syncthreads();
+      put_together();
+      __syncthreads();
+      window += count;
+    }
+  }
+}
+
+#endif  // __CUDACC__
+
+}  // namespace fl
+}  // namespace rb200

@@ -1,5 +1,5 @@
 // Host side of the small-batch kernel: scale source, grid, launch.
-#include "gemv_rk.cuh"
+#include "gemv_flat.cuh"
 
 #include <cstring>
 
@@ -42,10 +42,11 @@ int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const in
   pp.s_n = (int)p.s_n;
   pp.s_g = (int)p.s_g;
   const long long blocks = (long long)(p.n / 16) * (indptr ? num_experts : 1);
+  const int flat = indptr ? -1 : fl::source(pp, bits, zmode, src);
   // Eight k slices while an SM has few row blocks (its 16 warps are two CTAs), four once there are
   // enough for four CTAs: half the passes per byte.  Measured: k 8192 x n 28672 int8 (12 row blocks
   // per SM) 44 -> 41 us, k 4096 x n 22016 int4 (9.3) 13.7 -> 13.9 us, k = n = 4096 (1.7) 3.9 -> 5.8 us.
-  const int warps = blocks >= (long long)sm_count * 12 ? 4 : 8;
+  const int warps = flat < 0 && blocks >= (long long)sm_count * 12 ? 4 : 8;
   long long grid = (long long)sm_count * (16 / warps);
   if (grid > blocks) grid = blocks;
   // the kernel numbers row blocks entry by entry: an expert may have several, and most have none
@@ -53,6 +54,7 @@ int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const in
   RB200_CHECK(numbered * grid < (1ll << 32), "too many row blocks for the small-batch kernel (n=%d)", p.n);
   pp.per_cta = (unsigned)(blocks / grid);
   pp.extra = (unsigned)(blocks % grid);
+  if (flat >= 0) return fl::launch(pp, zmode, flat, (int)grid, stream);
   return bits == 4 ? launch_i4(pp, zmode, src, warps, (int)grid, stream) : launch_i8(pp, zmode, src, warps, (int)grid, stream);
 }
 

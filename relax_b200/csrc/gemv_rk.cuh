@@ -1,4 +1,5 @@
-// Decode-path kernel for at most sixteen batch rows: row blocks per CTA, k split over its warps.
+// Decode-path kernel for at most sixteen batch rows: row blocks per CTA, k split over its warps.  (Most int4 calls of
+// up to four rows, and some of up to eight, are taken by gemv_flat.cuh, which has the figures of both.)
 //
 //   out[m, n] = epilogue(sum_k x[m, k] * wq[n, k]),  m <= 8 or 16 (one or two m16n8k16 MMAs wide)
 //
@@ -57,9 +58,8 @@ enum ScaleSrc : int {
 // int4 instead of 13, or 17 with zero points.  Measured at k 4096 x n 11008 int4, four rows, decoded against
 // this: group 128 with zero points 12.9 / 10.3 us, without 10.7 / 9.3, group 64 12.0 / 10.1, one scale per row
 // 8.8 / 8.2.  Two m-tiles decode (measured only for the form that kept the sums apart, which was slower
-// there: 16 rows, group 128 12.8 / 14.6), and so does group 32: two groups in a tile, four batch rows of one
-// beside the same rows of the other in the MMA's eight columns, was no faster (k 4096 x n 12288 8.9 / 9.1,
-// k 11008 x n 4096 8.0 / 8.6).
+// there: 16 rows, group 128 12.8 / 14.6), and so does group 32 here: its two groups of a
+// tile are kept apart by the columns of the MMA in gemv_flat.cuh, which takes up to four rows of it.
 constexpr bool folds(int src, int m_tiles) { return src != kRow32 && src != kGeneral && m_tiles == 1; }
 
 // Row blocks of one pass: activations fetched once serve both.  With a scale and a zero point per group of 32 the two

@@ -1,0 +1,106 @@
+"""The int4 kernel for at most eight rows where its split can go wrong: warps without a chunk, chunks that k ends in,
+short last row tiles, more row blocks than one meeting of the warps holds, every source of scales and zero points at
+either side of its rule, and zero points that do not fit the codes' units."""
+import numpy as np
+import pytest
+import torch
+
+from relax_b200 import get_launch_overlap, ops, set_launch_overlap
+from tests.test_gemv_gpu import _check_status
+from tests.util import to_dev, u32_to_dev
+
+pytestmark = pytest.mark.gpu
+
+
+def _exact(case, group, x):
+    """Unrounded: codes, zero points and scales in 64 bits."""
+    n, k = case.w.shape[0], case.w.shape[1] * 8
+    codes = ((case.w[:, :, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15).reshape(n, k).astype(np.float64)
+    z = 7.0 if case.zeros is None else np.repeat(case.zeros.astype(np.float64), group, axis=1)
+    return x.astype(np.float64) @ ((codes - z) * np.repeat(case.scales.astype(np.float64), group, axis=1)).T
+
+
+# Weights that are not rounded to fp16 leave the output's own rounding, at most 2^-11 of a value; where calls of up to
+# eight rows stay with decoded weights another 2^-11 a weight, 2.8e-4 in the mean square.  Zero points that are no
+# integers round u - z once more.  3e-5 for fp32 sums.
+BOUND = 6e-4
+
+
+@pytest.mark.parametrize("m,overlap", [(1, False), (4, True), (7, False)])
+@pytest.mark.parametrize("zeros", [None, "int", "any"])
+@pytest.mark.parametrize("k,n,group", [(64, 16, 32), (192, 48, 32), (2304, 400, 32), (1856, 144, 32), (4096, 4752, 32), (256, 47632, 32),
+                                       (256, 16, 64), (320, 48, 64), (2304, 400, 64), (4096, 1040, 64), (5504, 144, 64), (256, 47632, 64),
+                                       (256, 16, 128), (640, 48, 128), (4096, 400, 128), (1152, 9488, 128), (4352, 144, 128),
+                                       (512, 47632, 256), (320, 144, 320)])
+def test_rows_of_scales(k, n, group, zeros, m, overlap):
+    """scales [N, K / g]"""
+    from relax_b200 import synth
+    case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, group, asymmetric=zeros is not None)
+    if zeros == "any":  # of some row blocks only
+        case.zeros[n // 2::5, -1] = np.float16(7.3)
+    pre, s, x = ops.preprocess_weight_q4f16(u32_to_dev(case.w)), to_dev(case.scales), to_dev(case.x)
+    z = None if zeros is None else to_dev(case.zeros)
+    bias = torch.randn(n, device="cuda").half()
+    torch.cuda.synchronize()  # (overlap: the weights are not the preceding kernel's)
+    before = get_launch_overlap()
+    set_launch_overlap(overlap)
+    try:
+        out = ops.gemm_fp16_q4f16(x, pre, s, z, bias=bias, group_size=group)
+        _check_status()
+    finally:
+        set_launch_overlap(before)
+    exp = _exact(case, group, case.x) + bias.cpu().numpy().astype(np.float64)
+    got = out.cpu().numpy().astype(np.float64)
+    assert np.linalg.norm(got - exp) <= BOUND * np.linalg.norm(exp)
+    assert np.abs(got - exp).max() <= 4 * BOUND * np.abs(exp).max()
+
+
+@pytest.mark.parametrize("m", [1, 4, 8])
+@pytest.mark.parametrize("k,n,group,zeros", [(4096, 8208, 128, False), (1024, 1040, 128, True), (1152, 144, 128, True), (640, 48, 128, False),
+                                             (4096, 8208, 64, False), (960, 400, 64, False), (4096, 400, 64, True), (768, 144, 384, True),
+                                             (1088, 144, -1, False), (64, 16, -1, False)])
+def test_columns_of_scales(oracle, k, n, group, zeros, m):
+    """scales [K / g, N], zero points beside them"""
+    rs = np.random.RandomState(k + n + m)
+    x = rs.randn(m, k).astype(np.float16)
+    w = rs.randint(-128, 128, size=(k, n // 2)).astype(np.int8)
+    groups = 1 if group < 0 else k // group
+    s = rs.uniform(1e-3, 1e-2, size=(n,) if group < 0 else (groups, n)).astype(np.float16)
+    C = oracle.C()
+    if not zeros:
+        out = ops.gemm_fp16_ft(to_dev(x), ops.preprocess_weight_ft(to_dev(w), True), to_dev(s), 4, group_size=group)
+        wq = C.decode_ft_kn(w, s, 4, group).T.astype(np.float64)
+    else:
+        z = rs.randint(0, 16, size=(groups, n)).astype(np.float16)
+        z[-1, ::3] = 3.7  # (k slices of some warps only)
+        qw = rs.randint(0, 2 ** 32, size=(k // 8, n), dtype=np.uint32)
+        out = ops.gemm_fp16_autogptq(to_dev(x), ops.preprocess_weight_autogptq(u32_to_dev(qw)), to_dev(s), to_dev(z))
+        codes = ((qw[:, None, :] >> (4 * np.arange(8, dtype=np.uint32))[None, :, None]) & 15).reshape(k, n).astype(np.float64)
+        wq = ((codes - np.repeat(z.astype(np.float64), group, axis=0)) * np.repeat(s.astype(np.float64), group, axis=0)).T
+    _check_status()
+    exp = x.astype(np.float64) @ wq.T
+    got = out.cpu().numpy().astype(np.float64)
+    assert np.linalg.norm(got - exp) <= BOUND * np.linalg.norm(exp)
+
+
+@pytest.mark.parametrize("m", [1, 4])
+@pytest.mark.parametrize("k", [4096, 1856])
+def test_swiglu_and_residual(oracle, m, k):
+    """the epilogue's operands in the paired columns: gate and up rows, a residual of each row"""
+    ffn, group = 144, 32
+    rs = np.random.RandomState(k + m)
+    x = rs.randn(m, k).astype(np.float16)
+    w = rs.randint(0, 2 ** 32, size=(2 * ffn, k // 8), dtype=np.uint32)
+    s = rs.uniform(1e-3, 1e-2, size=(2 * ffn, k // group)).astype(np.float16)
+    pre, si = ops.preprocess_weight_gate_up(u32_to_dev(w)), ops.interleave_gate_up(to_dev(s))
+    got = ops.gemm_fp16_q4f16(to_dev(x), pre, si, activation="swiglu").cpu().numpy().astype(np.float64)
+    C = oracle.C()
+    y = C.matmul_f32(x, C.decode_q4_nk(w, s, None, 7.0, group)).astype(np.float64)
+    exp = y[:, :ffn] / (1 + np.exp(-y[:, :ffn])) * y[:, ffn:]
+    assert np.linalg.norm(got - exp) <= 1e-3 * np.linalg.norm(exp)
+    r = rs.randn(m, 2 * ffn).astype(np.float16)
+    got = ops.gemm_fp16_q4f16(to_dev(x), ops.preprocess_weight_q4f16(u32_to_dev(w)), to_dev(s), residual=to_dev(r),
+                              binary_op="plus").cpu().numpy().astype(np.float64)
+    _check_status()
+    exp = y + r
+    assert np.linalg.norm(got - exp) <= 1e-3 * np.linalg.norm(exp)
