@@ -196,9 +196,11 @@ int umma_run(const GemvParams& p, int bits, int zmode, int sm_count, const int64
   pp.cpt = (p.k / frag + 3) / 4;
   if (grouped) {
     // The split of the rows over the experts is known on the device only: the tile is an even share plus
-    // three standard deviations of a uniform routing wide (an expert above it takes a second tile).
+    // three standard deviations of a uniform routing (rows drawn one by one) wide; an expert above it takes a second
+    // tile.  With the deviation of a Poisson count 1024 rows over 8 experts had tiles of 192 columns, one accumulator,
+    // instead of 160, two: int4 group 128, k 4096 x n 14336 143.8 -> 131.5 us, int8 k 4096 x n 8192 96.9 -> 90.6.
     const double even = (double)p.m / num_experts;
-    int nb = (int)(even + 3.0 * std::sqrt(even)) + 1;
+    int nb = (int)(even + 3.0 * std::sqrt(even * (1.0 - 1.0 / num_experts))) + 1;
     if (nb > p.m) nb = p.m;
     pp.nb = nb > kMaxNb ? kMaxNb : nb;
     pp.m_tiles = 1;
