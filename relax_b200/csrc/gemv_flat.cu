@@ -10,10 +10,13 @@ int source(const rk::Params& pp, int bits, int zmode, int src) {
   if (bits != 4 || p.m > 8 || (z && !p.z)) return -1;
   const uintptr_t addr = reinterpret_cast<uintptr_t>(p.s) | reinterpret_cast<uintptr_t>(p.z);
   const int64_t weights = (int64_t)p.n * p.k;
-  // Groups of 32: four columns of one row each beside another four.  (Eight rows stay where two row blocks
-  // share a load of x.)
-  if (p.group == 32 && p.s_g == 1 && p.s_n % 2 == 0 && (addr & 3u) == 0 && p.m <= 4)
-    return src == rk::kRow32 || tail ? rk::kRow32 : (z && p.k % 64 == 0 ? rk::kRow32 : -1);
+  // Groups of 32.  Five to eight rows, where two row blocks cannot share a load of x: eight rows with zero points k 4096 x
+  // n 22016 21.3 / 16.9 us (here), k 11008 x n 4096 12.1 / 10.0, k = n = 4096 5.43 / 5.48, k 2048 x n 4096 3.53 / 4.17; without
+  // k 5504 x n 4096 8.6 / 6.5 and 1152 x 1040 3.33 / 2.88, but whole chunks k = n = 4096 4.66 / 5.24, n 22016 15.5 / 15.6.
+  if (p.group == 32 && p.s_g == 1 && p.s_n % 2 == 0 && (addr & 3u) == 0 && (tail || src == rk::kRow32)) {
+    if (p.m <= 4) return rk::kRow32;
+    return tail || (z && weights >= (16ll << 20)) ? kRow32Wide : -1;
+  }
   if (src == rk::kGeneral || src == rk::kRow32) return -1;
   if (!tail && p.s_g == 1 && p.group == 64 && p.s_n % 4 == 0 && (addr & 7u) == 0)
     // k 2048 x n 4096 without zero points 2.77 / 2.85 us (here), k = n = 4096 4.44 / 3.93; eight rows 3.13 / 3.5, 4.94 / 4.7
@@ -56,6 +59,8 @@ int launch(const rk::Params& rp, int zmode, int src, int grid, cudaStream_t stre
   switch (src) {
     case rk::kRow32:
       return launch_src<rk::kRow32>(pp, zmode, grid, stream);
+    case kRow32Wide:
+      return launch_src<kRow32Wide>(pp, zmode, grid, stream);
     case kRow64:
       return launch_src<kRow64, false>(pp, zmode, grid, stream);
     case kRow128:

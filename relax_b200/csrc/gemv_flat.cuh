@@ -9,7 +9,8 @@
 //   * u - z goes into the MMA in the codes' units and the scale is applied to the fp32 sums of a group (see
 //     folds() in gemv_rk.cuh), for groups of 32 too: an MMA's k slots reach over a whole tile, two groups, so
 //     the MMA's eight columns are up to four batch rows of the tile's first group beside the same rows of its
-//     second (a lane's x is zero where its k belong to the other group);
+//     second (a lane's x is zero where its k belong to the other group); five to eight rows have the lanes
+//     exchange half of their words, so that an MMA's k are of one group (eight instructions a tile more);
 //   * the groups of a chunk are one load of each row where they lie side by side ([N, K/g]);
 //   * a column without a batch row is never loaded (zeros stay in its registers): with the absent rows read as
 //     row 0 the loads of x took 70 % of what L1 passes on, now 20 %;
@@ -29,9 +30,9 @@
 //                                   one row          four rows        eight rows
 //   group 32, k = n = 4096          4.19 / 3.83      4.57 / 3.97      (stays there)
 //   group 32, k 4096 x n 22016      14.6 / 12.2      15.4 / 12.3
-//   group 32, k 5504 x n 4096       8.2 / 5.1        8.5 / 5.2
-//   the same with zero points       9.1 / 5.5        9.4 / 5.6
-//   group 32 + z, k 4096 x n 22016  20.1 / 13.2      20.9 / 13.5
+//   group 32, k 5504 x n 4096       8.2 / 5.1        8.5 / 5.2        8.6 / 6.5
+//   the same with zero points       9.1 / 5.7        9.4 / 6.0        9.6 / 7.3
+//   group 32 + z, k 4096 x n 22016  20.1 / 13.2      20.9 / 13.5      21.3 / 16.9
 //   group 64 + z, k 4096 x n 22016  23.4 / 13.5      24.3 / 14.0      24.8 / 15.1
 //   group 128 + z [K/g, N], x 11008 11.0 / 8.7       11.6 / 9.1       11.6 / 9.9
 #pragma once
@@ -45,6 +46,8 @@ constexpr int kWarps = 8;  // k slices of a row block; two CTAs per SM
 
 // Beside rk::ScaleSrc: [N, K/g] with groups of 64 or 128, the groups of a chunk are one load of each row.
 constexpr int kRow64 = 5, kRow128 = 6;
+// Groups of 32 as rk::kRow32, for up to eight rows.
+constexpr int kRow32Wide = 7;
 
 struct Params : rk::Params {
   unsigned s_last;  // offset of the last group's scales
@@ -99,8 +102,9 @@ __device__ __forceinline__ float2 halves(uint32_t v) { return __half22float2(*re
 constexpr float kUnitLo = 1.0f / (1 << 24), kUnitHi = 16.0f * kUnitLo;  // the codes' units, rows g and g + 8
 
 // A warp's sums of one row block once more, in the codes' units and the caller's columns: for zero points that are not
-// integers.  k blocks kb0 to kb1; x at kb0, read by the lanes that have a column.
-template <bool kPairs>
+// integers.  k blocks kb0 to kb1; x at kb0, read by the lanes that have a column.  (kWide: with the lanes' own groups,
+// the scales in the weights.)
+template <bool kPairs, bool kWide>
 __device__ __forceinline__ float4 again(const rk::Params& pp, const __half* x, bool mine, int nb, int kb0, int kb1) {
   const GemvParams& p = pp.g;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
@@ -113,21 +117,23 @@ __device__ __forceinline__ float4 again(const rk::Params& pp, const __half* x, b
     uint4 xv[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
     ld_x_if(xv[0], x, mine);
     ld_x_if(xv[1], x + 8, mine);
-    const unsigned grp = (unsigned)(kb * 64) / (unsigned)p.group;
-    uint32_t z[2];
+    const unsigned grp = (unsigned)(kb * 64 + (kWide ? t * 16 : 0)) / (unsigned)p.group;
+    uint32_t z[2], s2[2];
     float d[4], s[2][2];
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int64_t o = (int64_t)(nb * 16 + g + 8 * i) * pp.s_n + (int64_t)grp * pp.s_g;
       z[i] = ld_nc_u16(p.z + o + (kPairs ? t >> 1 : 0)) * 0x10001u;
-      s[i][0] = half_lo(ld_nc_u16(p.s + o));
+      s2[i] = ld_nc_u16(p.s + o) * 0x10001u;
+      s[i][0] = kWide ? 1.0f : half_lo(s2[i]);
       s[i][1] = kPairs ? half_lo(ld_nc_u16(p.s + o + 1)) : s[i][0];
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       constexpr uint32_t kOne = 0x3c003c00u;
       uint32_t a[4];
-      decode_int4_word<kZeroGeneral>(word(w, i), zc, kOne, kOne, z[0], z[1], a);
+      if (kWide) decode_int4_word<kZeroGeneral>(word(w, i), zc, s2[0], s2[1], z[0], z[1], a);
+      else decode_int4_word<kZeroGeneral>(word(w, i), zc, kOne, kOne, z[0], z[1], a);
       const uint4& xx = xv[i >> 1];
       if (i == 0) mma_16816_first(d, a, xx.x, xx.y);
       else mma_16816(d, a, (i & 1) ? xx.z : xx.x, (i & 1) ? xx.w : xx.y);
@@ -144,9 +150,9 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
   using namespace rk;
   constexpr int kFrag = 64, kChunkK = 4 * kFrag;
   constexpr bool kZ = ZMODE == kZeroGeneral;
-  constexpr bool kPairs = SRC == kRow32, kChan = SRC == kChannel, kRow = SRC == kRow64 || SRC == kRow128;
+  constexpr bool kPairs = SRC == kRow32, kWide = SRC == kRow32Wide, k32 = kPairs || kWide, kChan = SRC == kChannel, kRow = SRC == kRow64 || SRC == kRow128;
   constexpr int kSpans = kChan ? 1 : SRC == kHalf || SRC == kRow128 ? 2 : 4, kSpan = 4 / kSpans;  // of a chunk; tiles of one
-  constexpr bool kWords = kPairs && (kZ || kTail);  // scales by words: lane t has tile t's (registers, alignment)
+  constexpr bool kWords = k32 && (kZ || kTail);  // scales by words: lane t has tile t's (registers, alignment)
   constexpr int kVals = kPairs ? 2 : 4;
   __shared__ __align__(16) float red[kWarps][kWarps][32 * kVals];
   const GemvParams& p = pp.g;
@@ -190,7 +196,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
     to_load = (blocks - block) * nc;
     left = nc;
     aim();
-    const int o = (lnb * 16 + g) * pp.s_n + (kPairs ? c0 * 8 + (kWords ? 2 * t : 0) : kRow ? c0 * kSpans : 0);
+    const int o = (lnb * 16 + g) * pp.s_n + (k32 ? c0 * 8 + (kWords ? 2 * t : 0) : kRow ? c0 * kSpans : 0);
     sp = p.s + o;
     zp = kZ ? p.z + o : nullptr;
     s_at = s_at0;
@@ -198,7 +204,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
   };
   start_at(0);
   auto advance = [&]() {
-    constexpr int kStep = kPairs ? 8 : kRow ? kSpans : 0;  // scales of a chunk
+    constexpr int kStep = k32 ? 8 : kRow ? kSpans : 0;  // scales of a chunk
     --to_load;
     wp += stride;
     sp += kStep;
@@ -222,12 +228,12 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
   };
   auto load_s = [&](auto set, bool on) {
     constexpr int S = decltype(set)::value;
-    if (kPairs || kRow) {
+    if (k32 || kRow) {
       const bool there = on && (!kTail || !ends_short || left > 1 || t < nkb_last);
 #pragma unroll
       for (int i = 0; i < 2; ++i) {
         if (kWords) ld_nc_if(sw[S][i], sp + i * row8, there);
-        else if (kPairs) ld_nc_if(sq[S][i], sp + i * row8, on);
+        else if (k32) ld_nc_if(sq[S][i], sp + i * row8, on);
         else if (SRC == kRow128) ld_nc_if(sr[S][i].x, sp + i * row8, on);
         else ld_nc_if(sr[S][i], sp + i * row8, on);
         if (!kZ) continue;
@@ -306,7 +312,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
   // loads, that costs 5 % of a small matmul: a warp without chunks has no column.)
   const int m = kPairs ? g >> 1 : g;
   const bool mine = m < p.m && nc > 0 && (!kPairs || (t >> 1) == (g & 1));
-  const __half* const x0 = p.x + (m < p.m ? m : 0) * (unsigned)p.ldx + t * 16 + c0 * kChunkK;
+  const __half* const x0 = p.x + (m < p.m ? m : 0) * (unsigned)p.ldx + (kWide ? (t & 1) * 16 + (t >> 1) * 8 : t * 16) + c0 * kChunkK;
   const __half* xp = x0;
   uint4 x[4][2];
   auto clear_x = [&]() {
@@ -317,7 +323,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
   auto load_x = [&](int j, bool last) {
     const bool there = mine && (!kTail || !ends_short || !last || j < nkb_last);
 #pragma unroll
-    for (int i = 0; i < 2; ++i) ld_x_if(x[j][i], xp + j * kFrag + i * 8, there);
+    for (int i = 0; i < 2; ++i) ld_x_if(x[j][i], xp + j * kFrag + i * (kWide ? 32 : 8), there);
   };
 #pragma unroll
   for (int j = 0; j < 4; ++j) load_x(j, nc == 1);
@@ -342,6 +348,41 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
     }
     xp = done_left == 1 ? x0 : xp + kChunkK;
     const bool next_last = done_left == 2 || nc == 1;
+    if constexpr (kWide) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        // Lanes t < 2 hold words of the tile's first group, the others of its second: they exchange two each, and every
+        // MMA then sums over one group: lane t has the k from 16 (t & 1) + 8 (t >> 1) on of either.
+        const bool hi = t >> 1;
+        const uint4 v = w[S][j];
+        const uint32_t r0 = __shfl_xor_sync(0xffffffffu, hi ? v.x : v.z, 2), r1 = __shfl_xor_sync(0xffffffffu, hi ? v.y : v.w, 2);
+        const uint32_t ww[2][2] = {{hi ? r0 : v.x, hi ? r1 : v.y}, {hi ? v.z : r0, hi ? v.w : r1}};
+        uint32_t za = 0, zb = 0, s2[2];
+        if (kZ) {
+          za = __shfl_sync(0xffffffffu, zw[S][0], j, 4);
+          zb = __shfl_sync(0xffffffffu, zw[S][1], j, 4);
+        }
+#pragma unroll
+        for (int i = 0; i < 2; ++i) s2[i] = kWords ? __shfl_sync(0xffffffffu, sw[S][i], j, 4) : word(sq[S][i], j);
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          if (kZ) set_zero(prmt(za, zb, q ? 0x7632u : 0x5410u));
+          float d[4];
+          uint32_t a[4];
+          codes_int4_word(ww[q][0], z_g, z_g8, a);
+          mma_16816_first(d, a, x[j][q].x, x[j][q].y);
+          codes_int4_word(ww[q][1], z_g, z_g8, a);
+          mma_16816(d, a, x[j][q].z, x[j][q].w);
+#pragma unroll
+          for (int c = 0; c < 4; ++c) acc[c] += half_lo(s2[c >> 1] >> (q ? 16 : 0)) * d[c];
+        }
+        load_w(set, j, on);
+        load_x(j, next_last);
+      }
+      load_s(set, on);
+      advance();
+      return;
+    }
 #pragma unroll
     for (int q = 0; q < kSpans; ++q) {
       if (kZ) {
@@ -468,7 +509,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
     while (window < blocks) {
       count = min(kWarps, blocks - window);
       for (int i = 0; i < count; ++i) {
-        const float4 f = again<kPairs>(pp, x0, mine, pos + window + i, c0 * 4, min(KB, (c0 + nc) * 4));
+        const float4 f = again<kPairs, kWide>(pp, x0 + (kWide ? t * 16 - ((t & 1) * 16 + (t >> 1) * 8) : 0), mine, pos + window + i, c0 * 4,
+                                              min(KB, (c0 + nc) * 4));
         if (kPairs) *reinterpret_cast<float2*>(&red[i][warp][lane * 2]) = make_float2(f.x + f.y, f.z + f.w);
         else *reinterpret_cast<float4*>(&red[i][warp][lane * 4]) = f;
       }
