@@ -6,45 +6,51 @@ namespace fl {
 
 int source(const rk::Params& pp, int bits, int zmode, int src) {
   const GemvParams& p = pp.g;
-  const bool z = zmode == kZeroGeneral, tail = p.k % 256 != 0;
-  if (bits != 4 || p.m > 8 || (z && !p.z)) return -1;
-  const uintptr_t addr = reinterpret_cast<uintptr_t>(p.s) | reinterpret_cast<uintptr_t>(p.z);
+  const bool z = zmode == kZeroGeneral, tail = p.k % 256 != 0, experts = pp.indptr != nullptr;
+  if (bits != 4 || (p.m > 8 && !experts) || (z && !p.z)) return -1;
+  const uintptr_t addr = reinterpret_cast<uintptr_t>(p.s) | reinterpret_cast<uintptr_t>(p.z) | (uintptr_t)(pp.s_expert_stride * 2);
   const int64_t weights = (int64_t)p.n * p.k;
+  const bool few = p.m <= 4 || experts;  // (an expert's rows are seldom more)
   // Groups of 32.  Five to eight rows, where two row blocks cannot share a load of x: eight rows with zero points k 4096 x
   // n 22016 21.3 / 16.9 us (here), k 11008 x n 4096 12.1 / 10.0, k = n = 4096 5.43 / 5.48, k 2048 x n 4096 3.53 / 4.17; without
   // k 5504 x n 4096 8.6 / 6.5 and 1152 x 1040 3.33 / 2.88, but whole chunks k = n = 4096 4.66 / 5.24, n 22016 15.5 / 15.6.
   if (p.group == 32 && p.s_g == 1 && p.s_n % 2 == 0 && (addr & 3u) == 0 && (tail || src == rk::kRow32)) {
-    if (p.m <= 4) return rk::kRow32;
-    return tail || (z && weights >= (16ll << 20)) ? kRow32Wide : -1;
+    if (p.m <= 4 && !experts) return rk::kRow32;
+    return tail || experts || (z && weights >= (16ll << 20)) ? kRow32Wide : -1;
   }
   if (src == rk::kGeneral || src == rk::kRow32) return -1;
   if (!tail && p.s_g == 1 && p.group == 64 && p.s_n % 4 == 0 && (addr & 7u) == 0)
     // k 2048 x n 4096 without zero points 2.77 / 2.85 us (here), k = n = 4096 4.44 / 3.93; eight rows 3.13 / 3.5, 4.94 / 4.7
-    return z || p.k >= 4096 ? kRow64 : -1;
+    return z || experts || p.k >= 4096 ? kRow64 : -1;
   if (!tail && p.s_g == 1 && p.group == 128 && p.s_n % 2 == 0 && (addr & 3u) == 0)
     // eight rows: k 2048 x n 4096 with zero points 3.34 / 3.58, k = n = 4096 5.09 / 4.82, without 4.33 / 4.67
-    return p.m <= 4 || (z && p.k >= 4096) ? kRow128 : -1;
+    return few || (z && p.k >= 4096) ? kRow128 : -1;
   if (src == rk::kChannel) return tail && !z ? src : -1;  // whole chunks: k 8192 x n 28672 24.6 / 29
   if (src == rk::kTile && z) return -1;                   // spills 450 bytes: k 4096 x n 11008, one row 11.1 / 12.1
   if (tail) return src;
   // scales one by one, whole chunks: k = n = 4096 without zero points 3.88 / 4.06, x n 11008 7.77 / 6.88, eight rows
   // k 11008 x n 4096 8.28 / 8.59; groups of 64 with zero points k = n = 4096 5.34 / 5.81, x n 11008 11.0 / 10.4;
   // groups of 128 with zero points k = n = 4096 4.83 / 4.31, 1024 x 1024 2.49 / 2.41
-  if (src == rk::kHalf && z) return src;
-  return p.m <= 4 && weights >= (32ll << 20) ? src : -1;
+  if ((src == rk::kHalf && z) || experts) return src;
+  return few && weights >= (32ll << 20) ? src : -1;
 }
 
+template <int Z, int SRC, bool kTail>
+int launch_form(const Params& pp, int grid, cudaStream_t stream) {
+  const dim3 g((unsigned)grid);
+  if (pp.indptr) {
+    if constexpr (SRC != rk::kRow32) RB200_CUDA(launch_dependent(gemv_flat_experts_kernel<Z, SRC, kTail>, g, kWarps * 32, 0, stream, pp));
+  } else {
+    RB200_CUDA(launch_dependent(gemv_flat_kernel<Z, SRC, kTail>, g, kWarps * 32, 0, stream, pp));
+  }
+  return 0;
+}
 template <int Z, int SRC, bool kEither = true>
 int launch_tail(const Params& pp, int grid, cudaStream_t stream) {
-  const dim3 g((unsigned)grid);
   if constexpr (kEither) {
-    if (pp.g.k % 256) {
-      RB200_CUDA(launch_dependent(gemv_flat_kernel<Z, SRC, true>, g, kWarps * 32, 0, stream, pp));
-      return 0;
-    }
+    if (pp.g.k % 256) return launch_form<Z, SRC, true>(pp, grid, stream);
   }
-  RB200_CUDA(launch_dependent(gemv_flat_kernel<Z, SRC, false>, g, kWarps * 32, 0, stream, pp));
-  return 0;
+  return launch_form<Z, SRC, false>(pp, grid, stream);
 }
 template <int SRC, bool kEither = true>
 int launch_src(const Params& pp, int zmode, int grid, cudaStream_t stream) {
@@ -70,8 +76,7 @@ int launch(const rk::Params& rp, int zmode, int src, int grid, cudaStream_t stre
     case rk::kTile:
       return launch_tail<kZeroConstInt, rk::kTile>(pp, grid, stream);
   }
-  RB200_CUDA(launch_dependent(gemv_flat_kernel<kZeroConstInt, rk::kChannel, true>, dim3((unsigned)grid), kWarps * 32, 0, stream, pp));
-  return 0;
+  return launch_form<kZeroConstInt, rk::kChannel, true>(pp, grid, stream);
 }
 
 }  // namespace fl

@@ -55,7 +55,7 @@ struct Params : rk::Params {
 
 // Where this kernel takes its scales from for these operands, or -1: the kernel of gemv_rk.cuh.
 int source(const rk::Params& pp, int bits, int zmode, int src);
-int launch(const rk::Params& pp, int zmode, int src, int grid, cudaStream_t stream);
+int launch(const rk::Params& pp, int zmode, int src, int grid, cudaStream_t stream);  // (grouped where pp.indptr is set)
 
 #ifdef __CUDACC__
 
@@ -101,11 +101,41 @@ __device__ __forceinline__ float2 halves(uint32_t v) { return __half22float2(*re
 
 constexpr float kUnitLo = 1.0f / (1 << 24), kUnitHi = 16.0f * kUnitLo;  // the codes' units, rows g and g + 8
 
+// What run_blocks works on: the CTA's row blocks of the call's weight, straight from the parameters (as plain fields
+// of a run, like an expert's, they cost groups of 128 two to five per cent) ...
+struct Call {
+  static constexpr bool kWait = true;  // the previous kernel has to be waited for
+  const GemvParams& p;
+  int pos, blocks;
+  __device__ const uint8_t* w() const { return p.w; }
+  __device__ const __half* s() const { return p.s; }
+  __device__ const __half* z() const { return p.z; }
+  __device__ const __half* x() const { return p.x; }
+  __device__ __half* out() const { return p.out; }
+  __device__ int m() const { return p.m; }
+  __device__ int row(int i) const { return i; }
+};
+// ... or of one entry of an expert layer.
+struct Share {
+  static constexpr bool kWait = false;
+  const uint8_t* w_;
+  const __half *s_, *z_, *x_;
+  __half* out_;
+  int m_, m0, pos, blocks;
+  __device__ const uint8_t* w() const { return w_; }
+  __device__ const __half* s() const { return s_; }
+  __device__ const __half* z() const { return z_; }
+  __device__ const __half* x() const { return x_; }
+  __device__ __half* out() const { return out_; }
+  __device__ int m() const { return m_; }
+  __device__ int row(int i) const { return m0 + i; }
+};
+
 // A warp's sums of one row block once more, in the codes' units and the caller's columns: for zero points that are not
 // integers.  k blocks kb0 to kb1; x at kb0, read by the lanes that have a column.  (kWide: with the lanes' own groups,
 // the scales in the weights.)
-template <bool kPairs, bool kWide>
-__device__ __forceinline__ float4 again(const rk::Params& pp, const __half* x, bool mine, int nb, int kb0, int kb1) {
+template <bool kPairs, bool kWide, class Run>
+__device__ __forceinline__ float4 again(const Params& pp, const Run& run, const __half* x, bool mine, int nb, int kb0, int kb1) {
   const GemvParams& p = pp.g;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
   const int NB = p.n / 16, KB = p.k / 64;
@@ -113,7 +143,7 @@ __device__ __forceinline__ float4 again(const rk::Params& pp, const __half* x, b
   float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll 1
   for (int kb = kb0; kb < kb1; ++kb, x += 64) {
-    const uint4 w = rk::ld_stream_v4(p.w + frag_tile_offset(nb, kb, NB, KB) + frag_unit_pos(lane) * 16);
+    const uint4 w = rk::ld_stream_v4(run.w() + frag_tile_offset(nb, kb, NB, KB) + frag_unit_pos(lane) * 16);
     uint4 xv[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
     ld_x_if(xv[0], x, mine);
     ld_x_if(xv[1], x + 8, mine);
@@ -123,10 +153,10 @@ __device__ __forceinline__ float4 again(const rk::Params& pp, const __half* x, b
 #pragma unroll
     for (int i = 0; i < 2; ++i) {
       const int64_t o = (int64_t)(nb * 16 + g + 8 * i) * pp.s_n + (int64_t)grp * pp.s_g;
-      z[i] = ld_nc_u16(p.z + o + (kPairs ? t >> 1 : 0)) * 0x10001u;
-      s2[i] = ld_nc_u16(p.s + o) * 0x10001u;
+      z[i] = ld_nc_u16(run.z() + o + (kPairs ? t >> 1 : 0)) * 0x10001u;
+      s2[i] = ld_nc_u16(run.s() + o) * 0x10001u;
       s[i][0] = kWide ? 1.0f : half_lo(s2[i]);
-      s[i][1] = kPairs ? half_lo(ld_nc_u16(p.s + o + 1)) : s[i][0];
+      s[i][1] = kPairs ? half_lo(ld_nc_u16(run.s() + o + 1)) : s[i][0];
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -145,24 +175,21 @@ __device__ __forceinline__ float4 again(const rk::Params& pp, const __half* x, b
 }
 
 // kTail: k % 256 != 0
-template <int ZMODE, int SRC, bool kTail>
-__global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params pp) {
+constexpr int vals(int src) { return src == rk::kRow32 ? 2 : 4; }  // sums of a lane and row block
+template <int ZMODE, int SRC, bool kTail, class Run>
+__device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, float (&red)[kWarps][kWarps][32 * vals(SRC)]) {
   using namespace rk;
   constexpr int kFrag = 64, kChunkK = 4 * kFrag;
   constexpr bool kZ = ZMODE == kZeroGeneral;
   constexpr bool kPairs = SRC == kRow32, kWide = SRC == kRow32Wide, k32 = kPairs || kWide, kChan = SRC == kChannel, kRow = SRC == kRow64 || SRC == kRow128;
   constexpr int kSpans = kChan ? 1 : SRC == kHalf || SRC == kRow128 ? 2 : 4, kSpan = 4 / kSpans;  // of a chunk; tiles of one
   constexpr bool kWords = k32 && (kZ || kTail);  // scales by words: lane t has tile t's (registers, alignment)
-  constexpr int kVals = kPairs ? 2 : 4;
-  __shared__ __align__(16) float red[kWarps][kWarps][32 * kVals];
+  constexpr int kVals = vals(SRC);
   const GemvParams& p = pp.g;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
   const int NB = p.n / 16, KB = p.k / kFrag;
-
-  griddep_launch_dependents();
-  const int pos = (int)(blockIdx.x * pp.per_cta + min(blockIdx.x, pp.extra));
-  const int blocks = (int)(pp.per_cta + (blockIdx.x < pp.extra ? 1u : 0u));
+  const int pos = run.pos, blocks = run.blocks;
   const int chunks = (KB + 3) / 4, nkb_last = KB - (chunks - 1) * 4;
   const int c0 = warp * chunks / kWarps, nc = (warp + 1) * chunks / kWarps - c0;
   const bool ends_short = kTail && warp == kWarps - 1;  // (that warp has at least one chunk)
@@ -189,7 +216,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
   auto aim = [&]() {  // at chunk c0 of row block lnb
     const int nblk = min(8, NB - (lnb & ~7));
     stride = nblk * 2048;
-    wp = p.w + (int64_t)((lnb & ~7) * KB + c0 * 4 * nblk + (lnb & 7) * (kTail && c0 == chunks - 1 ? nkb_last : 4)) * 512 + unit16;
+    wp = run.w() + (int64_t)((lnb & ~7) * KB + c0 * 4 * nblk + (lnb & 7) * (kTail && c0 == chunks - 1 ? nkb_last : 4)) * 512 + unit16;
   };
   auto start_at = [&](int block) {  // at the first unit of the CTA's block
     lnb = pos + block;
@@ -197,8 +224,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
     left = nc;
     aim();
     const int o = (lnb * 16 + g) * pp.s_n + (k32 ? c0 * 8 + (kWords ? 2 * t : 0) : kRow ? c0 * kSpans : 0);
-    sp = p.s + o;
-    zp = kZ ? p.z + o : nullptr;
+    sp = run.s() + o;
+    zp = kZ ? run.z() + o : nullptr;
     s_at = s_at0;
     s_left = s_left0;
   };
@@ -286,12 +313,12 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
   uint32_t ch_s[2] = {0x3c00u, 0x3c00u};
   auto load_channel = [&](int first, int count) {
     if (kChan && warp < count) {
-      const __half* s = p.s + ((pos + first + warp) * 16 + g) * pp.s_n;
+      const __half* s = run.s() + ((pos + first + warp) * 16 + g) * pp.s_n;
 #pragma unroll
       for (int i = 0; i < 2; ++i) ld_nc16_if(ch_s[i], s + i * row8, true);
     }
   };
-  if (pp.early) {
+  if (!Run::kWait || pp.early) {
     load(I0{});
     load(I1{});
   } else if (lane < 16) {
@@ -300,8 +327,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
     const uint8_t* line = wp - unit16 + lane * 128;
     for (int c = 0; c < min(2, min(nc, KB / 4 - c0)); ++c, line += stride) prefetch_l2(line);
   }
-  griddep_wait();
-  if (!pp.early) {
+  if (Run::kWait) griddep_wait();
+  if (Run::kWait && !pp.early) {
     load(I0{});
     load(I1{});
   }
@@ -311,8 +338,8 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
   // ---- activations: each tile's are loaded for the next unit as it is used.  (No branch around the first
   // loads, that costs 5 % of a small matmul: a warp without chunks has no column.)
   const int m = kPairs ? g >> 1 : g;
-  const bool mine = m < p.m && nc > 0 && (!kPairs || (t >> 1) == (g & 1));
-  const __half* const x0 = p.x + (m < p.m ? m : 0) * (unsigned)p.ldx + (kWide ? (t & 1) * 16 + (t >> 1) * 8 : t * 16) + c0 * kChunkK;
+  const bool mine = m < run.m() && nc > 0 && (!kPairs || (t >> 1) == (g & 1));
+  const __half* const x0 = run.x() + (m < run.m() ? m : 0) * (unsigned)p.ldx + (kWide ? (t & 1) * 16 + (t >> 1) * 8 : t * 16) + c0 * kChunkK;
   const __half* xp = x0;
   uint4 x[4][2];
   auto clear_x = [&]() {
@@ -460,15 +487,15 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
 #pragma unroll
     for (int c = 0; c < kVals / 2; ++c) {
       const int mm = t * (kVals / 2) + c;
-      if (mm >= p.m) continue;
+      if (mm >= run.m()) continue;
       const float lo = v[c], hi = v[c + kVals / 2];
       if (p.epi.act == kActSwiglu) {
         // rows g / g + 8 of the block are gate_f / up_f of f = 8 nb + g (interleaved repack)
-        p.out[(int64_t)mm * p.ldo + nb * 8 + g] = __float2half_rn(silu_mul(lo, hi));
+        run.out()[(int64_t)mm * p.ldo + nb * 8 + g] = __float2half_rn(silu_mul(lo, hi));
       } else {
         const int64_t n = (int64_t)nb * 16 + g;
-        p.out[(int64_t)mm * p.ldo + n] = __float2half_rn(apply_epilogue(lo, p.epi, mm, n));
-        p.out[(int64_t)mm * p.ldo + n + 8] = __float2half_rn(apply_epilogue(hi, p.epi, mm, n + 8));
+        run.out()[(int64_t)mm * p.ldo + n] = __float2half_rn(apply_epilogue(lo, p.epi, run.row(mm), n));
+        run.out()[(int64_t)mm * p.ldo + n + 8] = __float2half_rn(apply_epilogue(hi, p.epi, run.row(mm), n + 8));
       }
     }
   };
@@ -509,7 +536,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
     while (window < blocks) {
       count = min(kWarps, blocks - window);
       for (int i = 0; i < count; ++i) {
-        const float4 f = again<kPairs, kWide>(pp, x0 + (kWide ? t * 16 - ((t & 1) * 16 + (t >> 1) * 8) : 0), mine, pos + window + i, c0 * 4,
+        const float4 f = again<kPairs, kWide>(pp, run, x0 + (kWide ? t * 16 - ((t & 1) * 16 + (t >> 1) * 8) : 0), mine, pos + window + i, c0 * 4,
                                               min(KB, (c0 + nc) * 4));
         if (kPairs) *reinterpret_cast<float2*>(&red[i][warp][lane * 2]) = make_float2(f.x + f.y, f.z + f.w);
         else *reinterpret_cast<float4*>(&red[i][warp][lane * 4]) = f;
@@ -519,6 +546,37 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params 
       __syncthreads();
       window += count;
     }
+  }
+}
+
+template <int ZMODE, int SRC, bool kTail>
+__global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params pp) {
+  __shared__ __align__(16) float red[kWarps][kWarps][32 * vals(SRC)];
+  griddep_launch_dependents();
+  const Call call = {pp.g, (int)(blockIdx.x * pp.per_cta + min(blockIdx.x, pp.extra)), (int)(pp.per_cta + (blockIdx.x < pp.extra ? 1u : 0u))};
+  run_blocks<ZMODE, SRC, kTail>(pp, call, red);
+}
+
+// Expert form: the row blocks of all entries (expert, up to eight of its rows) in one line, shared out evenly.
+template <int ZMODE, int SRC, bool kTail>
+__global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_experts_kernel(const Params pp) {
+  __shared__ __align__(16) float red[kWarps][kWarps][32 * vals(SRC)];
+  __shared__ rk::Entries tab;
+  griddep_launch_dependents();
+  griddep_wait();  // the row table is the routing kernel's output
+  rk::list_entries(pp, tab);
+  const unsigned NB = (unsigned)pp.g.n / 16u, total = (unsigned)tab.count * NB;  // total * grid fits 32 bits (checked by the host)
+  unsigned at = blockIdx.x * total / gridDim.x;
+  const unsigned end = (blockIdx.x + 1) * total / gridDim.x;
+#pragma unroll 1
+  while (at < end) {
+    const unsigned i = at / NB, first = at - i * NB, count = min(end - at, NB - first);
+    const int64_t so = tab.expert[i] * pp.s_expert_stride;
+    const Share share = {pp.g.w + tab.expert[i] * pp.w_expert_bytes, pp.g.s + so, pp.g.z + so, pp.g.x + (int64_t)tab.m_lo[i] * pp.g.ldx,
+                         pp.g.out + (int64_t)tab.m_lo[i] * pp.g.ldo, tab.m_n[i], tab.m_lo[i], (int)first, (int)count};
+    run_blocks<ZMODE, SRC, kTail>(pp, share, red);
+    at += count;
+    __syncthreads();
   }
 }
 

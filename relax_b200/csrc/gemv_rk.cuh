@@ -114,6 +114,44 @@ __device__ __forceinline__ void prefetch_l2(const void* p) {
   asm volatile("prefetch.global.L2 [%0];" ::"l"(p));
 }
 
+// Grouped form: the (expert, up to eight batch rows) pairs that have rows.
+struct Entries {
+  int count, m_lo[kMaxEntries], m_n[kMaxEntries], expert[kMaxEntries];
+};
+// ... from indptr (the whole CTA).
+__device__ __forceinline__ void list_entries(const Params& pp, Entries& tab) {
+  const int lane = threadIdx.x & 31;
+  if (threadIdx.x < 32) {
+    int n_e = 0;
+    for (int e0 = 0; e0 < pp.num_experts; e0 += 32) {
+      const int e = e0 + lane;
+      int r0 = 0, r1 = 0;
+      if (e < pp.num_experts) {
+        r0 = (e || pp.has_prev) ? (int)pp.indptr[e - 1] : 0;
+        r1 = min((int)pp.indptr[e], pp.g.m);  // never past the rows x / out hold
+      }
+      const int mine = r1 > r0 ? (r1 - r0 + kEntryRows - 1) / kEntryRows : 0;
+      int incl = mine;
+#pragma unroll
+      for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, incl, o);
+        if (lane >= o) incl += v;
+      }
+      for (int i = 0; i < mine; ++i) {
+        const int slot = n_e + incl - mine + i;
+        if (slot < kMaxEntries) {
+          tab.m_lo[slot] = r0 + i * kEntryRows;
+          tab.m_n[slot] = min(kEntryRows, r1 - r0 - i * kEntryRows);
+          tab.expert[slot] = e;
+        }
+      }
+      n_e += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    if (lane == 0) tab.count = min(n_e, kMaxEntries);
+  }
+  __syncthreads();
+}
+
 template <int kXV, int MT>
 struct XHalf {
   uint4 v[2][MT][kXV];
@@ -131,7 +169,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   constexpr bool kFold = folds(BITS, ZMODE, SRC, MT);
   constexpr bool kFoldAll = kFold && SRC == kChannel;  // the sums run over all of k
   __shared__ __align__(16) float4 red[2][kWarps][kRows * MT][32];
-  __shared__ int s_entries, s_m_lo[kMaxEntries], s_m_n[kMaxEntries], s_expert[kMaxEntries];
+  __shared__ Entries tab;
   const GemvParams& p = pp.g;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -142,36 +180,8 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   int entries = 1;
   if (grouped) {
     griddep_wait();  // the row table is the routing kernel's output
-    if (warp == 0) {
-      int n_e = 0;
-      for (int e0 = 0; e0 < pp.num_experts; e0 += 32) {
-        const int e = e0 + lane;
-        int r0 = 0, r1 = 0;
-        if (e < pp.num_experts) {
-          r0 = (e || pp.has_prev) ? (int)pp.indptr[e - 1] : 0;
-          r1 = min((int)pp.indptr[e], p.m);  // never past the rows x / out hold
-        }
-        const int mine = r1 > r0 ? (r1 - r0 + kEntryRows - 1) / kEntryRows : 0;
-        int incl = mine;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, incl, o);
-          if (lane >= o) incl += v;
-        }
-        for (int i = 0; i < mine; ++i) {
-          const int slot = n_e + incl - mine + i;
-          if (slot < kMaxEntries) {
-            s_m_lo[slot] = r0 + i * kEntryRows;
-            s_m_n[slot] = min(kEntryRows, r1 - r0 - i * kEntryRows);
-            s_expert[slot] = e;
-          }
-        }
-        n_e += __shfl_sync(0xffffffffu, incl, 31);
-      }
-      if (lane == 0) s_entries = min(n_e, kMaxEntries);
-    }
-    __syncthreads();
-    entries = s_entries;
+    list_entries(pp, tab);
+    entries = tab.count;
   }
   // this CTA's row blocks, numbered entry by entry
   unsigned pos, pos_end;
@@ -229,9 +239,9 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
     // a short last row tile has another chunk stride: a pass stays on one side of it
     const int to_tile_end = 8 - (q.nb0 & 7);
     q.rn = min(min(kRows, (int)(pos_end - at)), min(NB - q.nb0, to_tile_end));
-    q.e = grouped ? s_expert[entry] : 0;
-    q.m_lo = grouped ? s_m_lo[entry] : 0;
-    q.m_n = grouped ? s_m_n[entry] : p.m;
+    q.e = grouped ? tab.expert[entry] : 0;
+    q.m_lo = grouped ? tab.m_lo[entry] : 0;
+    q.m_n = grouped ? tab.m_n[entry] : p.m;
     return q;
   };
   const int row8 = pp.s_n * 8;  // elements from row g's scale to row g + 8's
@@ -368,11 +378,9 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   // L2 prefetch: a lane asks for one of the 16 lines of either row block's chunk.  int8 tiles take a
   // third of the arithmetic of int4 tiles per byte, so there the loads need this lead to keep HBM
   // busy (k 8192 x n 28672: 54 -> 38 us).  For int4 it only costs instructions in one matmul (14.8 against
-  // 13.7 us at k 4096 x n 22016; folded, k 4096 x n 57344 group 128 29.6 against 28.7), but an expert
-  // layer's weights are many times that, and its passes jump between experts: eight experts, 16 rows,
-  // k 4096 x n 28672 102.9 -> 98.6 us, k 14336 x n 4096 58.2 -> 51.7, one scale per row 80.5 -> 78.0 (scales
-  // per tile 28.2 -> 29.8: not there).
-  constexpr bool kLead = BITS == 8 || (GROUPED && kFold && !kZ && SRC != kTile);
+  // 13.7 us at k 4096 x n 22016), but an expert layer's weights are many times that, and its passes jump between
+  // experts: eight experts, 16 rows, k 4096 x n 28672, one scale per row 80.5 -> 78.0 us.
+  constexpr bool kLead = BITS == 8 || (GROUPED && kFoldAll && !kZ);
   const int ahead = min(kLeadChunks, c1 - c0);
   auto line_of = [&](const Pass& q, int c) -> const uint8_t* {
     const int st = min(8, NB - (q.nb0 & ~7)) * 4;
@@ -742,9 +750,15 @@ int launch_inst(const Params& pp, int warps, int grid, cudaStream_t stream) {
   cfg.attrs = attr;
   cfg.numAttrs = 1;
 #define RB200_RK(GR, W, M) RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, GR, W, M>, pp))
+  // (those experts are all gemv_flat.cuh's)
+  constexpr bool kExperts = !(BITS == 4 && ZMODE == kZeroConstInt && (SRC == kRow32 || SRC == kHalf || SRC == kTile));
   if (pp.indptr) {
-    if (warps == 8) RB200_RK(true, 8, 1);
-    else RB200_RK(true, 4, 1);
+    if constexpr (kExperts) {
+      if (warps == 8) RB200_RK(true, 8, 1);
+      else RB200_RK(true, 4, 1);
+    } else {
+      RB200_CHECK(false, "no expert kernel for this source of scales");
+    }
   } else if (pp.g.m <= 8) {
     if (warps == 8) RB200_RK(false, 8, 1);
     else RB200_RK(false, 4, 1);

@@ -104,3 +104,32 @@ def test_swiglu_and_residual(oracle, m, k):
     _check_status()
     exp = y + r
     assert np.linalg.norm(got - exp) <= 1e-3 * np.linalg.norm(exp)
+
+
+@pytest.mark.parametrize("rows", [[0, 9, 0, 23], [1, 2, 0, 5], [32, 0, 0, 0], [0, 0, 0, 0]])
+@pytest.mark.parametrize("k,n,group,zeros", [(512, 1040, 32, None), (320, 48, 32, "any"), (512, 9616, 64, "any"), (256, 144, 64, None),
+                                             (1024, 144, 128, "int"), (512, 48, 128, None), (640, 144, 128, "any"), (64, 16, 64, None)])
+def test_experts(k, n, group, zeros, rows):
+    """expert layers: entries of up to eight rows, a CTA's share over several of them, rows of no expert untouched"""
+    experts, total = len(rows), 32
+    rs = np.random.RandomState(k + n + sum(rows))
+    x = rs.randn(total, k).astype(np.float16)
+    w = rs.randint(0, 2 ** 32, size=(experts, n, k // 8), dtype=np.uint32)
+    s = rs.uniform(1e-3, 1e-2, size=(experts, n, k // group)).astype(np.float16)
+    z = None if zeros is None else rs.randint(0, 16, size=s.shape).astype(np.float16)
+    if zeros == "any":
+        z[1, ::7, -1] = 7.3
+    pre = torch.stack([ops.preprocess_weight_q4f16(u32_to_dev(w[e])) for e in range(experts)])
+    indptr = np.cumsum(rows).astype(np.int64)
+    out = torch.full((total, n), -7.0, dtype=torch.float16, device="cuda")
+    ops.moe_gemm_q4f16(to_dev(x), pre, to_dev(s), torch.from_numpy(indptr).cuda(), None if z is None else to_dev(z), group_size=group, out=out)
+    _check_status()
+    got = out.cpu().numpy().astype(np.float64)
+    assert np.all(got[indptr[-1]:] == -7.0)
+    codes = ((w[..., None] >> (4 * np.arange(8, dtype=np.uint32))) & 15).reshape(experts, n, k).astype(np.float64)
+    wq = (codes - (7.0 if z is None else np.repeat(z.astype(np.float64), group, axis=2))) * np.repeat(s.astype(np.float64), group, axis=2)
+    begin = 0
+    for e, end in enumerate(indptr):
+        exp = x[begin:end].astype(np.float64) @ wq[e].T
+        assert np.linalg.norm(got[begin:end] - exp) <= BOUND * np.linalg.norm(exp)
+        begin = end
