@@ -58,12 +58,14 @@ enum ScaleSrc : int {
 // int4 instead of 13, or 17 with zero points.  Measured at k 4096 x n 11008 int4, four rows, decoded against
 // this: group 128 with zero points 12.9 / 10.3 us, without 10.7 / 9.3, group 64 12.0 / 10.1, one scale per row
 // 8.8 / 8.2.  Two m-tiles decode (measured only for the form that kept the sums apart, which was slower
-// there: 16 rows, group 128 12.8 / 14.6) except int4 with one scale per row and an integer zero point: sixteen rows
-// k 4096 x n 22016 18.1 / 16.1, k 8192 x n 57344 66.7 / 57.5, k = n = 4096 5.81 / 5.51.  (With zero points 3 % slower to 19 %
-// faster, int8 4 % slower to 4 % faster: those decode.)  Group 32 decodes here: its two groups of a
+// there: 16 rows, group 128 12.8 / 14.6) except with one scale per row and an integer zero point: sixteen rows of int4
+// k 4096 x n 22016 18.1 / 16.1, k 8192 x n 57344 66.7 / 57.5, k = n = 4096 5.81 / 5.51; of int8, run for a quarter of a
+// second at a time, k 28672 x n 8192 52.6 / 47.6, k 8192 x n 57344 96.9 / 92.6, k 4096 x n 22016 22.0 / 21.7, k = n = 4096
+// 5.81 / 5.85 (alone, before the power cap is felt, 4 % slower to 4 % faster: what counts is the arithmetic's power).  With
+// zero points int4 is 3 % slower to 19 % faster, int8 10 % to 16 %: those decode.  Group 32 decodes here: its two groups of a
 // tile are kept apart by the columns of the MMA in gemv_flat.cuh, which takes up to four rows of it.
-constexpr bool folds(int bits, int zmode, int src, int m_tiles) {
-  if (m_tiles == 2) return src == kChannel && bits == 4 && zmode == kZeroConstInt;
+constexpr bool folds(int zmode, int src, int m_tiles) {
+  if (m_tiles == 2) return src == kChannel && zmode == kZeroConstInt;
   return src != kRow32 && src != kGeneral;
 }
 
@@ -166,7 +168,7 @@ __global__ void __launch_bounds__(kWarps * 32, 16 / kWarps) gemv_rk_kernel(const
   constexpr int kXV = BITS == 4 ? 2 : 1;  // 16-byte pieces of x per lane and tile
   constexpr bool kZ = ZMODE == kZeroGeneral;
   constexpr int kRows = pass_rows(SRC, ZMODE);
-  constexpr bool kFold = folds(BITS, ZMODE, SRC, MT);
+  constexpr bool kFold = folds(ZMODE, SRC, MT);
   constexpr bool kFoldAll = kFold && SRC == kChannel;  // the sums run over all of k
   __shared__ __align__(16) float4 red[2][kWarps][kRows * MT][32];
   __shared__ Entries tab;
