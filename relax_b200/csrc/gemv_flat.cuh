@@ -1,4 +1,4 @@
-// Decode-path kernel for at most eight batch rows of int4: one sequence of units per warp.
+// Decode-path kernel for at most sixteen batch rows of int4: one sequence of units per warp.
 //
 // The small-batch kernel of gemv_rk.cuh works through row blocks two at a time and starts each pair anew: its
 // loads are drained at a pass's end (two chunks of 256 k a warp at k 4096), the two-rounding decode of groups of
@@ -23,17 +23,20 @@
 // MMAs, 8 the scales; issue slots are half used and a warp mostly waits for its weights, but a third set of loads
 // in flight gave nothing, nor did L2 prefetches ahead of them, and with four warps a CTA instead of eight it was
 // up to 17 % slower.  Without the codes' arithmetic the loads alone would take 25 % less (k 4096 x n 22016).
+// Nine to sixteen rows are two m-tiles with two tiles of x in registers instead of four; their loads of x take 128 of
+// L1's clocks a unit, more than the arithmetic.
 // Replacing the subtraction of z by z times the sums of x, kept in shared memory, needed 12 % fewer
 // instructions and was 5 to 15 % slower: the sums come before the first unit.
 //
 // Measured against the two-row-block kernel (graphs of launches over 300 MB of weights, launch overlap on; us):
-//                                   one row          four rows        eight rows
+//                                   one row          four rows        eight rows       sixteen rows
 //   group 32, k = n = 4096          4.19 / 3.83      4.57 / 3.97      (stays there)
 //   group 32, k 4096 x n 22016      14.6 / 12.2      15.4 / 12.3
-//   group 32, k 5504 x n 4096       8.2 / 5.1        8.5 / 5.2        8.6 / 6.5
+//   group 32, k 5504 x n 4096       8.2 / 5.1        8.5 / 5.2        8.6 / 6.5        10.6 / 8.9
 //   the same with zero points       9.1 / 5.7        9.4 / 6.0        9.6 / 7.3
 //   group 32 + z, k 4096 x n 22016  20.1 / 13.2      20.9 / 13.5      21.3 / 16.9
-//   group 64 + z, k 4096 x n 22016  23.4 / 13.5      24.3 / 14.0      24.8 / 15.1
+//   group 64 + z, k 4096 x n 22016  23.4 / 13.5      24.3 / 14.0      24.8 / 15.1      30.2 / 25.1
+//   group 128, k 11008 x n 4096     7.7 / 7.2        8.1 / 7.5        (stays there)    11.7 / 10.7
 //   group 128 + z [K/g, N], x 11008 11.0 / 8.7       11.6 / 9.1       11.6 / 9.9
 #pragma once
 
@@ -46,7 +49,7 @@ constexpr int kWarps = 8;  // k slices of a row block; two CTAs per SM
 
 // Beside rk::ScaleSrc: [N, K/g] with groups of 64 or 128, the groups of a chunk are one load of each row.
 constexpr int kRow64 = 5, kRow128 = 6;
-// Groups of 32 as rk::kRow32, for up to eight rows.
+// Groups of 32 as rk::kRow32, for more than four rows.
 constexpr int kRow32Wide = 7;
 
 struct Params : rk::Params {
@@ -175,8 +178,9 @@ __device__ __forceinline__ float4 again(const Params& pp, const Run& run, const 
 }
 
 // kTail: k % 256 != 0
-constexpr int vals(int src) { return src == rk::kRow32 ? 2 : 4; }  // sums of a lane and row block
-template <int ZMODE, int SRC, bool kTail, class Run>
+constexpr int vals(int src) { return src == rk::kRow32 ? 2 : 4; }  // sums of a lane, row block and m-tile
+// MT: m-tiles of eight batch rows
+template <int ZMODE, int SRC, bool kTail, int MT, class Run>
 __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, float (&red)[kWarps][kWarps][32 * vals(SRC)]) {
   using namespace rk;
   constexpr int kFrag = 64, kChunkK = 4 * kFrag;
@@ -185,6 +189,9 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
   constexpr int kSpans = kChan ? 1 : SRC == kHalf || SRC == kRow128 ? 2 : 4, kSpan = 4 / kSpans;  // of a chunk; tiles of one
   constexpr bool kWords = k32 && (kZ || kTail);  // scales by words: lane t has tile t's (registers, alignment)
   constexpr int kVals = vals(SRC);
+  constexpr int kSlots = kWarps / MT;  // row blocks whose sums wait in shared memory: [row block, m-tile]
+  constexpr int kXTiles = MT == 1 ? 4 : 2;  // tiles of x in registers
+  static_assert(MT == 1 || (!kPairs && !kChan), "");
   const GemvParams& p = pp.g;
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int g = lane >> 2, t = lane & 3;
@@ -332,30 +339,39 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
     load(I0{});
     load(I1{});
   }
-  int count = min(kWarps, blocks);
+  int count = min(kSlots, blocks);
   load_channel(0, count);
 
   // ---- activations: each tile's are loaded for the next unit as it is used.  (No branch around the first
   // loads, that costs 5 % of a small matmul: a warp without chunks has no column.)
   const int m = kPairs ? g >> 1 : g;
-  const bool mine = m < run.m() && nc > 0 && (!kPairs || (t >> 1) == (g & 1));
+  bool mine[MT];
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) mine[mt] = m + 8 * mt < run.m() && nc > 0 && (!kPairs || (t >> 1) == (g & 1));
   const __half* const x0 = run.x() + (m < run.m() ? m : 0) * (unsigned)p.ldx + (kWide ? (t & 1) * 16 + (t >> 1) * 8 : t * 16) + c0 * kChunkK;
   const __half* xp = x0;
-  uint4 x[4][2];
-  auto clear_x = [&]() {
+  uint4 x[kXTiles][MT][2];
+  auto clear_x = [&](int j) {
 #pragma unroll
-    for (int j = 0; j < 4; ++j) x[j][0] = x[j][1] = make_uint4(0, 0, 0, 0);
+    for (int mt = 0; mt < MT; ++mt) x[j][mt][0] = x[j][mt][1] = make_uint4(0, 0, 0, 0);
   };
-  clear_x();
+#pragma unroll
+  for (int j = 0; j < kXTiles; ++j) clear_x(j);
   auto load_x = [&](int j, bool last) {
-    const bool there = mine && (!kTail || !ends_short || !last || j < nkb_last);
+    const bool there = !kTail || !ends_short || !last || j < nkb_last;
+    if (kTail && MT > 1) clear_x(j % kXTiles);  // (one m-tile: before the short unit)
 #pragma unroll
-    for (int i = 0; i < 2; ++i) ld_x_if(x[j][i], xp + j * kFrag + i * (kWide ? 32 : 8), there);
+    for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+      for (int i = 0; i < 2; ++i)
+        ld_x_if(x[j % kXTiles][mt][i], xp + mt * 8u * (unsigned)p.ldx + j * kFrag + i * (kWide ? 32 : 8), mine[mt] && there);
   };
 #pragma unroll
-  for (int j = 0; j < 4; ++j) load_x(j, nc == 1);
+  for (int j = 0; j < kXTiles; ++j) load_x(j, nc == 1);
 
-  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f}, acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  float acc[MT][4], acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+  for (int mt = 0; mt < MT; ++mt) acc[mt][0] = acc[mt][1] = acc[mt][2] = acc[mt][3] = 0.0f;
   int done_left = nc;  // chunks of the row block that are to be done
   uint32_t misfit = 0;  // not zero: a zero point was no integer
   uint32_t z_g, z_g8;
@@ -368,13 +384,18 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
   auto step = [&](auto set) {
     constexpr int S = decltype(set)::value;
     const bool on = to_load > 0;
-    if (kTail && ends_short && done_left == 1) {
+    const bool this_last = done_left == 1, next_last = done_left == 2 || nc == 1;
+    if constexpr (kTail && MT == 1) {
+      if (ends_short && this_last) {
 #pragma unroll
-      for (int j = 1; j < 4; ++j)
-        if (j >= nkb_last) x[j][0] = x[j][1] = make_uint4(0, 0, 0, 0);
+        for (int j = 1; j < 4; ++j)
+          if (j >= nkb_last) clear_x(j);
+      }
     }
-    xp = done_left == 1 ? x0 : xp + kChunkK;
-    const bool next_last = done_left == 2 || nc == 1;
+    auto next_x = [&](int j) {  // after tile j: what takes its place
+      if (j == 4 - kXTiles) xp = this_last ? x0 : xp + kChunkK;
+      load_x((j + kXTiles) & 3, j + kXTiles < 4 ? this_last : next_last);
+    };
     if constexpr (kWide) {
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
@@ -394,17 +415,23 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           if (kZ) set_zero(prmt(za, zb, q ? 0x7632u : 0x5410u));
-          float d[4];
+          float d[MT][4];
           uint32_t a[4];
+          const uint4(&xx)[MT][2] = x[j % kXTiles];
           codes_int4_word(ww[q][0], z_g, z_g8, a);
-          mma_16816_first(d, a, x[j][q].x, x[j][q].y);
-          codes_int4_word(ww[q][1], z_g, z_g8, a);
-          mma_16816(d, a, x[j][q].z, x[j][q].w);
 #pragma unroll
-          for (int c = 0; c < 4; ++c) acc[c] += half_lo(s2[c >> 1] >> (q ? 16 : 0)) * d[c];
+          for (int mt = 0; mt < MT; ++mt) mma_16816_first(d[mt], a, xx[mt][q].x, xx[mt][q].y);
+          codes_int4_word(ww[q][1], z_g, z_g8, a);
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) mma_16816(d[mt], a, xx[mt][q].z, xx[mt][q].w);
+          const float s_g = half_lo(s2[0] >> (q ? 16 : 0)), s_g8 = half_lo(s2[1] >> (q ? 16 : 0));
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+            for (int c = 0; c < 4; ++c) acc[mt][c] += (c < 2 ? s_g : s_g8) * d[mt][c];
         }
         load_w(set, j, on);
-        load_x(j, next_last);
+        next_x(j);
       }
       load_s(set, on);
       advance();
@@ -423,21 +450,24 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
           set_zero(zg[S][q][0] | (zg[S][q][1] << 16));
         }
       }
-      float d[4];
+      float d[MT][4];
 #pragma unroll
       for (int j = q * kSpan; j < (q + 1) * kSpan; ++j) {
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
           uint32_t a[4];
           codes_int4_word(word(w[S][j], i), z_g, z_g8, a);
-          const uint4& xx = x[j][i >> 1];
-          const uint32_t b0 = (i & 1) ? xx.z : xx.x, b1 = (i & 1) ? xx.w : xx.y;
-          if (kChan) mma_16816(j & 1 ? acc2 : acc, a, b0, b1);
-          else if (i == 0 && j == q * kSpan) mma_16816_first(d, a, b0, b1);
-          else mma_16816(d, a, b0, b1);
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            const uint4& xx = x[j % kXTiles][mt][i >> 1];
+            const uint32_t b0 = (i & 1) ? xx.z : xx.x, b1 = (i & 1) ? xx.w : xx.y;
+            if (kChan) mma_16816(j & 1 ? acc2 : acc[mt], a, b0, b1);
+            else if (i == 0 && j == q * kSpan) mma_16816_first(d[mt], a, b0, b1);
+            else mma_16816(d[mt], a, b0, b1);
+          }
         }
         load_w(set, j, on);
-        load_x(j, next_last);
+        next_x(j);
       }
       if (!kChan) {
 #pragma unroll
@@ -445,8 +475,11 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
           const uint32_t one = kRow ? (q < 2 ? sr[S][i].x : sr[S][i].y) >> (q & 1 ? 16 : 0) : sg[S][q][i];
           const float2 s = !kPairs ? make_float2(half_lo(one), half_lo(one))
                                    : halves(kWords ? __shfl_sync(0xffffffffu, sw[S][i], q, 4) : word(sq[S][i], q));
-          acc[2 * i] += s.x * d[2 * i];
-          acc[2 * i + 1] += s.y * d[2 * i + 1];
+#pragma unroll
+          for (int mt = 0; mt < MT; ++mt) {
+            acc[mt][2 * i] += s.x * d[mt][2 * i];
+            acc[mt][2 * i + 1] += s.y * d[mt][2 * i + 1];
+          }
         }
       }
     }
@@ -454,26 +487,30 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
     advance();
   };
 
-  // the sums of a row block are kept until kWarps blocks are done, or all
+  // the sums of a row block are kept until kSlots blocks are done, or all
   int slot = 0, window = 0;
   auto window_done = [&]() {
     if (--done_left != 0) return false;
     if (kChan) {
 #pragma unroll
       for (int c = 0; c < 4; ++c) {
-        acc[c] += acc2[c];
+        acc[0][c] += acc2[c];
         acc2[c] = 0.0f;
       }
     }
-    if (kPairs) *reinterpret_cast<float2*>(&red[slot][warp][lane * 2]) = make_float2(acc[0] + acc[1], acc[2] + acc[3]);
-    else *reinterpret_cast<float4*>(&red[slot][warp][lane * 4]) = make_float4(acc[0], acc[1], acc[2], acc[3]);
-    acc[0] = acc[1] = acc[2] = acc[3] = 0.0f;
+#pragma unroll
+    for (int mt = 0; mt < MT; ++mt) {
+      float(&f)[4] = acc[mt];
+      if (kPairs) *reinterpret_cast<float2*>(&red[slot][warp][lane * 2]) = make_float2(f[0] + f[1], f[2] + f[3]);
+      else *reinterpret_cast<float4*>(&red[slot * MT + mt][warp][lane * 4]) = make_float4(f[0], f[1], f[2], f[3]);
+      f[0] = f[1] = f[2] = f[3] = 0.0f;
+    }
     done_left = nc;
     return ++slot == count;
   };
   // the k slices meet in warp order
   auto put_together = [&]() {
-    if (warp >= count) return;
+    if (warp >= count * MT) return;
     float v[kVals];
 #pragma unroll
     for (int c = 0; c < kVals; ++c) v[c] = 0.0f;
@@ -483,10 +520,10 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
       for (int c = 0; c < kVals; ++c) v[c] += red[warp][i][lane * kVals + c];
 #pragma unroll
     for (int c = 0; c < kVals; ++c) v[c] *= (c < kVals / 2 ? 1.0f / kUnitLo : 1.0f / kUnitHi) * half_lo(ch_s[c / (kVals / 2)]);
-    const int nb = pos + window + warp;
+    const int nb = pos + window + warp / MT;
 #pragma unroll
     for (int c = 0; c < kVals / 2; ++c) {
-      const int mm = t * (kVals / 2) + c;
+      const int mm = (warp % MT) * 8 + t * (kVals / 2) + c;
       if (mm >= run.m()) continue;
       const float lo = v[c], hi = v[c + kVals / 2];
       if (p.epi.act == kActSwiglu) {
@@ -502,7 +539,7 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
   bool odd = false;  // which set is next
   for (;;) {
     if (nc == 0) {
-      for (int i = 0; i < count; ++i)
+      for (int i = 0; i < count * MT; ++i)
 #pragma unroll
         for (int v = 0; v < kVals; ++v) red[i][warp][lane * kVals + v] = 0.0f;
     } else {
@@ -526,7 +563,7 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
     put_together();
     window += count;
     if (window >= blocks) break;
-    count = min(kWarps, blocks - window);
+    count = min(kSlots, blocks - window);
     load_channel(window, count);
     slot = 0;
     __syncthreads();
@@ -534,12 +571,15 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
   if (kZ) {
     // left early: these row blocks and the rest once more
     while (window < blocks) {
-      count = min(kWarps, blocks - window);
+      count = min(kSlots, blocks - window);
       for (int i = 0; i < count; ++i) {
-        const float4 f = again<kPairs, kWide>(pp, run, x0 + (kWide ? t * 16 - ((t & 1) * 16 + (t >> 1) * 8) : 0), mine, pos + window + i, c0 * 4,
-                                              min(KB, (c0 + nc) * 4));
-        if (kPairs) *reinterpret_cast<float2*>(&red[i][warp][lane * 2]) = make_float2(f.x + f.y, f.z + f.w);
-        else *reinterpret_cast<float4*>(&red[i][warp][lane * 4]) = f;
+#pragma unroll 1
+        for (int mt = 0; mt < MT; ++mt) {
+          const __half* xa = x0 + (kWide ? t * 16 - ((t & 1) * 16 + (t >> 1) * 8) : 0) + mt * 8u * (unsigned)p.ldx;
+          const float4 f = again<kPairs, kWide>(pp, run, xa, mt ? mine[MT - 1] : mine[0], pos + window + i, c0 * 4, min(KB, (c0 + nc) * 4));
+          if (kPairs) *reinterpret_cast<float2*>(&red[i][warp][lane * 2]) = make_float2(f.x + f.y, f.z + f.w);
+          else *reinterpret_cast<float4*>(&red[i * MT + mt][warp][lane * 4]) = f;
+        }
       }
       __syncthreads();
       put_together();
@@ -549,12 +589,12 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
   }
 }
 
-template <int ZMODE, int SRC, bool kTail>
+template <int ZMODE, int SRC, bool kTail, int MT>
 __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_kernel(const Params pp) {
   __shared__ __align__(16) float red[kWarps][kWarps][32 * vals(SRC)];
   griddep_launch_dependents();
   const Call call = {pp.g, (int)(blockIdx.x * pp.per_cta + min(blockIdx.x, pp.extra)), (int)(pp.per_cta + (blockIdx.x < pp.extra ? 1u : 0u))};
-  run_blocks<ZMODE, SRC, kTail>(pp, call, red);
+  run_blocks<ZMODE, SRC, kTail, MT>(pp, call, red);
 }
 
 // Expert form: the row blocks of all entries (expert, up to eight of its rows) in one line, shared out evenly.
@@ -574,7 +614,7 @@ __global__ void __launch_bounds__(kWarps * 32, 2) gemv_flat_experts_kernel(const
     const int64_t so = tab.expert[i] * pp.s_expert_stride;
     const Share share = {pp.g.w + tab.expert[i] * pp.w_expert_bytes, pp.g.s + so, pp.g.z + so, pp.g.x + (int64_t)tab.m_lo[i] * pp.g.ldx,
                          pp.g.out + (int64_t)tab.m_lo[i] * pp.g.ldo, tab.m_n[i], tab.m_lo[i], (int)first, (int)count};
-    run_blocks<ZMODE, SRC, kTail>(pp, share, red);
+    run_blocks<ZMODE, SRC, kTail, 1>(pp, share, red);
     at += count;
     __syncthreads();
   }

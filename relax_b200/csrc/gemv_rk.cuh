@@ -1,5 +1,6 @@
-// Decode-path kernel for at most sixteen batch rows: row blocks per CTA, k split over its warps.  (Most int4 calls of
-// up to four rows, and some of up to eight, are taken by gemv_flat.cuh, which has the figures of both.)
+// Decode-path kernel for at most sixteen batch rows: row blocks per CTA, k split over its warps.  (Most int4 calls are
+// taken by gemv_flat.cuh, which has the figures of both; what stays here of them are one scale per row, groups of 32
+// above four rows, and group sizes that are no whole tiles.)
 //
 //   out[m, n] = epilogue(sum_k x[m, k] * wq[n, k]),  m <= 8 or 16 (one or two m16n8k16 MMAs wide)
 //
@@ -765,8 +766,12 @@ int launch_inst(const Params& pp, int warps, int grid, cudaStream_t stream) {
     if (warps == 8) RB200_RK(false, 8, 1);
     else RB200_RK(false, 4, 1);
   } else {
-    if (warps == 8) RB200_RK(false, 8, 2);
-    else RB200_RK(false, 4, 2);
+    if constexpr (!(BITS == 4 && ZMODE == kZeroConstInt && SRC == kHalf)) {  // (gemv_flat.cuh's)
+      if (warps == 8) RB200_RK(false, 8, 2);
+      else RB200_RK(false, 4, 2);
+    } else {
+      RB200_CHECK(false, "no kernel of two m-tiles for this source of scales");
+    }
   }
 #undef RB200_RK
   return 0;

@@ -1,4 +1,4 @@
-"""The int4 kernel for at most eight rows where its split can go wrong: warps without a chunk, chunks that k ends in,
+"""The int4 kernel of one sequence of units per warp where its split can go wrong: warps without a chunk, chunks that k ends in,
 short last row tiles, more row blocks than one meeting of the warps holds, every source of scales and zero points at
 either side of its rule, and zero points that do not fit the codes' units."""
 import numpy as np
@@ -20,13 +20,13 @@ def _exact(case, group, x):
     return x.astype(np.float64) @ ((codes - z) * np.repeat(case.scales.astype(np.float64), group, axis=1)).T
 
 
-# Weights that are not rounded to fp16 leave the output's own rounding, at most 2^-11 of a value; where calls of up to
-# eight rows stay with decoded weights another 2^-11 a weight, 2.8e-4 in the mean square.  Zero points that are no
+# Weights that are not rounded to fp16 leave the output's own rounding, at most 2^-11 of a value; where calls
+# stay with decoded weights another 2^-11 a weight, 2.8e-4 in the mean square.  Zero points that are no
 # integers round u - z once more.  3e-5 for fp32 sums.
 BOUND = 6e-4
 
 
-@pytest.mark.parametrize("m,overlap", [(1, False), (4, True), (7, False)])
+@pytest.mark.parametrize("m,overlap", [(1, False), (4, True), (7, False), (13, True)])
 @pytest.mark.parametrize("zeros", [None, "int", "any"])
 @pytest.mark.parametrize("k,n,group", [(64, 16, 32), (192, 48, 32), (2304, 400, 32), (1856, 144, 32), (4096, 4752, 32), (256, 47632, 32),
                                        (256, 16, 64), (320, 48, 64), (2304, 400, 64), (4096, 1040, 64), (5504, 144, 64), (256, 47632, 64),
@@ -55,9 +55,9 @@ def test_rows_of_scales(k, n, group, zeros, m, overlap):
     assert np.abs(got - exp).max() <= 4 * BOUND * np.abs(exp).max()
 
 
-@pytest.mark.parametrize("m", [1, 4, 8])
-@pytest.mark.parametrize("k,n,group,zeros", [(4096, 8208, 128, False), (1024, 1040, 128, True), (1152, 144, 128, True), (640, 48, 128, False),
-                                             (4096, 8208, 64, False), (960, 400, 64, False), (4096, 400, 64, True), (768, 144, 384, True),
+@pytest.mark.parametrize("m", [1, 4, 8, 16])
+@pytest.mark.parametrize("k,n,group,zeros", [(4096, 8208, 128, False), (8192, 80, 128, True), (1024, 1040, 128, True), (1152, 144, 128, True), (640, 48, 128, False),
+                                             (4096, 8208, 64, False), (4096, 1040, 64, False), (960, 400, 64, False), (4096, 400, 64, True), (768, 144, 384, True),
                                              (1088, 144, -1, False), (64, 16, -1, False)])
 def test_columns_of_scales(oracle, k, n, group, zeros, m):
     """scales [K / g, N], zero points beside them"""
