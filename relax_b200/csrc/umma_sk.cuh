@@ -157,8 +157,11 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   const unsigned step = pp.partial ? 1u : (unsigned)cpt, units = pp.partial ? total : items;
   // (experts without rows can leave fewer units than CTAs: the surplus CTAs stay out of the split)
   const unsigned ctas = min(gridDim.x, units);
-  const unsigned u_begin = blockIdx.x < ctas ? blockIdx.x * units / ctas * step : 0u;
-  const unsigned u_end = blockIdx.x < ctas ? (blockIdx.x + 1) * units / ctas * step : 0u;
+  // the first `whole` CTAs take a tile each, the others equal runs of the rest
+  const unsigned whole = (unsigned)pp.whole, base = whole * (unsigned)cpt;
+  const unsigned rest = units - base, takers = min(ctas - whole, rest), idx = blockIdx.x - whole;
+  const unsigned u_begin = blockIdx.x < whole ? blockIdx.x * (unsigned)cpt : (idx < takers ? base + idx * rest / takers * step : 0u);
+  const unsigned u_end = blockIdx.x < whole ? (blockIdx.x + 1) * (unsigned)cpt : (idx < takers ? base + (idx + 1) * rest / takers * step : 0u);
 
   auto get_item = [&](int item) {
     Item it;
@@ -436,7 +439,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
         if (w.c1 < cpt) {
           // this CTA owns the tile, later ones hold the rest
           const unsigned hi_u = (unsigned)w.item * (unsigned)cpt + (unsigned)cpt - 1u;
-          last = (int)(((hi_u + 1u) * ctas - 1u) / total);
+          last = (int)(whole + ((hi_u - base + 1u) * takers - 1u) / rest);
         }
         ok = drain_store<false, folds<ZMODE, SRC>()>(pp, dt, me, last, 1, e_stage + grp * kStageBytes, step, group_sync);
         if (!ok) break;

@@ -139,6 +139,13 @@ int run_single(Params& pp, int bits, int zmode, int src, int sm_count, cudaStrea
   RB200_CHECK(units * grid < (1ll << 31), "problem too large for the 32-bit work split (n=%d, k=%d, m=%d)", p.n, p.k, p.m);
   // (one CTA per tile cuts none)
   if (pp.indptr || grid != items) pp.partial = handover_words(stream, sm_count, (size_t)grid * pp.nb * kTileRows * sizeof(float));
+  // A tile per SM is not cut: its first CTA makes one, the second a run of the rest.  That saves a quarter of the pieces
+  // where the tiles come near two per SM; with fewer the second CTA is done long before the first (int8 per row, 48 rows,
+  // k 4096: n 32016 26.6 us in equal runs, 25.3 so, n 36000 28.3 / 27.9, n 22016 27.5 / 27.9, 24 rows 24.4 / 26.1; int4
+  // group 32, 32 rows: n 32016 28.6 / 27.6, n 26624 25.0 / 26.1, n 22016 21.9 / 21.0).
+  // (Run for a quarter of a second at a time, 238 tiles, 24 rows of int4 lose 1 to 2 %, 48 and 64 rows gain 2 to 4.)
+  if (!pp.indptr && pp.partial && grid == 2ll * sm_count && items < grid && (pp.nb > 32 ? items * 5 >= sm_count * 8ll : items * 3 >= sm_count * 5ll))
+    pp.whole = sm_count;
   l.grid = (int)grid;
   CUtensorMap tx;
   if (x_map(&tx, p, pp.nb) != 0) return -1;

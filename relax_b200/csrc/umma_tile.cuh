@@ -34,6 +34,7 @@ struct Params {
   GemvParams g;
   int nb, m_tiles;             // batch rows per tile (multiple of 16), batch tiles (ungrouped)
   int cpt;                     // chunks per tile
+  int whole;                   // umma_sk: CTAs that take a whole tile each
   int x_stages, w_stages;
   int nd, d_stride, a_base, na, tmem_cols;  // accumulators and A slots in tensor memory
   int s_n, s_g;                // scale strides in elements

@@ -89,3 +89,16 @@ def test_int4_groups_of_32_by_columns(oracle, m, k, n):
     got = _twice(lambda: ops.gemm_fp16_autogptq(xd, pre, sd, zeros, bias=bd))
     C = oracle.C()
     assert_close(got, C.epilogue(C.matmul_f32(x, C.decode_autogptq(qweight, qzeros, scales, (np.arange(k) // 32).astype(np.uint32)), False), bias))
+
+
+@pytest.mark.parametrize("m", [24, 64])
+@pytest.mark.parametrize("tiles", [236, 238, 246, 248, 295])
+@pytest.mark.parametrize("k", [64, 1088])
+def test_a_tile_per_sm_and_runs_of_the_rest(oracle, m, tiles, k):
+    """either side of the tile counts from which an SM's first CTA keeps a whole tile, with more CTAs than chunks left and fewer"""
+    n = tiles * 128 - 48
+    case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, 32)
+    pre, s, x = ops.preprocess_weight_q4f16(u32_to_dev(case.w)), to_dev(case.scales), to_dev(case.x)
+    got = _twice(lambda: ops.gemm_fp16_q4f16(x, pre, s, group_size=32))
+    C = oracle.C()
+    assert_close(got, C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, None, 7.0, 32))))
