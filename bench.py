@@ -838,9 +838,9 @@ def run_gpu(args):
                          # DRAM bytes per launch: the ncu capture of the gate_up M=1 launch read + wrote
                          # 50.77 MB for 50.78 MB of algorithmic bytes (x 0.9998); scaled to the mean launch
                          "traffic": 0.9998 * sum(c for _, c in per_shape.values()) / len(per_shape),
-                         "traffic_source": "profiles/gemv_rk_kernel_gate_up_m1.md, scaled by algorithmic bytes",
+                         "traffic_source": "profiles/gemv_flat_kernel_gate_up_m1.md, scaled by algorithmic bytes",
                          "peak_kind": peak_kind,
-                         "kernel": "gemv_rk_kernel (M <= 16), umma_sk_kernel (M = 32)",
+                         "kernel": "gemv_flat_kernel (M = 1), gemv_rk_kernel (M = 8), umma_sk_kernel (M = 32)",
                          "per_shape_gbs": shape_gbs, "per_shape_us": shape_us},
             "cpu_baseline": cpu,
             "clocks": {"sm_mhz": clk["sm_mhz"], "sm_max_mhz": clk["sm_max_mhz"], "reasons": clk["reasons"]},
