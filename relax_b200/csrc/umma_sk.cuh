@@ -17,6 +17,9 @@
 // their own flags: at rest they hold a NaN pattern that no sum has (kVacant), the owner polls them -
 // several contributors' words requested together, one trip to memory per try - and puts the pattern
 // back.  (A fence, a flag and a second trip per contributor cost 6 us at k = n = 4096.)
+// Where a tile is cut into equal parts that are many or large, its CTAs form a cluster instead and each adds up its
+// share of the columns (CLUSTER; the rule and its figures are beside the split in umma_tile.cu): the owner's trips to
+// memory, one per part, were up to a third of such a launch, and the registers for several parts a trip spill.
 //
 //   warp 0  packed weights, one 16 KB bulk copy per chunk (128 rows x 256 | 128 k)
 //   warp 1  MMA: four per 64-k block, by an elected thread
@@ -40,6 +43,7 @@ namespace us {
 
 constexpr int kSmallNb = 64;            // up to here two CTAs share an SM
 constexpr int kGroups = 2;              // decode groups of four warps
+constexpr size_t kCtaSmem = 228 * 1024 / 2 - 1024;  // the most for two CTAs per SM
 
 inline size_t bar_bytes() { return (size_t)(4 * kMaxStages + 2 * kMaxA + 4 + kGroups) * 8 + 16 + (3 * kMaxExperts + 4) * sizeof(int); }
 inline size_t smem_bytes(int nb, int x_stages, int w_stages) {
@@ -48,9 +52,11 @@ inline size_t smem_bytes(int nb, int x_stages, int w_stages) {
 
 struct Launch {
   int grid, zmode, src;
+  int ranges;  // every tile is shared by a cluster of as many CTAs, 0: parts go through global scratch
   size_t smem;
 };
 int launch_i4(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream);
+int cluster_places(int ranges);  // clusters of so many CTAs that run at a time
 int launch_i8(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream);
 
 #ifdef __CUDACC__
@@ -66,7 +72,85 @@ __device__ __forceinline__ void tma_load_x(void* smem_dst, const CUtensorMap* ma
       : "memory");
 }
 
-template <int BITS, int ZMODE, int SRC>
+__device__ __forceinline__ uint32_t cluster_nctarank() {
+  uint32_t r;
+  asm("mov.u32 %0, %%cluster_nctaid.x;" : "=r"(r));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
+// Parts of a tile in one cluster: each CTA sends column c of its accumulator to the CTA that adds it up, in place of that
+// CTA's ring of weights (at most 64 + 7 columns of 512 bytes; the ring has at least three stages of 16 KB).  A CTA whose
+// waits ran out sends NaN.  Columns and not weight rows: a thread's sixteen values go to few CTAs, 128 bytes a warp each.
+__device__ __forceinline__ void exchange_send(const Params& pp, uint32_t ring, uint32_t d, int cols, int rank, int ranks, int grp, int gj,
+                                              bool ok) {
+  const int most = (cols + ranks - 1) / ranks;
+  for (int c0 = grp * 16; c0 < cols; c0 += kGroups * 16) {
+    float v[16];
+    tc_ld16(d + (uint32_t)c0, v);
+    int to = ((c0 + 1) * ranks - 1) / cols, lo = cols * to / ranks, hi = cols * (to + 1) / ranks;
+    uint32_t dst = 0;
+    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(ring), "r"(to));
+#pragma unroll
+    for (int i = 0; i < 16; ++i) {
+      const int c = c0 + i;
+      if (c >= cols) break;
+      if (c >= hi) {
+        do {
+          ++to;
+          lo = hi;
+          hi = cols * (to + 1) / ranks;
+        } while (c >= hi);
+        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(ring), "r"(to));
+      }
+      asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + (uint32_t)(((rank * most + c - lo) * kTileRows + gj) * 4)),
+                   "f"(ok ? v[i] : __int_as_float(0x7fffffff))
+                   : "memory");
+    }
+  }
+}
+// This CTA's columns, half of them each group's, a weight row per thread; parts in the order of the CTAs as in drain_store.
+template <bool SCALED>
+__device__ __forceinline__ void exchange_store(const Params& pp, const float* parts, const float* scales, int n0, int m0, int cols, int rank,
+                                               int ranks, int grp, int row) {
+  const GemvParams& p = pp.g;
+  const int most = (cols + ranks - 1) / ranks, lo = cols * rank / ranks, hi = cols * (rank + 1) / ranks, half = (hi - lo + 1) / 2;
+  const int first = lo + grp * half, end = grp ? hi : lo + half;
+  // where the sending thread of this weight row put it: its tensor-memory lane
+  const int blk = row >> 4, lane = (((row >> 3) & 1) + 2 * (blk >> 2)) * 32 + (blk & 3) * 8 + (row & 7);
+  const float scale = SCALED ? scales[lane] : 1.0f;
+  const int n = n0 + row;
+  for (int c = first; c < end; c += 4) {
+    float v[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i) v[i] = parts[(min(c + i, end - 1) - lo) * kTileRows + lane];
+    for (int s = 1; s < ranks; ++s)
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] += parts[(s * most + min(c + i, end - 1) - lo) * kTileRows + lane];
+    if (SCALED) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) v[i] *= scale;
+    }
+    const int m = m0 + c, m_end = m0 + end;
+    if (p.epi.act == kActSwiglu) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float up = __shfl_down_sync(0xffffffffu, v[i], 8);
+        if (m + i < m_end && n < p.n && !(row & 8))
+          p.out[(int64_t)(m + i) * p.ldo + n0 / 2 + blk * 8 + (row & 7)] = __float2half_rn(silu_mul(v[i], up));
+      }
+    } else {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        if (m + i < m_end && n < p.n) p.out[(int64_t)(m + i) * p.ldo + n] = __float2half_rn(apply_epilogue(v[i], p.epi, m + i, n));
+    }
+  }
+}
+
+template <int BITS, int ZMODE, int SRC, bool CLUSTER>
 __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
     umma_sk_kernel(const Params pp, const __grid_constant__ CUtensorMap tmap_x) {
   constexpr int kBlkPerChunk = BITS == 8 ? 2 : 4;   // 64-k blocks per weight stage
@@ -97,7 +181,8 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   Tables& tt = *reinterpret_cast<Tables*>(tmem_holder + 4);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool grouped = pp.indptr != nullptr;
+  const bool grouped = !CLUSTER && pp.indptr != nullptr;
+  bool fine = true;
   if (tid == 0) {
     for (int s = 0; s < w_stages; ++s) {
       mbar_init(&w_full[s], 1);
@@ -154,7 +239,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   const unsigned items = grouped ? (unsigned)tt.base[pp.num_experts] : (unsigned)(n_tiles * pp.m_tiles);
   const unsigned total = items * (unsigned)cpt;  // total * grid fits 31 bits (checked by the host)
   // what the cuts fall between: chunks, or tiles where there are no words to hand over a part of one
-  const unsigned step = pp.partial ? 1u : (unsigned)cpt, units = pp.partial ? total : items;
+  const unsigned step = CLUSTER || pp.partial ? 1u : (unsigned)cpt, units = CLUSTER || pp.partial ? total : items;
   // (experts without rows can leave fewer units than CTAs: the surplus CTAs stay out of the split)
   const unsigned ctas = min(gridDim.x, units);
   // the first `whole` CTAs take a tile each, the others equal runs of the rest
@@ -424,6 +509,10 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
         break;
       }
       tc_fence_after();
+      if (CLUSTER) {
+        if (folds<ZMODE, SRC>()) reinterpret_cast<float*>(e_stage)[gj] = drain_scale<BITS>(feed.s_row, hi);  // (both groups the same)
+        break;
+      }
       if (!waited) {
         griddep_wait();  // outputs and scratch may be in use by the previous kernel until it has ended
         waited = true;
@@ -452,8 +541,24 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
         dph ^= 1u;
       }
     }
+    fine = ok;
   }
 
+  if (CLUSTER) {
+    const int grp = (warp - 4) >> 2, w4 = warp & 3, ranks = (int)cluster_nctarank(), rank = (int)blockIdx.x % ranks;
+    const Item it = get_item((int)blockIdx.x / ranks);
+    const int cols = min(nb, it.m_end - it.m0);
+    cluster_sync();  // no CTA reads its ring of weights any more
+    if (warp >= 4) {
+      exchange_send(pp, smem_u32(w_ring), ((uint32_t)(32 * w4) << 16) | tmem, cols, rank, ranks, grp, w4 * 32 + lane, fine);
+      tc_fence_before();
+      if (pp.early) griddep_wait();  // outputs may be in use by the previous kernel until it has ended
+    }
+    cluster_sync();
+    if (warp >= 4)
+      exchange_store<folds<ZMODE, SRC>()>(pp, reinterpret_cast<const float*>(w_ring), reinterpret_cast<const float*>(e_stage),
+                                          it.n_tile * kTileRows, it.m0, cols, rank, ranks, grp, w4 * 32 + lane);
+  }
   __syncthreads();
   if (warp == 1) {
     tc_fence_after();
@@ -461,9 +566,9 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   }
 }
 
-template <int BITS, int ZMODE, int SRC>
-int launch_inst(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream) {
-  auto kern = umma_sk_kernel<BITS, ZMODE, SRC>;
+template <int BITS, int ZMODE, int SRC, bool CLUSTER>
+int launch_form(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream) {
+  auto kern = umma_sk_kernel<BITS, ZMODE, SRC, CLUSTER>;
   static thread_local int configured_device = -1;
   int dev = 0;
   RB200_CUDA(cudaGetDevice(&dev));
@@ -476,15 +581,26 @@ int launch_inst(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaSt
   cfg.blockDim = dim3((4 + 4 * kGroups) * 32, 1, 1);
   cfg.dynamicSmemBytes = l.smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
+  if (CLUSTER) {
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = (unsigned)l.ranges;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cfg.numAttrs = 1;
+  }
   // always a programmatic dependent: before its wait the kernel only prefetches, unless the host
   // switched launch overlap on
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[cfg.numAttrs].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  ++cfg.numAttrs;
   RB200_CUDA(cudaLaunchKernelEx(&cfg, kern, pp, tx));
   return 0;
+}
+template <int BITS, int ZMODE, int SRC>
+int launch_inst(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream) {
+  if (l.ranges > 1) return launch_form<BITS, ZMODE, SRC, true>(pp, l, tx, stream);
+  return launch_form<BITS, ZMODE, SRC, false>(pp, l, tx, stream);
 }
 
 template <int BITS, int ZMODE>

@@ -107,7 +107,7 @@ int run_single(Params& pp, int bits, int zmode, int src, int sm_count, cudaStrea
   pp.na = (pp.tmem_cols - pp.a_base) / (32 * own);
   if (pp.na > kMaxA) pp.na = kMaxA;
   // rings: x stages first (one 64-k block each), then as many weight stages as fit
-  const size_t budget = (size_t)(228 * 1024) / 2 - 1024;
+  const size_t budget = kCtaSmem;
   pp.x_stages = 4;
   pp.w_stages = kMaxStages;
   while (pp.w_stages > 3 && smem_bytes(pp.nb, pp.x_stages, pp.w_stages) > budget) --pp.w_stages;
@@ -132,13 +132,29 @@ int run_single(Params& pp, int bits, int zmode, int src, int sm_count, cudaStrea
     if (ranges > longest) ranges = longest;
     if (ranges > 8) ranges = 8;
     if (ranges >= 2 || items <= sm_count) grid = items * (ranges > 1 ? ranges : 1);
+    // Where the parts of a tile are many or large they are added inside a cluster: one exchange through shared memory in
+    // place of a trip to memory per part.  Without overlap of launches, us before / now: k 4096 x n 4096 int4 group 32,
+    // 32 rows 12.2 / 11.4, 64 rows 14.8 / 13.3; k 11008 x n 4096 32 rows 17.5 / 16.8, 64 rows 23.4 / 18.7; k 8192 x
+    // n 1024 64 rows 18.6 / 11.7; int8 per row k 8192 x n 4096 64 rows 22.7 / 17.6.  Fewer or smaller parts lose to the
+    // two cluster barriers (32 rows: k 2048 x n 4096 in three CTAs a tile 9.3 / 11.1, k 14336 x n 4096 in seven 13.9 / 14.7;
+    // 48 rows of int8 in four 1 % slower), and clusters that do not all run at once to the second wave (k 4096 x n 12288,
+    // 96 x 3: 15.0 / 27.3).  Overlapped launches of up to 32 rows start late in an SM that is full of them: there only up
+    // to a CTA per SM (k 4096 x n 2048 9.6 / 8.3; n 4096, 256 CTAs, 10.4 / 11.0).
+    const int k_blocks = p.k / kKBlock;
+    int wide = k_blocks / 8 < 8 ? k_blocks / 8 : 8;
+    while (wide >= 4 && cluster_places(wide) < items) --wide;
+    if (pp.nb <= 32 ? wide == 8 && (!pp.early || items * wide <= sm_count)
+                    : (wide > 4 || (wide == 4 && k_blocks >= 64)) && wide * pp.nb >= (bits == 4 ? 192 : 256)) {
+      l.ranges = wide;
+      grid = items * wide;
+    }
   } else if (units < 3 * grid) {
     grid = sm_count;  // a tile cut into many short ranges spends its time in the hand-over
   }
   if (grid > units) grid = units;
   RB200_CHECK(units * grid < (1ll << 31), "problem too large for the 32-bit work split (n=%d, k=%d, m=%d)", p.n, p.k, p.m);
   // (one CTA per tile cuts none)
-  if (pp.indptr || grid != items) pp.partial = handover_words(stream, sm_count, (size_t)grid * pp.nb * kTileRows * sizeof(float));
+  if (!l.ranges && (pp.indptr || grid != items)) pp.partial = handover_words(stream, sm_count, (size_t)grid * pp.nb * kTileRows * sizeof(float));
   // A tile per SM is not cut: its first CTA makes one, the second a run of the rest.  That saves a quarter of the pieces
   // where the tiles come near two per SM; with fewer the second CTA is done long before the first (int8 per row, 48 rows,
   // k 4096: n 32016 26.6 us in equal runs, 25.3 so, n 36000 28.3 / 27.9, n 22016 27.5 / 27.9, 24 rows 24.4 / 26.1; int4

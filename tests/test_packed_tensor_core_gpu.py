@@ -7,7 +7,7 @@ import numpy as np
 import pytest
 import torch
 
-from relax_b200 import ops, synth
+from relax_b200 import get_launch_overlap, ops, set_launch_overlap, synth
 from tests.test_autogptq_gpu import _case as gptq_case
 from tests.test_gemv_gpu import _check_status
 from tests.util import assert_close, bits16, to_dev, u32_to_dev
@@ -102,3 +102,42 @@ def test_a_tile_per_sm_and_runs_of_the_rest(oracle, m, tiles, k):
     got = _twice(lambda: ops.gemm_fp16_q4f16(x, pre, s, group_size=32))
     C = oracle.C()
     assert_close(got, C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, None, 7.0, 32))))
+
+
+@pytest.mark.parametrize("m", [17, 31, 33, 50, 64, 81])
+@pytest.mark.parametrize("k,n", [(2560, 144), (3136, 272), (4160, 1040), (11008, 16)])
+def test_parts_of_a_tile_in_a_cluster(oracle, m, k, n):
+    """columns that do not divide by the CTAs of a tile, a last tile of few weight rows, a last batch tile of few rows"""
+    rs = np.random.RandomState(m + k + n)
+    C = oracle.C()
+    case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, 32)
+    pre, s, x = ops.preprocess_weight_q4f16(u32_to_dev(case.w)), to_dev(case.scales), to_dev(case.x)
+    acc = C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, None, 7.0, 32))
+    assert_close(_twice(lambda: ops.gemm_fp16_q4f16(x, pre, s, group_size=32)), C.epilogue(acc))
+    bias, res = rs.randn(n).astype(np.float16), rs.randn(m, n).astype(np.float16)
+    b, r = to_dev(bias), to_dev(res)
+    got = _twice(lambda: ops.gemm_fp16_q4f16(x, pre, s, bias=b, residual=r, activation="relu", binary_op="plus", group_size=32))
+    assert_close(got, C.epilogue(acc, bias, res, "relu", "plus"))
+    w, s8 = rs.randint(-128, 128, size=(k, n)).astype(np.int8), rs.uniform(1e-4, 1e-3, size=(n,)).astype(np.float16)
+    pre, s = ops.preprocess_weight_ft(to_dev(w), False), to_dev(s8)
+    assert_close(_twice(lambda: ops.gemm_fp16_ft(x, pre, s, 8, group_size=-1)),
+                 C.epilogue(C.matmul_f32(case.x, C.decode_ft_kn(w, s8, 8, -1), False)))
+
+
+@pytest.mark.parametrize("m,overlap", [(19, False), (32, True), (64, False)])
+def test_gate_and_up_rows_of_a_cluster(oracle, m, overlap):
+    """the gated activation, gate and up rows eight lanes apart, with overlap of launches where that is switched on"""
+    k, ffn = 4096, 144
+    rs = np.random.RandomState(m)
+    x, w = rs.randn(m, k).astype(np.float16), rs.randint(0, 2 ** 32, size=(2 * ffn, k // 8), dtype=np.uint32)
+    s = rs.uniform(1e-3, 1e-2, size=(2 * ffn, k // 32)).astype(np.float16)
+    pre, si, xd = ops.preprocess_weight_gate_up(u32_to_dev(w)), ops.interleave_gate_up(to_dev(s)), to_dev(x)
+    before = get_launch_overlap()
+    set_launch_overlap(overlap)
+    try:
+        got = _twice(lambda: ops.gemm_fp16_q4f16(xd, pre, si, activation="swiglu")).astype(np.float64)
+    finally:
+        set_launch_overlap(before)
+    y = oracle.C().matmul_f32(x, oracle.C().decode_q4_nk(w, s, None, 7.0, 32)).astype(np.float64)
+    exp = y[:, :ffn] / (1 + np.exp(-y[:, :ffn])) * y[:, ffn:]
+    assert np.linalg.norm(got - exp) <= 1e-3 * np.linalg.norm(exp)
