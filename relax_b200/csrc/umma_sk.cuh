@@ -18,7 +18,7 @@
 // several contributors' words requested together, one trip to memory per try - and puts the pattern
 // back.  (A fence, a flag and a second trip per contributor cost 6 us at k = n = 4096.)
 // Where a tile is cut into equal parts that are many or large, its CTAs form a cluster instead and each adds up its
-// share of the columns (CLUSTER; the rule and its figures are beside the split in umma_tile.cu): the owner's trips to
+// share of the columns (kCluster; the rule and its figures are beside the split in umma_tile.cu): the owner's trips to
 // memory, one per part, were up to a third of such a launch, and the registers for several parts a trip spill.
 //
 //   warp 0  packed weights, one 16 KB bulk copy per chunk (128 rows x 256 | 128 k)
@@ -50,6 +50,9 @@ inline size_t smem_bytes(int nb, int x_stages, int w_stages) {
   return 1024 + (size_t)x_stages * nb * 128 + (size_t)w_stages * kWBytes + kGroups * kStageBytes + bar_bytes();
 }
 
+// How the tiles are cut: equal runs of chunks, a tile each for the first CTAs and runs of the rest (Params::whole), or
+// every tile over a cluster.
+enum Split { kRuns, kWholeFirst, kCluster };
 struct Launch {
   int grid, zmode, src;
   int ranges;  // every tile is shared by a cluster of as many CTAs, 0: parts go through global scratch
@@ -150,14 +153,14 @@ __device__ __forceinline__ void exchange_store(const Params& pp, const float* pa
   }
 }
 
-template <int BITS, int ZMODE, int SRC, bool CLUSTER>
+template <int BITS, int ZMODE, int SRC, int SPLIT>
 __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
     umma_sk_kernel(const Params pp, const __grid_constant__ CUtensorMap tmap_x) {
   constexpr int kBlkPerChunk = BITS == 8 ? 2 : 4;   // 64-k blocks per weight stage
   constexpr int kTilesPerBlk = BITS == 8 ? 2 : 1;
   constexpr int kFragK = BITS == 8 ? 32 : 64;
   constexpr int kOwn = kBlkPerChunk / kGroups;  // adjacent blocks of a chunk one group decodes: an A slot
-  constexpr bool kZ = ZMODE == kZeroGeneral;
+  constexpr bool kExchange = SPLIT == kCluster;
   extern __shared__ uint8_t smem_raw[];
   const GemvParams& p = pp.g;
   // 1 KB alignment as an offset from the array (a pointer rebuilt from an integer would turn every
@@ -181,7 +184,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   Tables& tt = *reinterpret_cast<Tables*>(tmem_holder + 4);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  const bool grouped = !CLUSTER && pp.indptr != nullptr;
+  const bool grouped = !kExchange && pp.indptr != nullptr;
   bool fine = true;
   if (tid == 0) {
     for (int s = 0; s < w_stages; ++s) {
@@ -239,14 +242,18 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   const unsigned items = grouped ? (unsigned)tt.base[pp.num_experts] : (unsigned)(n_tiles * pp.m_tiles);
   const unsigned total = items * (unsigned)cpt;  // total * grid fits 31 bits (checked by the host)
   // what the cuts fall between: chunks, or tiles where there are no words to hand over a part of one
-  const unsigned step = CLUSTER || pp.partial ? 1u : (unsigned)cpt, units = CLUSTER || pp.partial ? total : items;
+  const unsigned step = kExchange || pp.partial ? 1u : (unsigned)cpt, units = kExchange || pp.partial ? total : items;
   // (experts without rows can leave fewer units than CTAs: the surplus CTAs stay out of the split)
   const unsigned ctas = min(gridDim.x, units);
-  // the first `whole` CTAs take a tile each, the others equal runs of the rest
-  const unsigned whole = (unsigned)pp.whole, base = whole * (unsigned)cpt;
-  const unsigned rest = units - base, takers = min(ctas - whole, rest), idx = blockIdx.x - whole;
-  const unsigned u_begin = blockIdx.x < whole ? blockIdx.x * (unsigned)cpt : (idx < takers ? base + idx * rest / takers * step : 0u);
-  const unsigned u_end = blockIdx.x < whole ? (blockIdx.x + 1) * (unsigned)cpt : (idx < takers ? base + (idx + 1) * rest / takers * step : 0u);
+  unsigned u_begin = blockIdx.x < ctas ? blockIdx.x * units / ctas * step : 0u;
+  unsigned u_end = blockIdx.x < ctas ? (blockIdx.x + 1) * units / ctas * step : 0u;
+  [[maybe_unused]] unsigned whole = 0u, base = 0u, rest = 0u, takers = 0u;
+  if constexpr (SPLIT == kWholeFirst) {
+    whole = (unsigned)pp.whole, base = whole * (unsigned)cpt, rest = total - base, takers = min(ctas - whole, rest);
+    const unsigned idx = blockIdx.x - whole;
+    u_begin = blockIdx.x < whole ? blockIdx.x * (unsigned)cpt : (idx < takers ? base + idx * rest / takers : 0u);
+    u_end = blockIdx.x < whole ? u_begin + (unsigned)cpt : (idx < takers ? base + (idx + 1) * rest / takers : 0u);
+  }
 
   auto get_item = [&](int item) {
     Item it;
@@ -509,7 +516,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
         break;
       }
       tc_fence_after();
-      if (CLUSTER) {
+      if (kExchange) {
         if (folds<ZMODE, SRC>()) reinterpret_cast<float*>(e_stage)[gj] = drain_scale<BITS>(feed.s_row, hi);  // (both groups the same)
         break;
       }
@@ -528,7 +535,8 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
         if (w.c1 < cpt) {
           // this CTA owns the tile, later ones hold the rest
           const unsigned hi_u = (unsigned)w.item * (unsigned)cpt + (unsigned)cpt - 1u;
-          last = (int)(whole + ((hi_u - base + 1u) * takers - 1u) / rest);
+          if constexpr (SPLIT == kWholeFirst) last = (int)(whole + ((hi_u - base + 1u) * takers - 1u) / rest);
+          else last = (int)(((hi_u + 1u) * ctas - 1u) / total);
         }
         ok = drain_store<false, folds<ZMODE, SRC>()>(pp, dt, me, last, 1, e_stage + grp * kStageBytes, step, group_sync);
         if (!ok) break;
@@ -544,7 +552,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
     fine = ok;
   }
 
-  if (CLUSTER) {
+  if (kExchange) {
     const int grp = (warp - 4) >> 2, w4 = warp & 3, ranks = (int)cluster_nctarank(), rank = (int)blockIdx.x % ranks;
     const Item it = get_item((int)blockIdx.x / ranks);
     const int cols = min(nb, it.m_end - it.m0);
@@ -566,9 +574,9 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   }
 }
 
-template <int BITS, int ZMODE, int SRC, bool CLUSTER>
-int launch_form(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream) {
-  auto kern = umma_sk_kernel<BITS, ZMODE, SRC, CLUSTER>;
+template <int BITS, int ZMODE, int SRC, int SPLIT>
+int launch_split(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream) {
+  auto kern = umma_sk_kernel<BITS, ZMODE, SRC, SPLIT>;
   static thread_local int configured_device = -1;
   int dev = 0;
   RB200_CUDA(cudaGetDevice(&dev));
@@ -582,7 +590,7 @@ int launch_form(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaSt
   cfg.dynamicSmemBytes = l.smem;
   cfg.stream = stream;
   cudaLaunchAttribute attr[2];
-  if (CLUSTER) {
+  if (SPLIT == kCluster) {
     attr[0].id = cudaLaunchAttributeClusterDimension;
     attr[0].val.clusterDim.x = (unsigned)l.ranges;
     attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
@@ -599,8 +607,9 @@ int launch_form(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaSt
 }
 template <int BITS, int ZMODE, int SRC>
 int launch_inst(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream) {
-  if (l.ranges > 1) return launch_form<BITS, ZMODE, SRC, true>(pp, l, tx, stream);
-  return launch_form<BITS, ZMODE, SRC, false>(pp, l, tx, stream);
+  if (l.ranges > 1) return launch_split<BITS, ZMODE, SRC, kCluster>(pp, l, tx, stream);
+  if (pp.whole) return launch_split<BITS, ZMODE, SRC, kWholeFirst>(pp, l, tx, stream);
+  return launch_split<BITS, ZMODE, SRC, kRuns>(pp, l, tx, stream);
 }
 
 template <int BITS, int ZMODE>

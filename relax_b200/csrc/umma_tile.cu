@@ -136,7 +136,7 @@ int run_single(Params& pp, int bits, int zmode, int src, int sm_count, cudaStrea
     // place of a trip to memory per part.  Without overlap of launches, us before / now: k 4096 x n 4096 int4 group 32,
     // 32 rows 12.2 / 11.4, 64 rows 14.8 / 13.3; k 11008 x n 4096 32 rows 17.5 / 16.8, 64 rows 23.4 / 18.7; k 8192 x
     // n 1024 64 rows 18.6 / 11.7; int8 per row k 8192 x n 4096 64 rows 22.7 / 17.6.  Fewer or smaller parts lose to the
-    // two cluster barriers (32 rows: k 2048 x n 4096 in three CTAs a tile 9.3 / 11.1, k 14336 x n 4096 in seven 13.9 / 14.7;
+    // two cluster barriers (32 rows: k 2048 x n 4096 in three CTAs a tile 9.3 / 11.1, k 14336 x n 4096 in seven 20.2 / 21.3;
     // 48 rows of int8 in four 1 % slower), and clusters that do not all run at once to the second wave (k 4096 x n 12288,
     // 96 x 3: 15.0 / 27.3).  Overlapped launches of up to 32 rows start late in an SM that is full of them: there only up
     // to a CTA per SM (k 4096 x n 2048 9.6 / 8.3; n 4096, 256 CTAs, 10.4 / 11.0).
