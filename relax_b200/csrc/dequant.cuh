@@ -82,6 +82,11 @@ __device__ __forceinline__ uint32_t h2_mul(uint32_t a, uint32_t b) {
   asm("mul.rn.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
   return r;
 }
+__device__ __forceinline__ uint32_t h2_min(uint32_t a, uint32_t b) {  // (of a NaN and a number the number)
+  uint32_t r;
+  asm("min.f16x2 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(b));
+  return r;
+}
 __device__ __forceinline__ uint32_t h2_fma(uint32_t a, uint32_t b, uint32_t c) {
   uint32_t r;
   asm("fma.rn.f16x2 %0, %1, %2, %3;" : "=r"(r) : "r"(a), "r"(b), "r"(c));
@@ -216,12 +221,23 @@ __device__ __forceinline__ void codes_int8_pair(uint32_t w_g, uint32_t w_g8, uin
 // Zero points of rows g (low half) and g + 8 in those units, and whether they fit (integers do): a
 // subnormal has no room for a fraction.  misfit gets bits where they don't.
 template <int BITS>
+__device__ __forceinline__ uint32_t zero_in_codes(uint32_t z_pair) {
+  return h2_mul(z_pair, BITS == 4 ? 0x00100001u : 0x00010001u);  // f16x2(2^-24, 2^-20 | 2^-24)
+}
+template <int BITS>
+__device__ __forceinline__ uint32_t zero_from_codes(uint32_t z) {
+  return h2_mul(h2_mul(z, 0x6c006c00u), BITS == 4 ? 0x5c006c00u : 0x6c006c00u);  // times 4096, and the rest
+}
+template <int BITS>
 __device__ __forceinline__ uint32_t zero_in_codes(uint32_t z_pair, uint32_t& misfit) {
-  constexpr uint32_t kUnits = BITS == 4 ? 0x00100001u : 0x00010001u;  // f16x2(2^-24, 2^-20 | 2^-24)
-  constexpr uint32_t k4096 = 0x6c006c00u, kRest = BITS == 4 ? 0x5c006c00u : 0x6c006c00u;
-  const uint32_t z = h2_mul(z_pair, kUnits);
-  misfit |= h2_mul(h2_mul(z, k4096), kRest) ^ z_pair;
+  const uint32_t z = zero_in_codes<BITS>(z_pair);
+  misfit |= zero_from_codes<BITS>(z) ^ z_pair;
   return z;
+}
+// What does not fit, exactly; of infinities and NaN something finite.
+template <int BITS>
+__device__ __forceinline__ uint32_t zero_rest(uint32_t z_pair) {
+  return h2_min(h2_sub(z_pair, zero_from_codes<BITS>(zero_in_codes<BITS>(z_pair))), 0x3c003c00u);
 }
 template <int BITS>
 __device__ __forceinline__ uint32_t zero_in_codes(uint32_t z_pair, bool& fits) {

@@ -15,9 +15,8 @@
 //   * a column without a batch row is never loaded (zeros stay in its registers): with the absent rows read as
 //     row 0 the loads of x took 70 % of what L1 passes on, now 20 %;
 //   * k may end within a chunk (k % 256 != 0): the last unit of a row block is shorter.
-// Zero points that are not integers do not fit the codes' units.  Row blocks that met one are computed again
-// before they are stored, by the decode without scales (again(), never reached with integers; inside the loop, or
-// called, it cost the kernels with zero points 300 to 700 bytes of spills).
+// Zero points that are not integers do not fit the codes' units.  The loop takes what fits of them, and a warp that met one
+// adds the rest to its sums before they are put together (add_fractions, never reached with integers).
 //
 // Bound: instruction issue and latency, then HBM.  Of 65 instructions a 512-byte tile needs 36 are the codes, 4
 // MMAs, 8 the scales; issue slots are half used and a warp mostly waits for its weights, but a third set of loads
@@ -134,52 +133,143 @@ struct Share {
   __device__ int row(int i) const { return m0 + i; }
 };
 
-// A warp's sums of one row block once more, in the codes' units and the caller's columns: for zero points that are not
-// integers.  k blocks kb0 to kb1; x at kb0, read by the lanes that have a column.  (kWide: with the lanes' own groups,
-// the scales in the weights.)
-template <bool kPairs, bool kWide, class Run>
-__device__ __forceinline__ float4 again(const Params& pp, const Run& run, const __half* x, bool mine, int nb, int kb0, int kb1) {
-  const GemvParams& p = pp.g;
+constexpr int vals(int src) { return src == rk::kRow32 ? 2 : 4; }  // sums of a lane, row block and m-tile
+
+// D(16x8) += A(16x8 tf32) * B(8x8 tf32): row g, columns t, t + 4 of A and rows t, t + 4, column g of B by lane
+__device__ __forceinline__ void mma_1688(float (&d)[4], const float (&a)[4], float b0, float b1) {
+  asm volatile("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+               : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
+               : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
+                 "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+}
+__device__ __forceinline__ float tf32_of(float v) { return __uint_as_float(__float_as_uint(v) & 0xffffe000u); }
+
+// A zero point that is no integer fits the codes' units but for a fraction (of row g + 8, whose units are finer, for what
+// is left of sixteenths): z = r + f, sum (u - z) x = sum (u - r) x - f sum x.  The loop has the first part, this adds the
+// second to a warp's sums of `count` row blocks, from x, the scales and the zero points and without the weights.  Sums of x
+// of a chunk's tiles (groups of 32: of each group) come out of MMAs with a column of ones each in the places of the B of a
+// product with -f s (tf32: x in two parts, the fraction, a few per cent of the result, rounded to 11 bits).  k blocks kb0 to
+// kb1; x (this lane's sixteen k of a tile), its row eight further and the scales and zero points of the first block's row g.
+// Bound: L1, which passes x on once more for each window of row blocks.  Reading and decoding the weights again instead, with
+// fractions everywhere (before / now; with integers; gemv_rk.cuh's kernel, which decodes either), us: k 4096 x n 22016, groups
+// of 64, one row 43.2 / 17.3; 13.8; 30.3, sixteen rows 76.1 / 33.2; 22.2; 31.2, groups of 32, eight rows 49.1 / 23.1; 18.6;
+// 21.9; k = n = 4096, groups of 32, one row 10.2 / 6.3; 4.8; 5.4, eight rows 11.4 / 8.0; 5.9; 6.0, groups of 128 10.1 / 6.9;
+// 4.8; 6.0.  One fraction in the whole weight, groups of 128, k 4096 x n 22016, one row: 30.4 / 13.4; 13.0; 16.3.
+struct Fractions {
+  const __half *x, *x8, *s, *z;
+  int kb0, kb1, count, s_n, s_g, group, group_shift;
+};
+template <int SRC, bool kTail, int MT>
+__device__ __forceinline__ void add_fractions_inline(Fractions a, float (*red)[kWarps][32 * vals(SRC)]) {
+  constexpr bool kPairs = SRC == rk::kRow32, k32 = kPairs || SRC == kRow32Wide;
   const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
-  const int NB = p.n / 16, KB = p.k / 64;
-  const ZeroConsts zc = make_zero_consts(kZeroGeneral, 0.0f);
-  float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+  float* const sums = &red[0][threadIdx.x >> 5][lane * vals(SRC)];
+  constexpr int kBlock = MT * kWarps * 32 * vals(SRC);  // from a row block's sums to the next one's
+  const uint32_t ones = (k32 ? (g & 1) == t >> 1 : !(g & 1)) ? 0x3c003c00u : 0u;
 #pragma unroll 1
-  for (int kb = kb0; kb < kb1; ++kb, x += 64) {
-    const uint4 w = rk::ld_stream_v4(run.w() + frag_tile_offset(nb, kb, NB, KB) + frag_unit_pos(lane) * 16);
-    uint4 xv[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
-    ld_x_if(xv[0], x, mine);
-    ld_x_if(xv[1], x + 8, mine);
-    const unsigned grp = (unsigned)(kb * 64 + (kWide ? t * 16 : 0)) / (unsigned)p.group;
-    uint32_t z[2], s2[2];
-    float d[4], s[2][2];
+  for (; a.kb0 < a.kb1; a.kb0 += 4, a.x += 256, a.x8 += 256) {
+    // lane t has the scales and zero points of tile t
+    const int kb = a.kb0 + t;
+    const bool there = !kTail || kb < a.kb1;
+    const unsigned o = k32 ? (unsigned)kb * 2u
+                           : (a.group_shift >= 0 ? (unsigned)(kb * 64) >> a.group_shift : (unsigned)(kb * 64) / (unsigned)a.group) * (unsigned)a.s_g;
+    const __half *sp = a.s + o, *zp = a.z + o;
+    uint32_t s[2], z[2];  // rows g, g + 8
+    auto load = [&]() {
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      const int64_t o = (int64_t)(nb * 16 + g + 8 * i) * pp.s_n + (int64_t)grp * pp.s_g;
-      z[i] = ld_nc_u16(run.z() + o + (kPairs ? t >> 1 : 0)) * 0x10001u;
-      s2[i] = ld_nc_u16(run.s() + o) * 0x10001u;
-      s[i][0] = kWide ? 1.0f : half_lo(s2[i]);
-      s[i][1] = kPairs ? half_lo(ld_nc_u16(run.s() + o + 1)) : s[i][0];
+      for (int i = 0; i < 2; ++i) {
+        if (kTail) s[i] = z[i] = 0u;
+        if (k32) {
+          ld_nc_if(s[i], sp + i * 8 * a.s_n, there);
+          ld_nc_if(z[i], zp + i * 8 * a.s_n, there);
+        } else {
+          ld_nc16_if(s[i], sp + i * 8 * a.s_n, there);
+          ld_nc16_if(z[i], zp + i * 8 * a.s_n, there);
+        }
+      }
+      sp += 16 * a.s_n;
+      zp += 16 * a.s_n;
+    };
+    load();
+    float xh[MT][2], xl[MT][2];  // of tile t's groups
+    {
+      uint4 v[MT][4][2];
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          if (kTail) v[mt][j][0] = v[mt][j][1] = make_uint4(0, 0, 0, 0);
+          if (!kTail || a.kb0 + j < a.kb1) {
+            v[mt][j][0] = rk::ld_x_v4((mt ? a.x8 : a.x) + j * 64);
+            v[mt][j][1] = rk::ld_x_v4((mt ? a.x8 : a.x) + j * 64 + 8);
+          }
+        }
+      // rows g of A are batch rows g, rows g + 8 batch rows g + 8 - or, in one m-tile, rows g of the next tile, so that
+      // tiles of either parity are in rows of their own
+      float d[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll
+      for (int j = 0; j < 4; j += 3 - MT) {
+        const uint32_t one = (MT == 1 ? g >> 2 == j >> 1 : g >> 1 == j) ? ones : 0u;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const uint4 &lo = v[0][j][i >> 1], &hi = v[MT - 1][j + 2 - MT][i >> 1];
+          const uint32_t w[4] = {(i & 1) ? lo.z : lo.x, (i & 1) ? hi.z : hi.x, (i & 1) ? lo.w : lo.y, (i & 1) ? hi.w : hi.y};
+          mma_16816(d, w, one, one);
+        }
+      }
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt)
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+          float sum = MT == 1 ? ((t & 1) ? d[2 + q] : d[q]) : d[2 * mt + q];
+          // (an infinite activation has made its rows' sums infinite already)
+          if ((kPairs && (g & 1) != q) || !(fabsf(sum) <= 3.4e38f)) sum = 0.0f;
+          xh[mt][q] = tf32_of(sum);
+          xl[mt][q] = sum - xh[mt][q];
+        }
     }
+    float* sum = sums;
+#pragma unroll 1
+    for (int left = a.count;; sum += kBlock) {
+      float f[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      constexpr uint32_t kOne = 0x3c003c00u;
-      uint32_t a[4];
-      if (kWide) decode_int4_word<kZeroGeneral>(word(w, i), zc, s2[0], s2[1], z[0], z[1], a);
-      else decode_int4_word<kZeroGeneral>(word(w, i), zc, kOne, kOne, z[0], z[1], a);
-      const uint4& xx = xv[i >> 1];
-      if (i == 0) mma_16816_first(d, a, xx.x, xx.y);
-      else mma_16816(d, a, (i & 1) ? xx.z : xx.x, (i & 1) ? xx.w : xx.y);
+      for (int q = 0; q < (k32 ? 2 : 1); ++q) {
+        const float2 r = halves(zero_rest<4>(prmt(z[0], z[1], q ? 0x7632u : 0x5410u)));
+        const float s0 = kUnitLo * half_lo(s[0] >> (16 * q)), s1 = kUnitHi * half_lo(s[1] >> (16 * q));
+        if (r.x != 0.0f) f[2 * q] = __uint_as_float(__float_as_uint(-r.x * s0) + 0x1000u);
+        if (r.y != 0.0f) f[2 * q + 1] = __uint_as_float(__float_as_uint(-r.y * s1) + 0x1000u);
+      }
+      const bool more = --left > 0;
+      if (more) load();
+#pragma unroll
+      for (int mt = 0; mt < MT; ++mt) {
+        float* at = sum + mt * (kBlock / MT);
+        if (kPairs) {
+          float2 v = *reinterpret_cast<float2*>(at);
+          float d[4] = {v.x, 0.0f, v.y, 0.0f};
+          mma_1688(d, f, xl[mt][0], xl[mt][1]);
+          mma_1688(d, f, xh[mt][0], xh[mt][1]);
+          *reinterpret_cast<float2*>(at) = make_float2(d[0] + d[1], d[2] + d[3]);
+        } else {
+          const float4 v = *reinterpret_cast<float4*>(at);
+          float d[4] = {v.x, v.y, v.z, v.w};
+          mma_1688(d, f, xl[mt][0], xl[mt][1]);
+          mma_1688(d, f, xh[mt][0], xh[mt][1]);
+          *reinterpret_cast<float4*>(at) = make_float4(d[0], d[1], d[2], d[3]);
+        }
+      }
+      if (!more) break;
     }
-#pragma unroll
-    for (int c = 0; c < 4; ++c) acc[c] += (c < 2 ? kUnitLo : kUnitHi) * s[c >> 1][c & 1] * d[c];
   }
-  return make_float4(acc[0], acc[1], acc[2], acc[3]);
+}
+// (Called for kRow32: written into that kernel it cost integers 6 %, k 4096 x n 22016, one row; a call costs the others
+// up to 10 % of a call with fractions.)
+template <int SRC, bool kTail, int MT>
+__device__ __noinline__ void add_fractions_call(Fractions a, float (*red)[kWarps][32 * vals(SRC)]) {
+  add_fractions_inline<SRC, kTail, MT>(a, red);
 }
 
-// kTail: k % 256 != 0
-constexpr int vals(int src) { return src == rk::kRow32 ? 2 : 4; }  // sums of a lane, row block and m-tile
-// MT: m-tiles of eight batch rows
+// kTail: k % 256 != 0; MT: m-tiles of eight batch rows
 template <int ZMODE, int SRC, bool kTail, int MT, class Run>
 __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, float (&red)[kWarps][kWarps][32 * vals(SRC)]) {
   using namespace rk;
@@ -236,7 +326,6 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
     s_at = s_at0;
     s_left = s_left0;
   };
-  start_at(0);
   auto advance = [&]() {
     constexpr int kStep = k32 ? 8 : kRow ? kSpans : 0;  // scales of a chunk
     --to_load;
@@ -315,7 +404,27 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
       }
     }
   };
-  clear();
+  // What a sequence begins with.  With zero points it may have to begin again (below), so that these loads are the head of a
+  // loop there; otherwise they leave as early as they can (1 to 2 % of a small matmul).
+  auto first_weights = [&](int block) {
+    start_at(block);
+    clear();
+    if (!Run::kWait || pp.early) {
+      load(I0{});
+      load(I1{});
+    } else if (lane < 16) {
+      // before the wait: a prefetch returns nothing to this kernel, so it is safe whatever the previous
+      // kernel still writes
+      const uint8_t* line = wp - unit16 + lane * 128;
+      for (int c = 0; c < min(2, min(nc, KB / 4 - c0)); ++c, line += stride) prefetch_l2(line);
+    }
+    if (Run::kWait) griddep_wait();
+    if (Run::kWait && !pp.early) {
+      load(I0{});
+      load(I1{});
+    }
+  };
+  if (!kZ) first_weights(0);
   // kChannel: the scales of the row block whose sums this warp puts together
   uint32_t ch_s[2] = {0x3c00u, 0x3c00u};
   auto load_channel = [&](int first, int count) {
@@ -325,20 +434,6 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
       for (int i = 0; i < 2; ++i) ld_nc16_if(ch_s[i], s + i * row8, true);
     }
   };
-  if (!Run::kWait || pp.early) {
-    load(I0{});
-    load(I1{});
-  } else if (lane < 16) {
-    // before the wait: a prefetch returns nothing to this kernel, so it is safe whatever the previous
-    // kernel still writes
-    const uint8_t* line = wp - unit16 + lane * 128;
-    for (int c = 0; c < min(2, min(nc, KB / 4 - c0)); ++c, line += stride) prefetch_l2(line);
-  }
-  if (Run::kWait) griddep_wait();
-  if (Run::kWait && !pp.early) {
-    load(I0{});
-    load(I1{});
-  }
   int count = min(kSlots, blocks);
   load_channel(0, count);
 
@@ -349,14 +444,12 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
 #pragma unroll
   for (int mt = 0; mt < MT; ++mt) mine[mt] = m + 8 * mt < run.m() && nc > 0 && (!kPairs || (t >> 1) == (g & 1));
   const __half* const x0 = run.x() + (m < run.m() ? m : 0) * (unsigned)p.ldx + (kWide ? (t & 1) * 16 + (t >> 1) * 8 : t * 16) + c0 * kChunkK;
-  const __half* xp = x0;
+  const __half* xp;
   uint4 x[kXTiles][MT][2];
   auto clear_x = [&](int j) {
 #pragma unroll
     for (int mt = 0; mt < MT; ++mt) x[j][mt][0] = x[j][mt][1] = make_uint4(0, 0, 0, 0);
   };
-#pragma unroll
-  for (int j = 0; j < kXTiles; ++j) clear_x(j);
   auto load_x = [&](int j, bool last) {
     const bool there = !kTail || !ends_short || !last || j < nkb_last;
     if (kTail && MT > 1) clear_x(j % kXTiles);  // (one m-tile: before the short unit)
@@ -366,8 +459,15 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
       for (int i = 0; i < 2; ++i)
         ld_x_if(x[j % kXTiles][mt][i], xp + mt * 8u * (unsigned)p.ldx + j * kFrag + i * (kWide ? 32 : 8), mine[mt] && there);
   };
+  auto first_x = [&]() {
+    xp = x0;
 #pragma unroll
-  for (int j = 0; j < kXTiles; ++j) load_x(j, nc == 1);
+    for (int j = 0; j < kXTiles; ++j) {
+      clear_x(j);
+      load_x(j, nc == 1);
+    }
+  };
+  if (!kZ) first_x();
 
   float acc[MT][4], acc2[4] = {0.0f, 0.0f, 0.0f, 0.0f};
 #pragma unroll
@@ -536,56 +636,53 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
       }
     }
   };
-  bool odd = false;  // which set is next
-  for (;;) {
-    if (nc == 0) {
-      for (int i = 0; i < count * MT; ++i)
-#pragma unroll
-        for (int v = 0; v < kVals; ++v) red[i][warp][lane * kVals + v] = 0.0f;
-    } else {
-#pragma unroll 1
-      for (;;) {
-        if (!odd) {
-          step(I0{});
-          odd = true;
-          if (window_done()) break;
-        }
-        step(I1{});
-        odd = false;
-        if (window_done()) break;
-      }
-    }
-    if (kZ) {
-      if (__syncthreads_or(misfit != 0)) break;
-    } else {
-      __syncthreads();
-    }
+  auto window_stored = [&]() {  // true: that was the last
+    __syncthreads();
     put_together();
     window += count;
-    if (window >= blocks) break;
+    if (window >= blocks) return true;
     count = min(kSlots, blocks - window);
     load_channel(window, count);
     slot = 0;
     __syncthreads();
-  }
-  if (kZ) {
-    // left early: these row blocks and the rest once more
-    while (window < blocks) {
-      count = min(kSlots, blocks - window);
-      for (int i = 0; i < count; ++i) {
+    return false;
+  };
+  for (;;) {
+    if (kZ) {
+      first_weights(window);
+      first_x();
+    }
+    bool odd = false;  // which set is next
+    for (;;) {
+      if (nc == 0) {
+        for (int i = 0; i < count * MT; ++i)
+#pragma unroll
+          for (int v = 0; v < kVals; ++v) red[i][warp][lane * kVals + v] = 0.0f;
+      } else {
 #pragma unroll 1
-        for (int mt = 0; mt < MT; ++mt) {
-          const __half* xa = x0 + (kWide ? t * 16 - ((t & 1) * 16 + (t >> 1) * 8) : 0) + mt * 8u * (unsigned)p.ldx;
-          const float4 f = again<kPairs, kWide>(pp, run, xa, mt ? mine[MT - 1] : mine[0], pos + window + i, c0 * 4, min(KB, (c0 + nc) * 4));
-          if (kPairs) *reinterpret_cast<float2*>(&red[i][warp][lane * 2]) = make_float2(f.x + f.y, f.z + f.w);
-          else *reinterpret_cast<float4*>(&red[i * MT + mt][warp][lane * 4]) = f;
+        for (;;) {
+          if (!odd) {
+            step(I0{});
+            odd = true;
+            if (window_done()) break;
+          }
+          step(I1{});
+          odd = false;
+          if (window_done()) break;
         }
       }
-      __syncthreads();
-      put_together();
-      __syncthreads();
-      window += count;
+      if (kZ && __any_sync(0xffffffffu, misfit != 0)) break;
+      if (window_stored()) return;
     }
+    // A zero point was no integer.  What is loaded ahead is loaded again: kept over this it would spill.
+    const unsigned at = (unsigned)((pos + window) * 16 + g) * (unsigned)pp.s_n;
+    const __half* xa = x0 + (kWide ? t * 16 - ((t & 1) * 16 + (t >> 1) * 8) : 0);
+    const Fractions a = {xa, MT > 1 && mine[MT - 1] ? xa + 8u * (unsigned)p.ldx : xa, run.s() + at, run.z() + at, c0 * 4, min(KB, (c0 + nc) * 4),
+                         count, pp.s_n, pp.s_g, p.group, pp.group_shift};
+    if (kPairs) add_fractions_call<SRC, kTail, MT>(a, red);
+    else add_fractions_inline<SRC, kTail, MT>(a, red);
+    misfit = 0;
+    if (window_stored()) return;
   }
 }
 

@@ -133,3 +133,96 @@ def test_experts(k, n, group, zeros, rows):
         exp = x[begin:end].astype(np.float64) @ wq[e].T
         assert np.linalg.norm(got[begin:end] - exp) <= BOUND * np.linalg.norm(exp)
         begin = end
+
+
+def _zeros_of(kind, rs, shape):
+    z = rs.randint(0, 16, size=shape).astype(np.float16)
+    if kind == "all":  # sixteenths, below zero and large ones among them
+        z = (rs.uniform(0, 15, size=shape)).astype(np.float16)
+        z.reshape(-1)[::7] = 5.0625
+        z.reshape(-1)[3::11] = -2.7
+        z.reshape(-1)[5::13] = 71.3
+    return z
+
+
+@pytest.mark.parametrize("m", [1, 3, 4, 8, 11, 16])
+@pytest.mark.parametrize("k,n,group,columns", [(4096, 1040, 32, False), (192, 48, 32, False), (4096, 8208, 32, False), (2368, 400, 32, False),
+                                               (4096, 1040, 64, False), (256, 47632, 64, False), (4096, 1040, 128, False), (1152, 9488, 128, False),
+                                               (8192, 4112, 128, True), (768, 144, 384, True), (11008, 4112, 128, True)])
+def test_fractional_zero_points(k, n, group, columns, m):
+    """Every zero point with a fraction: what the codes' units cannot hold is taken off afterwards, from more row blocks than one
+    meeting of the warps holds, warps without a chunk and short last chunks among them.  Outputs round to fp16, 2^-11 of a
+    value at most; the fractions' 12 bits are less than a tenth of that."""
+    rs = np.random.RandomState(m + k + n + group)
+    x = rs.randn(m, k).astype(np.float16)
+    w = rs.randint(0, 2 ** 32, size=(n, k // 8), dtype=np.uint32)
+    s = rs.uniform(1e-3, 1e-2, size=(n, k // group)).astype(np.float16)
+    z = _zeros_of("all", rs, s.shape)
+    if columns:
+        codes = ((w[:, :, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15).reshape(n, k)
+        qw = np.zeros((k // 8, n), dtype=np.uint32)
+        for i in range(8):
+            qw |= codes.T[i::8].astype(np.uint32) << np.uint32(4 * i)
+        out = ops.gemm_fp16_autogptq(to_dev(x), ops.preprocess_weight_autogptq(u32_to_dev(qw)), to_dev(np.ascontiguousarray(s.T)),
+                                     to_dev(np.ascontiguousarray(z.T)))
+    else:
+        out = ops.gemm_fp16_q4f16(to_dev(x), ops.preprocess_weight_q4f16(u32_to_dev(w)), to_dev(s), to_dev(z), group_size=group)
+        codes = ((w[:, :, None] >> (4 * np.arange(8, dtype=np.uint32))) & 15).reshape(n, k)
+    _check_status()
+    wq = (codes - np.repeat(z.astype(np.float64), group, axis=1)) * np.repeat(s.astype(np.float64), group, axis=1)
+    exp = x.astype(np.float64) @ wq.T
+    got = out.cpu().numpy().astype(np.float64)
+    assert np.linalg.norm(got - exp) <= BOUND * np.linalg.norm(exp)
+    assert np.abs(got - exp).max() <= 4 * BOUND * np.abs(exp).max()
+
+
+@pytest.mark.parametrize("group", [32, 64, 128])
+@pytest.mark.parametrize("m", [1, 8])
+def test_infinities_beside_fractional_zero_points(group, m):
+    """An infinite scale, zero point or activation stays with its row or column, and the sums that it takes part in are not finite."""
+    k, n = 1024, 64
+    rs = np.random.RandomState(m + group)
+    x = rs.randn(m, k).astype(np.float16)
+    x[m - 1, 700] = np.inf
+    w = rs.randint(0, 2 ** 32, size=(n, k // 8), dtype=np.uint32)
+    s, z = rs.uniform(1e-3, 1e-2, size=(n, k // group)).astype(np.float16), None
+    z = _zeros_of("all", rs, s.shape)
+    s[5, 1], z[18, 2], z[40, 3] = np.inf, np.inf, np.nan
+    got = ops.gemm_fp16_q4f16(to_dev(x), ops.preprocess_weight_q4f16(u32_to_dev(w)), to_dev(s), to_dev(z), group_size=group).cpu().numpy()
+    finite = np.ones((m, n), dtype=bool)
+    finite[m - 1], finite[:, [5, 18, 40]] = False, False
+    assert np.array_equal(np.isfinite(got), finite)
+
+
+@pytest.mark.parametrize("group", [32, 64, 128])
+@pytest.mark.parametrize("m", [1, 8, 16])
+def test_fractional_zero_points_take_no_second_pass(group, m):
+    """Weights are read once whatever the zero points are: a matmul took 2.6 to 3.4 times as long with fractions in all of them and
+    2.3 times with a single one while they were read and decoded again; now 1.2 to 1.5 times and 1.1."""
+    k, n = 4096, 22016
+    g = torch.Generator(device="cuda")
+    g.manual_seed(m + group)
+    pre = ops.preprocess_weight_q4f16(torch.randint(-2 ** 31, 2 ** 31 - 1, (n, k // 8), dtype=torch.int32, device="cuda", generator=g))
+    s = (torch.rand(n, k // group, device="cuda", generator=g) * 0.009 + 0.001).half()
+    whole = torch.randint(0, 16, s.shape, device="cuda", generator=g).half()
+    one = whole.clone()
+    one[n // 2, 3] = 7.3
+    x, out = torch.randn(m, k, device="cuda", generator=g).half(), torch.empty(m, n, dtype=torch.float16, device="cuda")
+    times = {}
+    graphs = {}
+    for name, z in (("whole", whole), ("one", one), ("all", whole + 0.3)):
+        graphs[name] = torch.cuda.CUDAGraph()
+        with torch.cuda.graph(graphs[name]):
+            for _ in range(20):
+                ops.gemm_fp16_q4f16(x, pre, s, z, group_size=group, out=out)
+        times[name] = []
+    for _ in range(8):
+        for name, graph in graphs.items():
+            a, b = torch.cuda.Event(enable_timing=True), torch.cuda.Event(enable_timing=True)
+            a.record()
+            graph.replay()
+            b.record()
+            b.synchronize()
+            times[name].append(a.elapsed_time(b))
+    best = {name: min(t) for name, t in times.items()}
+    assert best["all"] <= 2.0 * best["whole"] and best["one"] <= 1.5 * best["whole"], best
