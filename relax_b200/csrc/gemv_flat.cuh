@@ -157,8 +157,64 @@ __device__ __forceinline__ float tf32_of(float v) { return __uint_as_float(__flo
 // 4.8; 6.0.  One fraction in the whole weight, groups of 128, k 4096 x n 22016, one row: 30.4 / 13.4; 13.0; 16.3.
 struct Fractions {
   const __half *x, *x8, *s, *z;
-  int kb0, kb1, count, s_n, s_g, group, group_shift;
+  const uint8_t* w;
+  int kb0, kb1, first, count, NB, KB, s_n, s_g, group, group_shift;
 };
+// Where an activation is not finite its product with u - r is none where the code is r (0 inf) and u - z is not 0: those sums
+// anew, from u - z itself.
+template <int SRC, int MT>
+__device__ __noinline__ void sums_of_infinities(Fractions a, float (*red)[kWarps][32 * vals(SRC)]) {
+  constexpr bool kPairs = SRC == rk::kRow32, k32 = kPairs || SRC == kRow32Wide;
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const ZeroConsts zc = make_zero_consts(kZeroGeneral, 0.0f);
+#pragma unroll 1
+  for (int i = 0; i < a.count * MT; ++i) {
+    const int b = i / MT;
+    const __half* x = MT > 1 && (i & 1) ? a.x8 : a.x;
+    float acc[4] = {0.0f, 0.0f, 0.0f, 0.0f};
+#pragma unroll 1
+    for (int kb = a.kb0; kb < a.kb1; ++kb, x += 64) {
+      const uint4 w = rk::ld_stream_v4(a.w + frag_tile_offset(a.first + b, kb, a.NB, a.KB) + frag_unit_pos(lane) * 16);
+#pragma unroll 1
+      for (int q = 0; q < (SRC == kRow32Wide ? 2 : 1); ++q) {  // groups of 32: one at a time, or in columns of their own
+        const bool mine = !k32 || (t >> 1) == (kPairs ? g & 1 : q);
+        uint4 xv[2] = {make_uint4(0, 0, 0, 0), make_uint4(0, 0, 0, 0)};
+        ld_x_if(xv[0], x, mine);
+        ld_x_if(xv[1], x + 8, mine);
+        const unsigned grp = (unsigned)(kb * 64) / (unsigned)a.group;
+        float d[4], s[2][2];
+        uint32_t z[2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+          const int64_t o = (int64_t)(b * 16 + 8 * h) * a.s_n + (int64_t)grp * a.s_g;
+          z[h] = ld_nc_u16(a.z + o + (k32 ? t >> 1 : 0)) * 0x10001u;
+          s[h][0] = half_lo(ld_nc_u16(a.s + o + (SRC == kRow32Wide ? q : 0)));
+          s[h][1] = kPairs ? half_lo(ld_nc_u16(a.s + o + 1)) : s[h][0];
+        }
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          constexpr uint32_t kOne = 0x3c003c00u;
+          uint32_t c[4];
+          decode_int4_word<kZeroGeneral>(word(w, j), zc, kOne, kOne, z[0], z[1], c);
+          if (SRC == kRow32Wide && !mine) c[0] = c[1] = c[2] = c[3] = 0u;  // (an infinite zero point of the other group)
+          const uint4& xx = xv[j >> 1];
+          if (j == 0) mma_16816_first(d, c, xx.x, xx.y);
+          else mma_16816(d, c, (j & 1) ? xx.z : xx.x, (j & 1) ? xx.w : xx.y);
+        }
+#pragma unroll
+        for (int c = 0; c < 4; ++c) acc[c] += (c < 2 ? kUnitLo : kUnitHi) * s[c >> 1][c & 1] * d[c];
+      }
+    }
+    float* sum = &red[i][threadIdx.x >> 5][lane * vals(SRC)];
+    if (kPairs) {
+      sum[0] = acc[0] + acc[1];
+      sum[1] = acc[2] + acc[3];
+    } else {
+#pragma unroll
+      for (int c = 0; c < 4; ++c) sum[c] = acc[c];
+    }
+  }
+}
 template <int SRC, bool kTail, int MT>
 __device__ __forceinline__ void add_fractions_inline(Fractions a, float (*red)[kWarps][32 * vals(SRC)]) {
   constexpr bool kPairs = SRC == rk::kRow32, k32 = kPairs || SRC == kRow32Wide;
@@ -166,6 +222,8 @@ __device__ __forceinline__ void add_fractions_inline(Fractions a, float (*red)[k
   float* const sums = &red[0][threadIdx.x >> 5][lane * vals(SRC)];
   constexpr int kBlock = MT * kWarps * 32 * vals(SRC);  // from a row block's sums to the next one's
   const uint32_t ones = (k32 ? (g & 1) == t >> 1 : !(g & 1)) ? 0x3c003c00u : 0u;
+  const Fractions begin = a;
+  bool finite = true;
 #pragma unroll 1
   for (; a.kb0 < a.kb1; a.kb0 += 4, a.x += 256, a.x8 += 256) {
     // lane t has the scales and zero points of tile t
@@ -222,8 +280,8 @@ __device__ __forceinline__ void add_fractions_inline(Fractions a, float (*red)[k
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
           float sum = MT == 1 ? ((t & 1) ? d[2 + q] : d[q]) : d[2 * mt + q];
-          // (an infinite activation has made its rows' sums infinite already)
-          if ((kPairs && (g & 1) != q) || !(fabsf(sum) <= 3.4e38f)) sum = 0.0f;
+          if (kPairs && (g & 1) != q) sum = 0.0f;
+          finite = finite && fabsf(sum) <= 3.4e38f;
           xh[mt][q] = tf32_of(sum);
           xl[mt][q] = sum - xh[mt][q];
         }
@@ -261,9 +319,10 @@ __device__ __forceinline__ void add_fractions_inline(Fractions a, float (*red)[k
       if (!more) break;
     }
   }
+  if (!__all_sync(0xffffffffu, finite)) sums_of_infinities<SRC, MT>(begin, red);
 }
-// (Called for kRow32: written into that kernel it cost integers 6 %, k 4096 x n 22016, one row; a call costs the others
-// up to 10 % of a call with fractions.)
+// (Called for kRow32 and by experts: written into those kernels it cost integers 6 %, k 4096 x n 22016, one row, and 2 to 7 %;
+// a call costs the others up to 10 % where there are fractions.)
 template <int SRC, bool kTail, int MT>
 __device__ __noinline__ void add_fractions_call(Fractions a, float (*red)[kWarps][32 * vals(SRC)]) {
   add_fractions_inline<SRC, kTail, MT>(a, red);
@@ -677,9 +736,9 @@ __device__ __forceinline__ void run_blocks(const Params& pp, const Run& run, flo
     // A zero point was no integer.  What is loaded ahead is loaded again: kept over this it would spill.
     const unsigned at = (unsigned)((pos + window) * 16 + g) * (unsigned)pp.s_n;
     const __half* xa = x0 + (kWide ? t * 16 - ((t & 1) * 16 + (t >> 1) * 8) : 0);
-    const Fractions a = {xa, MT > 1 && mine[MT - 1] ? xa + 8u * (unsigned)p.ldx : xa, run.s() + at, run.z() + at, c0 * 4, min(KB, (c0 + nc) * 4),
-                         count, pp.s_n, pp.s_g, p.group, pp.group_shift};
-    if (kPairs) add_fractions_call<SRC, kTail, MT>(a, red);
+    const Fractions a = {xa, MT > 1 && mine[MT - 1] ? xa + 8u * (unsigned)p.ldx : xa, run.s() + at, run.z() + at, run.w(), c0 * 4,
+                         min(KB, (c0 + nc) * 4), pos + window, count, NB, KB, pp.s_n, pp.s_g, p.group, pp.group_shift};
+    if (kPairs || !Run::kWait) add_fractions_call<SRC, kTail, MT>(a, red);
     else add_fractions_inline<SRC, kTail, MT>(a, red);
     misfit = 0;
     if (window_stored()) return;

@@ -176,22 +176,32 @@ def test_fractional_zero_points(k, n, group, columns, m):
     assert np.abs(got - exp).max() <= 4 * BOUND * np.abs(exp).max()
 
 
-@pytest.mark.parametrize("group", [32, 64, 128])
-@pytest.mark.parametrize("m", [1, 8])
-def test_infinities_beside_fractional_zero_points(group, m):
-    """An infinite scale, zero point or activation stays with its row or column, and the sums that it takes part in are not finite."""
-    k, n = 1024, 64
+@pytest.mark.parametrize("k,group", [(1024, 32), (1088, 32), (1024, 64), (1024, 128), (1152, 128), (1024, 256)])
+@pytest.mark.parametrize("m", [1, 4, 8, 16])
+def test_infinities_beside_fractional_zero_points(k, group, m):
+    """An infinite activation has the sign of its weight, also where its code is the zero point's integer; an infinite scale or zero
+    point stays with its row."""
+    n = 272
     rs = np.random.RandomState(m + group)
     x = rs.randn(m, k).astype(np.float16)
     x[m - 1, 700] = np.inf
     w = rs.randint(0, 2 ** 32, size=(n, k // 8), dtype=np.uint32)
-    s, z = rs.uniform(1e-3, 1e-2, size=(n, k // group)).astype(np.float16), None
+    s = rs.uniform(1e-3, 1e-2, size=(n, k // group)).astype(np.float16)
     z = _zeros_of("all", rs, s.shape)
+    z[::2, 700 // group] = np.float16(7.3)
+
+    def call(s, z):
+        return ops.gemm_fp16_q4f16(to_dev(x), ops.preprocess_weight_q4f16(u32_to_dev(w)), to_dev(s), to_dev(z), group_size=group).cpu().numpy()
+
+    got = call(s, z)
+    with np.errstate(invalid="ignore"):
+        exp = (((w[:, 700 // 8] >> (4 * (700 % 8))) & 15) - z[:, 700 // group].astype(np.float64)) * np.inf
+    assert np.array_equal(got[m - 1].astype(np.float64), exp, equal_nan=True)
+    assert np.isfinite(got[:m - 1]).all()
     s[5, 1], z[18, 2], z[40, 3] = np.inf, np.inf, np.nan
-    got = ops.gemm_fp16_q4f16(to_dev(x), ops.preprocess_weight_q4f16(u32_to_dev(w)), to_dev(s), to_dev(z), group_size=group).cpu().numpy()
     finite = np.ones((m, n), dtype=bool)
     finite[m - 1], finite[:, [5, 18, 40]] = False, False
-    assert np.array_equal(np.isfinite(got), finite)
+    assert np.array_equal(np.isfinite(call(s, z)), finite)
 
 
 @pytest.mark.parametrize("group", [32, 64, 128])
