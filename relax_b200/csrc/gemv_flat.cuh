@@ -56,7 +56,7 @@ struct Params : rk::Params {
 };
 
 // Where this kernel takes its scales from for these operands, or -1: the kernel of gemv_rk.cuh.
-int source(const rk::Params& pp, int bits, int zmode, int src);
+int source(const rk::Params& pp, int bits, int zmode, int src, int sm_count);
 int launch(const rk::Params& pp, int zmode, int src, int grid, cudaStream_t stream);  // (grouped where pp.indptr is set)
 
 #ifdef __CUDACC__

@@ -42,7 +42,7 @@ int gemv_rk_run(const GemvParams& p, int bits, int zmode, int sm_count, const in
   pp.s_n = (int)p.s_n;
   pp.s_g = (int)p.s_g;
   const long long blocks = (long long)(p.n / 16) * (indptr ? num_experts : 1);
-  const int flat = fl::source(pp, bits, zmode, src);
+  const int flat = fl::source(pp, bits, zmode, src, sm_count);
   // Eight k slices while an SM has few row blocks (its 16 warps are two CTAs), four once there are
   // enough for four CTAs: half the passes per byte.  Measured: k 8192 x n 28672 int8 (12 row blocks
   // per SM) 44 -> 41 us, k 4096 x n 22016 int4 (9.3) 13.7 -> 13.9 us, k = n = 4096 (1.7) 3.9 -> 5.8 us.

@@ -754,7 +754,7 @@ int launch_inst(const Params& pp, int warps, int grid, cudaStream_t stream) {
   cfg.numAttrs = 1;
 #define RB200_RK(GR, W, M) RB200_CUDA(cudaLaunchKernelEx(&cfg, gemv_rk_kernel<BITS, ZMODE, SRC, GR, W, M>, pp))
   // (those experts are all gemv_flat.cuh's)
-  constexpr bool kExperts = !(BITS == 4 && ZMODE == kZeroConstInt && (SRC == kRow32 || SRC == kHalf || SRC == kTile));
+  constexpr bool kExperts = !(BITS == 4 && ZMODE == kZeroConstInt && (SRC == kRow32 || SRC == kHalf));
   if (pp.indptr) {
     if constexpr (kExperts) {
       if (warps == 8) RB200_RK(true, 8, 1);
@@ -766,12 +766,8 @@ int launch_inst(const Params& pp, int warps, int grid, cudaStream_t stream) {
     if (warps == 8) RB200_RK(false, 8, 1);
     else RB200_RK(false, 4, 1);
   } else {
-    if constexpr (!(BITS == 4 && ZMODE == kZeroConstInt && SRC == kHalf)) {  // (gemv_flat.cuh's)
-      if (warps == 8) RB200_RK(false, 8, 2);
-      else RB200_RK(false, 4, 2);
-    } else {
-      RB200_CHECK(false, "no kernel of two m-tiles for this source of scales");
-    }
+    if (warps == 8) RB200_RK(false, 8, 2);
+    else RB200_RK(false, 4, 2);
   }
 #undef RB200_RK
   return 0;

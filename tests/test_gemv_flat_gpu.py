@@ -83,6 +83,15 @@ def test_columns_of_scales(oracle, k, n, group, zeros, m):
     assert np.linalg.norm(got - exp) <= BOUND * np.linalg.norm(exp)
 
 
+@pytest.mark.parametrize("m", [4, 7, 12, 16])
+@pytest.mark.parametrize("k,n,group,zeros", [(512, 4736, 128, True), (512, 4752, 128, True), (512, 9488, 128, False), (512, 14224, 128, False),
+                                             (512, 4752, 128, False), (1088, 4752, 64, False), (1088, 9488, 64, False), (1152, 4752, 128, True),
+                                             (2112, 400, 64, False), (4352, 4752, 128, True)])
+def test_either_side_of_the_lines(oracle, k, n, group, zeros, m):
+    """one to four row blocks a CTA, and last chunks of one k block, with scales [K / g, N]"""
+    test_columns_of_scales(oracle, k, n, group, zeros, m)
+
+
 @pytest.mark.parametrize("m", [1, 4])
 @pytest.mark.parametrize("k", [4096, 1856])
 def test_swiglu_and_residual(oracle, m, k):
