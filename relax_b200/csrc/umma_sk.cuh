@@ -84,19 +84,23 @@ __device__ __forceinline__ void cluster_sync() {
   __syncwarp();
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// An address of this CTA's shared memory in that of the cluster's CTA `rank`.
+__device__ __forceinline__ uint32_t map_to(uint32_t addr, int rank) {
+  uint32_t to;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(to) : "r"(addr), "r"(rank));
+  return to;
+}
 
 // Parts of a tile in one cluster: each CTA sends column c of its accumulator to the CTA that adds it up, in place of that
-// CTA's ring of weights (at most 64 + 7 columns of 512 bytes; the ring has at least three stages of 16 KB).  A CTA whose
-// waits ran out sends NaN.  Columns and not weight rows: a thread's sixteen values go to few CTAs, 128 bytes a warp each.
-__device__ __forceinline__ void exchange_send(const Params& pp, uint32_t ring, uint32_t d, int cols, int rank, int ranks, int grp, int gj,
-                                              bool ok) {
+// CTA's ring of weights (at most 64 + 7 columns of 512 bytes; the ring has at least three stages of 16 KB).  Columns and not
+// weight rows: a thread's sixteen values go to few CTAs, 128 bytes a warp each.
+__device__ __forceinline__ void exchange_send(uint32_t ring, uint32_t d, int cols, int rank, int ranks, int grp, int gj) {
   const int most = (cols + ranks - 1) / ranks;
   for (int c0 = grp * 16; c0 < cols; c0 += kGroups * 16) {
     float v[16];
     tc_ld16(d + (uint32_t)c0, v);
     int to = ((c0 + 1) * ranks - 1) / cols, lo = cols * to / ranks, hi = cols * (to + 1) / ranks;
-    uint32_t dst = 0;
-    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(ring), "r"(to));
+    uint32_t dst = map_to(ring, to);
 #pragma unroll
     for (int i = 0; i < 16; ++i) {
       const int c = c0 + i;
@@ -107,10 +111,10 @@ __device__ __forceinline__ void exchange_send(const Params& pp, uint32_t ring, u
           lo = hi;
           hi = cols * (to + 1) / ranks;
         } while (c >= hi);
-        asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(dst) : "r"(ring), "r"(to));
+        dst = map_to(ring, to);
       }
       asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(dst + (uint32_t)(((rank * most + c - lo) * kTileRows + gj) * 4)),
-                   "f"(ok ? v[i] : __int_as_float(0x7fffffff))
+                   "f"(v[i])
                    : "memory");
     }
   }
@@ -181,6 +185,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   uint64_t* d_empty = d_full + 2;
   uint64_t* e_bar = d_empty + 2;
   uint32_t* tmem_holder = reinterpret_cast<uint32_t*>(e_bar + kGroups);
+  volatile uint32_t* const gave_up = tmem_holder + 1;  // kCluster: a wait of one of its CTAs ran out
   Tables& tt = *reinterpret_cast<Tables*>(tmem_holder + 4);
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
@@ -205,6 +210,7 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
     }
     for (int i = 0; i < kGroups; ++i) mbar_init(&e_bar[i], 4);
     mbar_fence_init();
+    *gave_up = 0u;
   }
   if (warp == 1) {
     ug::tmem_alloc(tmem_holder, (uint32_t)pp.tmem_cols);
@@ -558,12 +564,16 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
     const int cols = min(nb, it.m_end - it.m0);
     cluster_sync();  // no CTA reads its ring of weights any more
     if (warp >= 4) {
-      exchange_send(pp, smem_u32(w_ring), ((uint32_t)(32 * w4) << 16) | tmem, cols, rank, ranks, grp, w4 * 32 + lane, fine);
+      // After a wait that ran out bulk copies may still be on their way into a ring: the cluster's CTAs leave the tile unwritten.
+      // (Told before the first barrier, which takes one more for the flags to be at rest, it cost 3 to 6 % at 256 CTAs.)
+      if (!__all_sync(0xffffffffu, fine) && lane < ranks)
+        asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map_to(smem_u32(tmem_holder + 1), lane)), "r"(1u) : "memory");
+      exchange_send(smem_u32(w_ring), ((uint32_t)(32 * w4) << 16) | tmem, cols, rank, ranks, grp, w4 * 32 + lane);
       tc_fence_before();
       if (pp.early) griddep_wait();  // outputs may be in use by the previous kernel until it has ended
     }
     cluster_sync();
-    if (warp >= 4)
+    if (warp >= 4 && *gave_up == 0u)
       exchange_store<folds<ZMODE, SRC>()>(pp, reinterpret_cast<const float*>(w_ring), reinterpret_cast<const float*>(e_stage),
                                           it.n_tile * kTileRows, it.m0, cols, rank, ranks, grp, w4 * 32 + lane);
   }
