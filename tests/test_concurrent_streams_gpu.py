@@ -27,10 +27,15 @@ def _calls(seed):
         return (torch.rand(shape, device="cuda", generator=g) * (hi - lo) + lo).half()
 
     calls = []
-    for m, k, n in [(24, 4096, 4096), (64, 4096, 2048), (128, 4096, 1536), (300, 2048, 3072)]:
+    # tiles shared by a cluster (no words), cut into three, runs beside whole tiles, CTA pairs
+    for m, k, n in [(24, 4096, 4096), (64, 4096, 2048), (32, 2048, 8192), (64, 1088, 31696), (128, 4096, 1536), (300, 2048, 3072)]:
         w, s = ops.preprocess_weight_q4f16(words(n, k // 8)), half(1e-3, 1e-2, n, k // 32)
         x, out = torch.randn(m, k, device="cuda", generator=g).half(), torch.empty(m, n, dtype=torch.float16, device="cuda")
         calls.append((lambda x=x, w=w, s=s, out=out: ops.gemm_fp16_q4f16(x, w, s, out=out), out))
+    # the same of another decode and drain: int8, one scale per row
+    w, s = ops.preprocess_weight_ft(torch.randint(-128, 128, (2048, 3072), dtype=torch.int8, device="cuda", generator=g), False), half(1e-4, 1e-3, 3072)
+    x, out = torch.randn(24, 2048, device="cuda", generator=g).half(), torch.empty(24, 3072, dtype=torch.float16, device="cuda")
+    calls.append((lambda x=x, w=w, s=s, out=out: ops.gemm_fp16_ft(x, w, s, 8, group_size=-1, out=out), out))
     for rows in (96, 640):
         w = ops.preprocess_weight_ft(torch.randint(-128, 128, (4, 2048, 512), dtype=torch.int8, device="cuda", generator=g), True)
         s, indptr = half(1e-3, 1e-2, 4, 1024), torch.tensor([rows // 4, rows // 2, rows // 2, rows], device="cuda")

@@ -13,7 +13,7 @@ ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 CHILD = """
 import torch
 from relax_b200 import ops
-m, k, n = %d, 4096, 4096
+m, k, n = %d, %d, %d
 g = torch.Generator(device="cuda")
 g.manual_seed(3)
 w = ops.preprocess_weight_q4f16(torch.randint(-2 ** 31, 2 ** 31 - 1, (n, k // 8), dtype=torch.int32, device="cuda", generator=g))
@@ -34,9 +34,10 @@ print("held" if held else "not held")
 """
 
 
-@pytest.mark.parametrize("m", [32, 128])
-def test_first_call_beside_a_busy_default_stream(m):
-    r = subprocess.run([sys.executable, "-c", CHILD % m], cwd=ROOT, capture_output=True, text=True, timeout=300,
+# (32 rows of 4096 x 4096 are added up in clusters, without scratch; the others go through it: cut tiles, runs beside whole tiles, pairs)
+@pytest.mark.parametrize("m,k,n", [(32, 4096, 4096), (32, 2048, 8192), (64, 1088, 31696), (128, 4096, 4096)])
+def test_first_call_beside_a_busy_default_stream(m, k, n):
+    r = subprocess.run([sys.executable, "-c", CHILD % (m, k, n)], cwd=ROOT, capture_output=True, text=True, timeout=300,
                        env=dict(os.environ, CUDA_MODULE_LOADING="EAGER"))  # loading a kernel waits for the device
     assert r.returncode == 0, r.stdout + r.stderr
     assert r.stdout.strip() == "held", "the default stream was over too early to show anything"

@@ -93,9 +93,10 @@ def test_int4_groups_of_32_by_columns(oracle, m, k, n):
 
 @pytest.mark.parametrize("m", [24, 64])
 @pytest.mark.parametrize("tiles", [236, 238, 246, 248, 295])
-@pytest.mark.parametrize("k", [64, 1088])
+@pytest.mark.parametrize("k", [64, 320, 1088])
 def test_a_tile_per_sm_and_runs_of_the_rest(oracle, m, tiles, k):
-    """either side of the tile counts from which an SM's first CTA keeps a whole tile, with more CTAs than chunks left and fewer"""
+    """either side of the tile counts from which an SM's first CTA keeps a whole tile: two chunks a tile (no fewer CTAs than chunks are
+    left then), five, and one, where no tile is cut"""
     n = tiles * 128 - 48
     case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, 32)
     pre, s, x = ops.preprocess_weight_q4f16(u32_to_dev(case.w)), to_dev(case.scales), to_dev(case.x)
@@ -104,10 +105,33 @@ def test_a_tile_per_sm_and_runs_of_the_rest(oracle, m, tiles, k):
     assert_close(got, C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, None, 7.0, 32))))
 
 
+@pytest.mark.parametrize("m", [24, 64])
+def test_other_forms_of_runs_beside_whole_tiles(oracle, m):
+    """zero points, the scale left to the sums, the epilogue's operands and the gated activation behind the same split"""
+    k, n = 576, 248 * 128 - 32
+    rs, C = np.random.RandomState(m), oracle.C()
+    case = synth.q4_case(np.random.Generator(np.random.PCG64(m)), m, k, n, 64, asymmetric=True)
+    bias, res = rs.randn(n).astype(np.float16), rs.randn(m, n).astype(np.float16)
+    pre, s, z, x = ops.preprocess_weight_q4f16(u32_to_dev(case.w)), to_dev(case.scales), to_dev(case.zeros), to_dev(case.x)
+    b, r = to_dev(bias), to_dev(res)
+    got = _twice(lambda: ops.gemm_fp16_q4f16(x, pre, s, z, bias=b, residual=r, activation="relu", binary_op="plus", group_size=64))
+    assert_close(got, C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, case.zeros, 7.0, 64)), bias, res, "relu", "plus"))
+    w8, s8 = rs.randint(-128, 128, size=(k, n)).astype(np.int8), rs.uniform(1e-4, 1e-3, size=(n,)).astype(np.float16)
+    pre8, s8d = ops.preprocess_weight_ft(to_dev(w8), False), to_dev(s8)
+    assert_close(_twice(lambda: ops.gemm_fp16_ft(x, pre8, s8d, 8, group_size=-1)),
+                 C.epilogue(C.matmul_f32(case.x, C.decode_ft_kn(w8, s8, 8, -1), False)))
+    ffn, sg = n // 2, rs.uniform(1e-3, 1e-2, size=(n, k // 32)).astype(np.float16)
+    pre, si = ops.preprocess_weight_gate_up(u32_to_dev(case.w)), ops.interleave_gate_up(to_dev(sg))
+    got = _twice(lambda: ops.gemm_fp16_q4f16(x, pre, si, activation="swiglu")).astype(np.float64)
+    y = C.matmul_f32(case.x, C.decode_q4_nk(case.w, sg, None, 7.0, 32)).astype(np.float64)
+    exp = y[:, :ffn] / (1 + np.exp(-y[:, :ffn])) * y[:, ffn:]
+    assert np.linalg.norm(got - exp) <= 1e-3 * np.linalg.norm(exp)
+
+
 @pytest.mark.parametrize("m", [17, 31, 33, 50, 64, 81])
 @pytest.mark.parametrize("k,n", [(2560, 144), (3136, 272), (4160, 1040), (11008, 16)])
 def test_parts_of_a_tile_in_a_cluster(oracle, m, k, n):
-    """columns that do not divide by the CTAs of a tile, a last tile of few weight rows, a last batch tile of few rows"""
+    """columns that do not divide by the CTAs of a tile, a last tile of few weight rows (81 rows are the pair kernel's)"""
     rs = np.random.RandomState(m + k + n)
     C = oracle.C()
     case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, 32)
@@ -122,6 +146,17 @@ def test_parts_of_a_tile_in_a_cluster(oracle, m, k, n):
     pre, s = ops.preprocess_weight_ft(to_dev(w), False), to_dev(s8)
     assert_close(_twice(lambda: ops.gemm_fp16_ft(x, pre, s, 8, group_size=-1)),
                  C.epilogue(C.matmul_f32(case.x, C.decode_ft_kn(w, s8, 8, -1), False)))
+
+
+@pytest.mark.parametrize("m,k,n,group", [(20, 4160, 1040, 64), (50, 4096, 272, 128), (64, 3072, 144, 32), (12, 14336, 4096, 32)])
+def test_zero_points_in_a_cluster(oracle, m, k, n, group):
+    """and nine to sixteen rows, which groups of 32 with zero points bring here"""
+    case = synth.q4_case(np.random.Generator(np.random.PCG64(m + k + n)), m, k, n, group, asymmetric=True)
+    case.zeros[::5, -1] = np.float16(7.3)
+    pre, s, z, x = ops.preprocess_weight_q4f16(u32_to_dev(case.w)), to_dev(case.scales), to_dev(case.zeros), to_dev(case.x)
+    got = _twice(lambda: ops.gemm_fp16_q4f16(x, pre, s, z, group_size=group))
+    C = oracle.C()
+    assert_close(got, C.epilogue(C.matmul_f32(case.x, C.decode_q4_nk(case.w, case.scales, case.zeros, 7.0, group))))
 
 
 @pytest.mark.parametrize("m,overlap", [(19, False), (32, True), (64, False)])
