@@ -75,7 +75,7 @@ int source(const rk::Params& pp, int bits, int zmode, int src, int sm_count) {
     // nine / sixteen rows without zero points: k = n = 4096 1.09 / 1.0, n 12288 (three blocks) 1.17 / 1.06, n 14336 (four)
     // 1.12 / 0.92, k 8192 x n 28672 (seven) 1.05 / 0.94
     if (two && !z) return odd || !many ? src : -1;
-    // with them k 11008 x n 4096 16.8 / 14.6, k 8192 x n 10240 (three) 1.08 / 0.97, 14336 (four) 1.0 / 0.89, k 4096 x n 22016
+    // with them (200 bytes of spills, 250 in the form for short last chunks) k 11008 x n 4096 16.8 / 14.6, k 8192 x n 10240 (three) 1.08 / 0.97, 14336 (four) 1.0 / 0.89, k 4096 x n 22016
     // 25.4 / 26.9
     if (two) return p.k >= 8192 && odd ? src : -1;
     // with them k = n = 4096 4.9 / 4.8, n 12288 1.20, 14336 1.12, k 2048 x n 4096 3.56 / 3.77, 1024 x 1024 3.25 / 3.03

@@ -34,7 +34,7 @@
 //   group 32, k 5504 x n 4096       8.2 / 5.1        8.5 / 5.2        8.6 / 6.5        10.6 / 8.9
 //   the same with zero points       9.1 / 5.7        9.4 / 6.0        9.6 / 7.3
 //   group 32 + z, k 4096 x n 22016  20.1 / 13.2      20.9 / 13.5      21.3 / 16.9
-//   group 64 + z, k 4096 x n 22016  23.4 / 13.5      24.3 / 14.0      24.8 / 15.1      30.2 / 25.1
+//   group 64 + z, k 4096 x n 22016  23.4 / 13.5      24.3 / 14.0      24.8 / 15.1      (without overlap 31.1 / 22.2)
 //   group 128, k 11008 x n 4096     7.7 / 7.2        8.1 / 7.5        (stays there)    11.7 / 10.7
 //   group 128 + z [K/g, N], x 11008 11.0 / 8.7       11.6 / 9.1       11.6 / 9.9
 #pragma once

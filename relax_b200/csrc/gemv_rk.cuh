@@ -1,6 +1,5 @@
 // Decode-path kernel for at most sixteen batch rows: row blocks per CTA, k split over its warps.  (Most int4 calls are
-// taken by gemv_flat.cuh, which has the figures of both; what stays here of them are one scale per row, groups of 32
-// above four rows, and group sizes that are no whole tiles.)
+// taken by gemv_flat.cuh; the rules, with the figures of both, are in gemv_flat.cu.)
 //
 //   out[m, n] = epilogue(sum_k x[m, k] * wq[n, k]),  m <= 8 or 16 (one or two m16n8k16 MMAs wide)
 //
@@ -63,8 +62,8 @@ enum ScaleSrc : int {
 // k 4096 x n 22016 18.1 / 16.1, k 8192 x n 57344 66.7 / 57.5, k = n = 4096 5.81 / 5.51; of int8, run for a quarter of a
 // second at a time, k 28672 x n 8192 52.6 / 47.6, k 8192 x n 57344 96.9 / 92.6, k 4096 x n 22016 22.0 / 21.7, k = n = 4096
 // 5.81 / 5.85 (alone, before the power cap is felt, 4 % slower to 4 % faster: what counts is the arithmetic's power).  With
-// zero points int4 is 3 % slower to 19 % faster, int8 10 % to 16 %: those decode.  Group 32 decodes here: its two groups of a
-// tile are kept apart by the columns of the MMA in gemv_flat.cuh, which takes up to four rows of it.
+// zero points int4 is 3 % slower to 19 % faster, int8 10 % to 16 %: those decode.  Group 32 decodes here; gemv_flat.cuh
+// keeps its two groups of a tile apart.
 constexpr bool folds(int zmode, int src, int m_tiles) {
   if (m_tiles == 2) return src == kChannel && zmode == kZeroConstInt;
   return src != kRow32 && src != kGeneral;

@@ -255,10 +255,11 @@ __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2)
   unsigned u_end = blockIdx.x < ctas ? (blockIdx.x + 1) * units / ctas * step : 0u;
   [[maybe_unused]] unsigned whole = 0u, base = 0u, rest = 0u, takers = 0u;
   if constexpr (SPLIT == kWholeFirst) {
-    whole = (unsigned)pp.whole, base = whole * (unsigned)cpt, rest = total - base, takers = min(ctas - whole, rest);
+    // (rest >= takers: see the rule in umma_tile.cu; a CTA without a chunk inside an owner's range would be waited for)
+    whole = (unsigned)pp.whole, base = whole * (unsigned)cpt, rest = total - base, takers = ctas - whole;
     const unsigned idx = blockIdx.x - whole;
-    u_begin = blockIdx.x < whole ? blockIdx.x * (unsigned)cpt : (idx < takers ? base + idx * rest / takers : 0u);
-    u_end = blockIdx.x < whole ? u_begin + (unsigned)cpt : (idx < takers ? base + (idx + 1) * rest / takers : 0u);
+    u_begin = blockIdx.x < whole ? blockIdx.x * (unsigned)cpt : base + idx * rest / takers;
+    u_end = blockIdx.x < whole ? u_begin + (unsigned)cpt : base + (idx + 1) * rest / takers;
   }
 
   auto get_item = [&](int item) {

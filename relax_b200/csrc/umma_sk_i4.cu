@@ -4,8 +4,8 @@ namespace us {
 int launch_i4(const Params& pp, const Launch& l, const CUtensorMap& tx, cudaStream_t stream) {
   return launch_bits<4>(pp, l, tx, stream);
 }
-// Asked of a kernel with the same block, registers and shared memory but no tensor memory, and never launched: of kernels
-// that allocate tensor memory the query sees one CTA per SM whatever they take.
+// Asked of a kernel of the same block and shared memory but without tensor memory, and never launched: of kernels that allocate
+// tensor memory the query sees one CTA per SM whatever they take.  (Registers allow two by the launch bounds; shared memory decides.)
 __global__ void __launch_bounds__((4 + 4 * kGroups) * 32, 2) places_kernel() {}
 int cluster_places(int ranges) {
   static thread_local int device = -1, places[9];

@@ -133,13 +133,14 @@ int run_single(Params& pp, int bits, int zmode, int src, int sm_count, cudaStrea
     if (ranges > 8) ranges = 8;
     if (ranges >= 2 || items <= sm_count) grid = items * (ranges > 1 ? ranges : 1);
     // Where the parts of a tile are many or large they are added inside a cluster: one exchange through shared memory in
-    // place of a trip to memory per part.  Without overlap of launches, us before / now: k 4096 x n 4096 int4 group 32,
-    // 32 rows 12.2 / 11.4, 64 rows 14.8 / 13.3; k 11008 x n 4096 32 rows 17.5 / 16.8, 64 rows 23.4 / 18.7; k 8192 x
-    // n 1024 64 rows 18.6 / 11.7; int8 per row k 8192 x n 4096 64 rows 22.7 / 17.6.  Fewer or smaller parts lose to the
-    // two cluster barriers (32 rows: k 2048 x n 4096 in three CTAs a tile 9.3 / 11.1, k 14336 x n 4096 in seven 20.2 / 21.3;
-    // 48 rows of int8 in four 1 % slower), and clusters that do not all run at once to the second wave (k 4096 x n 12288,
-    // 96 x 3: 15.0 / 27.3).  Overlapped launches of up to 32 rows start late in an SM that is full of them: there only up
-    // to a CTA per SM (k 4096 x n 2048 9.6 / 8.3; n 4096, 256 CTAs, 10.4 / 11.0).
+    // place of a trip to memory per part.  Without overlap of launches, us without / with: k 4096 x n 4096 int4 group 32,
+    // 32 rows 12.2 / 11.5, 64 rows 14.8 / 13.3; k 14336 x n 4096 32 rows 20.3 / 18.5; k 11008 x n 4096 64 rows 23.4 / 18.7;
+    // k 8192 x n 1024 64 rows 18.6 / 11.7; int8 per row k 8192 x n 4096 64 rows 22.7 / 17.6.  Nine to sixteen rows come here with
+    // groups of 32 and zero points: sixteen, k 14336 x n 4096 23.1 / 21.8, k 28672 x n 2048 32.0 / 31.4, k 57344 x n 1024
+    // 48.3 / 37.4.  Fewer or smaller parts lose to the two cluster barriers (32 rows, k 2048 x n 4096 in three CTAs a tile
+    // 9.3 / 11.1; 48 rows of int8 in four 1 % slower), and clusters that do not all run at once to the second wave (k 4096 x
+    // n 12288, 96 x 3: 15.0 / 27.3).  Overlapped launches of up to 32 rows start late in an SM that is full of them: there only
+    // up to a CTA per SM (k 4096 x n 2048 9.6 / 8.3; n 4096, 256 CTAs, 10.4 / 11.0).
     const int k_blocks = p.k / kKBlock;
     int wide = k_blocks / 8 < 8 ? k_blocks / 8 : 8;
     while (wide >= 4 && cluster_places(wide) < items) --wide;
@@ -156,10 +157,13 @@ int run_single(Params& pp, int bits, int zmode, int src, int sm_count, cudaStrea
   // (one CTA per tile cuts none)
   if (!l.ranges && (pp.indptr || grid != items)) pp.partial = handover_words(stream, sm_count, (size_t)grid * pp.nb * kTileRows * sizeof(float));
   // A tile per SM is not cut: its first CTA makes one, the second a run of the rest.  That saves a quarter of the pieces
-  // where the tiles come near two per SM; with fewer the second CTA is done long before the first (int8 per row, 48 rows,
-  // k 4096: n 32016 26.6 us in equal runs, 25.3 so, n 36000 28.3 / 27.9, n 22016 27.5 / 27.9, 24 rows 24.4 / 26.1; int4
-  // group 32, 32 rows: n 32016 28.6 / 27.6, n 26624 25.0 / 26.1, n 22016 21.9 / 21.0).
-  // (Run for a quarter of a second at a time, 238 tiles, 24 rows of int4 lose 1 to 2 %, 48 and 64 rows gain 2 to 4.)
+  // where the tiles come near two per SM; with fewer the second CTA is done before the first, by more or less as the equal
+  // runs' cuts fall.  k 4096, us in equal runs / so, 32 and 64 rows: int4 group 32 n 20480 (160 tiles) 21.9 / 24.5 and 24.9 / 29.1,
+  // n 22016 (172) 23.1 / 21.9 and 26.1 / 28.9, n 26624 (208) 26.4 / 28.3 and 29.4 / 29.7, n 30208 (236) 28.0 / 29.0 and 31.1 /
+  // 30.4, n 31616 (247) 29.6 / 29.6 and 32.7 / 31.1, n 32016 (251) 29.9 / 29.7 and 32.9 / 31.2, n 36000 (282) 32.1 / 32.0 and 34.8 /
+  // 34.5; int8 per row n 22016 25.5 / 27.0 and 28.8 / 31.3, n 26624 30.0 / 28.9 and 33.5 / 33.5, n 32016 33.1 / 32.2 and 37.2 / 35.4,
+  // n 36000 35.9 / 35.2 and 39.7 / 38.5.
+  // (More CTAs than tiles, so two chunks a tile at least, and no fewer chunks are left than second CTAs.)
   if (!pp.indptr && pp.partial && grid == 2ll * sm_count && items < grid && (pp.nb > 32 ? items * 5 >= sm_count * 8ll : items * 3 >= sm_count * 5ll))
     pp.whole = sm_count;
   l.grid = (int)grid;
